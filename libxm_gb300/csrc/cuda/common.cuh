@@ -14,6 +14,11 @@ extern "C" int xmg_seterr(int code, const char *fmt, ...);
 namespace xmg {
 
 cudaStream_t stream();          /* engine compute stream */
+/* the engine's second compute stream, between fork_aux (it waits for what
+ * the engine stream holds so far) and join_aux (the engine stream waits for
+ * it); also under stream capture */
+int fork_aux(cudaStream_t *aux);
+int join_aux();
 int device();                   /* engine device ordinal */
 int num_sms();
 int check(cudaError_t e, const char *what);

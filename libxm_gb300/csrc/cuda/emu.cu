@@ -80,8 +80,10 @@ template <> struct fin<double> {
 		if (eb == 0) eb = 1; else m |= 1ll << 52;
 		neg = b < 0;
 	}
-	__device__ static inline int bexp(double x)
-	{ return (int)((__double_as_longlong(x) >> 52) & 0x7ff); }
+	/* the 32-bit word that holds the exponent, and the exponent in it */
+	__device__ static inline int eword(const double *p)
+	{ return __ldg(reinterpret_cast<const int *>(p) + 1); }
+	__device__ static inline int bexp(int w) { return (w >> 20) & 0x7ff; }
 };
 template <> struct fin<float> {
 	static constexpr int S = 3, KEEP = 2, T1 = 23, MANT = 23, EMAX = 0xff;
@@ -94,8 +96,9 @@ template <> struct fin<float> {
 		if (eb == 0) eb = 1; else m |= 1ll << 23;
 		neg = (b >> 31) != 0;
 	}
-	__device__ static inline int bexp(float x)
-	{ return (int)((__float_as_uint(x) >> 23) & 0xff); }
+	__device__ static inline int eword(const float *p)
+	{ return __ldg(reinterpret_cast<const int *>(p)); }
+	__device__ static inline int bexp(int w) { return (w >> 23) & 0xff; }
 };
 
 /* One work item: up to EMU_MAXMEM output blocks (members mfirst ..
@@ -127,12 +130,19 @@ struct view_meta {
 	int64_t first_cta;
 };
 
+/* The view of a CTA: the last one whose first CTA is <= cta.  Every lane of
+ * a warp searches for the same cta, so each step compares 32 candidates: two
+ * dependent loads up to 1024 views, where a binary search chains ten. */
 __device__ __forceinline__ int find_view(const view_meta *m, int n, int64_t cta)
 {
-	int lo = 0, hi = n - 1;
-	while (lo < hi) {
-		int mid = (lo + hi + 1) >> 1;
-		if (m[mid].first_cta <= cta) lo = mid; else hi = mid - 1;
+	const int lane = threadIdx.x & 31;
+	int lo = 0;
+	while (n > 1) {
+		const int step = (n + 31) / 32, o = lane * step;
+		const bool le = o < n && m[lo + o].first_cta <= cta;
+		const int c = __popc(__ballot_sync(0xffffffffu, le)) - 1;
+		lo += c * step;
+		n = min(step, n - c * step);
 	}
 	return lo;
 }
@@ -154,81 +164,112 @@ __device__ __forceinline__ T fetch(const T *X, const int32_t *rowt, int32_t co,
 /* ------------------------------------------------------------------ */
 /* 1. exponent tables                                                  */
 
-/* CTA = (view, 128-row tile, 256-wide K range) */
+/* CTA = (view, 128-row tile, K range of kr elements).  The kernel is bound
+ * by HBM on large operands and by the latency of its loads on small ones,
+ * so a thread's loads are issued in batches of eight before any of them is
+ * used (only the word with the exponent is loaded), and the host halves kr
+ * until the grid covers the chip.  Indices past the range are clamped: a
+ * maximum may see an element twice. */
 template <typename T>
 __global__ void __launch_bounds__(256)
 emu_exp_kernel(const xmgd_view_t *__restrict__ views,
-    const view_meta *__restrict__ meta, int nviews,
+    const view_meta *__restrict__ meta, int nviews, int kr,
     const int32_t *__restrict__ tabs, int32_t *__restrict__ E,
     int *__restrict__ flags)
 {
 	const int v = find_view(meta, nviews, blockIdx.x);
 	const xmgd_view_t w = views[v];
-	const int64_t local = blockIdx.x - meta[v].first_cta;
-	const int kall = w.n_ks * EMU_KS;
-	const int nkb = (kall + 255) / 256;
-	const int rt = (int)(local / nkb), kb = (int)(local % nkb);
+	const int local = (int)(blockIdx.x - meta[v].first_cta);
+	const int nkb = (w.k + kr - 1) / kr;
+	const int rt = local / nkb, kb = local % nkb;
 	const T *X = reinterpret_cast<const T *>(w.ptr);
 	const int32_t *rowt = tabs + w.rowtab, *colt = tabs + w.coltab;
-	const int k0 = kb * 256, k1 = min(kall, k0 + 256);
+	const int k0 = kb * kr, klast = min(w.k, k0 + kr) - 1;
+	const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
 	int bad = 0;
 
-	if (w.kcontig && !w.cplx) {
-		/* K one contiguous run per row: a warp walks it directly (no
-		 * offset table), four loads in flight per lane; the padding past
-		 * w.k is zero and needs no reading */
-		const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+	if (w.kfast) {
+		/* K runs along memory: a warp walks K for four rows at a time,
+		 * directly when K is one contiguous run */
+		const bool direct = w.kcontig && !w.cplx;
 		const T *base = X + rowt[0];
-		const int kend = min(k1, w.k);
-		for (int rr = warp; rr < EMU_TM; rr += 8) {
-			int r = rt * EMU_TM + rr;
-			if (r >= w.mn)
-				break;
-			const T *xr = base + colt[r];
-			int e = 0;
-#pragma unroll 4
-			for (int k = k0 + lane; k < kend; k += 32) {
-				int b = fin<T>::bexp(xr[k]);
-				bad |= b == fin<T>::EMAX;
-				e = max(e, b);
+		for (int r0 = rt * EMU_TM + warp * 16; r0 < min(w.mn, rt * EMU_TM +
+		    warp * 16 + 16); r0 += 4) {
+			int32_t co[4];
+			int e[4] = {0, 0, 0, 0};
+#pragma unroll
+			for (int j = 0; j < 4; j++)
+				co[j] = colt[min(r0 + j, w.mn - 1)];
+			for (int k = k0 + lane; k <= klast; k += 64) {
+				const int ka = k, kc = min(k + 32, klast);
+				int x[4][2];
+				if (direct) {
+#pragma unroll
+					for (int j = 0; j < 4; j++) {
+						x[j][0] = fin<T>::eword(base + co[j] + ka);
+						x[j][1] = fin<T>::eword(base + co[j] + kc);
+					}
+				} else if (!w.cplx) {
+					const int32_t ra = rowt[ka], rc = rowt[kc];
+#pragma unroll
+					for (int j = 0; j < 4; j++) {
+						x[j][0] = fin<T>::eword(X + ra + co[j]);
+						x[j][1] = fin<T>::eword(X + rc + co[j]);
+					}
+				} else {
+					const int32_t ra = rowt[ka], rc = rowt[kc];
+#pragma unroll
+					for (int j = 0; j < 4; j++) {
+						const int a = fin<T>::eword(X + 2 * (ra + co[j]));
+						const int b = fin<T>::eword(X + 2 * (rc + co[j]));
+						const int p = fin<T>::eword(X + 2 * (ra + co[j]) + 1);
+						const int q = fin<T>::eword(X + 2 * (rc + co[j]) + 1);
+						x[j][0] = fin<T>::bexp(a) > fin<T>::bexp(p) ? a : p;
+						x[j][1] = fin<T>::bexp(b) > fin<T>::bexp(q) ? b : q;
+					}
+				}
+#pragma unroll
+				for (int j = 0; j < 4; j++)
+					e[j] = max(e[j], max(fin<T>::bexp(x[j][0]),
+					    fin<T>::bexp(x[j][1])));
 			}
-			for (int off = 16; off > 0; off >>= 1)
-				e = max(e, __shfl_xor_sync(0xffffffffu, e, off));
-			if (lane == 0 && e > 0)
-				atomicMax(&E[w.exptab + r], e);
-		}
-	} else if (w.kfast) {
-		/* K unit-stride: a warp walks K for one row at a time */
-		const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-		for (int rr = warp; rr < EMU_TM; rr += 8) {
-			int r = rt * EMU_TM + rr;
-			if (r >= w.mn)
-				break;
-			int32_t co = colt[r];
-			int e = 0;
-			for (int k = k0 + lane; k < k1; k += 32) {
-				int b = fin<T>::bexp(fetch(X, rowt, co, w, k));
-				bad |= b == fin<T>::EMAX;
-				e = max(e, b);
+			int mine = 0;
+#pragma unroll
+			for (int j = 0; j < 4; j++) {
+				const int m = __reduce_max_sync(0xffffffffu, e[j]);
+				bad |= m == fin<T>::EMAX;
+				mine = lane == j ? m : mine;
 			}
-			for (int off = 16; off > 0; off >>= 1)
-				e = max(e, __shfl_xor_sync(0xffffffffu, e, off));
-			if (lane == 0 && e > 0)
-				atomicMax(&E[w.exptab + r], e);
+			if (lane < 4 && r0 + lane < w.mn && mine > E[w.exptab + r0 + lane])
+				atomicMax(&E[w.exptab + r0 + lane], mine);
 		}
 	} else {
 		/* free index contiguous: a thread per row, two K halves */
 		const int rr = threadIdx.x % EMU_TM, half = threadIdx.x / EMU_TM;
 		const int r = rt * EMU_TM + rr;
 		if (r < w.mn) {
-			int32_t co = colt[r];
+			const T *xr = X + (w.cplx ? 2 : 1) * (int64_t)colt[r];
 			int e = 0;
-			for (int k = k0 + half; k < k1; k += 2) {
-				int b = fin<T>::bexp(fetch(X, rowt, co, w, k));
-				bad |= b == fin<T>::EMAX;
-				e = max(e, b);
+			for (int k = k0 + half; k <= klast; k += 16) {
+				int x[8];
+				if (!w.cplx) {
+#pragma unroll
+					for (int j = 0; j < 8; j++)
+						x[j] = fin<T>::eword(xr + rowt[min(k + 2 * j, klast)]);
+				} else {
+#pragma unroll
+					for (int j = 0; j < 8; j++) {
+						const T *p = xr + 2 * (int64_t)rowt[min(k + 2 * j, klast)];
+						const int a = fin<T>::eword(p), b = fin<T>::eword(p + 1);
+						x[j] = fin<T>::bexp(a) > fin<T>::bexp(b) ? a : b;
+					}
+				}
+#pragma unroll
+				for (int j = 0; j < 8; j++)
+					e = max(e, fin<T>::bexp(x[j]));
 			}
-			if (e > 0)
+			bad |= e == fin<T>::EMAX;
+			if (e > 0 && e > E[w.exptab + r])
 				atomicMax(&E[w.exptab + r], e);
 		}
 	}
@@ -1273,6 +1314,7 @@ struct emu_plan {
 	std::vector<char> useA, useB;
 	uint64_t d_va = 0, d_vb = 0, d_meta[2][2] = {{0, 0}, {0, 0}};
 	int64_t nctas[2][2] = {{0, 0}, {0, 0}};
+	int kr[2] = {256, 256};              /* exponent pass: K per CTA */
 	uint64_t d_E = 0, d_F = 0;
 	int64_t nE = 0;
 	int32_t nexp_a = 0;
@@ -1294,58 +1336,71 @@ struct emu_plan {
 	int (*gemm)(emu_plan *) = nullptr;
 };
 
-/* exponent tables, then unfold + split of every used view of both sides */
+/* the exponent pass, or the unfold + split, of one side on a stream */
+template <typename TIN>
+static int
+launch_side(emu_plan *e, int side, int kind, int32_t *E, int *flags, cudaStream_t st)
+{
+	const xmgd_view_t *dv = (const xmgd_view_t *)(side ? e->d_vb : e->d_va);
+	const int nv = (int)(side ? e->VB.size() : e->VA.size());
+	const view_meta *m = (const view_meta *)e->d_meta[side][kind];
+	const unsigned n = (unsigned)e->nctas[side][kind];
+
+	if (n == 0)
+		return XMG_OK;
+	if (kind == 0)
+		emu_exp_kernel<TIN><<<n, 256, 0, st>>>(dv, m, nv, e->kr[side], e->d_tabs, E,
+		    flags);
+	else
+		emu_split_kernel<TIN><<<n, 256, 0, st>>>(dv, m, nv, e->d_tabs, E);
+	g_launches++;
+	XMG_CK(cudaGetLastError());
+	return XMG_OK;
+}
+
+/* exponent tables, then unfold + split of every used view of both sides.
+ * The two sides are independent chains of two kernels: a's runs on a second
+ * stream beside b's (two branches of the captured graph), since on small
+ * operands each kernel is shorter than the time its launch takes to fill
+ * and drain the chip.  A shared a side (streamed batches) keeps one chain:
+ * its flag is copied between the kernels. */
 template <typename TIN>
 static int
 launch_split(emu_plan *e)
 {
 	int32_t *EA = (int32_t *)e->d_E, *EB = EA + e->nexp_a;
 	int *flags = (int *)(EA + e->nE);
+	int st;
 
 	XMG_CK(cudaMemsetAsync((void *)e->d_E, 0, (e->nE + 64) * sizeof(int32_t),
 	    stream()));
+	if (!e->a_mode) {
+		cudaStream_t aux;
+		if ((st = fork_aux(&aux)) ||
+		    (st = launch_side<TIN>(e, 0, 0, EA, flags, aux)) ||
+		    (st = launch_side<TIN>(e, 0, 1, EA, flags, aux)) ||
+		    (st = launch_side<TIN>(e, 1, 0, EB, flags, stream())) ||
+		    (st = launch_side<TIN>(e, 1, 1, EB, flags, stream())))
+			return st;
+		return join_aux();
+	}
 	/* a shared a side: the preparing plan fills the shared exponent table
-	 * and flag, every plan takes the flag's Inf/NaN bit into its own */
-	int *aflags = flags;
-	if (e->a_mode) {
-		EA = (int32_t *)e->a_E;
-		aflags = (int *)e->a_flag;
-		if (e->a_mode == 1) {
-			XMG_CK(cudaMemsetAsync(EA, 0, e->nexp_a * sizeof(int32_t), stream()));
-			XMG_CK(cudaMemsetAsync(aflags, 0, sizeof(int), stream()));
-		}
+	 * and flag; every plan, the preparing one and the ones that use it,
+	 * takes the flag's Inf/NaN bit into its own */
+	EA = (int32_t *)e->a_E;
+	int *aflags = (int *)e->a_flag;
+	if (e->a_mode == 1) {
+		XMG_CK(cudaMemsetAsync(EA, 0, e->nexp_a * sizeof(int32_t), stream()));
+		XMG_CK(cudaMemsetAsync(aflags, 0, sizeof(int), stream()));
+		if ((st = launch_side<TIN>(e, 0, 0, EA, aflags, stream())))
+			return st;
 	}
-	for (int side = 0; side < 2; side++) {
-		const xmgd_view_t *dv = (const xmgd_view_t *)(side ? e->d_vb : e->d_va);
-		const int nv = (int)(side ? e->VB.size() : e->VA.size());
-		int32_t *E = side ? EB : EA;
-		if (e->nctas[side][0] > 0 && !(side == 0 && e->a_mode == 2)) {
-			emu_exp_kernel<TIN><<<(unsigned)e->nctas[side][0], 256, 0, stream()>>>(
-			    dv, (const view_meta *)e->d_meta[side][0], nv, e->d_tabs, E,
-			    side ? flags : aflags);
-			g_launches++;
-			XMG_CK(cudaGetLastError());
-		}
-		/* every plan of a shared a side, the preparing one and the
-		 * ones that use it, takes its Inf/NaN bit */
-		if (side == 0 && e->a_mode)
-			XMG_CK(cudaMemcpyAsync(flags, aflags, sizeof(int),
-			    cudaMemcpyDeviceToDevice, stream()));
-	}
-	for (int side = 0; side < 2; side++) {
-		const xmgd_view_t *dv = (const xmgd_view_t *)(side ? e->d_vb : e->d_va);
-		const int nv = (int)(side ? e->VB.size() : e->VA.size());
-		const int32_t *E = side ? EB : EA;
-		if (side == 0 && e->a_mode == 2)
-			continue;
-		if (e->nctas[side][1] > 0) {
-			emu_split_kernel<TIN><<<(unsigned)e->nctas[side][1], 256, 0, stream()>>>(
-			    dv, (const view_meta *)e->d_meta[side][1], nv, e->d_tabs, E);
-			g_launches++;
-			XMG_CK(cudaGetLastError());
-		}
-	}
-	return XMG_OK;
+	XMG_CK(cudaMemcpyAsync(flags, aflags, sizeof(int), cudaMemcpyDeviceToDevice,
+	    stream()));
+	if ((st = launch_side<TIN>(e, 1, 0, EB, flags, stream())) ||
+	    (e->a_mode == 1 && (st = launch_side<TIN>(e, 0, 1, EA, aflags, stream()))))
+		return st;
+	return launch_side<TIN>(e, 1, 1, EB, flags, stream());
 }
 
 /* the persistent grouped GEMM of the current candidate, then the flags */
@@ -1858,6 +1913,17 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 	for (int side = 0; side < 2; side++) {
 		std::vector<xmgd_view_t> &V = side ? e->VB : e->VA;
 		std::vector<char> &use = side ? e->useB : e->useA;
+		/* the exponent pass: K ranges of 256 (one atomic per row and CTA
+		 * from the fewest CTAs), halved down to 32 while the grid is
+		 * below eight CTAs per SM */
+		for (int &kr = e->kr[side]; kr > 32; kr /= 2) {
+			int64_t n = 0;
+			for (size_t v = 0; v < V.size(); v++)
+				if (use[v])
+					n += (int64_t)V[v].n_rt * ((V[v].k + kr - 1) / kr);
+			if (n >= 8 * num_sms())
+				break;
+		}
 		for (int kind = 0; kind < 2; kind++) {
 			std::vector<view_meta> meta(V.size());
 			int64_t n = 0;
@@ -1866,7 +1932,7 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 				if (!use[v])
 					continue;
 				if (kind == 0)
-					n += (int64_t)V[v].n_rt * ((V[v].n_ks * EMU_KS + 255) / 256);
+					n += (int64_t)V[v].n_rt * ((V[v].k + e->kr[side] - 1) / e->kr[side]);
 				else
 					n += (int64_t)V[v].n_rt * ((V[v].n_ks + 3) / 4);
 			}

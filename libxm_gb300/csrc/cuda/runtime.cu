@@ -18,6 +18,8 @@ static int g_ready = 0;
 static int g_dev = 0;
 static int g_sms = 0;
 static cudaStream_t g_stream = nullptr;
+static cudaStream_t g_aux = nullptr;
+static cudaEvent_t g_fork = nullptr, g_join = nullptr;
 static size_t g_in_use = 0;
 static cudaEvent_t g_t0 = nullptr, g_t1 = nullptr;
 long long g_launches = 0;
@@ -34,6 +36,24 @@ static bool g_side_rec[XMGD_SIDE_SLOTS];
 static buf g_chunk[XMGD_SIDE_SLOTS];
 
 cudaStream_t stream() { return g_stream; }
+
+int
+fork_aux(cudaStream_t *aux)
+{
+	XMG_CK(cudaEventRecord(g_fork, g_stream));
+	XMG_CK(cudaStreamWaitEvent(g_aux, g_fork, 0));
+	*aux = g_aux;
+	return XMG_OK;
+}
+
+int
+join_aux()
+{
+	XMG_CK(cudaEventRecord(g_join, g_aux));
+	XMG_CK(cudaStreamWaitEvent(g_stream, g_join, 0));
+	return XMG_OK;
+}
+
 int device() { return g_dev; }
 int num_sms() { return g_sms; }
 
@@ -79,6 +99,9 @@ xmgd_init(void)
 	XMG_CK(cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount,
 	    g_dev));
 	XMG_CK(cudaStreamCreateWithFlags(&g_stream, cudaStreamNonBlocking));
+	XMG_CK(cudaStreamCreateWithFlags(&g_aux, cudaStreamNonBlocking));
+	XMG_CK(cudaEventCreateWithFlags(&g_fork, cudaEventDisableTiming));
+	XMG_CK(cudaEventCreateWithFlags(&g_join, cudaEventDisableTiming));
 	XMG_CK(cudaStreamCreateWithFlags(&g_side, cudaStreamNonBlocking));
 	for (int i = 0; i < XMGD_SIDE_SLOTS; i++)
 		XMG_CK(cudaEventCreateWithFlags(&g_side_ev[i], cudaEventDisableTiming));
