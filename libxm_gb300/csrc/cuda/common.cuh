@@ -6,6 +6,7 @@
 #include <cuComplex.h>
 #include <stdint.h>
 
+#include "div.cuh"
 #include "xmg_dev.h"
 #include "xmg.h"
 
@@ -45,7 +46,7 @@ template <> struct num<double> {
 	__device__ static double mul(double a, double b) { return a * b; }
 	__device__ static double fma(double a, double b, double c) { return ::fma(a, b, c); }
 	__device__ static double add(double a, double b) { return a + b; }
-	__device__ static double div(double a, double b) { return a / b; }
+	__device__ static double div(double a, double b) { return div_f64(a, b); }
 	__device__ static double zero() { return 0.0; }
 	__device__ static double re(double a) { return a; }
 	__device__ static double im(double) { return 0; }

@@ -41,7 +41,8 @@ namespace xmg {
 
 constexpr int PT_THREADS = 256;
 constexpr int ROW_ELEMS = 4096;    /* elements per CTA in row mode */
-constexpr int FLAT_ELEMS = 8192;   /* elements per CTA in flat mode */
+constexpr int FLAT_ELEMS = 8192;   /* elements per CTA in flat mode, at most */
+constexpr int FLAT_MIN = 1024;     /* ... and at least */
 constexpr int TILE = 32;
 /* matrix mode: whole s0 x s1 slices (both <= MT) per CTA; a source and a
  * destination tile of both types fit the 48 KB of static shared memory */
@@ -63,7 +64,8 @@ constexpr int64_t SLAB_SMEM = 64 * 1024;
 struct task_meta {
 	int64_t first_cta;
 	int32_t mode;          /* 0 row, 1 tile, 2 flat, 3 matrix, 4 slab */
-	int32_t rows_per_cta;  /* row mode: outer rows per CTA */
+	int32_t rows_per_cta;  /* row mode: outer rows per CTA; flat mode:
+	                          elements per CTA */
 	int64_t nouter;        /* row: product of dims 1..; tile: dims 2.. */
 	int32_t ctas_d0, ctas_d1;
 };
@@ -108,16 +110,20 @@ struct elem_op {
  * Flat runs with 16-byte accesses.  Each thread issues the loads of U
  * vectors (of both runs) before any of its stores: stores to dst may alias
  * src as far as the compiler knows, so a plain loop keeps one iteration's
- * loads in flight at a time.
+ * loads in flight at a time.  ONE: alpha is 1 (real types), so that its
+ * product is left out: at 2 FP64 instructions a cycle and SM against one
+ * element a cycle from memory, two of them per element (alpha x and
+ * + beta y) already take the time of the traffic.
  */
 template <typename D> struct alignas(16) vec16 { D v[16 / sizeof(D)]; };
 
-template <int OP, typename D>
+template <int OP, bool ONE, typename D>
 __device__ inline void
 flat_vec(vec16<D> *dv, const vec16<D> *sv, int nv, const D al, const D be,
     double &dre, double &dim_)
 {
-	constexpr int W = 16 / sizeof(D), U = 4;
+	/* (a division needs the registers of two vectors more) */
+	constexpr int W = 16 / sizeof(D), U = OP == XMGD_OP_DIV ? 2 : 4;
 	constexpr bool RD = OP != XMGD_OP_COPY && OP != XMGD_OP_SET;
 	constexpr bool RS = OP != XMGD_OP_SET && OP != XMGD_OP_SCALE;
 	constexpr bool WR = OP != XMGD_OP_DOT;
@@ -145,16 +151,18 @@ flat_vec(vec16<D> *dv, const vec16<D> *sv, int nv, const D al, const D be,
 				if (OP == XMGD_OP_SET)
 					xv = al;
 				else if (OP == XMGD_OP_SCALE)
-					xv = num<D>::mul(al, xv);
+					xv = ONE ? xv : num<D>::mul(al, xv);
 				else if (OP == XMGD_OP_AXPY)
-					xv = num<D>::add(num<D>::mul(al, xv),
+					xv = num<D>::add(ONE ? xv : num<D>::mul(al, xv),
 					    num<D>::mul(be, y[u].v[w]));
 				else if (OP == XMGD_OP_COPY)
-					xv = num<D>::mul(al, y[u].v[w]);
+					xv = ONE ? y[u].v[w] : num<D>::mul(al, y[u].v[w]);
 				else if (OP == XMGD_OP_MUL)
-					xv = num<D>::mul(num<D>::mul(al, xv), y[u].v[w]);
+					xv = num<D>::mul(ONE ? xv : num<D>::mul(al, xv),
+					    y[u].v[w]);
 				else if (OP == XMGD_OP_DIV)
-					xv = num<D>::div(xv, num<D>::mul(al, y[u].v[w]));
+					xv = num<D>::div(xv, ONE ? y[u].v[w] :
+					    num<D>::mul(al, y[u].v[w]));
 				else {
 					const D pr = num<D>::mul(xv, y[u].v[w]);
 					dre += num<D>::re(pr);
@@ -210,13 +218,13 @@ ptask_kernel(const xmgd_ptask_t *__restrict__ tasks,
 	if constexpr (MODE == 2) {
 		/* flat: consecutive threads take consecutive elements, the op
 		 * resolved outside the loop */
-		const int64_t base = local * FLAT_ELEMS;
-		const int n = (int)(t.size[0] - base < FLAT_ELEMS ? t.size[0] - base :
-		    FLAT_ELEMS);
+		const int chunk = m.rows_per_cta;
+		const int64_t base = local * chunk;
+		const int n = (int)(t.size[0] - base < chunk ? t.size[0] - base : chunk);
 		D *dp = dst + base;
 		const S *sp = src + base;
 		bool done = false;
-		if constexpr (std::is_same<D, S>::value && sizeof(D) < 16) {
+		if constexpr (std::is_same<D, S>::value && sizeof(D) <= 16) {
 			/* 16-byte accesses when both runs start on a 16-byte
 			 * boundary (whole blocks do), scalar tail */
 			constexpr int W = 16 / sizeof(D);
@@ -226,32 +234,33 @@ ptask_kernel(const xmgd_ptask_t *__restrict__ tasks,
 			vec16<D> *dv = reinterpret_cast<vec16<D> *>(dp);
 			const vec16<D> *sv = reinterpret_cast<const vec16<D> *>(sp);
 			done = al16;
+			/* alpha == 1 of a real type, by its bits (a compare would
+			 * be an FP64 instruction) */
+			const bool one = !std::is_same<D, cf>::value &&
+			    !std::is_same<D, cd>::value &&
+			    __double_as_longlong(t.alpha[0]) == 0x3ff0000000000000ll;
 			if (al16) {
+#define FLAT_VEC(OP, AL) do { \
+	if (one) flat_vec<OP, true>(dv, sv, nv, AL, be, dre, dim_); \
+	else flat_vec<OP, false>(dv, sv, nv, AL, be, dre, dim_); } while (0)
 				switch (op) {
 				case XMGD_OP_SET:
-					flat_vec<XMGD_OP_SET>(dv, sv, nv, al, be, dre, dim_);
+					flat_vec<XMGD_OP_SET, false>(dv, sv, nv, al, be, dre, dim_);
 					break;
 				case XMGD_OP_SCALE:
-					flat_vec<XMGD_OP_SCALE>(dv, sv, nv, al, be, dre, dim_);
+					flat_vec<XMGD_OP_SCALE, false>(dv, sv, nv, al, be, dre, dim_);
 					break;
-				case XMGD_OP_AXPY:
-					flat_vec<XMGD_OP_AXPY>(dv, sv, nv, al, be, dre, dim_);
-					break;
-				case XMGD_OP_COPY:
-					flat_vec<XMGD_OP_COPY>(dv, sv, nv, als, be, dre, dim_);
-					break;
-				case XMGD_OP_MUL:
-					flat_vec<XMGD_OP_MUL>(dv, sv, nv, al, be, dre, dim_);
-					break;
-				case XMGD_OP_DIV:
-					flat_vec<XMGD_OP_DIV>(dv, sv, nv, al, be, dre, dim_);
-					break;
+				case XMGD_OP_AXPY: FLAT_VEC(XMGD_OP_AXPY, al); break;
+				case XMGD_OP_COPY: FLAT_VEC(XMGD_OP_COPY, als); break;
+				case XMGD_OP_MUL: FLAT_VEC(XMGD_OP_MUL, al); break;
+				case XMGD_OP_DIV: FLAT_VEC(XMGD_OP_DIV, al); break;
 				case XMGD_OP_DOT:
-					flat_vec<XMGD_OP_DOT>(dv, sv, nv, al, be, dre, dim_);
+					flat_vec<XMGD_OP_DOT, false>(dv, sv, nv, al, be, dre, dim_);
 					break;
 				default:
 					done = false;
 				}
+#undef FLAT_VEC
 			}
 			if (done)
 				for (int e = nv * W + threadIdx.x; e < n; e += PT_THREADS)
@@ -644,6 +653,7 @@ plan_tasks(const xmgd_ptask_t *tasks, int ntasks, int dtype, int stype,
 	const char *e = getenv("XMG_PTASK_SLAB");
 	const bool slab_on = !(e && strcmp(e, "0") == 0);
 
+	int64_t nflat = 0;
 	/* the slab launch's shared memory: the largest of its CTAs' */
 	*slab_smem = 0;
 	for (int i = 0; i < ntasks; i++) {
@@ -671,10 +681,8 @@ plan_tasks(const xmgd_ptask_t *tasks, int ntasks, int dtype, int stype,
 		    t.size[1] <= mt;
 		if (flat) {
 			m.mode = 2;
-			m.ctas_d0 = (int32_t)((t.size[0] + FLAT_ELEMS - 1) / FLAT_ELEMS);
 			m.nouter = 1;
-			m.rows_per_cta = 1;
-			cnt[i] = m.ctas_d0;
+			nflat += t.size[0];
 		} else if (mat) {
 			m.mode = 3;
 			m.nouter = 1;
@@ -708,6 +716,18 @@ plan_tasks(const xmgd_ptask_t *tasks, int ntasks, int dtype, int stype,
 			cnt[i] = (int64_t)m.ctas_d0 * ((m.nouter + rows - 1) / rows);
 		}
 	}
+	/* flat CTAs of 8192 elements, halved while they leave SMs without
+	 * four of them (a small batch is bound by the latency of a CTA's
+	 * passes: 33 000 elements divided in 6 CTAs took 52 us) */
+	int32_t chunk = FLAT_ELEMS;
+	while (chunk > FLAT_MIN && nflat < (int64_t)chunk * 4 * num_sms())
+		chunk /= 2;
+	for (int i = 0; i < ntasks; i++)
+		if (m0[i].mode == 2) {
+			m0[i].rows_per_cta = chunk;
+			m0[i].ctas_d0 = (int32_t)((tasks[i].size[0] + chunk - 1) / chunk);
+			cnt[i] = m0[i].ctas_d0;
+		}
 	sorted.clear();
 	meta.clear();
 	order.clear();
