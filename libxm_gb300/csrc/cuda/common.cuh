@@ -89,6 +89,25 @@ template <> __device__ inline cd conv<cd, cd>(cd s) { return s; }
 template <> __device__ inline cf conv<cf, cd>(cd s) { return cf{(float)s.x, (float)s.y}; }
 template <> __device__ inline cd conv<cd, cf>(cf s) { return cd{s.x, s.y}; }
 
+/* The last i in [0, n) with first(i) <= x (first ascending, first(0) <= x).
+ * Every lane of a warp searches for the same x, so each step compares 32
+ * candidates: two dependent loads up to 1024 entries, where a binary search
+ * chains ten. */
+template <typename F>
+__device__ __forceinline__ int last_at_most(int n, int64_t x, F first)
+{
+	const int lane = threadIdx.x & 31;
+	int lo = 0;
+	while (n > 1) {
+		const int step = (n + 31) / 32, o = lane * step;
+		const bool le = o < n && first(lo + o) <= x;
+		const int c = __popc(__ballot_sync(0xffffffffu, le)) - 1;
+		lo += c * step;
+		n = min(step, n - c * step);
+	}
+	return lo;
+}
+
 /* asynchronous global -> shared copy of one element (cp.async: no
  * register holds the value while it is in flight) */
 template <int B> __device__ __forceinline__ void cp_async_b(void *s, const void *g);

@@ -130,21 +130,10 @@ struct view_meta {
 	int64_t first_cta;
 };
 
-/* The view of a CTA: the last one whose first CTA is <= cta.  Every lane of
- * a warp searches for the same cta, so each step compares 32 candidates: two
- * dependent loads up to 1024 views, where a binary search chains ten. */
+/* the view of a CTA: the last one whose first CTA is <= cta */
 __device__ __forceinline__ int find_view(const view_meta *m, int n, int64_t cta)
 {
-	const int lane = threadIdx.x & 31;
-	int lo = 0;
-	while (n > 1) {
-		const int step = (n + 31) / 32, o = lane * step;
-		const bool le = o < n && m[lo + o].first_cta <= cta;
-		const int c = __popc(__ballot_sync(0xffffffffu, le)) - 1;
-		lo += c * step;
-		n = min(step, n - c * step);
-	}
-	return lo;
+	return last_at_most(n, cta, [&](int i) { return m[i].first_cta; });
 }
 
 /* Element (k', r) of a view: real views directly, complex views realified

@@ -70,6 +70,16 @@ struct task_meta {
 	int32_t ctas_d0, ctas_d1;
 };
 
+/* A batch of up to PACK tasks travels in the kernel's parameters, which
+ * spares a small call its host-to-device copy; larger batches are read
+ * from device memory. */
+constexpr int PACK = 14;
+struct task_pack {
+	xmgd_ptask_t t[PACK];
+	task_meta m[PACK];
+};
+static_assert(sizeof(task_pack) <= 3584, "kernel parameters");
+
 template <typename D, typename S>
 struct elem_op {
 	__device__ static inline void
@@ -192,19 +202,18 @@ outer_offsets(const xmgd_ptask_t &t, int first_dim, int64_t o, int64_t &od,
 
 template <typename D, typename S, int MODE>
 __global__ void __launch_bounds__(PT_THREADS, MODE == 0 ? 6 : MODE == 3 ? 5 : MODE == 2 ? 5 : 1)
-ptask_kernel(const xmgd_ptask_t *__restrict__ tasks,
-    const task_meta *__restrict__ meta, int ntasks, int64_t cta0,
+ptask_kernel(const __grid_constant__ task_pack pack,
+    const xmgd_ptask_t *__restrict__ dtasks,
+    const task_meta *__restrict__ dmeta, int ntasks, int64_t cta0,
     double *__restrict__ partial)
 {
 	__shared__ double s_red[2][PT_THREADS / 32];
 
-	/* locate the task of this CTA (binary search over first_cta) */
+	/* locate the task of this CTA */
 	const int64_t cta = cta0 + blockIdx.x;
-	int lo = 0, hi = ntasks - 1;
-	while (lo < hi) {
-		int mid = (lo + hi + 1) >> 1;
-		if (meta[mid].first_cta <= cta) lo = mid; else hi = mid - 1;
-	}
+	const xmgd_ptask_t *tasks = dtasks ? dtasks : pack.t;
+	const task_meta *meta = dtasks ? dmeta : pack.m;
+	const int lo = last_at_most(ntasks, cta, [&](int i) { return meta[i].first_cta; });
 	const xmgd_ptask_t &t = tasks[lo];
 	const task_meta &m = meta[lo];
 	int64_t local = cta - m.first_cta;
@@ -460,6 +469,35 @@ ptask_kernel(const xmgd_ptask_t *__restrict__ tasks,
 	}
 }
 
+/* Sums of the per-CTA partial dot products: a warp per task (in the
+ * caller's order, order[]), lanes striding over its CTAs, so the order of
+ * the additions depends on the batch alone. */
+__global__ void __launch_bounds__(256)
+dot_sum_kernel(const __grid_constant__ task_pack pack,
+    const task_meta *__restrict__ dmeta, const int *__restrict__ order, int ntasks,
+    int64_t nctas, const double *__restrict__ partial, double *__restrict__ out)
+{
+	const task_meta *meta = dmeta ? dmeta : pack.m;
+	const int t = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x & 31;
+	if (t >= ntasks)
+		return;
+	const int64_t end = t + 1 < ntasks ? meta[t + 1].first_cta : nctas;
+	double a = 0, b = 0;
+	for (int64_t c = meta[t].first_cta + lane; c < end; c += 32) {
+		a += partial[2 * c];
+		b += partial[2 * c + 1];
+	}
+	for (int off = 16; off > 0; off >>= 1) {
+		a += __shfl_down_sync(0xffffffffu, a, off);
+		b += __shfl_down_sync(0xffffffffu, b, off);
+	}
+	if (lane == 0) {
+		const int o = order ? order[t] : t;
+		out[2 * o] = a;
+		out[2 * o + 1] = b;
+	}
+}
+
 /* a bounded wait of the slab schedule gave up (set on the device, read
  * and cleared by the host after the launches) */
 __device__ int g_slab_err;
@@ -477,19 +515,18 @@ __device__ int g_slab_err;
  */
 template <typename T>
 __global__ void __launch_bounds__(PT_THREADS, 6)
-slab_kernel(const xmgd_ptask_t *__restrict__ tasks,
-    const task_meta *__restrict__ meta, int ntasks, int64_t cta0)
+slab_kernel(const __grid_constant__ task_pack pack,
+    const xmgd_ptask_t *__restrict__ dtasks,
+    const task_meta *__restrict__ dmeta, int ntasks, int64_t cta0)
 {
 	extern __shared__ __align__(16) unsigned char dsm[];
 	__shared__ __align__(8) uint64_t bar;
 	__shared__ int s_err;
 
 	const int64_t cta = cta0 + blockIdx.x;
-	int lo = 0, hi = ntasks - 1;
-	while (lo < hi) {
-		int mid = (lo + hi + 1) >> 1;
-		if (meta[mid].first_cta <= cta) lo = mid; else hi = mid - 1;
-	}
+	const xmgd_ptask_t *tasks = dtasks ? dtasks : pack.t;
+	const task_meta *meta = dtasks ? dmeta : pack.m;
+	const int lo = last_at_most(ntasks, cta, [&](int i) { return meta[i].first_cta; });
 	const xmgd_ptask_t &t = tasks[lo];
 	const task_meta &m = meta[lo];
 	const int s0 = (int)t.size[0], s1 = (int)t.size[1], n = s0 * s1;
@@ -578,7 +615,7 @@ slab_shape(const xmgd_ptask_t &t, int dbytes, int sbytes, int mt,
 
 template <typename D, typename S>
 static int
-launch_slab(const xmgd_ptask_t *dtasks, const task_meta *dmeta, int ntasks,
+launch_slab(const task_pack &pack, const xmgd_ptask_t *dtasks, const task_meta *dmeta, int ntasks,
     int64_t cta0, int64_t n, int64_t smem)
 {
 	if constexpr (std::is_same<D, S>::value) {
@@ -589,7 +626,7 @@ launch_slab(const xmgd_ptask_t *dtasks, const task_meta *dmeta, int ntasks,
 			attr = true;
 		}
 		slab_kernel<D><<<(unsigned)n, PT_THREADS, (size_t)smem, stream()>>>(
-		    dtasks, dmeta, ntasks, cta0);
+		    pack, dtasks, dmeta, ntasks, cta0);
 		g_launches++;
 		XMG_CK(cudaGetLastError());
 		return XMG_OK;
@@ -600,11 +637,11 @@ launch_slab(const xmgd_ptask_t *dtasks, const task_meta *dmeta, int ntasks,
 
 template <typename D, typename S>
 static int
-launch(const xmgd_ptask_t *dtasks, const task_meta *dmeta, int ntasks,
-    const int64_t *begin, int64_t slab_smem, double *dpartial)
+launch(const task_pack &pack, const xmgd_ptask_t *dtasks, const task_meta *dmeta,
+    int ntasks, const int64_t *begin, int64_t slab_smem, double *dpartial)
 {
 	if (begin[5] > begin[4]) {
-		int st = launch_slab<D, S>(dtasks, dmeta, ntasks, begin[4],
+		int st = launch_slab<D, S>(pack, dtasks, dmeta, ntasks, begin[4],
 		    begin[5] - begin[4], slab_smem);
 		if (st)
 			return st;
@@ -616,13 +653,13 @@ launch(const xmgd_ptask_t *dtasks, const task_meta *dmeta, int ntasks,
 			continue;
 		switch (mode) {
 		case 0: ptask_kernel<D, S, 0><<<(unsigned)n, PT_THREADS, 0, stream()>>>(
-		    dtasks, dmeta, ntasks, begin[mode], dpartial); break;
+		    pack, dtasks, dmeta, ntasks, begin[mode], dpartial); break;
 		case 1: ptask_kernel<D, S, 1><<<(unsigned)n, PT_THREADS, 0, stream()>>>(
-		    dtasks, dmeta, ntasks, begin[mode], dpartial); break;
+		    pack, dtasks, dmeta, ntasks, begin[mode], dpartial); break;
 		case 2: ptask_kernel<D, S, 2><<<(unsigned)n, PT_THREADS, 0, stream()>>>(
-		    dtasks, dmeta, ntasks, begin[mode], dpartial); break;
+		    pack, dtasks, dmeta, ntasks, begin[mode], dpartial); break;
 		case 3: ptask_kernel<D, S, 3><<<(unsigned)n, PT_THREADS, 0, stream()>>>(
-		    dtasks, dmeta, ntasks, begin[mode], dpartial); break;
+		    pack, dtasks, dmeta, ntasks, begin[mode], dpartial); break;
 		}
 		g_launches++;
 		XMG_CK(cudaGetLastError());
@@ -748,12 +785,12 @@ plan_tasks(const xmgd_ptask_t *tasks, int ntasks, int dtype, int stype,
 }
 
 static int
-launch_types(int dtype, int stype, const xmgd_ptask_t *dt, const task_meta *dm,
+launch_types(int dtype, int stype, const task_pack &pack, const xmgd_ptask_t *dt, const task_meta *dm,
     int ntasks, const int64_t *begin, int64_t slab_smem, double *dp)
 {
 	int st;
 
-#define L(D, S) st = launch<D, S>(dt, dm, ntasks, begin, slab_smem, dp)
+#define L(D, S) st = launch<D, S>(pack, dt, dm, ntasks, begin, slab_smem, dp)
 	if (dtype == stype) {
 		switch (dtype) {
 		case 0: L(float, float); break;
@@ -814,9 +851,31 @@ xmgd_ptask_launch(int dtype, int stype, const xmgd_ptask_batch_t *b)
 {
 	if (b->ntasks <= 0)
 		return XMG_OK;
-	return launch_types(dtype, stype, (const xmgd_ptask_t *)b->dbuf,
+	static const task_pack none = {};
+	return launch_types(dtype, stype, none, (const xmgd_ptask_t *)b->dbuf,
 	    (const task_meta *)(b->dbuf + task_bytes(b->ntasks)), b->ntasks,
 	    b->begin, b->slab_smem, nullptr);
+}
+
+/* page-locked host memory of the element-wise calls: the batch on its way
+ * to the device, or the sums a dot product's last kernel writes.  Grow-only;
+ * every call that uses it waits for its kernels before it returns. */
+static int
+batch_pinned(size_t bytes, void **p)
+{
+	static void *buf;
+	static size_t cap;
+
+	if (cap < bytes) {
+		if (buf)
+			XMG_CK(cudaFreeHost(buf));
+		buf = nullptr;
+		cap = 0;
+		XMG_CK(cudaMallocHost(&buf, bytes + bytes / 2 + 65536));
+		cap = bytes + bytes / 2 + 65536;
+	}
+	*p = buf;
+	return XMG_OK;
 }
 
 extern "C" int
@@ -826,9 +885,13 @@ xmgd_ptasks(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks,
 	std::vector<xmgd_ptask_t> sorted;
 	std::vector<task_meta> meta;
 	std::vector<int> order;
+	task_pack pack;
 	int64_t begin[6], nctas, slab_smem;
-	uint64_t dbuf, dpart = 0;
-	size_t tb, mb;
+	uint64_t dbuf = 0, dpart = 0;
+	const task_meta *dmeta = nullptr;
+	const int *dorder = nullptr;
+	void *pin = nullptr;
+	double *sums = nullptr;
 	int st;
 
 	if (ntasks <= 0)
@@ -836,23 +899,50 @@ xmgd_ptasks(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks,
 	plan_tasks(tasks, ntasks, dtype, stype, sorted, meta, order, begin,
 	    &slab_smem);
 	nctas = begin[5];
-	tb = task_bytes(ntasks);
-	mb = (size_t)ntasks * sizeof(task_meta);
-	if ((st = xmgd_scratch(2, tb + mb, &dbuf)) != XMG_OK)
-		return st;
-	XMG_CK(cudaMemcpyAsync((void *)dbuf, sorted.data(), (size_t)ntasks *
-	    sizeof(xmgd_ptask_t), cudaMemcpyHostToDevice, stream()));
-	XMG_CK(cudaMemcpyAsync((void *)(dbuf + tb), meta.data(), mb,
-	    cudaMemcpyHostToDevice, stream()));
+	const size_t tb = task_bytes(ntasks);
+	const size_t mb = ((size_t)ntasks * sizeof(task_meta) + 255) & ~(size_t)255;
+	const size_t ob = ((size_t)ntasks * sizeof(int) + 255) & ~(size_t)255;
+	const size_t db = dots ? 2 * (size_t)ntasks * sizeof(double) : 0;
+	const bool small = ntasks <= PACK;
+	bool inorder = true;
+	for (int i = 0; i < ntasks; i++)
+		inorder = inorder && order[i] == i;
+	/* an out-of-order batch of dots needs its order on the device */
+	const size_t up = small && (inorder || !dots) ? 0 : tb + mb + ob;
+	if (up + db > 0) {
+		if ((st = batch_pinned(up + db, &pin)) != XMG_OK)
+			return st;
+		sums = (double *)((char *)pin + up);
+	}
+	if (up > 0) {
+		char *h = (char *)pin;
+		memcpy(h, sorted.data(), (size_t)ntasks * sizeof(xmgd_ptask_t));
+		memcpy(h + tb, meta.data(), (size_t)ntasks * sizeof(task_meta));
+		memcpy(h + tb + mb, order.data(), (size_t)ntasks * sizeof(int));
+		if ((st = xmgd_scratch(2, up, &dbuf)) != XMG_OK)
+			return st;
+		XMG_CK(cudaMemcpyAsync((void *)dbuf, pin, up, cudaMemcpyHostToDevice,
+		    stream()));
+		dmeta = (const task_meta *)(dbuf + tb);
+		dorder = (const int *)(dbuf + tb + mb);
+	} else {
+		memcpy(pack.t, sorted.data(), (size_t)ntasks * sizeof(xmgd_ptask_t));
+		memcpy(pack.m, meta.data(), (size_t)ntasks * sizeof(task_meta));
+	}
 	if (dots && (st = xmgd_scratch(3, (size_t)nctas * 2 * sizeof(double),
 	    &dpart)) != XMG_OK)
 		return st;
-	if ((st = launch_types(dtype, stype, (const xmgd_ptask_t *)dbuf,
-	    (const task_meta *)(dbuf + tb), ntasks, begin, slab_smem,
-	    (double *)dpart)))
-		return st;
-	/* the task buffers are reused by the next batch: wait here */
-	if ((st = check(cudaStreamSynchronize(stream()), "ptask_kernel")))
+	st = launch_types(dtype, stype, pack, (const xmgd_ptask_t *)dbuf, dmeta, ntasks,
+	    begin, slab_smem, (double *)dpart);
+	if (st == XMG_OK && dots) {
+		dot_sum_kernel<<<(unsigned)((ntasks + 7) / 8), 256, 0, stream()>>>(pack,
+		    dmeta, dorder, ntasks, nctas, (const double *)dpart, sums);
+		g_launches++;
+		st = check(cudaGetLastError(), "dot_sum_kernel");
+	}
+	/* the buffers are reused by the next batch: wait here */
+	const int st2 = check(cudaStreamSynchronize(stream()), "ptask_kernel");
+	if (st != XMG_OK || (st = st2) != XMG_OK)
 		return st;
 	if (begin[5] > begin[4]) {
 		int err = 0;
@@ -864,20 +954,7 @@ xmgd_ptasks(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks,
 			    "did not complete within the bounded wait");
 		}
 	}
-	if (dots) {
-		std::vector<double> h((size_t)nctas * 2);
-		if ((st = xmgd_d2h(h.data(), dpart, h.size() * sizeof(double))))
-			return st;
-		for (int j = 0; j < ntasks; j++) {
-			const int64_t e = j + 1 < ntasks ? meta[j + 1].first_cta : nctas;
-			double a = 0, b = 0;
-			for (int64_t c = meta[j].first_cta; c < e; c++) {
-				a += h[2 * c];
-				b += h[2 * c + 1];
-			}
-			dots[2 * order[j]] = a;
-			dots[2 * order[j] + 1] = b;
-		}
-	}
+	if (dots)
+		memcpy(dots, sums, db);
 	return XMG_OK;
 }

@@ -150,6 +150,12 @@ xmg_block_space_autosplit_tiles(xm_block_space_t *bs, size_t target,
 	return XMG_OK;
 }
 
+const size_t *
+xmg_block_space_splits(const xm_block_space_t *bs, size_t dim)
+{
+	return bs->splits[dim];
+}
+
 size_t
 xm_block_space_get_split(xm_block_space_t *bs, size_t dim, size_t i)
 {

@@ -69,6 +69,9 @@ size_t xmg_tensor_block_linear(const xm_tensor_t *t, xm_dim_t blkidx);
 void xmg_tensor_block_strides(const xm_tensor_t *t, xm_dim_t blkidx,
     int64_t strides[XM_MAX_DIM]);
 
+/* split points of a dimension: block i covers [s[i], s[i + 1]) */
+const size_t *xmg_block_space_splits(const xm_block_space_t *bs, size_t dim);
+
 /* element-type helpers */
 static inline int xmg_is_complex(xm_scalar_type_t t)
 { return t == XM_SCALAR_FLOAT_COMPLEX || t == XM_SCALAR_DOUBLE_COMPLEX; }
