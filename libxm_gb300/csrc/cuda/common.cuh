@@ -70,7 +70,22 @@ template <> struct num<cd> {
 	__device__ static cd fma(cd a, cd b, cd c) {
 		return cd{::fma(a.x, b.x, ::fma(-a.y, b.y, c.x)), ::fma(a.x, b.y, ::fma(a.y, b.x, c.y))}; }
 	__device__ static cd add(cd a, cd b) { return cd{a.x + b.x, a.y + b.y}; }
+	/* a conj(b) / |b|^2: six FP64 instructions and two divisions on the
+	 * integer pipe, where no product or square can leave the normal range
+	 * (each part zero or between 2^-400 and 2^400); elsewhere cuCdiv, which
+	 * scales */
+	__device__ static bool tame(double v) {
+		const uint32_t h = (uint32_t)__double2hiint(v) & 0x7fffffffu;
+		return h - (623u << 20) < (800u << 20) || (h | (uint32_t)__double2loint(v)) == 0; }
 	__device__ static cd div(cd a, cd b) {
+		if (tame(a.x) && tame(a.y) && tame(b.x) && tame(b.y) &&
+		    (((uint32_t)__double2hiint(b.x) | (uint32_t)__double2hiint(b.y)) & 0x7fffffffu)) {
+			const double d = ::fma(b.x, b.x, b.y * b.y);
+			return cd{div_f64(::fma(a.x, b.x, a.y * b.y), d),
+			    div_f64(::fma(a.y, b.x, -a.x * b.y), d)};
+		}
+		return div_any(a, b); }
+	static __device__ __noinline__ cd div_any(cd a, cd b) {
 		cuDoubleComplex q = cuCdiv(make_cuDoubleComplex(a.x, a.y), make_cuDoubleComplex(b.x, b.y));
 		return cd{cuCreal(q), cuCimag(q)}; }
 	__device__ static cd zero() { return cd{0.0, 0.0}; }
@@ -106,33 +121,6 @@ __device__ __forceinline__ int last_at_most(int n, int64_t x, F first)
 		n = min(step, n - c * step);
 	}
 	return lo;
-}
-
-/* asynchronous global -> shared copy of one element (cp.async: no
- * register holds the value while it is in flight) */
-template <int B> __device__ __forceinline__ void cp_async_b(void *s, const void *g);
-template <> __device__ __forceinline__ void cp_async_b<4>(void *s, const void *g)
-{
-	asm volatile("cp.async.ca.shared.global [%0], [%1], 4;"
-	    :: "r"((uint32_t)__cvta_generic_to_shared(s)), "l"(g) : "memory");
-}
-template <> __device__ __forceinline__ void cp_async_b<8>(void *s, const void *g)
-{
-	asm volatile("cp.async.ca.shared.global [%0], [%1], 8;"
-	    :: "r"((uint32_t)__cvta_generic_to_shared(s)), "l"(g) : "memory");
-}
-template <> __device__ __forceinline__ void cp_async_b<16>(void *s, const void *g)
-{
-	asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
-	    :: "r"((uint32_t)__cvta_generic_to_shared(s)), "l"(g) : "memory");
-}
-template <typename T> __device__ __forceinline__ void cp_async_elem(T *s, const T *g)
-{
-	cp_async_b<sizeof(T)>(s, g);
-}
-__device__ __forceinline__ void cp_async_wait_all()
-{
-	asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
 } /* namespace xmg */

@@ -11,31 +11,24 @@
  *
  * Four schedules, chosen per task on the host after xmg_ptask_shape has
  * normalised the iteration space; each schedule is its own kernel
- * instantiation (so the lean ones keep few registers and full occupancy),
+ * instantiation (so the lean ones keep few registers),
  * and a batch launches one kernel per schedule present:
  *  - flat: one contiguous run on both sides (whole canonical blocks);
  *  - row: dimension 0 unit-stride on the destination side; a CTA covers
  *    ROW_ELEMS elements along dim 0 for as many outer rows as fit, with
  *    per-row outer offsets precomputed in shared memory;
- *  - matrix: the source's unit-stride dimension is dim 1 and both extents
- *    fit one tile; a CTA moves whole s0 x s1 slices through padded shared
+ *  - slices: the source's unit-stride dimension is dim 1 and both extents
+ *    are small: a CTA moves whole s0 x s1 slices through padded shared
  *    memory (loads along the source's runs, stores along the
  *    destination's): the gather-transpose of unfold/fold;
- *  - tile: the same for larger extents, TILE x TILE tiles;
- *  - slab: xm_copy's transposes when each s0 x s1 slice lies contiguously
- *    on both sides and consecutive slices follow one another (whole
- *    blocks whose permutation swaps the two leading dimensions): a CTA
- *    brings its slices in with one bulk copy into shared memory,
- *    transposes there and stores along the destination's run.
+ *  - tile: the same for larger extents, a t0 x t1 tile per CTA;
  */
-#include <stdlib.h>
 #include <string.h>
 #include <algorithm>
 #include <type_traits>
 #include <vector>
 
 #include "common.cuh"
-#include "tc.cuh"
 
 namespace xmg {
 
@@ -43,147 +36,228 @@ constexpr int PT_THREADS = 256;
 constexpr int ROW_ELEMS = 4096;    /* elements per CTA in row mode */
 constexpr int FLAT_ELEMS = 8192;   /* elements per CTA in flat mode, at most */
 constexpr int FLAT_MIN = 1024;     /* ... and at least */
-constexpr int TILE = 32;
-/* matrix mode: whole s0 x s1 slices (both <= MT) per CTA; a source and a
- * destination tile of both types fit the 48 KB of static shared memory */
-template <typename D, typename S> struct mt_of {
-	static constexpr int v = sizeof(S) <= 8 && sizeof(D) <= 8 ? 48 : 32;
-};
-static inline int mt_host(int dbytes, int sbytes)
+constexpr int SLICE_MAX = 48;      /* slices: extents at most */
+constexpr int SLICE_MAXQ = 64;     /* slices per CTA at most */
+/* tile and slices: elements per CTA (eight per thread; sixteen of the
+ * 4-byte type, four of the 16-byte ones), and the shared tile with the
+ * padding of its rows */
+static constexpr int tile_elems(int dbytes, int sbytes)
 {
-	return sbytes <= 8 && dbytes <= 8 ? 48 : 32;
+	return dbytes == 4 && sbytes == 4 ? 4096 : dbytes <= 8 && sbytes <= 8 ? 2048 : 1024;
 }
-constexpr int MAT_MAXQ = 64;       /* slices per CTA at most */
-/* slab schedule: about SLAB_CHUNK bytes of slices per CTA (one slice at
- * least), at most SLAB_SMEM bytes of shared memory (the source's slices
- * and the padded tile) */
-constexpr int64_t SLAB_CHUNK = 16384;
-constexpr int64_t SLAB_SMEM = 64 * 1024;
-
+static constexpr int tile_cap(int n) { return n + 256; }
+/* log2 of the lanes along a run of n <= 32 elements: 8 to 32 */
+static inline int lanes_log2(int n) { return n <= 8 ? 3 : n <= 16 ? 4 : 5; }
 
 struct task_meta {
 	int64_t first_cta;
-	int32_t mode;          /* 0 row, 1 tile, 2 flat, 3 matrix, 4 slab */
+	int32_t mode;          /* 0 row, 1 tile, 2 flat, 3 slices */
 	int32_t rows_per_cta;  /* row mode: outer rows per CTA; flat mode:
-	                          elements per CTA */
+	                          elements per CTA; slices: slices */
 	int64_t nouter;        /* row: product of dims 1..; tile: dims 2.. */
 	int32_t ctas_d0, ctas_d1;
+	int32_t t0, t1;        /* tile mode: extents of a tile */
+	int32_t l1, lb;        /* tile mode: log2 of the lanes along dim 1, of
+	                          the 32-lane blocks along dim 0 */
 };
 
 /* A batch of up to PACK tasks travels in the kernel's parameters, which
  * spares a small call its host-to-device copy; larger batches are read
  * from device memory. */
-constexpr int PACK = 14;
+constexpr int PACK = 13;
 struct task_pack {
 	xmgd_ptask_t t[PACK];
 	task_meta m[PACK];
 };
 static_assert(sizeof(task_pack) <= 3584, "kernel parameters");
 
+/* a task's scalars (als: alpha in the source's type) */
 template <typename D, typename S>
-struct elem_op {
-	__device__ static inline void
-	apply(int op, D *dp, const S *sp, const D &al, const S &als, const D &be,
-	    double &dre, double &dim_)
-	{
-		switch (op) {
-		case XMGD_OP_SET: *dp = al; break;
-		case XMGD_OP_COPY: *dp = conv<D, S>(num<S>::mul(als, *sp)); break;
-		case XMGD_OP_SCALE: *dp = num<D>::mul(al, *dp); break;
-		case XMGD_OP_AXPY: {
-			D s = conv<D, S>(*sp);
-			*dp = num<D>::add(num<D>::mul(al, *dp), num<D>::mul(be, s));
-			break;
-		}
-		case XMGD_OP_MUL: {
-			D s = conv<D, S>(*sp);
-			*dp = num<D>::mul(num<D>::mul(al, *dp), s);
-			break;
-		}
-		case XMGD_OP_DIV: {
-			D s = conv<D, S>(*sp);
-			*dp = num<D>::div(*dp, num<D>::mul(al, s));
-			break;
-		}
-		case XMGD_OP_DOT: {
-			D s = conv<D, S>(*sp);
-			D pr = num<D>::mul(*dp, s);
-			dre += num<D>::re(pr);
-			dim_ += num<D>::im(pr);
-			break;
-		}
-		}
-	}
+struct scalars {
+	D al, be;
+	S als;
+	__device__ __forceinline__ explicit scalars(const xmgd_ptask_t &t) :
+	    al(num<D>::mk(t.alpha)), be(num<D>::mk(t.beta)), als(num<S>::mk(t.alpha)) {}
 };
 
+__device__ __forceinline__ bool finite(const cd &v)
+{
+	return (__double2hiint(v.x) & 0x7ff00000) != 0x7ff00000 &&
+	    (__double2hiint(v.y) & 0x7ff00000) != 0x7ff00000;
+}
+
+/* the whole complex expression, out of line: Inf and NaN alone take it */
+static __device__ __noinline__ cd axpy_any(cd al, cd x, cd be, cd y)
+{
+	return num<cd>::add(num<cd>::mul(al, x), num<cd>::mul(be, y));
+}
+
+static __device__ __noinline__ cd mul_any(cd a, cd b) { return num<cd>::mul(a, b); }
+
+/* s * v; ONE: s is 1, left out for real types and for finite complex ones
+ * (Inf and NaN take the product, which spreads NaN to both parts) */
+template <bool ONE, typename T>
+__device__ __forceinline__ T unit(const T &s, const T &v)
+{
+	if constexpr (!ONE)
+		return num<T>::mul(s, v);
+	else if constexpr (std::is_same<T, cd>::value)
+		return finite(v) ? v : mul_any(s, v);
+	else
+		return v;
+}
+
+/* The new value of a destination element x from a source element y (dot:
+ * its product added to the sums).  ONE: alpha is 1 (and a complex beta
+ * real), so that products with 1 and 0 are left out: the FP64 pipe issues 2
+ * instructions a cycle and SM against one 8-byte element a cycle from
+ * memory, so that two of them per element (alpha x and + beta y), ten of a
+ * complex one, already take the time of the traffic or more. */
+template <int OP, bool ONE, typename D, typename S>
+__device__ __forceinline__ D
+combine(D x, S y, const scalars<D, S> &c, double &dre, double &dim_)
+{
+	if constexpr (OP == XMGD_OP_SET)
+		return c.al;
+	else if constexpr (OP == XMGD_OP_SCALE)
+		return num<D>::mul(c.al, x);
+	else if constexpr (OP == XMGD_OP_AXPY && ONE && std::is_same<D, cd>::value)
+		return finite(x) && finite(y) ?
+		    cd{::fma(c.be.x, y.x, x.x), ::fma(c.be.x, y.y, x.y)} :
+		    axpy_any(c.al, x, c.be, y);
+	else if constexpr (OP == XMGD_OP_AXPY)
+		return num<D>::add(unit<ONE>(c.al, x), num<D>::mul(c.be, conv<D, S>(y)));
+	else if constexpr (OP == XMGD_OP_COPY)
+		return conv<D, S>(unit<ONE>(c.als, y));
+	else if constexpr (OP == XMGD_OP_MUL)
+		return num<D>::mul(unit<ONE>(c.al, x), conv<D, S>(y));
+	else if constexpr (OP == XMGD_OP_DIV)
+		return num<D>::div(x, unit<ONE>(c.al, conv<D, S>(y)));
+	else if constexpr (std::is_same<D, cd>::value) {
+		/* four fused steps, no product rounded on its own */
+		const cd z = conv<D, S>(y);
+		dre = ::fma(x.x, z.x, ::fma(-x.y, z.y, dre));
+		dim_ = ::fma(x.x, z.y, ::fma(x.y, z.x, dim_));
+		return x;
+	} else {
+		const D pr = num<D>::mul(x, conv<D, S>(y));
+		dre += num<D>::re(pr);
+		dim_ += num<D>::im(pr);
+		return x;
+	}
+}
+
+/* f.run<OP, ONE>() for a task's operation; scalar conversions exist for
+ * xm_copy alone, and ONE is set apart where FP64 work bounds the kernel or
+ * costs nothing to leave out */
+template <typename D, typename S, typename F>
+__device__ __forceinline__ void
+with_op(const xmgd_ptask_t &t, F f)
+{
+	constexpr bool special = !std::is_same<D, cf>::value;
+	/* by their bits: a compare would be an FP64 instruction */
+	bool one = special && __double_as_longlong(t.alpha[0]) == 0x3ff0000000000000ll;
+	if (std::is_same<D, cd>::value)
+		one = one && __double_as_longlong(t.alpha[1]) == 0 &&
+		    __double_as_longlong(t.beta[1]) == 0;
+#define WITH(OP) case OP: \
+	if (one) f.template run<OP, special>(); else f.template run<OP, false>(); break
+	switch (t.op) {
+	case XMGD_OP_SET: f.template run<XMGD_OP_SET, false>(); break;
+	WITH(XMGD_OP_COPY);
+	default:
+		if constexpr (std::is_same<D, S>::value) {
+			switch (t.op) {
+			case XMGD_OP_SCALE: f.template run<XMGD_OP_SCALE, false>(); break;
+			WITH(XMGD_OP_AXPY);
+			WITH(XMGD_OP_MUL);
+			WITH(XMGD_OP_DIV);
+			case XMGD_OP_DOT: f.template run<XMGD_OP_DOT, false>(); break;
+			}
+		}
+	}
+#undef WITH
+}
+
+constexpr bool op_reads_dst(int op) { return op != XMGD_OP_COPY && op != XMGD_OP_SET; }
+constexpr bool op_reads_src(int op) { return op != XMGD_OP_SET && op != XMGD_OP_SCALE; }
+
 /*
- * Flat runs with 16-byte accesses.  Each thread issues the loads of U
- * vectors (of both runs) before any of its stores: stores to dst may alias
- * src as far as the compiler knows, so a plain loop keeps one iteration's
- * loads in flight at a time.  ONE: alpha is 1 (real types), so that its
- * product is left out: at 2 FP64 instructions a cycle and SM against one
- * element a cycle from memory, two of them per element (alpha x and
- * + beta y) already take the time of the traffic.
+ * Flat runs with 16-byte accesses where both runs start on a 16-byte
+ * boundary (whole blocks do), else one element at a time.  Each thread
+ * issues the loads of U vectors (of both runs) before any of its stores:
+ * stores to dst may alias src as far as the compiler knows, so a plain loop
+ * keeps one iteration's loads in flight at a time.
  */
 template <typename D> struct alignas(16) vec16 { D v[16 / sizeof(D)]; };
 
-template <int OP, bool ONE, typename D>
-__device__ inline void
-flat_vec(vec16<D> *dv, const vec16<D> *sv, int nv, const D al, const D be,
-    double &dre, double &dim_)
-{
-	/* (a division needs the registers of two vectors more) */
-	constexpr int W = 16 / sizeof(D), U = OP == XMGD_OP_DIV ? 2 : 4;
-	constexpr bool RD = OP != XMGD_OP_COPY && OP != XMGD_OP_SET;
-	constexpr bool RS = OP != XMGD_OP_SET && OP != XMGD_OP_SCALE;
-	constexpr bool WR = OP != XMGD_OP_DOT;
+template <typename D, typename S>
+struct flat_run {
+	D *dp;
+	const S *sp;
+	int n;
+	const xmgd_ptask_t &t;
+	double &dre, &dim_;
 
-	for (int e0 = threadIdx.x; e0 < nv; e0 += U * PT_THREADS) {
-		vec16<D> x[U], y[U];
-#pragma unroll
-		for (int u = 0; u < U; u++) {
-			const int e = e0 + u * PT_THREADS;
-			if (e < nv) {
-				if (RD)
-					x[u] = dv[e];
-				if (RS)
-					y[u] = sv[e];
-			}
+	template <int OP, bool ONE>
+	__device__ __forceinline__ void run()
+	{
+		int e0 = 0;
+		if constexpr (std::is_same<D, S>::value) {
+			if (((reinterpret_cast<uintptr_t>(dp) |
+			    reinterpret_cast<uintptr_t>(sp)) & 15) == 0)
+				e0 = vectors<OP, ONE>();
 		}
-#pragma unroll
-		for (int u = 0; u < U; u++) {
-			const int e = e0 + u * PT_THREADS;
-			if (e >= nv)
-				break;
-#pragma unroll
-			for (int w = 0; w < W; w++) {
-				D &xv = x[u].v[w];
-				if (OP == XMGD_OP_SET)
-					xv = al;
-				else if (OP == XMGD_OP_SCALE)
-					xv = ONE ? xv : num<D>::mul(al, xv);
-				else if (OP == XMGD_OP_AXPY)
-					xv = num<D>::add(ONE ? xv : num<D>::mul(al, xv),
-					    num<D>::mul(be, y[u].v[w]));
-				else if (OP == XMGD_OP_COPY)
-					xv = ONE ? y[u].v[w] : num<D>::mul(al, y[u].v[w]);
-				else if (OP == XMGD_OP_MUL)
-					xv = num<D>::mul(ONE ? xv : num<D>::mul(al, xv),
-					    y[u].v[w]);
-				else if (OP == XMGD_OP_DIV)
-					xv = num<D>::div(xv, ONE ? y[u].v[w] :
-					    num<D>::mul(al, y[u].v[w]));
-				else {
-					const D pr = num<D>::mul(xv, y[u].v[w]);
-					dre += num<D>::re(pr);
-					dim_ += num<D>::im(pr);
-				}
-			}
-			if (WR)
-				dv[e] = x[u];
+		const scalars<D, S> c(t);
+#pragma unroll 4
+		for (int e = e0 + threadIdx.x; e < n; e += PT_THREADS) {
+			const S y = op_reads_src(OP) ? sp[e] : S();
+			const D x = combine<OP, ONE>(op_reads_dst(OP) ? dp[e] : D(), y, c, dre,
+			    dim_);
+			if (OP != XMGD_OP_DOT)
+				dp[e] = x;
 		}
 	}
-}
+
+	/* whole vectors; the number of elements done */
+	template <int OP, bool ONE>
+	__device__ __forceinline__ int vectors()
+	{
+		/* (a division needs the registers of two vectors more) */
+		constexpr int W = 16 / sizeof(D), U = OP == XMGD_OP_DIV ? 2 : 4;
+		vec16<D> *dv = reinterpret_cast<vec16<D> *>(dp);
+		const vec16<D> *sv = reinterpret_cast<const vec16<D> *>(sp);
+		const int nv = n / W;
+		const scalars<D, S> c(t);
+
+		for (int e0 = threadIdx.x; e0 < nv; e0 += U * PT_THREADS) {
+			vec16<D> x[U], y[U];
+#pragma unroll
+			for (int u = 0; u < U; u++) {
+				const int e = e0 + u * PT_THREADS;
+				if (e < nv) {
+					if (op_reads_dst(OP))
+						x[u] = dv[e];
+					if (op_reads_src(OP))
+						y[u] = sv[e];
+				}
+			}
+#pragma unroll
+			for (int u = 0; u < U; u++) {
+				const int e = e0 + u * PT_THREADS;
+				if (e >= nv)
+					break;
+#pragma unroll
+				for (int w = 0; w < W; w++)
+					x[u].v[w] = combine<OP, ONE>(x[u].v[w], y[u].v[w], c, dre,
+					    dim_);
+				if (OP != XMGD_OP_DOT)
+					dv[e] = x[u];
+			}
+		}
+		return nv * W;
+	}
+};
 
 static __device__ inline void
 outer_offsets(const xmgd_ptask_t &t, int first_dim, int64_t o, int64_t &od,
@@ -192,16 +266,228 @@ outer_offsets(const xmgd_ptask_t &t, int first_dim, int64_t o, int64_t &od,
 	od = 0;
 	os = 0;
 	for (int d = first_dim; d < t.ndim; d++) {
-		int64_t sz = t.size[d];
-		int64_t q = o % sz;
-		o /= sz;
+		const uint32_t sz = (uint32_t)t.size[d];
+		int64_t q;
+		if ((uint64_t)o >> 32) {
+			q = o % sz;
+			o /= sz;
+		} else {	/* a 64-bit division costs about a hundred instructions */
+			q = (uint32_t)o % sz;
+			o = (uint32_t)o / sz;
+		}
 		od += q * t.dst_stride[d];
 		os += q * t.src_stride[d];
 	}
 }
 
+/* e / d by one multiplication, exact for e, d < 2^16 */
+struct fastdiv {
+	uint32_t d, mg;
+	__device__ __forceinline__ explicit fastdiv(uint32_t d_) : d(d_), mg(0xffffffffu / d_ + 1) {}
+	__device__ __forceinline__ uint32_t operator()(uint32_t e) const
+	{ return d == 1 ? e : __umulhi(e, mg); }
+};
+
+/*
+ * Tile schedule: a w0 x w1 tile of dims 0 (the destination's smallest
+ * stride) and 1 (unit stride in src, w1 <= 32).  Loads have 2^l1 lanes along
+ * dim 1, stores a warp along dim 0 in 2^lb blocks; a thread's loads of both
+ * sides are issued together, and the source goes through shared memory with
+ * an odd row pitch.  The kernel is bound by instruction issue, then HBM: a
+ * flattened walk (multiplications to find each element's place, 165 issue
+ * slots per element in all) moved 2 x 0.76 GB in 440 us; with fixed lanes
+ * places advance by additions.
+ */
+template <typename D, typename S>
+struct tile_run {
+	D *dst;
+	const S *src;
+	int w0, w1, l1, lb;
+	int64_t ss0, ds0, ds1;
+	S *tile;
+	const xmgd_ptask_t &t;
+	double &dre, &dim_;
+
+	template <int OP, bool ONE>
+	__device__ __forceinline__ void run()
+	{
+		constexpr int U = tile_elems(sizeof(D), sizeof(S)) / PT_THREADS;
+		constexpr int NW = PT_THREADS / 32;
+		const int ld = w0 | 1;
+		const int lx = threadIdx.x & 31, wy = threadIdx.x >> 5;
+		const int l = threadIdx.x & ((1 << l1) - 1), r0 = threadIdx.x >> l1;
+		const int rs = PT_THREADS >> l1, mask = (1 << lb) - 1;
+		S y[U];
+		D x[U];
+		{
+			const S *p = src + r0 * ss0 + l;
+			const int64_t step = rs * ss0;
+#pragma unroll
+			for (int u = 0; u < U; u++, p += step)
+				if (r0 + u * rs < w0 && l < w1)
+					y[u] = *p;
+		}
+		/* store steps: block u & mask of dim 0, then dim 1 by NW */
+		const int64_t da = 32 * ds0, db = NW * ds1 - mask * da;
+		D *dp = dst + wy * ds1 + lx * ds0;
+		if (op_reads_dst(OP)) {
+			const D *p = dp;
+#pragma unroll
+			for (int u = 0; u < U; u++) {
+				if (wy + NW * (u >> lb) < w1 && lx + 32 * (u & mask) < w0)
+					x[u] = *p;
+				p += ((u + 1) & mask) ? da : db;
+			}
+		}
+		{
+			S *p = tile + l * ld + r0;
+#pragma unroll
+			for (int u = 0; u < U; u++, p += rs)
+				if (r0 + u * rs < w0 && l < w1)
+					*p = y[u];
+		}
+		__syncthreads();
+		const scalars<D, S> c(t);
+		const S *tp = tile + wy * ld + lx;
+		const int ta = 32, tb = NW * ld - mask * 32;
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			if (wy + NW * (u >> lb) < w1 && lx + 32 * (u & mask) < w0) {
+				x[u] = combine<OP, ONE>(x[u], *tp, c, dre, dim_);
+				if (OP != XMGD_OP_DOT)
+					*dp = x[u];
+			}
+			const bool in = ((u + 1) & mask) != 0;
+			dp += in ? da : db;
+			tp += in ? ta : tb;
+		}
+	}
+};
+
+/*
+ * Slices schedule: k whole s0 x s1 slices (dims as above, both extents
+ * small), flattened over the threads: with 16 x 16 slices, fixed lanes along
+ * either run would leave half of them idle.  Strides fit 32 bits (checked on
+ * the host), so that an element's place in its slice does too.
+ */
+template <typename D, typename S>
+struct slice_run {
+	D *dst;
+	const S *src;
+	int w0, w1, total;
+	int ss0, ds0, ds1;
+	const int64_t (*so)[SLICE_MAXQ];     /* slice offsets: dst, src */
+	S *tile;
+	const xmgd_ptask_t &t;
+	double &dre, &dim_;
+
+	template <int OP, bool ONE>
+	__device__ __forceinline__ void run()
+	{
+		constexpr int U = tile_elems(sizeof(D), sizeof(S)) / PT_THREADS;
+		const int n = w0 * w1, ld = w0 | 1;
+		const fastdiv by_n(n), by_w1(w1), by_w0(w0);
+		S y[U];
+		D x[U];
+		uint32_t e0 = threadIdx.x;
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			const uint32_t e = e0 + u * PT_THREADS;
+			if ((int)e < total) {
+				const uint32_t q = by_n(e), r = e - q * n;
+				const int i0 = by_w1(r), i1 = r - i0 * w1;
+				y[u] = (src + so[1][q])[i0 * ss0 + i1];
+			}
+		}
+		if (op_reads_dst(OP)) {
+#pragma unroll
+			for (int u = 0; u < U; u++) {
+				const uint32_t e = e0 + u * PT_THREADS;
+				if ((int)e < total) {
+					const uint32_t q = by_n(e), r = e - q * n;
+					const int i1 = by_w0(r), i0 = r - i1 * w0;
+					x[u] = (dst + so[0][q])[i1 * ds1 + i0 * ds0];
+				}
+			}
+		}
+		/* the places are computed again below: kept from above they
+		 * would not fit the registers */
+		asm volatile("" : "+r"(e0));
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			const uint32_t e = e0 + u * PT_THREADS;
+			if ((int)e < total) {
+				const uint32_t q = by_n(e), r = e - q * n;
+				const int i0 = by_w1(r), i1 = r - i0 * w1;
+				tile[(q * w1 + i1) * ld + i0] = y[u];
+			}
+		}
+		__syncthreads();
+		const scalars<D, S> c(t);
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			const uint32_t e = e0 + u * PT_THREADS;
+			if ((int)e < total) {
+				const uint32_t g = by_w0(e), q = by_n(e);
+				const int i0 = e - g * w0, i1 = g - q * w1;
+				x[u] = combine<OP, ONE>(x[u], tile[g * ld + i0], c, dre, dim_);
+				if (OP != XMGD_OP_DOT)
+					(dst + so[0][q])[i1 * ds1 + i0 * ds0] = x[u];
+			}
+		}
+	}
+};
+
+/* Row schedule: rows of w0 elements along dim 0, one after the other over
+ * the CTA's threads; eight elements of a thread in flight at a time (four
+ * of the 16-byte types). */
+template <typename D, typename S>
+struct row_run {
+	D *dst;
+	const S *src;
+	int rows, w0;
+	int64_t ds0, ss0;
+	const int64_t (*so)[PT_THREADS];     /* row offsets: dst, src */
+	const xmgd_ptask_t &t;
+	double &dre, &dim_;
+
+	template <int OP, bool ONE>
+	__device__ __forceinline__ void run()
+	{
+		constexpr int U = sizeof(D) <= 8 && OP != XMGD_OP_DIV ? 8 : 4;
+		const scalars<D, S> c(t);
+		const int n = rows * w0;
+		const fastdiv by_w0(w0);
+		for (int e0 = threadIdx.x; e0 < n; e0 += U * PT_THREADS) {
+			S y[U];
+			D x[U];
+#pragma unroll
+			for (int u = 0; u < U; u++) {
+				const uint32_t e = e0 + u * PT_THREADS;
+				if ((int)e < n) {
+					const uint32_t r = by_w0(e), i = e - r * w0;
+					if (op_reads_src(OP))
+						y[u] = src[so[1][r] + i * ss0];
+					if (op_reads_dst(OP))
+						x[u] = dst[so[0][r] + i * ds0];
+				}
+			}
+#pragma unroll
+			for (int u = 0; u < U; u++) {
+				const uint32_t e = e0 + u * PT_THREADS;
+				if ((int)e < n) {
+					const uint32_t r = by_w0(e), i = e - r * w0;
+					x[u] = combine<OP, ONE>(x[u], y[u], c, dre, dim_);
+					if (OP != XMGD_OP_DOT)
+						dst[so[0][r] + i * ds0] = x[u];
+				}
+			}
+		}
+	}
+};
+
 template <typename D, typename S, int MODE>
-__global__ void __launch_bounds__(PT_THREADS, MODE == 0 ? 6 : MODE == 3 ? 5 : MODE == 2 ? 5 : 1)
+__global__ void __launch_bounds__(PT_THREADS, 4)
 ptask_kernel(const __grid_constant__ task_pack pack,
     const xmgd_ptask_t *__restrict__ dtasks,
     const task_meta *__restrict__ dmeta, int ntasks, int64_t cta0,
@@ -219,94 +505,17 @@ ptask_kernel(const __grid_constant__ task_pack pack,
 	int64_t local = cta - m.first_cta;
 	D *dst = reinterpret_cast<D *>(t.dst);
 	const S *src = reinterpret_cast<const S *>(t.src);
-	const D al = num<D>::mk(t.alpha), be = num<D>::mk(t.beta);
-	const S als = num<S>::mk(t.alpha);
 	const int op = t.op;
 	double dre = 0, dim_ = 0;
 
 	if constexpr (MODE == 2) {
-		/* flat: consecutive threads take consecutive elements, the op
-		 * resolved outside the loop */
+		/* flat: consecutive threads take consecutive elements */
 		const int chunk = m.rows_per_cta;
 		const int64_t base = local * chunk;
 		const int n = (int)(t.size[0] - base < chunk ? t.size[0] - base : chunk);
-		D *dp = dst + base;
-		const S *sp = src + base;
-		bool done = false;
-		if constexpr (std::is_same<D, S>::value && sizeof(D) <= 16) {
-			/* 16-byte accesses when both runs start on a 16-byte
-			 * boundary (whole blocks do), scalar tail */
-			constexpr int W = 16 / sizeof(D);
-			const bool al16 = ((reinterpret_cast<uintptr_t>(dp) |
-			    reinterpret_cast<uintptr_t>(sp)) & 15) == 0;
-			const int nv = n / W;
-			vec16<D> *dv = reinterpret_cast<vec16<D> *>(dp);
-			const vec16<D> *sv = reinterpret_cast<const vec16<D> *>(sp);
-			done = al16;
-			/* alpha == 1 of a real type, by its bits (a compare would
-			 * be an FP64 instruction) */
-			const bool one = !std::is_same<D, cf>::value &&
-			    !std::is_same<D, cd>::value &&
-			    __double_as_longlong(t.alpha[0]) == 0x3ff0000000000000ll;
-			if (al16) {
-#define FLAT_VEC(OP, AL) do { \
-	if (one) flat_vec<OP, true>(dv, sv, nv, AL, be, dre, dim_); \
-	else flat_vec<OP, false>(dv, sv, nv, AL, be, dre, dim_); } while (0)
-				switch (op) {
-				case XMGD_OP_SET:
-					flat_vec<XMGD_OP_SET, false>(dv, sv, nv, al, be, dre, dim_);
-					break;
-				case XMGD_OP_SCALE:
-					flat_vec<XMGD_OP_SCALE, false>(dv, sv, nv, al, be, dre, dim_);
-					break;
-				case XMGD_OP_AXPY: FLAT_VEC(XMGD_OP_AXPY, al); break;
-				case XMGD_OP_COPY: FLAT_VEC(XMGD_OP_COPY, als); break;
-				case XMGD_OP_MUL: FLAT_VEC(XMGD_OP_MUL, al); break;
-				case XMGD_OP_DIV: FLAT_VEC(XMGD_OP_DIV, al); break;
-				case XMGD_OP_DOT:
-					flat_vec<XMGD_OP_DOT, false>(dv, sv, nv, al, be, dre, dim_);
-					break;
-				default:
-					done = false;
-				}
-#undef FLAT_VEC
-			}
-			if (done)
-				for (int e = nv * W + threadIdx.x; e < n; e += PT_THREADS)
-					elem_op<D, S>::apply(op, dp + e, sp + e, al, als, be, dre, dim_);
-		}
-		if (!done)
-		switch (op) {
-		case XMGD_OP_SET:
-#pragma unroll 4
-			for (int e = threadIdx.x; e < n; e += PT_THREADS)
-				dp[e] = al;
-			break;
-		case XMGD_OP_SCALE:
-#pragma unroll 4
-			for (int e = threadIdx.x; e < n; e += PT_THREADS)
-				dp[e] = num<D>::mul(al, dp[e]);
-			break;
-		case XMGD_OP_AXPY:
-#pragma unroll 4
-			for (int e = threadIdx.x; e < n; e += PT_THREADS) {
-				const D x = conv<D, S>(sp[e]);
-				dp[e] = num<D>::add(num<D>::mul(al, dp[e]), num<D>::mul(be, x));
-			}
-			break;
-		case XMGD_OP_COPY:
-#pragma unroll 4
-			for (int e = threadIdx.x; e < n; e += PT_THREADS)
-				dp[e] = conv<D, S>(num<S>::mul(als, sp[e]));
-			break;
-		default:
-#pragma unroll 4
-			for (int e = threadIdx.x; e < n; e += PT_THREADS)
-				elem_op<D, S>::apply(op, dp + e, sp + e, al, als, be, dre, dim_);
-		}
+		with_op<D, S>(t, flat_run<D, S>{dst + base, src + base, n, t, dre, dim_});
 	} else if constexpr (MODE == 0) {
-		/* row */
-		__shared__ int64_t s_od[PT_THREADS], s_os[PT_THREADS];
+		__shared__ int64_t so[2][PT_THREADS];
 		int64_t s0 = t.size[0];
 		int64_t c0 = local % m.ctas_d0;
 		int64_t orow = (local / m.ctas_d0) * m.rows_per_cta;
@@ -315,136 +524,41 @@ ptask_kernel(const __grid_constant__ task_pack pack,
 		int rows = m.rows_per_cta;
 		if (orow + rows > m.nouter)
 			rows = (int)(m.nouter - orow);
-		for (int r = threadIdx.x; r < rows; r += PT_THREADS)
-			outer_offsets(t, 1, orow + r, s_od[r], s_os[r]);
+		for (int r = threadIdx.x; r < rows; r += PT_THREADS) {
+			int64_t od, os;
+			outer_offsets(t, 1, orow + r, od, os);
+			so[0][r] = od + i0beg * t.dst_stride[0];
+			so[1][r] = os + i0beg * t.src_stride[0];
+		}
 		__syncthreads();
-		const int64_t ds0 = t.dst_stride[0], ss0 = t.src_stride[0];
-		if (w0 >= 32) {
-			/* long rows: wpr warps per row (all eight on one row), lanes
-			 * along it */
-			const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-			const int wpr = rows >= PT_THREADS / 32 ? 1 : (PT_THREADS / 32) / rows;
-			const int step = 32 * wpr;
-			for (int r = warp / wpr; r < rows; r += (PT_THREADS / 32) / wpr) {
-				D *dr = dst + s_od[r];
-				const S *sr = src + s_os[r];
-#pragma unroll 4
-				for (int64_t i0 = i0beg + (warp % wpr) * 32 + lane;
-				    i0 < i0beg + w0; i0 += step)
-					elem_op<D, S>::apply(op, dr + i0 * ds0, sr + i0 * ss0, al,
-					    als, be, dre, dim_);
-			}
-		} else {
-			/* short rows: flattened, 32-bit index arithmetic */
-			const int w0i = (int)w0, n = w0i * rows;
-#pragma unroll 4
-			for (int e = threadIdx.x; e < n; e += PT_THREADS) {
-				const int r = e / w0i;
-				const int64_t i0 = i0beg + (e - r * w0i);
-				elem_op<D, S>::apply(op, dst + s_od[r] + i0 * ds0,
-				    src + s_os[r] + i0 * ss0, al, als, be, dre, dim_);
-			}
-		}
-	} else if constexpr (MODE == 3) {
-		/* matrix: whole s0 x s1 slices (dim 0 unit-stride in dst, dim 1
-		 * in src); rows_per_cta slices per CTA.  Every load of the CTA is
-		 * in flight at once as a cp.async copy: the source transposed
-		 * into a padded tile (row pitch s0 + 1), the destination (when
-		 * the op reads it) into a second tile in its own order; one wait;
-		 * then the op from shared memory and stores along the
-		 * destination's runs */
-		constexpr int MT = mt_of<D, S>::v;
-		__shared__ __align__(16) S mtile[MT * (MT + 1)];
-		__shared__ __align__(16) D dtile[MT * MT];
-		__shared__ int64_t s_o[2][MAT_MAXQ];
-		const int s0 = (int)t.size[0], s1 = (int)t.size[1], n = s0 * s1;
-		const int ld = s0 + 1, pitch = s1 * ld;
-		const int64_t ss0 = t.src_stride[0], ds1 = t.dst_stride[1];
-		const int64_t o0 = local * m.rows_per_cta;
-		const int k = (int)(m.nouter - o0 < m.rows_per_cta ? m.nouter - o0 :
-		    m.rows_per_cta);
-		const bool rd = op != XMGD_OP_COPY;	/* the op reads dst */
-		for (int q = threadIdx.x; q < k; q += PT_THREADS)
-			outer_offsets(t, 2, o0 + q, s_o[0][q], s_o[1][q]);
-		__syncthreads();
-		const int kn = k * n;
-		/* flattened walks with the mixed-radix digits advanced by the
-		 * thread stride (one division per CTA, not per element) */
-		{
-			/* source: e = q n + i0 s1 + i1 (runs along i1) */
-			int q = threadIdx.x / n, r = threadIdx.x - q * n;
-			int i0 = r / s1, i1 = r - i0 * s1;
-			const int dq = PT_THREADS / n, dr = PT_THREADS - dq * n;
-			const int d0 = dr / s1, d1 = dr - d0 * s1;
-			for (int e = threadIdx.x; e < kn; e += PT_THREADS) {
-				cp_async_elem(&mtile[q * pitch + i1 * ld + i0],
-				    &src[s_o[1][q] + i0 * ss0 + i1]);
-				i1 += d1;
-				if (i1 >= s1) { i1 -= s1; i0++; }
-				i0 += d0;
-				if (i0 >= s0) { i0 -= s0; q++; }
-				q += dq;
-			}
-		}
-		/* destination: e = q n + i1 s0 + i0 (runs along i0); tile slot e */
-		int q = threadIdx.x / n, r = threadIdx.x - q * n;
-		int i1 = r / s0, i0 = r - i1 * s0;
-		const int dq = PT_THREADS / n, dr = PT_THREADS - dq * n;
-		const int d1 = dr / s0, d0 = dr - d1 * s0;
-		if (rd) {
-			int qq = q, j0 = i0, j1 = i1;
-			for (int e = threadIdx.x; e < kn; e += PT_THREADS) {
-				cp_async_elem(&dtile[e], dst + s_o[0][qq] + j0 + j1 * ds1);
-				j0 += d0;
-				if (j0 >= s0) { j0 -= s0; j1++; }
-				j1 += d1;
-				if (j1 >= s1) { j1 -= s1; qq++; }
-				qq += dq;
-			}
-		}
-		cp_async_wait_all();
-		__syncthreads();
-		for (int e = threadIdx.x; e < kn; e += PT_THREADS) {
-			D v = rd ? dtile[e] : D();
-			elem_op<D, S>::apply(op, &v, &mtile[q * pitch + i1 * ld + i0], al,
-			    als, be, dre, dim_);
-			if (op != XMGD_OP_DOT)
-				dst[s_o[0][q] + i0 + i1 * ds1] = v;
-			i0 += d0;
-			if (i0 >= s0) { i0 -= s0; i1++; }
-			i1 += d1;
-			if (i1 >= s1) { i1 -= s1; q++; }
-			q += dq;
-		}
+		with_op<D, S>(t, row_run<D, S>{dst, src, rows, (int)w0, t.dst_stride[0],
+		    t.src_stride[0], so, t, dre, dim_});
 	} else {
-		/* tile: dims 0 (dst unit stride) and 1 (src unit stride) */
-		__shared__ S tile[TILE][TILE + 1];
-		int64_t c0 = local % m.ctas_d0;
-		int64_t rest = local / m.ctas_d0;
-		int64_t c1 = rest % m.ctas_d1;
-		int64_t o = rest / m.ctas_d1;
-		int64_t od, os;
-		outer_offsets(t, 2, o, od, os);
-		int64_t b0 = c0 * TILE, b1 = c1 * TILE;
-		int w0 = (int)(t.size[0] - b0 < TILE ? t.size[0] - b0 : TILE);
-		int w1 = (int)(t.size[1] - b1 < TILE ? t.size[1] - b1 : TILE);
-		/* load: consecutive threads walk dim 1 (source contiguous) */
-		for (int e = threadIdx.x; e < TILE * TILE; e += PT_THREADS) {
-			int i1 = e % TILE, i0 = e / TILE;
-			if (i0 < w0 && i1 < w1)
-				tile[i1][i0] = src[os + (b0 + i0) * t.src_stride[0] +
-				    (b1 + i1)];
-		}
-		__syncthreads();
-		/* store: consecutive threads walk dim 0 (destination contiguous) */
-		for (int e = threadIdx.x; e < TILE * TILE; e += PT_THREADS) {
-			int i0 = e % TILE, i1 = e / TILE;
-			if (i0 < w0 && i1 < w1) {
-				D *dp = dst + od + (b0 + i0) * t.dst_stride[0] +
-				    (b1 + i1) * t.dst_stride[1];
-				elem_op<D, S>::apply(op, dp, &tile[i1][i0], al, als, be,
-				    dre, dim_);
-			}
+		__shared__ S tile[tile_cap(tile_elems(sizeof(D), sizeof(S)))];
+		if constexpr (MODE == 1) {
+			const uint32_t x = (uint32_t)local, d0 = m.ctas_d0, d1 = m.ctas_d1;
+			const uint32_t y = x / d0, c0 = x - y * d0, o = y / d1, c1 = y - o * d1;
+			const int b0 = c0 * m.t0, b1 = c1 * m.t1;
+			int64_t od, os;
+			outer_offsets(t, 2, o, od, os);
+			od += b0 * t.dst_stride[0] + b1 * t.dst_stride[1];
+			os += b0 * t.src_stride[0] + b1;
+			with_op<D, S>(t, tile_run<D, S>{dst + od, src + os,
+			    min(m.t0, t.size[0] - b0), min(m.t1, t.size[1] - b1), m.l1, m.lb,
+			    t.src_stride[0], t.dst_stride[0], t.dst_stride[1], tile, t, dre,
+			    dim_});
+		} else {
+			__shared__ int64_t so[2][SLICE_MAXQ];
+			const int64_t o0 = local * m.rows_per_cta;
+			const int k = (int)(m.nouter - o0 < m.rows_per_cta ? m.nouter - o0 :
+			    m.rows_per_cta);
+			if ((int)threadIdx.x < k)
+				outer_offsets(t, 2, o0 + threadIdx.x, so[0][threadIdx.x],
+				    so[1][threadIdx.x]);
+			__syncthreads();
+			with_op<D, S>(t, slice_run<D, S>{dst, src, t.size[0], t.size[1],
+			    k * t.size[0] * t.size[1], (int)t.src_stride[0],
+			    (int)t.dst_stride[0], (int)t.dst_stride[1], so, tile, t, dre, dim_});
 		}
 	}
 	if (op == XMGD_OP_DOT) {
@@ -498,154 +612,11 @@ dot_sum_kernel(const __grid_constant__ task_pack pack,
 	}
 }
 
-/* a bounded wait of the slab schedule gave up (set on the device, read
- * and cleared by the host after the launches) */
-__device__ int g_slab_err;
-
-/*
- * Slab schedule: rows_per_cta consecutive s0 x s1 slices per CTA, each
- * contiguous on both sides (source: dim 1 unit stride, dim 0 stride s1;
- * destination: dim 0 unit stride, dim 1 stride s0; slice q at q * s0 * s1
- * on both), 16-byte aligned.  One bulk copy brings the CTA's slices of the
- * source into shared memory (one instruction, where the matrix schedule
- * issues a copy per element); the source goes into a tile with an odd row
- * pitch, so that both the transposing pass (threads along the source's
- * run) and the storing pass (threads along the destination's run) touch
- * distinct banks; stores follow the destination's run.
- */
-template <typename T>
-__global__ void __launch_bounds__(PT_THREADS, 6)
-slab_kernel(const __grid_constant__ task_pack pack,
-    const xmgd_ptask_t *__restrict__ dtasks,
-    const task_meta *__restrict__ dmeta, int ntasks, int64_t cta0)
-{
-	extern __shared__ __align__(16) unsigned char dsm[];
-	__shared__ __align__(8) uint64_t bar;
-	__shared__ int s_err;
-
-	const int64_t cta = cta0 + blockIdx.x;
-	const xmgd_ptask_t *tasks = dtasks ? dtasks : pack.t;
-	const task_meta *meta = dtasks ? dmeta : pack.m;
-	const int lo = last_at_most(ntasks, cta, [&](int i) { return meta[i].first_cta; });
-	const xmgd_ptask_t &t = tasks[lo];
-	const task_meta &m = meta[lo];
-	const int s0 = (int)t.size[0], s1 = (int)t.size[1], n = s0 * s1;
-	const int ld = s0 | 1;
-	const int64_t o0 = (cta - m.first_cta) * m.rows_per_cta;
-	const int k = (int)(m.nouter - o0 < m.rows_per_cta ? m.nouter - o0 :
-	    m.rows_per_cta);
-	const int kn = k * n;
-	const uint32_t cbytes = (uint32_t)kn * (uint32_t)sizeof(T);
-	const T *sb = reinterpret_cast<const T *>(dsm);
-	T *tb = reinterpret_cast<T *>(dsm + cbytes);
-	T *dst = reinterpret_cast<T *>(t.dst) + o0 * n;
-	const T *src = reinterpret_cast<const T *>(t.src) + o0 * n;
-	const T al = num<T>::mk(t.alpha);
-
-	const uint32_t b = smem_u32(&bar);
-	if (threadIdx.x == 0) {
-		s_err = 0;
-		mbar_init(b, 1);
-		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-	}
-	__syncthreads();
-	if (threadIdx.x == 0) {
-		mbar_expect_tx(b, cbytes);
-		bulk_g2s(smem_u32(dsm), src, cbytes, b);
-	}
-	const bool ok = mbar_wait(b, 0, &s_err, &g_slab_err, 1);
-	/* every thread leaves together when the wait gave up */
-	if (__syncthreads_or(!ok))
-		return;
-	/* source order e = q n + i0 s1 + i1 -> tile q s1 ld + i1 ld + i0 */
-	{
-		int q = threadIdx.x / n, r = threadIdx.x - q * n;
-		int i0 = r / s1, i1 = r - i0 * s1;
-		const int dq = PT_THREADS / n, dr = PT_THREADS - dq * n;
-		const int d0 = dr / s1, d1 = dr - d0 * s1;
-		for (int e = threadIdx.x; e < kn; e += PT_THREADS) {
-			tb[(q * s1 + i1) * ld + i0] = sb[e];
-			i1 += d1;
-			if (i1 >= s1) { i1 -= s1; i0++; }
-			i0 += d0;
-			if (i0 >= s0) { i0 -= s0; q++; }
-			q += dq;
-		}
-	}
-	__syncthreads();
-	/* destination order e = q n + i1 s0 + i0 */
-	int q = threadIdx.x / n, r = threadIdx.x - q * n;
-	int i1 = r / s0, i0 = r - i1 * s0;
-	const int dq = PT_THREADS / n, dr = PT_THREADS - dq * n;
-	const int d1 = dr / s0, d0 = dr - d1 * s0;
-	for (int e = threadIdx.x; e < kn; e += PT_THREADS) {
-		dst[e] = num<T>::mul(al, tb[(q * s1 + i1) * ld + i0]);
-		i0 += d0;
-		if (i0 >= s0) { i0 -= s0; i1++; }
-		i1 += d1;
-		if (i1 >= s1) { i1 -= s1; q++; }
-		q += dq;
-	}
-}
-
-/* the slab schedule for a task: slices per CTA (0 when the schedule does
- * not apply: xm_copy of one scalar type only; an op that reads the
- * destination ran slower with its second bulk copy, 0.69 of HBM against
- * the matrix schedule's 0.71), and the CTA's shared memory */
-static int64_t
-slab_shape(const xmgd_ptask_t &t, int dbytes, int sbytes, int mt,
-    int64_t *smem)
-{
-	if (dbytes != sbytes || t.op != XMGD_OP_COPY || t.ndim < 2 || t.ndim > 3)
-		return 0;
-	const int64_t s0 = t.size[0], s1 = t.size[1], n = s0 * s1;
-	if (s0 > mt || s1 > mt || s0 < 2 || s1 < 2 ||
-	    t.dst_stride[0] != 1 || t.dst_stride[1] != s0 ||
-	    t.src_stride[1] != 1 || t.src_stride[0] != s1 ||
-	    (t.ndim == 3 && (t.dst_stride[2] != n || t.src_stride[2] != n)) ||
-	    (n * sbytes) % 16 != 0 || ((t.dst | t.src) & 15) != 0)
-		return 0;
-	int64_t k = n * sbytes >= SLAB_CHUNK ? 1 : SLAB_CHUNK / (n * sbytes);
-	const int64_t cap = t.ndim == 3 ? t.size[2] : 1;
-	if (k > cap)
-		k = cap;
-	*smem = k * n * sbytes + k * s1 * (s0 | 1) * sbytes;
-	return *smem <= SLAB_SMEM ? k : 0;
-}
-
-template <typename D, typename S>
-static int
-launch_slab(const task_pack &pack, const xmgd_ptask_t *dtasks, const task_meta *dmeta, int ntasks,
-    int64_t cta0, int64_t n, int64_t smem)
-{
-	if constexpr (std::is_same<D, S>::value) {
-		static bool attr = false;
-		if (!attr) {
-			XMG_CK(cudaFuncSetAttribute(slab_kernel<D>,
-			    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SLAB_SMEM));
-			attr = true;
-		}
-		slab_kernel<D><<<(unsigned)n, PT_THREADS, (size_t)smem, stream()>>>(
-		    pack, dtasks, dmeta, ntasks, cta0);
-		g_launches++;
-		XMG_CK(cudaGetLastError());
-		return XMG_OK;
-	} else {
-		return xmg_seterr(XMG_EINVAL, "slab schedule: scalar conversion");
-	}
-}
-
 template <typename D, typename S>
 static int
 launch(const task_pack &pack, const xmgd_ptask_t *dtasks, const task_meta *dmeta,
-    int ntasks, const int64_t *begin, int64_t slab_smem, double *dpartial)
+    int ntasks, const int64_t *begin, double *dpartial)
 {
-	if (begin[5] > begin[4]) {
-		int st = launch_slab<D, S>(pack, dtasks, dmeta, ntasks, begin[4],
-		    begin[5] - begin[4], slab_smem);
-		if (st)
-			return st;
-	}
 	/* one launch per schedule, over that schedule's CTA range */
 	for (int mode = 0; mode < 4; mode++) {
 		const int64_t n = begin[mode + 1] - begin[mode];
@@ -682,63 +653,57 @@ elem_bytes(int type)
 static void
 plan_tasks(const xmgd_ptask_t *tasks, int ntasks, int dtype, int stype,
     std::vector<xmgd_ptask_t> &sorted, std::vector<task_meta> &meta,
-    std::vector<int> &order, int64_t begin[6], int64_t *slab_smem)
+    std::vector<int> &order, int64_t begin[5])
 {
 	std::vector<task_meta> m0((size_t)ntasks);
 	std::vector<int64_t> cnt((size_t)ntasks);
-	const int mt = mt_host(elem_bytes(dtype), elem_bytes(stype));
-	const char *e = getenv("XMG_PTASK_SLAB");
-	const bool slab_on = !(e && strcmp(e, "0") == 0);
+	const int tile_n = tile_elems(elem_bytes(dtype), elem_bytes(stype));
 
 	int64_t nflat = 0;
-	/* the slab launch's shared memory: the largest of its CTAs' */
-	*slab_smem = 0;
 	for (int i = 0; i < ntasks; i++) {
 		const xmgd_ptask_t &t = tasks[i];
 		task_meta &m = m0[i];
 		memset(&m, 0, sizeof m);
-		int64_t need = 0;
-		const int64_t k = slab_on ? slab_shape(t, elem_bytes(dtype),
-		    elem_bytes(stype), mt, &need) : 0;
-		if (k > 0) {
-			m.mode = 4;
-			m.nouter = t.ndim == 3 ? t.size[2] : 1;
-			m.rows_per_cta = (int32_t)k;
-			m.ctas_d0 = 1;
-			cnt[i] = (m.nouter + k - 1) / k;
-			*slab_smem = std::max(*slab_smem, need);
-			continue;
-		}
 		const bool nosrc = t.op == XMGD_OP_SET || t.op == XMGD_OP_SCALE;
 		const bool tile = t.ndim >= 2 && t.src_stride[1] == 1 &&
 		    t.src_stride[0] != 1 && !nosrc;
 		const bool flat = t.ndim == 1 && t.dst_stride[0] == 1 &&
 		    (nosrc || t.src_stride[0] == 1);
-		const bool mat = tile && t.dst_stride[0] == 1 && t.size[0] <= mt &&
-		    t.size[1] <= mt;
 		if (flat) {
 			m.mode = 2;
 			m.nouter = 1;
 			nflat += t.size[0];
-		} else if (mat) {
-			m.mode = 3;
-			m.nouter = 1;
-			for (int d = 2; d < t.ndim; d++)
-				m.nouter *= t.size[d];
-			/* as many slices as the shared tile holds (pitch s0 + 1) */
-			const int64_t per = t.size[1] * (t.size[0] + 1);
-			int64_t q = (int64_t)mt * (mt + 1) / per;
-			m.rows_per_cta = (int32_t)(q < 1 ? 1 : q > MAT_MAXQ ? MAT_MAXQ : q);
-			m.ctas_d0 = 1;
-			cnt[i] = (m.nouter + m.rows_per_cta - 1) / m.rows_per_cta;
 		} else if (tile) {
-			m.mode = 1;
-			m.ctas_d0 = (t.size[0] + TILE - 1) / TILE;
-			m.ctas_d1 = (t.size[1] + TILE - 1) / TILE;
+			const int s0 = t.size[0], s1 = t.size[1];
+			const int64_t far = 1 << 24;
 			m.nouter = 1;
 			for (int d = 2; d < t.ndim; d++)
 				m.nouter *= t.size[d];
-			cnt[i] = (int64_t)m.ctas_d0 * m.ctas_d1 * m.nouter;
+			if (s0 <= SLICE_MAX && s1 <= SLICE_MAX && s0 * s1 <= tile_n &&
+			    t.src_stride[0] < far && t.dst_stride[0] < far &&
+			    t.dst_stride[1] < far) {
+				/* as many slices as the elements and the tile hold */
+				m.mode = 3;
+				const int q = std::min({tile_n / (s0 * s1),
+				    tile_cap(tile_n) / (s1 * (s0 | 1)), SLICE_MAXQ});
+				m.rows_per_cta = std::max(1, q);
+				cnt[i] = (m.nouter + m.rows_per_cta - 1) / m.rows_per_cta;
+			} else {
+				/* t1: the source's run in equal parts of at most 32;
+				 * t0: what fills the steps of 2^l1 lanes, in whole
+				 * 32-lane blocks */
+				m.mode = 1;
+				const int parts = (s1 + 31) / 32;
+				m.t1 = (s1 + parts - 1) / parts;
+				m.l1 = lanes_log2(m.t1);
+				const int most = tile_n >> m.l1;
+				m.t0 = std::min(s0, most);
+				for (m.lb = 0; (32 << m.lb) < most; m.lb++)
+					;
+				m.ctas_d0 = (s0 + m.t0 - 1) / m.t0;
+				m.ctas_d1 = (s1 + m.t1 - 1) / m.t1;
+				cnt[i] = (int64_t)m.ctas_d0 * m.ctas_d1 * m.nouter;
+			}
 		} else {
 			m.mode = 0;
 			m.ctas_d0 = (t.size[0] + ROW_ELEMS - 1) / ROW_ELEMS;
@@ -769,7 +734,7 @@ plan_tasks(const xmgd_ptask_t *tasks, int ntasks, int dtype, int stype,
 	meta.clear();
 	order.clear();
 	int64_t n = 0;
-	for (int mode = 0; mode < 5; mode++) {
+	for (int mode = 0; mode < 4; mode++) {
 		begin[mode] = n;
 		for (int i = 0; i < ntasks; i++)
 			if (m0[i].mode == mode) {
@@ -781,16 +746,16 @@ plan_tasks(const xmgd_ptask_t *tasks, int ntasks, int dtype, int stype,
 				order.push_back(i);
 			}
 	}
-	begin[5] = n;
+	begin[4] = n;
 }
 
 static int
 launch_types(int dtype, int stype, const task_pack &pack, const xmgd_ptask_t *dt, const task_meta *dm,
-    int ntasks, const int64_t *begin, int64_t slab_smem, double *dp)
+    int ntasks, const int64_t *begin, double *dp)
 {
 	int st;
 
-#define L(D, S) st = launch<D, S>(pack, dt, dm, ntasks, begin, slab_smem, dp)
+#define L(D, S) st = launch<D, S>(pack, dt, dm, ntasks, begin, dp)
 	if (dtype == stype) {
 		switch (dtype) {
 		case 0: L(float, float); break;
@@ -832,8 +797,7 @@ xmgd_ptask_stage(const xmgd_ptask_t *tasks, int ntasks, int stype,
 	if (ntasks <= 0)
 		return XMG_OK;
 	/* batches staged for replay carry one type on both sides */
-	plan_tasks(tasks, ntasks, stype, stype, sorted, meta, order, b->begin,
-	    &b->slab_smem);
+	plan_tasks(tasks, ntasks, stype, stype, sorted, meta, order, b->begin);
 	if ((st = xmgd_alloc(tb + meta.size() * sizeof(task_meta), &b->dbuf)))
 		return st;
 	b->ntasks = ntasks;
@@ -854,7 +818,7 @@ xmgd_ptask_launch(int dtype, int stype, const xmgd_ptask_batch_t *b)
 	static const task_pack none = {};
 	return launch_types(dtype, stype, none, (const xmgd_ptask_t *)b->dbuf,
 	    (const task_meta *)(b->dbuf + task_bytes(b->ntasks)), b->ntasks,
-	    b->begin, b->slab_smem, nullptr);
+	    b->begin, nullptr);
 }
 
 /* page-locked host memory of the element-wise calls: the batch on its way
@@ -886,7 +850,7 @@ xmgd_ptasks(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks,
 	std::vector<task_meta> meta;
 	std::vector<int> order;
 	task_pack pack;
-	int64_t begin[6], nctas, slab_smem;
+	int64_t begin[5], nctas;
 	uint64_t dbuf = 0, dpart = 0;
 	const task_meta *dmeta = nullptr;
 	const int *dorder = nullptr;
@@ -896,9 +860,8 @@ xmgd_ptasks(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks,
 
 	if (ntasks <= 0)
 		return XMG_OK;
-	plan_tasks(tasks, ntasks, dtype, stype, sorted, meta, order, begin,
-	    &slab_smem);
-	nctas = begin[5];
+	plan_tasks(tasks, ntasks, dtype, stype, sorted, meta, order, begin);
+	nctas = begin[4];
 	const size_t tb = task_bytes(ntasks);
 	const size_t mb = ((size_t)ntasks * sizeof(task_meta) + 255) & ~(size_t)255;
 	const size_t ob = ((size_t)ntasks * sizeof(int) + 255) & ~(size_t)255;
@@ -933,7 +896,7 @@ xmgd_ptasks(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks,
 	    &dpart)) != XMG_OK)
 		return st;
 	st = launch_types(dtype, stype, pack, (const xmgd_ptask_t *)dbuf, dmeta, ntasks,
-	    begin, slab_smem, (double *)dpart);
+	    begin, (double *)dpart);
 	if (st == XMG_OK && dots) {
 		dot_sum_kernel<<<(unsigned)((ntasks + 7) / 8), 256, 0, stream()>>>(pack,
 		    dmeta, dorder, ntasks, nctas, (const double *)dpart, sums);
@@ -944,16 +907,6 @@ xmgd_ptasks(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks,
 	const int st2 = check(cudaStreamSynchronize(stream()), "ptask_kernel");
 	if (st != XMG_OK || (st = st2) != XMG_OK)
 		return st;
-	if (begin[5] > begin[4]) {
-		int err = 0;
-		XMG_CK(cudaMemcpyFromSymbol(&err, g_slab_err, sizeof err));
-		if (err) {
-			const int zero = 0;
-			XMG_CK(cudaMemcpyToSymbol(g_slab_err, &zero, sizeof zero));
-			return xmg_seterr(XMG_ETIMEOUT, "slab schedule: a bulk copy "
-			    "did not complete within the bounded wait");
-		}
-	}
 	if (dots)
 		memcpy(dots, sums, db);
 	return XMG_OK;
