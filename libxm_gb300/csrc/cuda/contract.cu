@@ -21,8 +21,9 @@
 namespace xmg {
 
 template <typename T>
-int plain_gemm_launch(const void *items, int nitems, const xmgd_cblock_t *cbs,
+int plain_gemm_launch(const void *items, int nitems, int tile, const xmgd_cblock_t *cbs,
     const xmgd_pair_t *prs, const int32_t *tabs, const double *beta);
+int plain_tile(int dtype, int64_t tiles32);
 
 /* split-precision path (emu.cu) */
 struct emu_plan;
@@ -73,7 +74,7 @@ struct xmgd_plan {
 	xmgd_ptask_batch_t scale = {};       /* staged beta-only tasks */
 	int n_scale = 0;
 	uint64_t d_pg = 0;                   /* plain GEMM work list */
-	int n_pg = 0;
+	int n_pg = 0, pg_tile = 0;
 	emu_plan *ep = nullptr;
 	/* three captured segments, timed by events recorded between their
 	 * launches: 0 beta-only blocks + operand split, 1 split-precision
@@ -89,26 +90,30 @@ xmgd_last_timing(xmgd_timing_t *t)
 	*t = g_timing;
 }
 
-/* plain work list of a set of blocks: 64 x 64 tiles, longest K first */
+/* plain work list of a set of blocks: square tiles, longest K first */
 static int
-stage_plain(const std::vector<xmgd_cblock_t> &cbs,
+stage_plain(int dtype, const std::vector<xmgd_cblock_t> &cbs,
     const std::vector<xmgd_pair_t> &prs, const std::vector<int> &blocks,
-    uint64_t *d, int *n)
+    uint64_t *d, int *n, int *tile)
 {
 	std::vector<pg_item> items;
 	std::vector<int64_t> cost(cbs.size(), 0);
 	int st;
 
 	*d = 0;
-	*n = 0;
+	*n = *tile = 0;
 	if (blocks.empty())
 		return XMG_OK;
+	int64_t t32 = 0;
+	for (int ci : blocks)
+		t32 += (int64_t)((cbs[ci].m + 31) / 32) * ((cbs[ci].n + 31) / 32);
+	const int tb = *tile = plain_tile(dtype, t32);
 	for (int ci : blocks) {
 		const xmgd_cblock_t &cb = cbs[ci];
 		for (int q = 0; q < cb.npairs; q++)
 			cost[ci] += prs[cb.first_pair + q].k;
-		for (int m0 = 0; m0 < cb.m; m0 += 64)
-			for (int n0 = 0; n0 < cb.n; n0 += 64)
+		for (int m0 = 0; m0 < cb.m; m0 += tb)
+			for (int n0 = 0; n0 < cb.n; n0 += tb)
 				items.push_back(pg_item{ci, m0, n0, 0});
 	}
 	std::stable_sort(items.begin(), items.end(),
@@ -123,7 +128,7 @@ stage_plain(const std::vector<xmgd_cblock_t> &cbs,
 }
 
 static int
-launch_plain(xmgd_plan *dp, uint64_t items, int n)
+launch_plain(xmgd_plan *dp, uint64_t items, int n, int tile)
 {
 	const xmgd_cblock_t *dc = (const xmgd_cblock_t *)dp->d_cbs;
 	const xmgd_pair_t *pr = (const xmgd_pair_t *)dp->d_prs;
@@ -131,10 +136,10 @@ launch_plain(xmgd_plan *dp, uint64_t items, int n)
 	const void *di = (const void *)items;
 
 	switch (dp->dtype) {
-	case 0: return plain_gemm_launch<float>(di, n, dc, pr, dt, dp->beta);
-	case 1: return plain_gemm_launch<cf>(di, n, dc, pr, dt, dp->beta);
-	case 2: return plain_gemm_launch<double>(di, n, dc, pr, dt, dp->beta);
-	case 3: return plain_gemm_launch<cd>(di, n, dc, pr, dt, dp->beta);
+	case 0: return plain_gemm_launch<float>(di, n, tile, dc, pr, dt, dp->beta);
+	case 1: return plain_gemm_launch<cf>(di, n, tile, dc, pr, dt, dp->beta);
+	case 2: return plain_gemm_launch<double>(di, n, tile, dc, pr, dt, dp->beta);
+	case 3: return plain_gemm_launch<cd>(di, n, tile, dc, pr, dt, dp->beta);
 	}
 	return xmg_seterr(XMG_EINVAL, "bad scalar type");
 }
@@ -154,7 +159,7 @@ record(xmgd_plan *dp, int seg)
 	case 1:
 		return dp->ep ? emu_record_gemm(dp->ep) : XMG_OK;
 	default:
-		return dp->n_pg ? launch_plain(dp, dp->d_pg, dp->n_pg) : XMG_OK;
+		return dp->n_pg ? launch_plain(dp, dp->d_pg, dp->n_pg, dp->pg_tile) : XMG_OK;
 	}
 }
 
@@ -282,7 +287,8 @@ xmgd_plan_create(const xmgd_contract_t *p, xmgd_plan **out)
 		} else if (st != XMG_OK)
 			goto fail;
 	}
-	if ((st = stage_plain(dp->cbs, dp->prs, dp->plain, &dp->d_pg, &dp->n_pg)))
+	if ((st = stage_plain(dp->dtype, dp->cbs, dp->prs, dp->plain, &dp->d_pg, &dp->n_pg,
+	    &dp->pg_tile)))
 		goto fail;
 	dp->seg1.resize(dp->ep ? emu_ncand(dp->ep) : 1);
 	if ((st = check(cudaStreamSynchronize(stream()), "plan upload")))
@@ -400,10 +406,10 @@ xmgd_plan_run(xmgd_plan *dp, int *precision_used)
 			return xmg_seterr(XMG_ENOTSUP, "split-precision path: Inf/NaN "
 			    "in operands");
 		uint64_t d;
-		int n;
-		if ((st = stage_plain(dp->cbs, dp->prs, dp->emu, &d, &n)))
+		int n, tile;
+		if ((st = stage_plain(dp->dtype, dp->cbs, dp->prs, dp->emu, &d, &n, &tile)))
 			return st;
-		st = launch_plain(dp, d, n);
+		st = launch_plain(dp, d, n, tile);
 		xmgd_free(d);
 		if (st == XMG_OK)
 			st = check(cudaStreamSynchronize(stream()), "plain fallback");

@@ -11,73 +11,89 @@
  * epilogue scatters C the same way, so operands are read once from their
  * canonical storage and C is written once.
  *
- * Tile 64 x 64, K step 16, 256 threads, 4 x 4 accumulators per thread in
- * registers.  Work items (block, m-tile, n-tile) arrive sorted by cost.
+ * Work items (block, m-tile, n-tile) arrive sorted by cost.  The float forms
+ * run 64 x 64 tiles, 256 threads with 4 x 4 accumulators each.  The double
+ * forms are bound by the FP64 pipe (2 multiply-adds a cycle and SM: a warp's
+ * takes 64 cycles of its scheduler), beside which loads, shared memory and
+ * L2 traffic are free; what costs is work on padding and SMs left without
+ * work, so they run small tiles on 128 threads (a warp per scheduler):
+ * 16 x 16, or 32 x 32 where there are thousands of those; thread rows and
+ * columns past the block are skipped.  Ladder o20/v57 (2.6 GFLOP in 30
+ * blocks): 210 tiles of 64 x 64 on 152 SMs took 4.40 ms, 16 x 16 tiles 2.50
+ * (2.46 at the pipe's rate).
  */
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace xmg {
 
-constexpr int PG_BM = 64, PG_BN = 64, PG_BK = 16, PG_THREADS = 256;
+constexpr int PG_BK = 16;
 
 struct pg_item {
 	int32_t cblock, m0, n0, pad;
 };
 
-template <typename T>
-__device__ inline void
-load_tile(T (*S)[PG_BM + 1], const T *__restrict__ base,
-    const int32_t *__restrict__ rowt, const int32_t *__restrict__ colt,
-    int k0, int kmax, int c0, int cmax, bool kfast, const T &scale)
-{
-	int t = threadIdx.x;
-	if (kfast) {
-		/* consecutive threads walk k: contiguous when rows are unit-stride */
-		int kk = t % PG_BK, cc = t / PG_BK;
-		int k = k0 + kk;
-		int32_t ro = k < kmax ? rowt[k] : 0;
+/* TB x TB tile, TM x TN outputs per thread: rows tx + (TB / TM) i, columns
+ * ty + (TB / TN) j */
+template <typename T, int TB, int TM, int TN>
+struct pg {
+	static constexpr int NX = TB / TM, NY = TB / TN, THREADS = NX * NY;
+	static constexpr int NL = TB * PG_BK / THREADS;	/* loads per operand */
+
+	/* this thread's NL elements of the K x TB operand tile at (k0, c0):
+	 * consecutive threads walk k where K runs along memory, else the free
+	 * index */
+	static __device__ __forceinline__ void
+	fetch(T (&v)[NL], const T *__restrict__ base, const int32_t *__restrict__ rowt,
+	    const int32_t *__restrict__ colt, int k0, int kmax, int c0, int cmax,
+	    bool kfast)
+	{
+		const int t = threadIdx.x;
 #pragma unroll
-		for (int r = 0; r < PG_BM / (PG_THREADS / PG_BK); r++) {
-			int c = c0 + cc + r * (PG_THREADS / PG_BK);
-			T v = num<T>::zero();
-			if (k < kmax && c < cmax)
-				v = num<T>::mul(scale, base[ro + colt[c]]);
-			S[kk][cc + r * (PG_THREADS / PG_BK)] = v;
-		}
-	} else {
-		int cc = t % PG_BM, kk = t / PG_BM;
-		int c = c0 + cc;
-		int32_t co = c < cmax ? colt[c] : 0;
-#pragma unroll
-		for (int r = 0; r < PG_BK / (PG_THREADS / PG_BM); r++) {
-			int k = k0 + kk + r * (PG_THREADS / PG_BM);
-			T v = num<T>::zero();
-			if (k < kmax && c < cmax)
-				v = num<T>::mul(scale, base[rowt[k] + co]);
-			S[kk + r * (PG_THREADS / PG_BM)][cc] = v;
+		for (int r = 0; r < NL; r++) {
+			const int kk = kfast ? t % PG_BK : t / TB + r * (THREADS / TB);
+			const int cc = kfast ? t / PG_BK + r * (THREADS / PG_BK) : t % TB;
+			v[r] = k0 + kk < kmax && c0 + cc < cmax ?
+			    base[rowt[k0 + kk] + colt[c0 + cc]] : num<T>::zero();
 		}
 	}
-}
 
-template <typename T>
-__global__ void __launch_bounds__(PG_THREADS)
+	static __device__ __forceinline__ void
+	put(T (*S)[TB + 1], const T (&v)[NL], bool kfast, const T *scale)
+	{
+		const int t = threadIdx.x;
+#pragma unroll
+		for (int r = 0; r < NL; r++) {
+			const int kk = kfast ? t % PG_BK : t / TB + r * (THREADS / TB);
+			const int cc = kfast ? t / PG_BK + r * (THREADS / PG_BK) : t % TB;
+			S[kk][cc] = scale ? num<T>::mul(*scale, v[r]) : v[r];
+		}
+	}
+};
+
+template <typename T, int TB, int TM, int TN>
+__global__ void __launch_bounds__(pg<T, TB, TM, TN>::THREADS)
 plain_gemm_kernel(const pg_item *__restrict__ items,
     const xmgd_cblock_t *__restrict__ cbs, const xmgd_pair_t *__restrict__ prs,
     const int32_t *__restrict__ tabs, double2 beta2)
 {
-	__shared__ T As[PG_BK][PG_BM + 1];
-	__shared__ T Bs[PG_BK][PG_BN + 1];
+	using P = pg<T, TB, TM, TN>;
+	__shared__ T As[PG_BK][TB + 1];
+	__shared__ T Bs[PG_BK][TB + 1];
 
 	const pg_item it = items[blockIdx.x];
 	const xmgd_cblock_t cb = cbs[it.cblock];
-	const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-	T acc[4][4];
+	const int tx = threadIdx.x % P::NX, ty = threadIdx.x / P::NX;
+	/* rows and columns of threads that reach into the block */
+	const int mi = min(TM, (cb.m - it.m0 + P::NX - 1) / P::NX);
+	const int nj = min(TN, (cb.n - it.n0 + P::NY - 1) / P::NY);
+	T acc[TM][TN];
 #pragma unroll
-	for (int i = 0; i < 4; i++)
+	for (int i = 0; i < TM; i++)
 #pragma unroll
-		for (int j = 0; j < 4; j++)
+		for (int j = 0; j < TN; j++)
 			acc[i][j] = num<T>::zero();
-	const T one = num<T>::mk((const double[2]){1.0, 0.0});
 
 	for (int p = 0; p < cb.npairs; p++) {
 		const xmgd_pair_t pr = prs[cb.first_pair + p];
@@ -88,25 +104,37 @@ plain_gemm_kernel(const pg_item *__restrict__ items,
 		const bool akf = pr.k > 1 && arow[1] - arow[0] == 1;
 		const bool bkf = pr.k > 1 && brow[1] - brow[0] == 1;
 		const T al = num<T>::mk(pr.al);
+		T va[P::NL], vb[P::NL];
+		P::fetch(va, A, arow, acol, 0, pr.k, it.m0, cb.m, akf);
+		P::fetch(vb, B, brow, bcol, 0, pr.k, it.n0, cb.n, bkf);
 		for (int k0 = 0; k0 < pr.k; k0 += PG_BK) {
 			__syncthreads();
-			load_tile<T>(As, A, arow, acol, k0, pr.k, it.m0, cb.m, akf, al);
-			load_tile<T>(Bs, B, brow, bcol, k0, pr.k, it.n0, cb.n, bkf, one);
+			P::put(As, va, akf, &al);
+			P::put(Bs, vb, bkf, nullptr);
 			__syncthreads();
+			if (k0 + PG_BK < pr.k) {	/* the next tile, in flight below */
+				P::fetch(va, A, arow, acol, k0 + PG_BK, pr.k, it.m0, cb.m, akf);
+				P::fetch(vb, B, brow, bcol, k0 + PG_BK, pr.k, it.n0, cb.n, bkf);
+			}
+			const int kn = min(PG_BK, pr.k - k0);
+#pragma unroll 4
+			for (int kk = 0; kk < kn; kk++) {
+				T a[TM], b[TN];
 #pragma unroll
-			for (int kk = 0; kk < PG_BK; kk++) {
-				T a[4], b[4];
+				for (int i = 0; i < TM; i++)
+					a[i] = As[kk][tx + P::NX * i];
 #pragma unroll
-				for (int i = 0; i < 4; i++)
-					a[i] = As[kk][tx + 16 * i];
+				for (int j = 0; j < TN; j++)
+					b[j] = Bs[kk][ty + P::NY * j];
 #pragma unroll
-				for (int j = 0; j < 4; j++)
-					b[j] = Bs[kk][ty + 16 * j];
+				for (int i = 0; i < TM; i++) {
+					if (i >= mi)
+						break;
 #pragma unroll
-				for (int i = 0; i < 4; i++)
-#pragma unroll
-					for (int j = 0; j < 4; j++)
-						acc[i][j] = num<T>::fma(a[i], b[j], acc[i][j]);
+					for (int j = 0; j < TN; j++)
+						if (j < nj)
+							acc[i][j] = num<T>::fma(a[i], b[j], acc[i][j]);
+				}
 			}
 		}
 	}
@@ -118,14 +146,14 @@ plain_gemm_kernel(const pg_item *__restrict__ items,
 	const T beta = num<T>::mk(bb);
 	const bool bzero = beta2.x == 0 && beta2.y == 0;
 #pragma unroll
-	for (int j = 0; j < 4; j++) {
-		int n = it.n0 + ty + 16 * j;
+	for (int j = 0; j < TN; j++) {
+		int n = it.n0 + ty + P::NY * j;
 		if (n >= cb.n)
 			continue;
 		int32_t co = ccol[n];
 #pragma unroll
-		for (int i = 0; i < 4; i++) {
-			int m = it.m0 + tx + 16 * i;
+		for (int i = 0; i < TM; i++) {
+			int m = it.m0 + tx + P::NX * i;
 			if (m >= cb.m)
 				continue;
 			T *cp = C + crow[m] + co;
@@ -134,26 +162,45 @@ plain_gemm_kernel(const pg_item *__restrict__ items,
 	}
 }
 
+/* Tile side for a scalar type and the number of 32 x 32 tiles of the work:
+ * double types 16 while that is below 32 per SM, else 32. */
+int
+plain_tile(int dtype, int64_t tiles32)
+{
+	return dtype < 2 ? 64 : tiles32 < 32 * (int64_t)num_sms() ? 16 : 32;
+}
+
 template <typename T>
 int
-plain_gemm_launch(const void *items, int nitems, const xmgd_cblock_t *cbs,
+plain_gemm_launch(const void *items, int nitems, int tile, const xmgd_cblock_t *cbs,
     const xmgd_pair_t *prs, const int32_t *tabs, const double *beta)
 {
+	const pg_item *it = (const pg_item *)items;
+	const double2 b2 = make_double2(beta[0], beta[1]);
+
 	if (nitems == 0)
 		return XMG_OK;
-	plain_gemm_kernel<T><<<nitems, PG_THREADS, 0, stream()>>>(
-	    (const pg_item *)items, cbs, prs, tabs, make_double2(beta[0], beta[1]));
+	if constexpr (std::is_same<T, double>::value || std::is_same<T, cd>::value) {
+		if (tile == 16)
+			plain_gemm_kernel<T, 16, 2, 1><<<nitems, 128, 0, stream()>>>(it, cbs, prs,
+			    tabs, b2);
+		else
+			plain_gemm_kernel<T, 32, 4, 2><<<nitems, 128, 0, stream()>>>(it, cbs, prs,
+			    tabs, b2);
+	} else
+		plain_gemm_kernel<T, 64, 4, 4><<<nitems, 256, 0, stream()>>>(it, cbs, prs, tabs,
+		    b2);
 	g_launches++;
 	return check(cudaGetLastError(), "plain_gemm_kernel launch");
 }
 
-template int plain_gemm_launch<float>(const void *, int, const xmgd_cblock_t *,
+template int plain_gemm_launch<float>(const void *, int, int, const xmgd_cblock_t *,
     const xmgd_pair_t *, const int32_t *, const double *);
-template int plain_gemm_launch<double>(const void *, int, const xmgd_cblock_t *,
+template int plain_gemm_launch<double>(const void *, int, int, const xmgd_cblock_t *,
     const xmgd_pair_t *, const int32_t *, const double *);
-template int plain_gemm_launch<cf>(const void *, int, const xmgd_cblock_t *,
+template int plain_gemm_launch<cf>(const void *, int, int, const xmgd_cblock_t *,
     const xmgd_pair_t *, const int32_t *, const double *);
-template int plain_gemm_launch<cd>(const void *, int, const xmgd_cblock_t *,
+template int plain_gemm_launch<cd>(const void *, int, int, const xmgd_cblock_t *,
     const xmgd_pair_t *, const int32_t *, const double *);
 
 } /* namespace xmg */
