@@ -78,9 +78,10 @@ struct xmgd_plan {
 	emu_plan *ep = nullptr;
 	/* three captured segments, timed by events recorded between their
 	 * launches: 0 beta-only blocks + operand split, 1 split-precision
-	 * GEMM (one graph per autotuner candidate), 2 plain GEMM */
-	segment seg0, seg2;
-	std::vector<segment> seg1;
+	 * GEMM (one graph each per autotuner candidate, whose form fixes the
+	 * operands' layout), 2 plain GEMM */
+	segment seg2;
+	std::vector<segment> seg0, seg1;
 	cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
 };
 
@@ -184,8 +185,9 @@ drop(segment &g)
 static void
 drop_graphs(xmgd_plan *dp)
 {
-	drop(dp->seg0);
 	drop(dp->seg2);
+	for (segment &g : dp->seg0)
+		drop(g);
 	for (segment &g : dp->seg1)
 		drop(g);
 }
@@ -290,7 +292,8 @@ xmgd_plan_create(const xmgd_contract_t *p, xmgd_plan **out)
 	if ((st = stage_plain(dp->dtype, dp->cbs, dp->prs, dp->plain, &dp->d_pg, &dp->n_pg,
 	    &dp->pg_tile)))
 		goto fail;
-	dp->seg1.resize(dp->ep ? emu_ncand(dp->ep) : 1);
+	dp->seg0.resize(dp->ep ? emu_ncand(dp->ep) : 1);
+	dp->seg1.resize(dp->seg0.size());
 	if ((st = check(cudaStreamSynchronize(stream()), "plan upload")))
 		goto fail;
 	*out = dp;
@@ -361,7 +364,7 @@ xmgd_plan_run(xmgd_plan *dp, int *precision_used)
 		cand = emu_current(dp->ep);
 	}
 	XMG_CK(cudaEventRecord(dp->ev[0], stream()));
-	if ((st = run_segment(dp, 0, dp->seg0)))
+	if ((st = run_segment(dp, 0, dp->seg0[cand])))
 		return st;
 	XMG_CK(cudaEventRecord(dp->ev[1], stream()));
 	if ((st = run_segment(dp, 1, dp->seg1[cand])))
@@ -390,8 +393,10 @@ xmgd_plan_run(xmgd_plan *dp, int *precision_used)
 		/* tuning over: keep only the chosen candidate's graph */
 		if (!was_tuned && emu_tuned(dp->ep))
 			for (size_t i = 0; i < dp->seg1.size(); i++)
-				if ((int)i != emu_current(dp->ep))
+				if ((int)i != emu_current(dp->ep)) {
+					drop(dp->seg0[i]);
 					drop(dp->seg1[i]);
+				}
 		if (!nan)
 			*precision_used = XMG_PREC_EMU64;
 	}

@@ -30,7 +30,7 @@
  *     (exact).  Integer and FP32 arithmetic only -- GB300's FP64 pipe runs at
  *     ~1 TFLOP/s.  The output is pre-tiled in the exact shared-memory image
  *     the MMA reads (no-swizzle K-major core matrices), so the GEMM loads a
- *     pipeline stage with two 1-D bulk copies.
+ *     K step of a tile with one 1-D bulk copy per operand.
  *  3. emu_gemm_kernel  - one CTA per (output block, 128 x 128 tile, pass);
  *     warp 0 streams stages with cp.async.bulk, warp 1 issues the slice
  *     products per 16-wide K step with tcgen05.mma.kind::f16 (bf16 x bf16 ->
@@ -50,6 +50,7 @@
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -129,6 +130,14 @@ constexpr int EMU_MAXMEM = 4;
 struct view_meta {
 	int64_t first_cta;
 };
+
+/* rows of the tile that starts at row r0 of a view with mn rows: the live
+ * ones rounded up to 16, at most 128 */
+__host__ __device__ __forceinline__ int tile_rows(int mn, int r0)
+{
+	const int r = (mn - r0 + 15) / 16 * 16;
+	return r < EMU_TM ? r : EMU_TM;
+}
 
 /* the view of a CTA: the last one whose first CTA is <= cta */
 __device__ __forceinline__ int find_view(const view_meta *m, int n, int64_t cta)
@@ -282,7 +291,7 @@ template <typename T>
 __global__ void __launch_bounds__(256, 6)
 emu_split_kernel(const xmgd_view_t *__restrict__ views,
     const view_meta *__restrict__ meta, int nviews,
-    const int32_t *__restrict__ tabs, const int32_t *__restrict__ E)
+    const int32_t *__restrict__ tabs, const int32_t *__restrict__ E, int rowmajor)
 {
 	constexpr int S = fin<T>::S;
 	constexpr int CHUNK_ELEMS = S * SLICE_BYTES / 2;
@@ -292,7 +301,7 @@ emu_split_kernel(const xmgd_view_t *__restrict__ views,
 	const int ngrp = (w.n_ks + 3) / 4;
 	const int rt = (int)(local / ngrp), g = (int)(local % ngrp);
 	const int rr = threadIdx.x % EMU_TM, oct = threadIdx.x / EMU_TM;
-	const int r = rt * EMU_TM + rr;
+	const int r = rt * EMU_TM + rr, tr = tile_rows(w.mn, rt * EMU_TM);
 	const T *X = reinterpret_cast<const T *>(w.ptr);
 	const int32_t *rowt = tabs + w.rowtab, *colt = tabs + w.coltab;
 	const bool live = r < w.mn;
@@ -337,15 +346,22 @@ emu_split_kernel(const xmgd_view_t *__restrict__ views,
 				bits[t][e >> 1] |= h << (16 * (e & 1));
 			}
 		}
-		/* chunk layout [8-row group][slice][2 K core matrices][8 rows x
-		 * 16 B]: the first R rows of a tile are a contiguous prefix, and
-		 * one slice is K-major with SBO = S * 256 B between row groups */
-		const size_t chunk = ((size_t)rt * w.n_ks + ks) * CHUNK_ELEMS;
-		const size_t within = (size_t)(rr >> 3) * (S * 128) + oct * 64 + (rr & 7) * 8;
+		/* chunk of a tile's live rows, rounded up to 16, in core matrices
+		 * of 8 rows x 16 B, two per row group and slice.  Slice-major,
+		 * [slice][8-row group]: consecutive slices follow one another
+		 * like the rows of one wider operand.  Row-major, [8-row
+		 * group][slice]: members' chunks stack by plain concatenation */
+		if (rr >= tr)
+			continue;
+		const size_t chunk = (size_t)rt * w.n_ks * CHUNK_ELEMS +
+		    (size_t)ks * (tr * EMU_KS * S);
+		const size_t within = (size_t)(rr >> 3) * (rowmajor ? S * 128 : 128) +
+		    oct * 64 + (rr & 7) * 8;
+		const int ts = rowmajor ? 128 : tr * EMU_KS;
 #pragma unroll
 		for (int t = 0; t < S; t++) {
 			uint4 val = make_uint4(bits[t][0], bits[t][1], bits[t][2], bits[t][3]);
-			*reinterpret_cast<uint4 *>(out + chunk + t * 128 + within) = val;
+			*reinterpret_cast<uint4 *>(out + chunk + t * ts + within) = val;
 		}
 	}
 }
@@ -472,45 +488,109 @@ __device__ __forceinline__ int chunk_end(int c0, int nks, int cplx, int kchunk)
 	return min(lim, c0 + kchunk);
 }
 
-/* Accumulators: 0, 1, 2 hold the exact weight groups p + q = 0, 1, 2; 3
- * the low band p + q = 3..KEEP.  The top one (3 with a low band, else 2)
- * forms set X, the others set Y.  The drain reads X first and releases it,
- * so at a chunk boundary the MMA warp issues the X products of the next
- * chunk's first (already staged) K steps while the drain still reads Y. */
-template <int KEEP>
-struct acc_sets {
-	static constexpr int XACC = KEEP > 2 ? 3 : 2;
+/*
+ * Accumulators and MMAs of one K step.  Weight groups p + q = 0, 1, 2 have
+ * an accumulator each (exact), 3..KEEP form the rounded low band.  FP64: the
+ * low band is set X, the exact groups set Y; FP32: group 2 is X, 0 and 1 are
+ * Y.  A slice of the M side times w consecutive slices of the N side is one
+ * MMA of w * N columns when the accumulators of its w groups lie side by
+ * side, since the slices of the N side follow one another in shared memory.
+ * An MMA reads its operands from shared memory at 128 B per cycle, the
+ * M-side slice (4 KiB) again each time, and costs max(cols / 2, 32 + cols /
+ * 4) + 6 cycles (measured), so fewer, wider ones win: a step of 21 products
+ * took 1450 cycles at N = 128, 1311 at 96, 1210 at 64 and 32 as single
+ * products; as below 1353, 1125, 698 and 560.  By the width N of a tile:
+ *   class 0 (N <= 80): six accumulators, up to three slices: 9 MMAs;
+ *   class 1 (N = 96): five (groups 4 and 5 share one), two slices: 15;
+ *   class 2 (N > 96): four (3, 4, 5 share one), two slices: 17 (19 where X
+ *     and Y are issued apart);
+ *   class 3 (FP32): three, two slices within Y: 5;
+ *   class 4: single products: CTA pairs (half of the N side in each CTA)
+ *     and stacked tiles, whose members' slices do not follow one another.
+ */
+enum { SET_Y, SET_X, SET_ALL };
+
+template <int S, int KEEP, int CLS, int SET>
+struct prod {
+	static constexpr int YTOP = KEEP > 2 ? 2 : 1;
+	static constexpr int GLO = SET == SET_X ? YTOP + 1 : 0;
+	static constexpr int GHI = SET == SET_Y ? YTOP : KEEP;
+	static constexpr int W = CLS == 0 ? 3 : CLS == 4 ? 1 : 2;
+	static constexpr int TOP = KEEP == 2 ? 2 : CLS == 0 ? 5 : CLS == 1 ? 4 : 3;
+	/* accumulator of weight group g */
+	static constexpr int acc(int g) { return g < TOP ? g : TOP; }
+	/* slices of the MMA that starts with product (p, q) */
+	static constexpr int width(int p, int q)
+	{
+		int w = 1;
+		while (w < W && p + q + w <= GHI && q + w < S &&
+		    acc(p + q + w) == acc(p + q + w - 1) + 1)
+			w++;
+		return w;
+	}
 };
 
-/* the slice products of one K step whose accumulator lies in `which`
- * (1: set X, 2: set Y, 3: both).  The two stage descriptors are built once;
- * each product adds its slice offset (>> 4) to the low word, which cannot
- * carry out of the 14-bit address field inside a < 256 KiB stage area. */
-template <int S, int KEEP, bool PAIR>
+/* what the MMAs of an item have in common */
+struct mma_item {
+	uint32_t idesc[3];           /* of one, two, three slices */
+	uint32_t sa, sb;             /* slice strides of the descriptors */
+	uint32_t sbo;                /* bytes between 8-row groups */
+	uint32_t n;                  /* columns per accumulator */
+};
+
+/* the products of a set for one K step whose stage step starts at base;
+ * acc0: 0 where they start the set's accumulators */
+template <int S, int KEEP, int CLS, int SET, bool PAIR, int P = 0, int Q = -1>
 __device__ __forceinline__ void
-issue_step(uint32_t tmem, uint32_t base, uint32_t a_off, uint32_t idesc,
-    int which, uint32_t &started)
+issue_set(const mma_item &m, uint32_t tmem, uint32_t xcol, uint32_t alo, uint32_t ahi,
+    uint32_t blo, uint32_t bhi, uint32_t acc0)
 {
-	const uint64_t da = sdesc(base, S * 256), db = sdesc(base + a_off, S * 256);
-	const uint32_t alo = (uint32_t)da, ahi = (uint32_t)(da >> 32);
-	const uint32_t blo = (uint32_t)db, bhi = (uint32_t)(db >> 32);
-#pragma unroll
-	for (int pa = 0; pa < S; pa++)
-#pragma unroll
-		for (int qb = 0; qb < S; qb++) {
-			if (pa + qb > KEEP)
-				continue;
-			const int acc = min(pa + qb, 3);
-			if (!(which & (acc == acc_sets<KEEP>::XACC ? 1 : 2)))
-				continue;
-			if constexpr (PAIR)
-				mma_bf16_pair(tmem + acc * 128, alo + qb * 16, ahi, blo + pa * 16,
-				    bhi, idesc, (started >> acc) & 1u);
-			else
-				mma_bf16_split(tmem + acc * 128, alo + qb * 16, ahi, blo + pa * 16,
-				    bhi, idesc, (started >> acc) & 1u);
-			started |= 1u << acc;
-		}
+	using R = prod<S, KEEP, CLS, SET>;
+	if constexpr (Q < 0) {
+		constexpr int q0 = R::GLO > P ? R::GLO - P : 0;
+		if constexpr (P < S)
+			issue_set<S, KEEP, CLS, SET, PAIR, P, q0>(m, tmem, xcol, alo, ahi, blo, bhi, acc0);
+	} else if constexpr (Q >= S || P + Q > R::GHI) {
+		issue_set<S, KEEP, CLS, SET, PAIR, P + 1, -1>(m, tmem, xcol, alo, ahi, blo, bhi, acc0);
+	} else {
+		constexpr int w = R::width(P, Q), a = R::acc(P + Q);
+		/* the first product of its accumulators: slice 0 of the M side
+		 * with the first slice of each accumulator */
+		constexpr bool first = P == 0 && (Q == R::GLO || R::acc(Q) != R::acc(Q - 1));
+		/* FP32 alternates X between two fixed places */
+		const uint32_t d = tmem + (KEEP == 2 && !PAIR && a == 2 ? xcol : a * m.n);
+		const uint32_t acc = first ? acc0 : 1u;
+		if constexpr (PAIR)
+			mma_bf16_pair(d, alo + P * m.sa, ahi, blo + Q * m.sb, bhi, m.idesc[0], acc);
+		else
+			mma_bf16_split(d, alo + P * m.sa, ahi, blo + Q * m.sb, bhi,
+			    m.idesc[w - 1], acc);
+		issue_set<S, KEEP, CLS, SET, PAIR, P, Q + w>(m, tmem, xcol, alo, ahi, blo, bhi, acc0);
+	}
+}
+
+/* K steps of a pair of contracted extent k */
+__device__ __forceinline__ int pair_steps(int k, int cplx)
+{
+	return (cplx ? 2 : 1) * ((k + EMU_KS - 1) / EMU_KS);
+}
+
+/*
+ * Drain arithmetic.  A value x is rounded to an integer by fp32 adds and a
+ * bit read, not by the conversion pipe (1/8 of the FMA pipe's rate): the
+ * bits of x + M, M = 1.5 * 2^23, are those of M plus rint(x) for |x| < 2^22.
+ * The bits of M stay in the sums and are subtracted once at the end.  64-bit
+ * sums take shifted words and carries; a 32 x 32 -> 64 multiply-add costs
+ * four issue slots (set Y of a chunk at N = 115: 4057 cycles with it, 3206 as
+ * below, 3598 with a conversion per group; FP32's set X 1879 -> 1168).
+ */
+constexpr float MAGICF = 12582912.0f;
+constexpr int MAGIC = 0x4B400000;
+
+/* V += (uint64)a << sh, 1 <= sh < 32 */
+__device__ __forceinline__ uint64_t shl64(uint32_t a, int sh)
+{
+	return ((uint64_t)(a >> (32 - sh)) << 32) | (uint32_t)(a << sh);
 }
 
 /* PAIR: a cluster of two CTAs runs each 256-row tile with cta_group::2
@@ -525,7 +605,7 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
     const xmgd_view_t *__restrict__ va, const xmgd_view_t *__restrict__ vb,
     const int32_t *__restrict__ tabs, const int32_t *__restrict__ EA,
     const int32_t *__restrict__ EB, const int32_t *__restrict__ cbF,
-    double alpha, double beta, int expoff2, int cplx, int hmax, int pfd, int kchunk,
+    double alpha, double beta, int expoff2, int cplx, int hmax, int kchunk, int rowmajor,
     int *__restrict__ flags)
 {
 	using C = stage_cfg<S>;
@@ -534,7 +614,11 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 	uint8_t *stages = reinterpret_cast<uint8_t *>(
 	    (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
 	__shared__ __align__(8) uint64_t bar_full[NST], bar_empty[NST];
-	__shared__ __align__(8) uint64_t bar_xfull, bar_yfull, bar_xempty, bar_yempty, bar_fin;
+	/* FP32 keeps two copies of set X (its third accumulator leaves room),
+	 * used by the chunks in turn */
+	constexpr bool XDB = KEEP == 2 && !PAIR;
+	constexpr uint32_t XCOL = 256;       /* their columns: 256, 384 */
+	__shared__ __align__(8) uint64_t bar_xfull, bar_yfull, bar_xempty[2], bar_yempty, bar_fin;
 	__shared__ __align__(8) uint64_t bar_ifull[2], bar_iempty[2];
 	__shared__ __align__(8) uint64_t bar_pfull[PAIR ? NST : 1];
 	__shared__ int s_item[2];
@@ -576,7 +660,8 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 		}
 		mbar_init(smem_u32(&bar_xfull), 1);
 		mbar_init(smem_u32(&bar_yfull), 1);
-		mbar_init(smem_u32(&bar_xempty), PAIR ? 2 * DW : DW);
+		for (int q = 0; q < 2; q++)
+			mbar_init(smem_u32(&bar_xempty[q]), PAIR ? 2 * DW : DW);
 		mbar_init(smem_u32(&bar_yempty), PAIR ? 2 * DW : DW);
 		mbar_init(smem_u32(&bar_fin), 1);
 		for (int q = 0; q < 2; q++) {
@@ -651,50 +736,60 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 				const xmgd_cblock_t cb = cbs[members[it.mfirst].cblock];
 				const int pass = it.pr & 1, swp = (it.pr >> 1) & 1;
 				const int mstk = (it.pr >> 2) & 1;
-				/* the shared side: the M side's 128 rows (this CTA's half
-				 * of 256 in a pair) or, M-stacked, the N side's live rows;
-				 * the members: their live rows at their first column or
-				 * lane (a pair: one member, this CTA's half of its rows) */
-				const uint32_t ntot = (uint32_t)(it.pr >> 8) * S * 32 / (PAIR ? 2 : 1);
-				const uint32_t noff = PAIR ? rank * ntot : 0;
-				const uint32_t shb = mstk ? ntot : C::CHUNK_BYTES;
+				constexpr uint32_t ROWB = S * EMU_KS * 2;  /* a row's slices */
+				/* the shared side: the M side's tile (this CTA's of the two
+				 * in a pair) or, M-stacked, the N side's */
+				const int stile = it.m0 / EMU_TM + (mstk ? 0 : (int)rank);
+				const int slen = mstk == swp ? cb.n : cb.m;
+				/* (a pair's second M tile may lie past the view: its rows
+				 * are then never stored) */
+				const uint32_t sby = stile * EMU_TM < slen ?
+				    tile_rows(slen, stile * EMU_TM) * ROWB : 0;
+				/* the members: bytes copied per K step, bytes of their
+				 * tile's chunk, place in the stage; one member, unless the
+				 * list is stacked (row-major chunks); a pair stages half of
+				 * its rows in each CTA */
 				int mfp[EMU_MAXMEM], mrt[EMU_MAXMEM];
-				uint32_t mby[EMU_MAXMEM], mdo[EMU_MAXMEM], stb = 0;
+				uint32_t mby[EMU_MAXMEM], mch[EMU_MAXMEM], mdo[EMU_MAXMEM], stb = 0;
 #pragma unroll
 				for (int j = 0; j < EMU_MAXMEM; j++) {
 					const emu_member mb = members[it.mfirst + (j < nmem ? j : 0)];
-					mfp[j] = cbs[mb.cblock].first_pair;
+					const xmgd_cblock_t cj = cbs[mb.cblock];
+					mfp[j] = cj.first_pair;
 					mrt[j] = mb.n0 / EMU_TM;
-					mby[j] = PAIR ? ntot : (uint32_t)mb.rows * S * 32;
-					mdo[j] = (mstk ? 0u : C::CHUNK_BYTES) + (uint32_t)mb.off * S * 32;
+					/* the stacked side: the N side (without swap a's rows)
+					 * or, M-stacked, the M side */
+					mch[j] = tile_rows(mstk == swp ? cj.m : cj.n, mb.n0) * ROWB;
+					mby[j] = PAIR ? mch[j] / 2 : mch[j];
+					mdo[j] = (mstk ? 0u : C::CHUNK_BYTES) + (uint32_t)mb.off * ROWB;
 					stb += j < nmem ? mby[j] : 0;
 				}
+				const uint32_t mso = PAIR ? rank * mby[0] : 0;
 				/* shared side from a's views when it is a's side */
 				const bool sha = (mstk ^ swp) != 0;
-				/* a pair's operand chunks: the shared side's tile (live
-				 * or past the view) and each member's */
+				/* a pair's operand chunks: the shared side's tile and each
+				 * member's */
 				struct pair_src {
 					const uint8_t *gs, *gn[EMU_MAXMEM];
 					int nks;
-					bool slive;
 				};
 				auto load_pair = [&](int p, pair_src &o) {
 					/* the members' pair lists run in step: pair p of
 					 * every member has member 0's view and K on the
 					 * shared side */
 					const xmgd_pair_t pr = prs[cb.first_pair + p];
-					const xmgd_view_t ws = sha ? va[pr.aview] : vb[pr.bview];
-					o.nks = vb[pr.bview].n_ks;
-					const int stile = it.m0 / EMU_TM + (mstk ? 0 : (int)rank);
-					o.slive = stile < ws.n_rt;
-					o.gs = reinterpret_cast<const uint8_t *>(ws.slices) +
+					o.nks = pair_steps(pr.k, cplx);
+					o.gs = reinterpret_cast<const uint8_t *>(sha ?
+					    va[pr.aview].slices : vb[pr.bview].slices) +
 					    (size_t)stile * o.nks * C::CHUNK_BYTES;
 #pragma unroll
 					for (int j = 0; j < EMU_MAXMEM; j++) {
+						if (j >= nmem)
+							break;
 						const xmgd_pair_t pj = prs[mfp[j] + p];
 						o.gn[j] = reinterpret_cast<const uint8_t *>(sha ?
 						    vb[pj.bview].slices : va[pj.aview].slices) +
-						    (size_t)mrt[j] * o.nks * C::CHUNK_BYTES + noff;
+						    (size_t)mrt[j] * o.nks * C::CHUNK_BYTES + mso;
 					}
 				};
 				/* K step ks of a pair: the shared side reads at its own
@@ -707,59 +802,47 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 					ksh = mstk ? kn : km;
 					kst = mstk ? km : kn;
 				};
-				/* L2 prefetch cursor, pfd steps ahead of the copies within
-				 * the item (XMG_EMU_PF; off by default: measured slower,
-				 * the ring's copies are not waiting on DRAM misses) */
-				pair_src pf;
-				int pfp = 0, pfk = 0;
-				if (pfd > 0)
-					load_pair(0, pf);
-				auto pf_step = [&]() {
-					if (pfd <= 0 || pfp >= cb.npairs)
-						return;
-					int ksh, kst;
-					kidx(pfk, pf.nks, ksh, kst);
-					if (pf.slive)
-						bulk_prefetch_l2(pf.gs + (size_t)ksh * C::CHUNK_BYTES, shb);
-#pragma unroll
-					for (int j = 0; j < EMU_MAXMEM; j++)
-						if (j < nmem)
-							bulk_prefetch_l2(pf.gn[j] + (size_t)kst * C::CHUNK_BYTES,
-							    mby[j]);
-					if (++pfk == pf.nks) {
-						pfk = 0;
-						if (++pfp < cb.npairs)
-							load_pair(pfp, pf);
-					}
-				};
-				for (int q = 0; q < pfd; q++)
-					pf_step();
-				pair_src cur;
+				/* the next pair's operand addresses are loaded while this
+				 * one's steps are staged (two dependent loads) */
+				pair_src cur, nxt;
+				load_pair(0, nxt);
 				for (int p = 0; p < cb.npairs && !s_err; p++) {
-					load_pair(p, cur);
+					cur = nxt;
+					if (p + 1 < cb.npairs)
+						load_pair(p + 1, nxt);
 					for (int ks = 0; ks < cur.nks; ) {
+						const int ke = super_end<S>(ks, cur.nks, cplx);
 						if (!wait(smem_u32(&bar_empty[s]), ph ^ 1, 1))
 							break;
-						const int ke = super_end<S>(ks, cur.nks, cplx);
 						uint32_t dst = smem_u32(stages + (size_t)s * C::STAGE_BYTES);
-						uint32_t fb = smem_u32(&bar_full[s]);
-						/* a pair's second M tile may lie past the view: its
-						 * rows are then never stored */
-						mbar_expect_tx(fb, (uint32_t)(ke - ks) *
-						    ((cur.slive ? shb : 0) + stb));
-						for (int k = ks; k < ke; k++, dst += C::STEP_BYTES) {
-							int ksh, kst;
-							kidx(k, cur.nks, ksh, kst);
-							if (cur.slive)
-								bulk_g2s(dst + (mstk ? C::CHUNK_BYTES : 0u),
-								    cur.gs + (size_t)ksh * C::CHUNK_BYTES, shb, fb);
+						const uint32_t fb = smem_u32(&bar_full[s]);
+						mbar_expect_tx(fb, (uint32_t)(ke - ks) * (sby + stb));
+						/* (a stage's steps lie in one half of a realified view,
+						 * so that both operands' chunks follow one another) */
+						int ksh, kst;
+						kidx(ks, cur.nks, ksh, kst);
+						const uint8_t *g = cur.gs + (size_t)ksh * sby;
+						if (nmem == 1 && !PAIR) {
+							const uint8_t *x = cur.gn[0] + (size_t)kst * mch[0];
+							const uint32_t xb = mch[0];
+							for (int k = ks; k < ke; k++) {
+								bulk_g2s(dst, g, sby, fb);
+								bulk_g2s(dst + C::CHUNK_BYTES, x, xb, fb);
+								dst += C::STEP_BYTES;
+								g += sby;
+								x += xb;
+							}
+						} else
+						for (int k = ks; k < ke; k++, kst++) {
+							if (!PAIR || sby)
+								bulk_g2s(dst + (mstk ? C::CHUNK_BYTES : 0u), g, sby, fb);
 #pragma unroll
 							for (int j = 0; j < EMU_MAXMEM; j++)
 								if (j < nmem)
 									bulk_g2s(dst + mdo[j],
-									    cur.gn[j] + (size_t)kst * C::CHUNK_BYTES,
-									    mby[j], fb);
-							pf_step();
+									    cur.gn[j] + (size_t)kst * mch[j], mby[j], fb);
+							dst += C::STEP_BYTES;
+							g += sby;
 						}
 #pragma unroll
 						for (int q = 0; q < NST; q++)
@@ -798,7 +881,7 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 					break;
 				const xmgd_cblock_t cb = cbs[members[items[t].mfirst].cblock];
 				for (int p = 0; p < cb.npairs && !s_err; p++) {
-					const int nst_p = stages_of<S>(vb[prs[cb.first_pair + p].bview].n_ks, cplx);
+					const int nst_p = stages_of<S>(pair_steps(prs[cb.first_pair + p].k, cplx), cplx);
 					for (int q = 0; q < nst_p; q++) {
 						if (!wait(smem_u32(&bar_full[s]), ph, 3))
 							break;
@@ -816,9 +899,9 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 	} else if (warp == 1) {
 		/* ---------------- MMA issuer ---------------- */
 		if (lane == 0) {
-			int s = 0;
+			int s = 0, prevn = 0;
 			bool first = true;
-			uint32_t ph = 0, xph = 0, yph = 0;
+			uint32_t ph = 0, xph = 0, yph = 0, nch = 0;
 			uint32_t iph = 0;
 			/* a stage is ready once this CTA's copies (and, in a pair,
 			 * the peer's, forwarded) have landed */
@@ -827,7 +910,155 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 					return false;
 				if (PAIR && !wait(smem_u32(&bar_pfull[st_]), par, 10))
 					return false;
+				tc_fence_after();
 				return true;
+			};
+			/* one item of a width class; returns on failure (s_err set) */
+			auto item = [&](auto cls, const emu_item &it, const xmgd_cblock_t &cb) {
+				constexpr int CLS = decltype(cls)::value;
+				constexpr int KS = C::KSTEPS;
+				mma_item mi;
+				mi.n = it.pr >> 8;
+				const int swp = (it.pr >> 1) & 1;
+				for (int w = 0; w < 3; w++)
+					mi.idesc[w] = PAIR ? idesc_pair_n(mi.n) : idesc_n((w + 1) * mi.n);
+				mi.sbo = rowmajor ? S * 256 : 256;
+				mi.sa = rowmajor ? 16 : 2 * tile_rows(swp ? cb.m : cb.n, it.m0);
+				mi.sb = rowmajor ? 16 : 2 * mi.n;
+				/* accumulators of another width than the last item's lie
+				 * across them: wait for both sets' drains */
+				bool both = !XDB && !first && (int)mi.n != prevn;
+				prevn = mi.n;
+				int knext = prs[cb.first_pair].k;
+				for (int p = 0; p < cb.npairs; p++) {
+					const int nks = pair_steps(knext, cplx);
+					if (p + 1 < cb.npairs)
+						knext = prs[cb.first_pair + p + 1].k;
+					for (int c0 = 0; c0 < nks; ) {
+						const int c1 = chunk_end<S>(c0, nks, cplx, kchunk);
+						/* the chunk's stages: KSTEPS steps each, the last
+						 * one shorter at a segment's end */
+						const int nss = (c1 - c0 + KS - 1) / KS;
+						const uint32_t xcol = XCOL + (nch & 1) * 128;
+						/* every accumulator restarts each chunk: the exact
+						 * groups for their 2^24 bound, the low band because
+						 * the tensor core's fp32 accumulation error grows
+						 * with the accumulation length (per-pair
+						 * accumulation measured 10x larger error) */
+						uint32_t ax = 0, ay = 0;
+						/* the products of stage sj, the chunk's j-th: set X
+						 * (1), set Y (2) or both (3) */
+						auto issue = [&](int sj, int j, auto which) {
+							constexpr int WH = decltype(which)::value;
+							const uint32_t base = smem_u32(stages + (size_t)sj * C::STAGE_BYTES);
+							const int nk = min(KS, c1 - c0 - j * KS);
+							for (int u = 0; u < nk; u++) {
+								const uint32_t b0 = base + u * C::STEP_BYTES;
+								const uint64_t da = sdesc(b0, mi.sbo);
+								const uint64_t db = sdesc(b0 + C::CHUNK_BYTES, mi.sbo);
+								const uint32_t alo = (uint32_t)da, ahi = (uint32_t)(da >> 32);
+								const uint32_t blo = (uint32_t)db, bhi = (uint32_t)(db >> 32);
+								if constexpr (WH == 3 && CLS == 2 && KEEP > 2) {
+									/* (a middle stage: both sets have started) */
+									issue_set<S, KEEP, CLS, SET_ALL, PAIR>(mi, tmem, xcol, alo,
+									    ahi, blo, bhi, 1u);
+									continue;
+								}
+								if constexpr (WH & 2) {
+									issue_set<S, KEEP, CLS, SET_Y, PAIR>(mi, tmem, xcol, alo, ahi,
+									    blo, bhi, ay);
+									ay = 1;
+								}
+								if constexpr (WH & 1) {
+									issue_set<S, KEEP, CLS, SET_X, PAIR>(mi, tmem, xcol, alo, ahi,
+									    blo, bhi, ax);
+									ax = 1;
+								}
+							}
+						};
+						const std::integral_constant<int, 1> X{};
+						const std::integral_constant<int, 2> Y{};
+						const std::integral_constant<int, 3> XY{};
+						/* head: the first H (staged) stages; tail: the last T
+						 * stages; middle: the rest.  H, T <= hmax <= NST: the
+						 * stages a head or tail holds are released only after
+						 * its set-Y products, so hmax < NST leaves stages for
+						 * the producer to prefetch the steps after them */
+						const int H = min(hmax, nss);
+						const int T = XDB ? 0 : min(hmax, nss - H);
+						/* head, set X, as soon as the drain has read X of
+						 * the previous chunk (of the one before it, where X
+						 * has two copies) */
+						if (XDB) {
+							if (nch >= 2 && !wait(smem_u32(&bar_xempty[nch & 1]),
+							    ((nch >> 1) - 1) & 1, 2))
+								return;
+						} else if (!first) {
+							if (!wait(smem_u32(&bar_xempty[0]), xph, 2))
+								return;
+							xph ^= 1;
+						}
+						if (both) {
+							if (!wait(smem_u32(&bar_yempty), yph, 8))
+								return;
+							yph ^= 1;
+						}
+						tc_fence_after();
+						for (int j = 0; j < H; j++) {
+							const int sj = s + j < NST ? s + j : s + j - NST;
+							if (!ready(sj, s + j < NST ? ph : ph ^ 1))
+								return;
+							issue(sj, j, X);
+						}
+						if (T == 0 && !XDB)
+							commit(&bar_xfull);
+						/* head, set Y, once Y is read too */
+						if (!first && !both) {
+							if (!wait(smem_u32(&bar_yempty), yph, 8))
+								return;
+							yph ^= 1;
+						}
+						first = both = false;
+						tc_fence_after();
+						for (int j = 0; j < H; j++) {
+							const int sj = s + j < NST ? s + j : s + j - NST;
+							issue(sj, j, Y);
+							commit(&bar_empty[sj]);
+						}
+						s += H;
+						if (s >= NST) { s -= NST; ph ^= 1; }
+						/* middle: every product per stage */
+						for (int j = H; j < nss - T; j++) {
+							if (!ready(s, ph))
+								return;
+							issue(s, j, XY);
+							commit(&bar_empty[s]);
+							if (++s == NST) { s = 0; ph ^= 1; }
+						}
+						/* tail: set X of the last T stages, then X is
+						 * complete and its drain can start while the
+						 * tensor core still works on set Y */
+						for (int j = 0; j < T; j++) {
+							const int sj = s + j < NST ? s + j : s + j - NST;
+							if (!ready(sj, s + j < NST ? ph : ph ^ 1))
+								return;
+							issue(sj, nss - T + j, X);
+						}
+						if (T > 0) {
+							commit(&bar_xfull);
+							for (int j = 0; j < T; j++) {
+								const int sj = s + j < NST ? s + j : s + j - NST;
+								issue(sj, nss - T + j, Y);
+								commit(&bar_empty[sj]);
+							}
+							s += T;
+							if (s >= NST) { s -= NST; ph ^= 1; }
+						}
+						commit(&bar_yfull);
+						nch++;
+						c0 = c1;
+					}
+				}
 			};
 			for (int slot = 0; !s_err; ) {
 				if (!wait(smem_u32(&bar_ifull[slot]), iph, 6))
@@ -839,115 +1070,22 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 					break;
 				const emu_item it = items[t];
 				const xmgd_cblock_t cb = cbs[members[it.mfirst].cblock];
-				const uint32_t idesc = PAIR ? idesc_pair_n(it.pr >> 8) : idesc_n(it.pr >> 8);
-				for (int p = 0; p < cb.npairs && !s_err; p++) {
-					const xmgd_pair_t pr = prs[cb.first_pair + p];
-					const int nks = vb[pr.bview].n_ks;
-					for (int c0 = 0; c0 < nks && !s_err; ) {
-						const int c1 = chunk_end<S>(c0, nks, cplx, kchunk);
-						/* the chunk's stages: KSTEPS steps each, the last
-						 * one shorter at a segment's end */
-						constexpr int KS = C::KSTEPS;
-						const int nss = (c1 - c0 + KS - 1) / KS;
-						/* every accumulator restarts each chunk: the exact
-						 * groups for their 2^24 bound, the low band because
-						 * the tensor core's fp32 accumulation error grows
-						 * with the accumulation length (per-pair
-						 * accumulation measured 10x larger error) */
-						uint32_t started = 0;
-						bool okc = true;
-						auto issue_stage = [&](int sj, int j, int which) {
-							const uint32_t base = smem_u32(stages + (size_t)sj * C::STAGE_BYTES);
-							const int nk = min(KS, c1 - c0 - j * KS);
-							for (int u = 0; u < nk; u++)
-								issue_step<S, KEEP, PAIR>(tmem, base + u * C::STEP_BYTES,
-								    C::CHUNK_BYTES, idesc, which, started);
-						};
-						/* head: the first H (staged) stages; tail: the last T
-						 * stages; middle: the rest.  H, T <= hmax <= NST: the
-						 * stages a head or tail holds are released only after
-						 * its set-Y products, so hmax < NST leaves stages for
-						 * the producer to prefetch the steps after them */
-						const int H = min(hmax, nss);
-						const int T = min(hmax, nss - H);
-						/* head, set X, as soon as the drain has read X of
-						 * the previous chunk */
-						if (!first) {
-							if (!wait(smem_u32(&bar_xempty), xph, 2))
-								break;
-							xph ^= 1;
-						}
-						tc_fence_after();
-						for (int j = 0; j < H; j++) {
-							const int sj = s + j < NST ? s + j : s + j - NST;
-							const uint32_t pj = s + j < NST ? ph : ph ^ 1;
-							if (!ready(sj, pj)) {
-								okc = false;
-								break;
-							}
-							tc_fence_after();
-							issue_stage(sj, j, 1);
-						}
-						if (!okc)
-							break;
-						if (T == 0)
-							commit(&bar_xfull);
-						/* head, set Y, once Y is read too */
-						if (!first) {
-							if (!wait(smem_u32(&bar_yempty), yph, 8))
-								break;
-							yph ^= 1;
-						}
-						first = false;
-						tc_fence_after();
-						for (int j = 0; j < H; j++) {
-							const int sj = s + j < NST ? s + j : s + j - NST;
-							issue_stage(sj, j, 2);
-							commit(&bar_empty[sj]);
-						}
-						s += H;
-						if (s >= NST) { s -= NST; ph ^= 1; }
-						/* middle: every product per stage */
-						for (int j = H; j < nss - T; j++) {
-							if (!ready(s, ph)) {
-								okc = false;
-								break;
-							}
-							tc_fence_after();
-							issue_stage(s, j, 3);
-							commit(&bar_empty[s]);
-							if (++s == NST) { s = 0; ph ^= 1; }
-						}
-						if (!okc)
-							break;
-						/* tail: set X of the last T stages, then X is
-						 * complete and its drain can start while the
-						 * tensor core still works on set Y */
-						for (int j = 0; j < T; j++) {
-							const int sj = s + j < NST ? s + j : s + j - NST;
-							const uint32_t pj = s + j < NST ? ph : ph ^ 1;
-							if (!ready(sj, pj)) {
-								okc = false;
-								break;
-							}
-							tc_fence_after();
-							issue_stage(sj, nss - T + j, 1);
-						}
-						if (!okc)
-							break;
-						if (T > 0) {
-							commit(&bar_xfull);
-							for (int j = 0; j < T; j++) {
-								const int sj = s + j < NST ? s + j : s + j - NST;
-								issue_stage(sj, nss - T + j, 2);
-								commit(&bar_empty[sj]);
-							}
-							s += T;
-							if (s >= NST) { s -= NST; ph ^= 1; }
-						}
-						commit(&bar_yfull);
-						c0 = c1;
-					}
+				if (PAIR || rowmajor) {
+					item(std::integral_constant<int, 4>{}, it, cb);
+					continue;
+				}
+				if constexpr (PAIR)
+					;
+				else if constexpr (KEEP == 2)
+					item(std::integral_constant<int, 3>{}, it, cb);
+				else {
+					const int n = it.pr >> 8;
+					if (n <= 80)
+						item(std::integral_constant<int, 0>{}, it, cb);
+					else if (n <= 96)
+						item(std::integral_constant<int, 1>{}, it, cb);
+					else
+						item(std::integral_constant<int, 2>{}, it, cb);
 				}
 			}
 			/* every MMA issued by this CTA has completed once bar_fin
@@ -965,10 +1103,27 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 		constexpr int NC = 128 / (DW / 4);
 		constexpr int NSEG = NC / 16;
 		const int quad = warp & 3, half = (warp - 2) >> 2;
-		const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16) + half * NC;
-		uint32_t fph = 0;
+		const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16);
+		uint32_t fph = 0, xb = 0;
 		bool ok = true;
 		uint32_t iph = 0;
+		/* one lane waits, the warp follows its verdict, so the
+		 * .sync.aligned TMEM loads stay convergent */
+		auto wait_warp = [&](uint64_t *bar, uint32_t par, int code) -> bool {
+			int w = 1;
+			if (lane == 0)
+				w = wait(smem_u32(bar), par, code);
+			w = __shfl_sync(0xffffffffu, w, 0);
+			tc_fence_after();
+			return w != 0;
+		};
+		/* this warp has read a set: the MMA warp may overwrite it */
+		auto release = [&](uint64_t *bar) {
+			tc_fence_before();
+			__syncwarp();
+			if (lane == 0)
+				arrive0(bar);
+		};
 		for (int slot = 0; ok; ) {
 			int t = -1;
 			if (lane == 0) {
@@ -985,8 +1140,13 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 			const emu_item it = items[t];
 			const int pass = it.pr & 1, swp = (it.pr >> 1) & 1, rows = it.pr >> 8;
 			const int mstk = (it.pr >> 2) & 1;
-			/* this warp's NC columns fall into NC / 16 segments of 16, each
-			 * inside one member's output block (N-stacked members hold
+			/* this warp's columns: 32, or 16 where the tile has at most
+			 * 64, so that every column group has work */
+			const int cw = rows <= 64 && NC == 32 ? 16 : NC;
+			const int col0 = half * cw;
+			const int nacc3 = KEEP == 2 || PAIR || rowmajor ? 1 : rows <= 80 ? 3 : rows <= 96 ? 2 : 1;
+			/* its columns fall into segments of 16, each inside one
+			 * member's output block (N-stacked members hold
 			 * multiples of 16 columns; M-stacked ones multiples of 32
 			 * lanes, so one member holds all of this warp's lanes): per
 			 * segment the output block, its first pair, its F and the
@@ -1004,13 +1164,13 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 					scb[g] = mb.cblock;
 					sfp[g] = cbs[mb.cblock].first_pair;
 					sF[g] = cbF[mb.cblock];
-					sq0[g] = it.m0 + half * NC + g * 16;
+					sq0[g] = it.m0 + col0 + g * 16;
 				}
 				mrow0 = mb.n0 + row0 - mb.off;
 			} else {
 #pragma unroll
 				for (int g = 0; g < NSEG; g++) {
-					const int col = half * NC + g * 16;
+					const int col = col0 + g * 16;
 					int j = 0;
 					for (int jj = 1; jj < it.mcount; jj++)
 						j += col >= members[it.mfirst + jj].off;
@@ -1023,18 +1183,113 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 				mrow0 = it.m0 + (int)rank * EMU_TM + quad * 32;
 			}
 			const int npairs = cbs[scb[0]].npairs;
-			long long V[NC];
+			uint64_t V[NC];                  /* two's complement */
 #pragma unroll
 			for (int c = 0; c < NC; c++)
 				V[c] = 0;
-			for (int p = 0; p < npairs && ok; p++) {
-				const int nks = vb[prs[sfp[0] + p].bview].n_ks;
-				int esg[NSEG], esh[NSEG];
+			/* set X.  FP64: the low band, L in units of 2^-16 (|L| <
+			 * 2^19: 15 products of 256 times 2^14 at 2^-24, with the pair
+			 * factor's 2), to units of 2^(-16-F): V += 2^F h + l, h =
+			 * rint(L), l = rint(2^F (L - h)).  FP32: group 2, an integer */
+			auto drain_x = [&](uint32_t at, const float *s0) {
 #pragma unroll
-				for (int g = 0; g < NSEG; g++) {
-					const xmgd_pair_t pg = prs[sfp[g] + p];
-					esg[g] = pg.esign;
-					esh[g] = pg.eshift;
+				for (int b4 = 0; b4 < NC / 4; b4++) {
+					if (b4 * 4 >= cw || col0 + b4 * 4 >= rows)
+						break;	/* warp-uniform: columns past the tile */
+					const int g = b4 / 4;
+					float ax[4];
+					tmem_ld4(trow + at + col0 + b4 * 4, ax);
+					if (LOW && nacc3 > 1) {
+						/* groups 4 (and 5) have their own accumulators,
+						 * in the same units */
+						float a4[4], a5[4] = {0, 0, 0, 0};
+						tmem_ld4(trow + at + rows + col0 + b4 * 4, a4);
+						if (nacc3 > 2)
+							tmem_ld4(trow + at + 2 * rows + col0 + b4 * 4, a5);
+						tmem_wait_ld();
+#pragma unroll
+						for (int c = 0; c < 4; c++)
+							ax[c] += a4[c] + a5[c];
+					} else
+						tmem_wait_ld();
+#pragma unroll
+					for (int c = 0; c < 4; c++) {
+						const float sx = s0[g] * 65536.0f;
+						if (LOW) {
+							const float t = fmaf(ax[c], sx, MAGICF);
+							const float r = fmaf(ax[c], sx, MAGICF - t);
+							const float l = fmaf(r, __int_as_float((127 + sF[g]) << 23),
+							    MAGICF);
+							V[b4 * 4 + c] += shl64(__float_as_uint(t), sF[g]) +
+							    __float_as_uint(l);
+						} else
+							V[b4 * 4 + c] += (long long)__float2int_rn(ax[c] * sx);
+					}
+				}
+			};
+			/* set Y: D0 2^16 + D1 2^8 (+ D2), the exact groups, read as
+			 * D0, D1 2^-8, D2 2^-16.  With h = rint(D1 2^-8), the sum is
+			 * 2^16 (D0 + h) + e, e = 2^8 (D1 - 2^8 h) + D2: both fit 24
+			 * bits (|D0| <= 2^22, |h| <= 2^15, |D2| < 3 * 2^22, each
+			 * twice that with the pair factor's 2, then even), so two
+			 * conversions serve three groups, one serves two in FP32 */
+			auto drain_y = [&](const float *s0) {
+#pragma unroll
+				for (int b4 = 0; b4 < NC / 4; b4++) {
+					if (b4 * 4 >= cw || col0 + b4 * 4 >= rows)
+						break;
+					const int g = b4 / 4, F = sF[g];
+					float a0[4], a1[4], a2[4];
+					tmem_ld4(trow + col0 + b4 * 4, a0);
+					tmem_ld4(trow + rows + col0 + b4 * 4, a1);
+					if (LOW)
+						tmem_ld4(trow + 2 * rows + col0 + b4 * 4, a2);
+					tmem_wait_ld();
+#pragma unroll
+					for (int c = 0; c < 4; c++) {
+						const float h = fmaf(a1[c], s0[g], MAGICF) - MAGICF;
+						const float r = fmaf(a1[c], s0[g], -h);
+						const int d = __float2int_rn(fmaf(a0[c], s0[g], h));
+						if (LOW) {
+							const int e = __float2int_rn(fmaf(a2[c], s0[g], r) * 65536.0f);
+							/* d 2^(16+F) + e 2^F, 1 <= F <= 15 */
+							const uint64_t dv = ((uint64_t)(uint32_t)(d >> (16 - F)) << 32) |
+							    ((uint32_t)d << (16 + F));
+							const uint64_t ev = ((uint64_t)(uint32_t)(e >> (32 - F)) << 32) |
+							    ((uint32_t)e << F);
+							V[b4 * 4 + c] += dv + ev;
+						} else {
+							const float l = fmaf(r, 65536.0f, MAGICF);
+							const uint64_t dv = ((uint64_t)(uint32_t)(d >> 16) << 32) |
+							    ((uint32_t)d << 16);
+							V[b4 * 4 + c] += dv + __float_as_uint(l);
+						}
+					}
+				}
+			};
+			int nchunk = 0;
+			/* the next pair's extent and factors are loaded during this
+			 * one's chunks */
+			int knext = prs[sfp[0]].k, esn[NSEG], ehn[NSEG];
+#pragma unroll
+			for (int g = 0; g < NSEG; g++) {
+				esn[g] = prs[sfp[g]].esign;
+				ehn[g] = prs[sfp[g]].eshift;
+			}
+			for (int p = 0; p < npairs && ok; p++) {
+				const int nks = pair_steps(knext, cplx);
+				float f0[NSEG];
+#pragma unroll
+				for (int g = 0; g < NSEG; g++)
+					f0[g] = (esn[g] > 0 ? 1.0f : -1.0f) *
+					    __int_as_float((127 + ehn[g]) << 23);
+				if (p + 1 < npairs) {
+					knext = prs[sfp[0] + p + 1].k;
+#pragma unroll
+					for (int g = 0; g < NSEG; g++) {
+						esn[g] = prs[sfp[g] + p + 1].esign;
+						ehn[g] = prs[sfp[g] + p + 1].eshift;
+					}
 				}
 				for (int c0 = 0; c0 < nks; ) {
 					const int c1 = chunk_end<S>(c0, nks, cplx, kchunk);
@@ -1046,110 +1301,39 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 					float s0[NSEG];
 #pragma unroll
 					for (int g = 0; g < NSEG; g++)
-						s0[g] = ((esg[g] > 0) != negh ? 1.0f : -1.0f) *
-						    __int_as_float((127 + esh[g]) << 23);
-					/* one lane waits, the warp follows its verdict, so the
-					 * .sync.aligned TMEM loads below stay convergent */
-					int w = 1;
-					if (lane == 0)
-						w = wait(smem_u32(&bar_xfull), fph, 4);
-					w = __shfl_sync(0xffffffffu, w, 0);
-					if (!w) {
-						ok = false;
-						break;
-					}
-					tc_fence_after();
-					/* set X first: the low band (or, without one, group 2),
-					 * then release it to the MMA warp */
-					constexpr int XACC = acc_sets<KEEP>::XACC;
-#pragma unroll
-					for (int b4 = 0; b4 < NC / 4; b4++) {
-						if (half * NC + b4 * 4 >= rows)
-							break;	/* warp-uniform: columns past the tile */
-						const int g = b4 / 4, F = sF[g];
-						const float s2 = s0[g] * 65536.0f;
-						const float s3 = s0[g] * __int_as_float((127 + 16 + F) << 23);
-						float ax[4];
-						tmem_ld4(trow + XACC * 128 + b4 * 4, ax);
-						tmem_wait_ld();
-#pragma unroll
-						for (int c = 0; c < 4; c++) {
-							if (LOW) {
-								/* low band in units of 2^(-16-F), rounded
-								 * to an integer with fp32 adds only (the
-								 * conversion pipe runs at 1/8 of the FMA
-								 * pipe's rate and bounded this drain):
-								 * x = h * 2^22 + l, h = rint(x / 2^22) read
-								 * from the bits of x / 2^22 + 1.5 * 2^23,
-								 * l = x - h * 2^22 exact (|l| <= 2^21) and
-								 * rounded the same way.  |x| < 2^42 (the
-								 * band is below 2 units of the leading
-								 * group per chunk, scaled by at most
-								 * 2^(16 + 24 + 1)), inside the 2^44 the
-								 * first add allows; the sum h * 2^22 +
-								 * rint(l) equals rint(x), ties to even,
-								 * as a direct conversion would give */
-								const float M = 12582912.0f;	/* 1.5 * 2^23 */
-								const float x = ax[c] * s3;
-								const float t = fmaf(x, 2.384185791015625e-7f, M);
-								const float l = fmaf(t - M, -4194304.0f, x);
-								const int hi = __float_as_int(t) - 0x4B400000;
-								const int lo = __float_as_int(l + M) - 0x4B400000;
-								V[b4 * 4 + c] += ((long long)hi << 22) + lo;
-							} else {
-								V[b4 * 4 + c] += (long long)__float2int_rn(ax[c] * s2) << F;
-							}
-						}
-					}
-					tc_fence_before();
-					__syncwarp();
-					if (lane == 0)
-						arrive0(&bar_xempty);
-					/* set Y: the exact groups below X, once their last
-					 * products have landed */
-					w = 1;
-					if (lane == 0)
-						w = wait(smem_u32(&bar_yfull), fph, 9);
-					w = __shfl_sync(0xffffffffu, w, 0);
-					if (!w) {
-						ok = false;
-						break;
+						s0[g] = negh ? -f0[g] : f0[g];
+					if (XDB) {
+						/* Y first: X's copy is not needed for a chunk yet */
+						if (!(ok = wait_warp(&bar_yfull, fph, 9)))
+							break;
+						drain_y(s0);
+						release(&bar_yempty);
+						drain_x(XCOL + xb * 128, s0);
+						release(&bar_xempty[xb]);
+						xb ^= 1;
+					} else {
+						/* X first, then it is free for the next chunk's head;
+						 * Y once its last products have landed */
+						if (!(ok = wait_warp(&bar_xfull, fph, 4)))
+							break;
+						drain_x((LOW ? 3 : 2) * rows, s0);
+						release(&bar_xempty[0]);
+						if (!(ok = wait_warp(&bar_yfull, fph, 9)))
+							break;
+						drain_y(s0);
+						release(&bar_yempty);
 					}
 					fph ^= 1;
-					tc_fence_after();
-#pragma unroll
-					for (int b4 = 0; b4 < NC / 4; b4++) {
-						if (half * NC + b4 * 4 >= rows)
-							break;
-						const int g = b4 / 4, F = sF[g];
-						const float sa = s0[g], sb = sa * 256.0f, sc = sa * 65536.0f;
-						float a0[4], a1[4], a2[4];
-						tmem_ld4(trow + 0 * 128 + b4 * 4, a0);
-						tmem_ld4(trow + 1 * 128 + b4 * 4, a1);
-						if (LOW)
-							tmem_ld4(trow + 2 * 128 + b4 * 4, a2);
-						tmem_wait_ld();
-#pragma unroll
-						for (int c = 0; c < 4; c++) {
-							/* exact integers: with the pair factor's 2^1,
-							 * |i0| <= 2^14 * 336 * 2 < 2^23.4 and |i1| <
-							 * 2^24.4; the packing is 64-bit */
-							int i0 = __float2int_rn(a0[c] * sa);
-							int i1 = __float2int_rn(a1[c] * sb);
-							long long d = ((long long)i0 * 256 + i1) << 8;
-							if (LOW)
-								d += __float2int_rn(a2[c] * sc);
-							V[b4 * 4 + c] += d << F;
-						}
-					}
-					tc_fence_before();
-					__syncwarp();
-					if (lane == 0)
-						arrive0(&bar_yempty);
+					nchunk++;
 					c0 = c1;
 				}
 			}
-			if (!ok || s_err)
+			/* the magic numbers' bits out of the sums (modulo 2^64) */
+#pragma unroll
+			for (int c = 0; c < NC; c++)
+				V[c] -= (uint64_t)nchunk * (LOW ?
+				    shl64(MAGIC, sF[c / 16]) + MAGIC : (uint64_t)MAGIC);
+			if (__any_sync(0xffffffffu, !ok || s_err))
 				break;
 			/* epilogue (overlaps the next item's first chunk of MMAs):
 			 * this thread's TMEM lane is one M-side row; its columns are
@@ -1168,6 +1352,8 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 			    (unsigned long long)ab & (1ull << 63) : 0ull;
 #pragma unroll
 			for (int g = 0; g < NSEG; g++) {
+				if (g * 16 >= cw)
+					break;
 				const xmgd_cblock_t cb = cbs[scb[g]];
 				const int flim = swp ? cb.m : cb.n, vlim = swp ? cb.n : cb.m;
 				if (ms >= flim)
@@ -1181,11 +1367,11 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 #pragma unroll
 				for (int c = 0; c < 16; c++) {
 					const int q = sq0[g] + c;
-					if (q < vlim && half * NC + g * 16 + c < rows) {
+					if (q < vlim && col0 + g * 16 + c < rows) {
 						const int e = vexp[q] + fe - expoff2 - 16 - F;
 						double v;
-						if (!pack_f64(V[g * 16 + c], e + esa, asx, v))
-							v = alpha * ldexp((double)V[g * 16 + c], e);
+						if (!pack_f64((long long)V[g * 16 + c], e + esa, asx, v))
+							v = alpha * ldexp((double)(long long)V[g * 16 + c], e);
 						else if (!apow2)
 							v *= alpha;
 						TOUT *cp = Cp + (size_t)cm * (vtab[q] + fo) + pass;
@@ -1235,10 +1421,11 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
  *      max(N / 2, 32 + N / 4) cycles: the M-side operand (4 KiB) and the
  *      N-side operand (N * 32 B) are read from shared memory at 128 B per
  *      cycle while the tensor core needs N / 2 cycles.
- * (and 6, the stacked form below, which runs first).  The first runs of a
- * plan replay each distinct policy once, timed with events, then keep the
- * fastest; the choice is remembered per block-size histogram so later
- * plans of the same shape start tuned.
+ * (and 6, the stacked form below).  The first runs of a plan replay each
+ * distinct policy within a quarter of the modelled best once, in the model's
+ * order (list_cycles), timed with events, then keep the fastest; the choice
+ * is remembered per block-size histogram so later plans of the same shape
+ * start tuned.
  */
 enum { EMU_NPOLICY = 3 };
 
@@ -1252,6 +1439,15 @@ static bool
 pair_policy(int pol)
 {
 	return pol >= EMU_NPOLICY && pol < 2 * EMU_NPOLICY;
+}
+
+/* The operands' layout a policy's kernel form takes (emu_split_kernel):
+ * row-major where a tile stacks members, and for pairs; slice-major where
+ * every tile is one block's. */
+static bool
+row_major(int pol)
+{
+	return pair_policy(pol) || pol == EMU_POL_MERGED;
 }
 
 /* CTA pairs (256-row M tiles, cta_group::2): policies 3..5 repeat 0..2 in
@@ -1315,7 +1511,6 @@ struct emu_plan {
 	std::vector<emu_cand> cand;
 	int cur = 0, tuned = 0;
 	int hmax = 4;                        /* head/tail steps (<= stages) */
-	int pfd = 0;                         /* L2 prefetch distance, steps */
 	int a_mode = 0;                      /* shared a side (xmgd_contract_t) */
 	uint64_t a_slices = 0, a_E = 0, a_flag = 0;
 	int kchunk = EMU_CHUNK;              /* FP64: K steps per chunk */
@@ -1341,7 +1536,8 @@ launch_side(emu_plan *e, int side, int kind, int32_t *E, int *flags, cudaStream_
 		emu_exp_kernel<TIN><<<n, 256, 0, st>>>(dv, m, nv, e->kr[side], e->d_tabs, E,
 		    flags);
 	else
-		emu_split_kernel<TIN><<<n, 256, 0, st>>>(dv, m, nv, e->d_tabs, E);
+		emu_split_kernel<TIN><<<n, 256, 0, st>>>(dv, m, nv, e->d_tabs, E,
+		    row_major(e->cand[e->cur].policy));
 	g_launches++;
 	XMG_CK(cudaGetLastError());
 	return XMG_OK;
@@ -1424,7 +1620,8 @@ launch_gemm(emu_plan *e)
 		    e->d_cbs, e->d_prs,
 		    (const xmgd_view_t *)e->d_va, (const xmgd_view_t *)e->d_vb, e->d_tabs,
 		    (const int32_t *)EA, (const int32_t *)EB, (const int32_t *)e->d_F,
-		    e->alpha, e->beta, 2 * fin<TIN>::EXPOFF, e->cplx, e->hmax, e->pfd, e->kchunk, flags));
+		    e->alpha, e->beta, 2 * fin<TIN>::EXPOFF, e->cplx, e->hmax, e->kchunk,
+		    (int)row_major(c.policy), flags));
 	} else {
 		emu_gemm_kernel<S, KEEP, LOW, TOUT, EMU_DW, false><<<(unsigned)c.grid,
 		    64 + 32 * EMU_DW, stage_cfg<S>::SMEM, stream()>>>(
@@ -1432,7 +1629,8 @@ launch_gemm(emu_plan *e)
 		    e->d_cbs, e->d_prs,
 		    (const xmgd_view_t *)e->d_va, (const xmgd_view_t *)e->d_vb, e->d_tabs,
 		    EA, EB, (const int32_t *)e->d_F, e->alpha, e->beta,
-		    2 * fin<TIN>::EXPOFF, e->cplx, e->hmax, e->pfd, e->kchunk, flags);
+		    2 * fin<TIN>::EXPOFF, e->cplx, e->hmax, e->kchunk,
+		    (int)row_major(c.policy), flags);
 	}
 	g_launches++;
 	XMG_CK(cudaGetLastError());
@@ -1778,6 +1976,61 @@ items_ok(const xmgd_contract_t *p, const std::vector<emu_item> &items,
 	return true;
 }
 
+/* Modelled cycles of one K step of a tile of n columns: its MMAs (issue_set)
+ * at max(columns / 2, 32 + columns / 4) + 6 cycles each, and the stage's
+ * bytes written to shared memory at the 128 per cycle the MMAs read with. */
+static double
+step_cycles(bool dbl, bool rowmajor, int n)
+{
+	double c = 0;
+	auto mma = [&](int slices, int count) {
+		c += count * (std::max(slices * n / 2.0, 32 + slices * n / 4.0) + 6);
+	};
+	if (rowmajor)
+		mma(1, dbl ? 21 : 6);
+	else if (!dbl) {
+		mma(2, 1);
+		mma(1, 4);
+	} else if (n <= 80) {
+		mma(3, 5);
+		mma(2, 2);
+		mma(1, 2);
+	} else {
+		mma(2, n <= 96 ? 6 : 4);
+		mma(1, n <= 96 ? 9 : 13);
+	}
+	return c + (dbl ? fin<double>::S : fin<float>::S) * (EMU_TM + n) / 4.0;
+}
+
+/* modelled cycles of a work list on the chip: the SMs' share, at least the
+ * longest item */
+static double
+list_cycles(const xmgd_contract_t *p, const std::vector<emu_item> &items,
+    const std::vector<emu_member> &mem, int cplx, bool rowmajor)
+{
+	double sum = 0, top = 0;
+	for (const emu_item &it : items) {
+		const xmgd_cblock_t &cb = p->cblocks[mem[it.mfirst].cblock];
+		double steps = 0;
+		for (int q = 0; q < cb.npairs; q++)
+			steps += (cplx ? 2 : 1) * ((p->pairs[cb.first_pair + q].k + EMU_KS - 1) / EMU_KS);
+		const double c = steps * step_cycles(p->dtype >= 2, rowmajor, it.pr >> 8);
+		sum += c;
+		top = std::max(top, c);
+	}
+	return std::max(top, sum / std::max(1, num_sms()));
+}
+
+/* bytes of one K step of a view with mn rows: whole tiles, then the last
+ * one's rows (tile_rows) */
+static size_t
+view_step_bytes(int mn, int chunk_bytes)
+{
+	const int full = (mn - 1) / EMU_TM;
+	return (size_t)full * chunk_bytes +
+	    (size_t)tile_rows(mn, full * EMU_TM) * chunk_bytes / EMU_TM;
+}
+
 int
 emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
     const xmgd_cblock_t *d_cbs, const xmgd_pair_t *d_prs,
@@ -1806,10 +2059,9 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 	e->cplx = cplx;
 	{
 		const int nst = dbl ? stage_cfg<fin<double>::S>::NST : stage_cfg<fin<float>::S>::NST;
-		/* head/tail length in stages: 2 two-step stages (FP64), 1
-		 * three-step stage (FP32) */
+		/* head/tail length in stages */
 		const char *h = getenv("XMG_EMU_HEAD");
-		e->hmax = h ? atoi(h) : (dbl ? 2 : 1);
+		e->hmax = h ? atoi(h) : 2;
 		e->hmax = std::max(1, std::min(nst, e->hmax));
 		/* FP64 chunks in whole stages (they start at a segment's first
 		 * step, as the stages do) */
@@ -1817,8 +2069,6 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 		constexpr int KS64 = stage_cfg<fin<double>::S>::KSTEPS;
 		e->kchunk = kc ? std::max(1, std::min(20, atoi(kc))) : EMU_CHUNK;
 		e->kchunk = std::max(KS64, e->kchunk / KS64 * KS64);
-		const char *f = getenv("XMG_EMU_PF");
-		e->pfd = f ? std::max(0, atoi(f)) : 0;
 	}
 	e->alpha = p->alpha[0];
 	e->beta = p->beta[0];
@@ -1841,7 +2091,7 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 
 	{
 	/* operand views used by the emulated blocks, and the fixed-point
-	 * scale F of every block (|V| <= K_eff * 2^(30+F) < 2^61) */
+	 * scale F of every block (|V| <= K_eff * 2^(30+F) <= 2^62) */
 	std::vector<int32_t> F(p->ncblocks, 0);
 	std::vector<uint64_t> hist;
 	for (int ci : cblocks) {
@@ -1860,7 +2110,8 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 			st = xmg_seterr(XMG_ENOTSUP, "split-precision path: K too large");
 			goto fail;
 		}
-		F[ci] = std::min(24, 31 - lg);
+		/* (FP32 has no rounded terms to place below its integers) */
+		F[ci] = dbl ? std::max(1, std::min(15, 31 - lg)) : 0;
 		hist.push_back(mix64(((uint64_t)cb.m << 40) ^ ((uint64_t)cb.n << 20) ^
 		    (uint64_t)ksum));
 	}
@@ -1891,7 +2142,7 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 				continue;
 			}
 			w.slices = off;
-			off += (size_t)w.n_rt * w.n_ks * chunk_bytes;
+			off += (size_t)w.n_ks * view_step_bytes(w.mn, chunk_bytes);
 		}
 	};
 	tile(e->VA, e->useA, p->a_mode ? p->a_off : nullptr);
@@ -1949,21 +2200,24 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 		known = EMU_POL_MERGED;
 	if (getenv("XMG_POLICY"))	/* one fixed work-list policy */
 		known = atoi(getenv("XMG_POLICY"));
-	/* a plan that runs once has no runs left to tune with: the first
-	 * list that passes its checks */
+	/* a plan that runs once has no runs left to tune with: the list the
+	 * model puts first */
 	const bool first_only = p->one_shot && known < 0;
-	/* the stacked list first: a plan that runs once (an out-of-core
-	 * batch) never finishes tuning and keeps its first candidate */
 	std::vector<int> pols = {EMU_POL_MERGED, 0, 1, 2};
 	if (pairs_enabled())
 		pols.insert(pols.end(), {EMU_NPOLICY, EMU_NPOLICY + 1, EMU_NPOLICY + 2});
+	/* batches that share a's operands agree on their layout */
+	if (p->a_mode && !getenv("XMG_POLICY")) {
+		known = known >= 0 && row_major(known) ? known : -1;
+		pols.erase(std::remove_if(pols.begin(), pols.end(),
+		    [](int q) { return !row_major(q); }), pols.end());
+	}
 	std::vector<std::vector<emu_item>> lists;
 	std::vector<std::vector<emu_member>> mlists;
+	std::vector<double> est;
 	for (int pol : pols) {
 		if (known >= 0 && pol != known)
 			continue;
-		if (first_only && !e->cand.empty())
-			break;
 		std::vector<emu_item> items;
 		std::vector<emu_member> mem;
 		make_items(p, cblocks, cplx, pol, items, mem);
@@ -1973,7 +2227,9 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 			continue;
 		bool dup = false;
 		for (size_t l = 0; l < lists.size(); l++)
-			dup |= lists[l].size() == items.size() && mlists[l].size() == mem.size() &&
+			dup |= row_major(e->cand[l].policy) == row_major(pol) &&
+			    pair_policy(e->cand[l].policy) == pair_policy(pol) &&
+			    lists[l].size() == items.size() && mlists[l].size() == mem.size() &&
 			    memcmp(lists[l].data(), items.data(), items.size() * sizeof(emu_item)) == 0 &&
 			    memcmp(mlists[l].data(), mem.data(), mem.size() * sizeof(emu_member)) == 0;
 		if (dup)
@@ -1985,15 +2241,34 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 		    std::min(c.nitems, num_sms());
 		c.ms = -1;
 		c.d_items = c.d_members = 0;
-		if ((st = upload_new(items.data(), items.size() * sizeof(emu_item),
-		    &c.d_items)) || (st = upload_new(mem.data(), mem.size() *
-		    sizeof(emu_member), &c.d_members))) {
-			e->cand.push_back(c);	/* freed with the plan */
-			goto fail;
-		}
+		est.push_back(list_cycles(p, items, mem, cplx, row_major(pol)));
 		e->cand.push_back(c);
 		lists.push_back(std::move(items));
 		mlists.push_back(std::move(mem));
+	}
+	/* in the model's order; lists a quarter above the best are not tried
+	 * (measured spread of the model's ratios: +-10 %) */
+	{
+		std::vector<int> ord(e->cand.size());
+		for (size_t i = 0; i < ord.size(); i++)
+			ord[i] = (int)i;
+		std::stable_sort(ord.begin(), ord.end(),
+		    [&](int x, int y) { return est[x] < est[y]; });
+		std::vector<emu_cand> keep;
+		for (int i : ord) {
+			if (!keep.empty() && (first_only || est[i] > 1.25 * est[ord[0]]))
+				continue;
+			emu_cand c = e->cand[i];
+			if ((st = upload_new(lists[i].data(), lists[i].size() * sizeof(emu_item),
+			    &c.d_items)) || (st = upload_new(mlists[i].data(), mlists[i].size() *
+			    sizeof(emu_member), &c.d_members))) {
+				keep.push_back(c);	/* freed with the plan */
+				e->cand = keep;
+				goto fail;
+			}
+			keep.push_back(c);
+		}
+		e->cand = keep;
 	}
 	if (e->cand.empty()) {
 		st = xmg_seterr(XMG_EINVAL, "split-precision path: no work list "
@@ -2092,9 +2367,8 @@ xmgd_emu_view_bytes(const xmgd_view_t *v, int dtype)
 	const bool cplx = dtype == 1 || dtype == 3;
 	const int chunk_bytes = (dtype >= 2 ? fin<double>::S : fin<float>::S) *
 	    SLICE_BYTES;
-	const int64_t n_rt = (v->mn + EMU_TM - 1) / EMU_TM;
 	const int64_t n_ks = (cplx ? 2 : 1) * ((v->k + EMU_KS - 1) / EMU_KS);
-	return n_rt * n_ks * chunk_bytes;
+	return n_ks * (int64_t)view_step_bytes(v->mn, chunk_bytes);
 }
 int emu_items(const emu_plan *e) { return e->cand[e->cur].nitems; }
 int emu_policy(const emu_plan *e) { return e->cand[e->cur].policy; }
