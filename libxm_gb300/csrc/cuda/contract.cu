@@ -145,6 +145,35 @@ launch_plain(xmgd_plan *dp, uint64_t items, int n, int tile)
 	return xmg_seterr(XMG_EINVAL, "bad scalar type");
 }
 
+/* Whether the plain FP64 GEMM takes a contraction that the split-precision
+ * path could: where the modelled time of its longest chain of tiles stays
+ * below what the other path's launches alone cost (about 45 us for exponent,
+ * split and GEMM kernels one after the other; this is one kernel).  A 16 x 16
+ * tile takes 128 cycles per K element on its SM's FP64 pipe (four times that
+ * for complex), and about 2000 per pair to reach its operands.  Ladder
+ * o4/v10: 61 us on the split path, 20 here; the result is the more accurate
+ * one. */
+static bool
+plain_is_faster(const xmgd_contract_t *p, const std::vector<int> &blocks)
+{
+	const double unit = p->dtype == 3 ? 512 : 128, limit = 15.0 * 1900;
+	double sum = 0, top = 0;
+
+	if (!p->in_core || p->precision != XMG_PREC_AUTO || p->dtype < 2)
+		return false;
+	for (int i : blocks) {
+		const xmgd_cblock_t &cb = p->cblocks[i];
+		double c = 0;
+		for (int q = 0; q < cb.npairs; q++)
+			c += 2000 + unit * p->pairs[cb.first_pair + q].k;
+		top = std::max(top, c);
+		sum += c * ((cb.m + 15) / 16) * ((cb.n + 15) / 16);
+		if (top > limit || sum > limit * num_sms())
+			return false;
+	}
+	return true;
+}
+
 /* the launches of one segment, on the engine stream */
 static int
 record(xmgd_plan *dp, int seg)
@@ -272,6 +301,10 @@ xmgd_plan_create(const xmgd_contract_t *p, xmgd_plan **out)
 		bool want_emu = p->precision != XMG_PREC_FP64 && p->emulatable[i];
 		(want_emu ? dp->emu : dp->plain).push_back(i);
 	}
+	if (plain_is_faster(p, dp->emu)) {
+		dp->plain.insert(dp->plain.end(), dp->emu.begin(), dp->emu.end());
+		dp->emu.clear();
+	}
 	if (!scale.empty()) {
 		dp->n_scale = (int)scale.size();
 		if ((st = xmgd_ptask_stage(scale.data(), dp->n_scale, dp->dtype,
@@ -337,7 +370,8 @@ run_segment(xmgd_plan *dp, int seg, segment &g)
 
 	if (seg_empty(dp, seg))
 		return XMG_OK;
-	if (!graphs_enabled() || dp->one_shot)
+	/* (the plain GEMM is one kernel: a graph of it costs more to launch) */
+	if (!graphs_enabled() || dp->one_shot || seg == 2)
 		return record(dp, seg);
 	if (!g.x && (st = capture(dp, seg, g)))
 		return st;
@@ -363,22 +397,28 @@ xmgd_plan_run(xmgd_plan *dp, int *precision_used)
 			drop_graphs(dp);
 		cand = emu_current(dp->ep);
 	}
+	/* an event after each segment that launches anything */
+	int at[4] = {0, 0, 0, 0};
 	XMG_CK(cudaEventRecord(dp->ev[0], stream()));
-	if ((st = run_segment(dp, 0, dp->seg0[cand])))
+	for (int seg = 0; seg < 3; seg++) {
+		at[seg + 1] = at[seg];
+		if (seg_empty(dp, seg))
+			continue;
+		if ((st = run_segment(dp, seg, seg == 0 ? dp->seg0[cand] :
+		    seg == 1 ? dp->seg1[cand] : dp->seg2)))
+			return st;
+		at[seg + 1] = seg + 1;
+		XMG_CK(cudaEventRecord(dp->ev[seg + 1], stream()));
+	}
+	if ((st = check(cudaEventSynchronize(dp->ev[at[3]]), "contraction kernels")))
 		return st;
-	XMG_CK(cudaEventRecord(dp->ev[1], stream()));
-	if ((st = run_segment(dp, 1, dp->seg1[cand])))
-		return st;
-	XMG_CK(cudaEventRecord(dp->ev[2], stream()));
-	if ((st = run_segment(dp, 2, dp->seg2)))
-		return st;
-	XMG_CK(cudaEventRecord(dp->ev[3], stream()));
-	if ((st = check(cudaEventSynchronize(dp->ev[3]), "contraction kernels")))
-		return st;
-	XMG_CK(cudaEventElapsedTime(&ms_split, dp->ev[0], dp->ev[1]));
-	XMG_CK(cudaEventElapsedTime(&ms_emu, dp->ev[1], dp->ev[2]));
-	XMG_CK(cudaEventElapsedTime(&ms_plain, dp->ev[2], dp->ev[3]));
-	XMG_CK(cudaEventElapsedTime(&ms, dp->ev[0], dp->ev[3]));
+	float *const took[3] = {&ms_split, &ms_emu, &ms_plain};
+	for (int seg = 0; seg < 3; seg++) {
+		if (at[seg + 1] > at[seg])
+			XMG_CK(cudaEventElapsedTime(took[seg], dp->ev[at[seg]],
+			    dp->ev[at[seg + 1]]));
+		ms += *took[seg];
+	}
 	g_timing.ms_total = ms;
 	if (dp->ep) {
 		const bool was_tuned = emu_tuned(dp->ep);

@@ -835,6 +835,7 @@ xmg_contract(xm_scalar_t alpha, const xm_tensor_t *a, const xm_tensor_t *b,
 		goto out;
 	}
 	fill_contract(&dp, &p, alpha, beta, prec);
+	dp.in_core = xmg_alloc_is_device(c->allocator);
 	if ((st = xmgd_plan_create(&dp, &h)) != XMG_OK) {
 		st = xmg_commit_c(c, st);
 		goto out;

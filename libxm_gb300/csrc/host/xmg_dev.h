@@ -148,6 +148,7 @@ typedef struct {
 	double flops;                /* useful flops (reference counting) */
 	const uint8_t *emulatable;   /* per cblock: every pair factor +-2^t */
 	int precision_used;          /* out: XMG_PREC_FP64 / XMG_PREC_EMU64 */
+	int in_core;                 /* the whole contraction, in GPU memory */
 	int one_shot;                /* the plan runs once (an out-of-core
 	                                batch): no graphs, no tuning runs */
 	/* a's split-precision operands shared by the batches of a streamed
