@@ -117,12 +117,15 @@ static void
 strides_of(const struct xmg_block *b, size_t nd, const int64_t *dims,
     int64_t *st)
 {
-	int64_t cs[XM_MAX_DIM], acc = 1;
+	int64_t cd[XM_MAX_DIM], cs[XM_MAX_DIM], acc = 1;
 	size_t k;
 
+	/* dimension k of the block is dimension perm[k] of its source */
+	for (k = 0; k < nd; k++)
+		cd[b->perm.i[k]] = dims[k];
 	for (k = 0; k < nd; k++) {
 		cs[k] = acc;
-		acc *= dims[b->perm.i[k]];
+		acc *= cd[k];
 	}
 	for (k = 0; k < nd; k++)
 		st[k] = cs[b->perm.i[k]];
