@@ -6,6 +6,9 @@
 #include <cuComplex.h>
 #include <stdint.h>
 
+#include <utility>
+#include <vector>
+
 #include "div.cuh"
 #include "xmg_dev.h"
 #include "xmg.h"
@@ -21,6 +24,21 @@ cudaStream_t stream();          /* engine compute stream */
 int fork_aux(cudaStream_t *aux);
 int join_aux();
 int device();                   /* engine device ordinal */
+
+/* Arrays that go to the device together: one allocation, one copy.  add()
+ * takes a copy of the data (none: the space is only reserved) and the
+ * address of the pointer that commit() sets. */
+class upload_batch {
+	std::vector<char> h;
+	std::vector<std::pair<size_t, uint64_t *>> at;
+public:
+	void add(const void *data, size_t bytes, uint64_t *dst);
+	int commit(uint64_t *base);
+};
+/* Two page-locked ints for a plan's flags, from a small pool: page-locking
+ * memory for each plan costs more than planning a small contraction. */
+int flag_pair(int **p);
+void flag_pair_release(int *p);
 int num_sms();
 int check(cudaError_t e, const char *what);
 extern long long g_launches;     /* kernels launched by the engine */

@@ -71,6 +71,8 @@ struct xmgd_plan {
 	std::vector<xmgd_pair_t> prs;
 	std::vector<int> emu, plain;
 	uint64_t d_cbs = 0, d_prs = 0, d_tabs = 0;
+	uint64_t dbuf = 0;                   /* the allocation of these three */
+	bool ran = false;
 	xmgd_ptask_batch_t scale = {};       /* staged beta-only tasks */
 	int n_scale = 0;
 	uint64_t d_pg = 0;                   /* plain GEMM work list */
@@ -229,7 +231,7 @@ xmgd_plan_free(xmgd_plan *dp)
 	cudaStreamSynchronize(stream());
 	drop_graphs(dp);
 	emu_free(dp->ep);
-	uint64_t bufs[] = {dp->d_cbs, dp->d_prs, dp->d_tabs, dp->scale.dbuf, dp->d_pg};
+	uint64_t bufs[] = {dp->dbuf, dp->scale.dbuf, dp->d_pg};
 	for (uint64_t b : bufs)
 		if (b)
 			xmgd_free(b);
@@ -239,24 +241,12 @@ xmgd_plan_free(xmgd_plan *dp)
 	delete dp;
 }
 
-static int
-upload(const void *h, size_t bytes, uint64_t *d)
-{
-	int st;
-
-	if ((st = xmgd_alloc(bytes ? bytes : 16, d)) != XMG_OK)
-		return st;
-	if (bytes)
-		XMG_CK(cudaMemcpyAsync((void *)*d, h, bytes, cudaMemcpyHostToDevice,
-		    stream()));
-	return XMG_OK;
-}
-
 extern "C" int
 xmgd_plan_create(const xmgd_contract_t *p, xmgd_plan **out)
 {
 	xmgd_plan *dp = new xmgd_plan();
 	std::vector<xmgd_ptask_t> scale;
+	upload_batch up;	/* (its copy is waited for at the end) */
 	int st;
 
 	*out = nullptr;
@@ -270,11 +260,13 @@ xmgd_plan_create(const xmgd_contract_t *p, xmgd_plan **out)
 	for (int i = 0; i < 4; i++)
 		if ((st = check(cudaEventCreate(&dp->ev[i]), "event")))
 			goto fail;
-	if ((st = upload(p->cblocks, (size_t)p->ncblocks * sizeof(xmgd_cblock_t),
-	    &dp->d_cbs)) || (st = upload(p->pairs, (size_t)p->npairs *
-	    sizeof(xmgd_pair_t), &dp->d_prs)) || (st = upload(p->tabs,
-	    (size_t)p->ntabs * sizeof(int32_t), &dp->d_tabs)))
-		goto fail;
+	{
+		up.add(p->cblocks, (size_t)p->ncblocks * sizeof(xmgd_cblock_t), &dp->d_cbs);
+		up.add(p->pairs, (size_t)p->npairs * sizeof(xmgd_pair_t), &dp->d_prs);
+		up.add(p->tabs, (size_t)p->ntabs * sizeof(int32_t), &dp->d_tabs);
+		if ((st = up.commit(&dp->dbuf)))
+			goto fail;
+	}
 
 	/* route the output blocks */
 	for (int i = 0; i < p->ncblocks; i++) {
@@ -370,8 +362,10 @@ run_segment(xmgd_plan *dp, int seg, segment &g)
 
 	if (seg_empty(dp, seg))
 		return XMG_OK;
-	/* (the plain GEMM is one kernel: a graph of it costs more to launch) */
-	if (!graphs_enabled() || dp->one_shot || seg == 2)
+	/* a graph pays from the third launch on: a plan's first run, its tuning
+	 * runs and the plain GEMM, one kernel, launch directly */
+	if (!graphs_enabled() || dp->one_shot || seg == 2 || !dp->ran ||
+	    (dp->ep && !emu_tuned(dp->ep)))
 		return record(dp, seg);
 	if (!g.x && (st = capture(dp, seg, g)))
 		return st;
@@ -412,6 +406,7 @@ xmgd_plan_run(xmgd_plan *dp, int *precision_used)
 	}
 	if ((st = check(cudaEventSynchronize(dp->ev[at[3]]), "contraction kernels")))
 		return st;
+	dp->ran = true;
 	float *const took[3] = {&ms_split, &ms_emu, &ms_plain};
 	for (int seg = 0; seg < 3; seg++) {
 		if (at[seg + 1] > at[seg])

@@ -1501,6 +1501,8 @@ struct emu_plan {
 	int64_t nctas[2][2] = {{0, 0}, {0, 0}};
 	int kr[2] = {256, 256};              /* exponent pass: K per CTA */
 	uint64_t d_E = 0, d_F = 0;
+	uint64_t dbuf = 0;                   /* the allocation of all of these */
+	std::vector<xmgd_view_t> vstage;     /* bound views on their way up */
 	int64_t nE = 0;
 	int32_t nexp_a = 0;
 	size_t slice_bytes = 0;
@@ -1655,37 +1657,14 @@ set_attrs()
 	return XMG_OK;
 }
 
-static int
-upload_new(const void *h, size_t bytes, uint64_t *d)
-{
-	int st;
-
-	if ((st = xmgd_alloc(bytes ? bytes : 16, d)) != XMG_OK)
-		return st;
-	if (bytes)
-		XMG_CK(cudaMemcpyAsync((void *)*d, h, bytes, cudaMemcpyHostToDevice,
-		    stream()));
-	return XMG_OK;
-}
-
 void
 emu_free(emu_plan *e)
 {
 	if (!e)
 		return;
-	uint64_t bufs[] = {e->d_va, e->d_vb, e->d_meta[0][0], e->d_meta[0][1],
-	    e->d_meta[1][0], e->d_meta[1][1], e->d_E, e->d_F};
-	for (uint64_t b : bufs)
-		if (b)
-			xmgd_free(b);
-	for (emu_cand &c : e->cand) {
-		if (c.d_items)
-			xmgd_free(c.d_items);
-		if (c.d_members)
-			xmgd_free(c.d_members);
-	}
-	if (e->h_flags)
-		cudaFreeHost(e->h_flags);
+	if (e->dbuf)
+		xmgd_free(e->dbuf);
+	flag_pair_release(e->h_flags);
 	delete e;
 }
 
@@ -2149,6 +2128,7 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 	tile(e->VB, e->useB, nullptr);
 	e->slice_bytes = off;
 
+	upload_batch up;
 	/* CTA ranges of the exponent and split launches of each side */
 	for (int side = 0; side < 2; side++) {
 		std::vector<xmgd_view_t> &V = side ? e->VB : e->VA;
@@ -2177,18 +2157,15 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 					n += (int64_t)V[v].n_rt * ((V[v].n_ks + 3) / 4);
 			}
 			e->nctas[side][kind] = n;
-			if ((st = upload_new(meta.data(), meta.size() * sizeof(view_meta),
-			    &e->d_meta[side][kind])))
-				goto fail;
+			up.add(meta.data(), meta.size() * sizeof(view_meta), &e->d_meta[side][kind]);
 		}
 	}
 	e->nexp_a = p->nexp_a;
 	e->nE = (int64_t)p->nexp_a + p->nexp_b;
-	if ((st = xmgd_alloc((e->nE + 64) * sizeof(int32_t), &e->d_E)) ||
-	    (st = upload_new(F.data(), F.size() * sizeof(int32_t), &e->d_F)) ||
-	    (st = xmgd_alloc(e->VA.size() * sizeof(xmgd_view_t) + 16, &e->d_va)) ||
-	    (st = xmgd_alloc(e->VB.size() * sizeof(xmgd_view_t) + 16, &e->d_vb)))
-		goto fail;
+	up.add(nullptr, (e->nE + 64) * sizeof(int32_t), &e->d_E);
+	up.add(F.data(), F.size() * sizeof(int32_t), &e->d_F);
+	/* (the views go up when bound: one array, a's then b's) */
+	up.add(nullptr, (e->VA.size() + e->VB.size()) * sizeof(xmgd_view_t) + 16, &e->d_va);
 
 	/* work lists: a remembered policy for this histogram, else every
 	 * distinct policy once */
@@ -2255,20 +2232,20 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 		std::stable_sort(ord.begin(), ord.end(),
 		    [&](int x, int y) { return est[x] < est[y]; });
 		std::vector<emu_cand> keep;
-		for (int i : ord) {
-			if (!keep.empty() && (first_only || est[i] > 1.25 * est[ord[0]]))
-				continue;
-			emu_cand c = e->cand[i];
-			if ((st = upload_new(lists[i].data(), lists[i].size() * sizeof(emu_item),
-			    &c.d_items)) || (st = upload_new(mlists[i].data(), mlists[i].size() *
-			    sizeof(emu_member), &c.d_members))) {
-				keep.push_back(c);	/* freed with the plan */
-				e->cand = keep;
-				goto fail;
+		std::vector<int> kept;
+		for (int i : ord)
+			if (keep.empty() || !(first_only || est[i] > 1.25 * est[ord[0]])) {
+				keep.push_back(e->cand[i]);
+				kept.push_back(i);
 			}
-			keep.push_back(c);
-		}
 		e->cand = keep;
+		for (size_t i = 0; i < kept.size(); i++) {
+			const int l = kept[i];
+			up.add(lists[l].data(), lists[l].size() * sizeof(emu_item),
+			    &e->cand[i].d_items);
+			up.add(mlists[l].data(), mlists[l].size() * sizeof(emu_member),
+			    &e->cand[i].d_members);
+		}
 	}
 	if (e->cand.empty()) {
 		st = xmg_seterr(XMG_EINVAL, "split-precision path: no work list "
@@ -2276,9 +2253,10 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 		goto fail;
 	}
 	e->tuned = e->cand.size() <= 1;
-	if ((st = check(cudaMallocHost(&e->h_flags, 2 * sizeof(int)), "flags")) ||
+	if ((st = flag_pair(&e->h_flags)) || (st = up.commit(&e->dbuf)) ||
 	    (st = check(cudaStreamSynchronize(stream()), "plan upload")))
 		goto fail;
+	e->d_vb = e->d_va + e->VA.size() * sizeof(xmgd_view_t);
 	e->h_flags[0] = e->h_flags[1] = 0;
 	}
 	*out = e;
@@ -2301,17 +2279,16 @@ emu_bind(emu_plan *e, bool *moved)
 		return st;
 	if (ws == e->ws)
 		return XMG_OK;
-	for (int side = 0; side < 2; side++) {
-		std::vector<xmgd_view_t> V = side ? e->VB : e->VA;
-		std::vector<char> &use = side ? e->useB : e->useA;
-		const uint64_t base = side == 0 && e->a_mode ? e->a_slices : ws;
-		for (size_t v = 0; v < V.size(); v++)
-			if (use[v])
-				V[v].slices += base;
-		XMG_CK(cudaMemcpyAsync((void *)(side ? e->d_vb : e->d_va), V.data(),
-		    V.size() * sizeof(xmgd_view_t), cudaMemcpyHostToDevice, stream()));
-		XMG_CK(cudaStreamSynchronize(stream()));
+	e->vstage = e->VA;
+	e->vstage.insert(e->vstage.end(), e->VB.begin(), e->VB.end());
+	for (size_t v = 0; v < e->vstage.size(); v++) {
+		const bool isa = v < e->VA.size();
+		if (isa ? e->useA[v] : e->useB[v - e->VA.size()])
+			e->vstage[v].slices += isa && e->a_mode ? e->a_slices : ws;
 	}
+	/* (the staged copy lives as long as the plan) */
+	XMG_CK(cudaMemcpyAsync((void *)e->d_va, e->vstage.data(), e->vstage.size() *
+	    sizeof(xmgd_view_t), cudaMemcpyHostToDevice, stream()));
 	e->ws = ws;
 	*moved = true;
 	return XMG_OK;

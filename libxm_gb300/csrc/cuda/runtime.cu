@@ -8,6 +8,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <mutex>
 #include <vector>
 
 #include "common.cuh"
@@ -36,6 +37,60 @@ static bool g_side_rec[XMGD_SIDE_SLOTS];
 static buf g_chunk[XMGD_SIDE_SLOTS];
 
 cudaStream_t stream() { return g_stream; }
+
+void
+upload_batch::add(const void *data, size_t bytes, uint64_t *dst)
+{
+	const size_t o = (h.size() + 255) & ~(size_t)255;
+
+	h.resize(o + bytes);
+	if (data && bytes)
+		memcpy(h.data() + o, data, bytes);
+	at.push_back({o, dst});
+}
+
+int
+upload_batch::commit(uint64_t *base)
+{
+	int st;
+
+	*base = 0;
+	if ((st = xmgd_alloc(h.size() + 256, base)) != XMG_OK)
+		return st;
+	XMG_CK(cudaMemcpyAsync((void *)(uintptr_t)*base, h.data(), h.size(),
+	    cudaMemcpyHostToDevice, g_stream));
+	for (const auto &x : at)
+		*x.second = *base + x.first;
+	return XMG_OK;
+}
+
+static std::mutex g_flag_lock;
+static std::vector<int *> g_flag_free;
+
+int
+flag_pair(int **p)
+{
+	std::lock_guard<std::mutex> l(g_flag_lock);
+
+	if (g_flag_free.empty()) {
+		void *page;
+		XMG_CK(cudaMallocHost(&page, 4096));
+		for (int i = 0; i < 64; i++)	/* a cache line each */
+			g_flag_free.push_back((int *)((char *)page + 64 * i));
+	}
+	*p = g_flag_free.back();
+	g_flag_free.pop_back();
+	return XMG_OK;
+}
+
+void
+flag_pair_release(int *p)
+{
+	std::lock_guard<std::mutex> l(g_flag_lock);
+
+	if (p)
+		g_flag_free.push_back(p);
+}
 
 int
 fork_aux(cudaStream_t *aux)

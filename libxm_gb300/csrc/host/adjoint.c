@@ -140,36 +140,64 @@ letter(const char *s, char ch)
 	return p != NULL && ch != '\0' ? (int)(p - s) : -1;
 }
 
-/* Block of operand o (letters io) at target position v (letters it) and
- * summed block indices u (in o's dims; the target's letters are taken
- * from v). */
-static xm_dim_t
-operand_block(const char *io, const char *it, xm_dim_t v, xm_dim_t u)
-{
-	size_t j;
+/* A tensor's block table in the words the checks compare: canonical source
+ * (linear index + 1, 0 for a zero block) and permutation, four bits each. */
+struct bcode {
+	size_t src;
+	uint32_t perm;
+};
 
-	for (j = 0; j < u.n; j++) {
-		int k = letter(it, io[j]);
-		if (k >= 0)
-			u.i[j] = v.i[k];
+static struct bcode *
+block_codes(const xm_tensor_t *t)
+{
+	struct bcode *c = malloc(t->nblocks_total * sizeof *c);
+	size_t i, k;
+
+	if (c == NULL)
+		xm_fatal("%s: out of memory", __func__);
+	for (i = 0; i < t->nblocks_total; i++) {
+		const struct xmg_block *b = &t->blocks[i];
+		c[i].src = b->type == XM_BLOCK_TYPE_ZERO ? 0 :
+		    (b->type == XM_BLOCK_TYPE_CANONICAL ? i : (size_t)b->data) + 1;
+		c[i].perm = 0;
+		for (k = 0; k < b->perm.n; k++)
+			c[i].perm |= (uint32_t)b->perm.i[k] << (4 * k);
 	}
-	return u;
+	return c;
 }
 
-/* canonical source (linear index) and element strides of block z of t;
- * 0 for a zero block */
-static int
-block_map(const xm_tensor_t *t, xm_dim_t z, size_t *src, int64_t *str,
-    xm_scalar_t *sc)
+/* block index of a linear position (index 0 fastest) */
+static xm_dim_t
+unlinear(const xm_tensor_t *t, size_t lin)
 {
-	struct xmg_block *b = xmg_tensor_block(t, z);
+	xm_dim_t nb = xm_block_space_get_nblocks(t->bs), r = xm_dim_zero(nb.n);
+	size_t k;
 
-	if (b->type == XM_BLOCK_TYPE_ZERO)
-		return 0;
-	*src = b->type == XM_BLOCK_TYPE_CANONICAL ?
-	    xmg_tensor_block_linear(t, z) : (size_t)b->data;
-	*sc = b->scalar;
-	xmg_tensor_block_strides(t, z, str);
+	for (k = 0; k < nb.n; k++) {
+		r.i[k] = lin % nb.i[k];
+		lin /= nb.i[k];
+	}
+	return r;
+}
+
+/* Blocks z and zq of t (linear positions, same canonical source), z's
+ * dimension j beside zq's jj[j]: same extents and element strides (of
+ * extents above 1). */
+static int
+same_strides(const xm_tensor_t *t, size_t z, size_t zq, const int *jj)
+{
+	xm_dim_t iz = unlinear(t, z), iq = unlinear(t, zq), dz, dq;
+	int64_t sz[XM_MAX_DIM], sq[XM_MAX_DIM];
+	size_t j;
+
+	dz = xm_block_space_get_block_dims(t->bs, iz);
+	dq = xm_block_space_get_block_dims(t->bs, iq);
+	xmg_tensor_block_strides(t, iz, sz);
+	xmg_tensor_block_strides(t, iq, sq);
+	for (j = 0; j < dz.n; j++)
+		if (dz.i[j] != dq.i[jj[j]] ||
+		    (dz.i[j] > 1 && sz[j] != sq[jj[j]]))
+			return 0;
 	return 1;
 }
 
@@ -178,90 +206,111 @@ block_map(const xm_tensor_t *t, xm_dim_t z, size_t *src, int64_t *str,
 #define EQV_EMPTY  2	/* no nonzero term at p or q */
 
 /* Equivariance of T = X * Y at derivative position p of T (letters it,
- * ix, iy); *sigma on EQV_YES. */
+ * ix, iy; codes of x's and y's blocks); *sigma on EQV_YES. */
 static int
 equivariant(const xm_tensor_t *t, const char *it, const xm_tensor_t *x,
-    const char *ix, const xm_tensor_t *y, const char *iy, xm_dim_t p,
-    xm_scalar_t *sigma)
+    const char *ix, const struct bcode *cx, const xm_tensor_t *y,
+    const char *iy, const struct bcode *cy, xm_dim_t p, xm_scalar_t *sigma)
 {
 	struct xmg_block *bp = xmg_tensor_block(t, p);
 	const xm_tensor_t *op[2] = { x, y };
 	const char *io[2] = { ix, iy };
-	xm_dim_t nbt = xm_block_space_get_nblocks(t->bs), q, nbx, u[2];
-	int sl[XM_MAX_DIM], ns = 0, have = 0;
-	size_t cnt[XM_MAX_DIM], cur[XM_MAX_DIM], k, j, lin;
+	const struct bcode *code[2] = { cx, cy };
+	xm_dim_t q = unlinear(t, (size_t)bp->data), nb;
+	/* per operand: linear positions at p and q (summed letters at 0),
+	 * step per summed letter, dimensions, zq's dimension beside z's */
+	size_t lz[2] = { 0, 0 }, lq[2] = { 0, 0 }, step[2][XM_MAX_DIM];
+	size_t cnt[XM_MAX_DIM], cur[XM_MAX_DIM], nd[2], k, j, st;
+	int jj[2][XM_MAX_DIM], bad[2] = { 0, 0 }, ns = 0, have = 0, o;
+	uint32_t map[2] = { 0, 0 };
 	xm_scalar_t s0 = 0;
 
-	/* q from the linear source index; block indices related like the
-	 * element indices; letter classes kept */
-	q = xm_dim_zero(nbt.n);
-	for (lin = (size_t)bp->data, k = 0; k < nbt.n; k++) {
-		q.i[k] = lin % nbt.i[k];
-		lin /= nbt.i[k];
-	}
-	for (k = 0; k < nbt.n; k++) {
+	/* block indices related like the element indices; letter classes
+	 * kept */
+	for (k = 0; k < p.n; k++) {
 		size_t pk = bp->perm.i[k];
 		if (p.i[k] != q.i[pk] ||
 		    (letter(ix, it[k]) >= 0) != (letter(ix, it[pk]) >= 0))
 			return EQV_NO;
 	}
 	/* summed letters: in x and y, not in t */
-	nbx = xm_block_space_get_nblocks(x->bs);
-	for (j = 0; j < nbx.n; j++)
+	nb = xm_block_space_get_nblocks(x->bs);
+	for (j = 0; j < nb.n; j++)
 		if (letter(it, ix[j]) < 0 && letter(iy, ix[j]) >= 0) {
-			sl[ns] = (int)j;
-			cnt[ns] = nbx.i[j];
+			cnt[ns] = nb.i[j];
 			cur[ns++] = 0;
 		}
-	for (;;) {
-		int zero[2] = { 0, 0 };
-		xm_scalar_t ratio[2];
-		u[0] = xm_dim_zero(strlen(ix));
-		u[1] = xm_dim_zero(strlen(iy));
-		for (k = 0; k < (size_t)ns; k++) {
-			u[0].i[sl[k]] = cur[k];
-			u[1].i[letter(iy, ix[sl[k]])] = cur[k];
+	for (o = 0; o < 2; o++) {
+		int n = 0;
+		nb = xm_block_space_get_nblocks(op[o]->bs);
+		nd[o] = nb.n;
+		/* (the summed letters in x's order) */
+		for (j = 0; ix[j] != '\0'; j++)
+			if (letter(it, ix[j]) < 0 && letter(iy, ix[j]) >= 0) {
+				int at = letter(io[o], ix[j]);
+				for (st = 1, k = 0; k < (size_t)at; k++)
+					st *= nb.i[k];
+				step[o][n++] = st;
+			}
+		for (st = 1, j = 0; j < nb.n; st *= nb.i[j], j++) {
+			int kt = letter(it, io[o][j]);
+			jj[o][j] = kt < 0 ? (int)j :
+			    letter(io[o], it[bp->perm.i[kt]]);
+			if (jj[o][j] < 0)
+				bad[o] = 1;
+			else
+				map[o] |= (uint32_t)jj[o][j] << (4 * j);
+			if (kt >= 0) {
+				lz[o] += p.i[kt] * st;
+				lq[o] += q.i[kt] * st;
+			}
 		}
-		for (int o = 0; o < 2; o++) {
-			xm_dim_t z = operand_block(io[o], it, p, u[o]);
-			xm_dim_t zq = operand_block(io[o], it, q, u[o]);
-			xm_dim_t dz, dq;
-			int64_t sz[XM_MAX_DIM], sq[XM_MAX_DIM];
-			size_t src, srcq;
+	}
+	for (;;) {
+		int zero = 0;
+		xm_scalar_t s = 1;
+		for (o = 0; o < 2; o++) {
+			const struct bcode *z = &code[o][lz[o]];
+			const struct bcode *zq = &code[o][lq[o]];
 			xm_scalar_t cz, cq;
-			int nz = block_map(op[o], z, &src, sz, &cz);
-			int nq = block_map(op[o], zq, &srcq, sq, &cq);
 
-			if (nz != nq)
+			if (z->src != zq->src)
 				return EQV_NO;
-			if (!nz) {
-				zero[o] = 1;
+			if (z->src == 0) {
+				zero = 1;
 				continue;
 			}
-			if (src != srcq || cq == 0)
+			cz = op[o]->blocks[lz[o]].scalar;
+			cq = op[o]->blocks[lq[o]].scalar;
+			if (cq == 0 || bad[o])
 				return EQV_NO;
-			dz = xm_block_space_get_block_dims(op[o]->bs, z);
-			dq = xm_block_space_get_block_dims(op[o]->bs, zq);
-			for (j = 0; j < dz.n; j++) {
-				int kt = letter(it, io[o][j]);
-				int jj = kt < 0 ? (int)j :
-				    letter(io[o], it[bp->perm.i[kt]]);
-				if (jj < 0 || dz.i[j] != dq.i[jj] ||
-				    (dz.i[j] > 1 && sz[j] != sq[jj]))
-					return EQV_NO;
-			}
-			ratio[o] = cz / cq;
+			/* the same source dimension along each pair: extents
+			 * and strides agree; else compare them */
+			for (j = 0; j < nd[o]; j++)
+				if (((z->perm >> (4 * j)) & 15) !=
+				    ((zq->perm >> (4 * ((map[o] >> (4 * j)) & 15))) & 15))
+					break;
+			if (j < nd[o] && !same_strides(op[o], lz[o], lq[o], jj[o]))
+				return EQV_NO;
+			s *= cz == cq ? 1 : cz / cq;
 		}
-		if (!zero[0] && !zero[1]) {
-			xm_scalar_t s = ratio[0] * ratio[1];
+		if (!zero) {
 			if (have && s != s0)
 				return EQV_NO;
 			s0 = s;
 			have = 1;
 		}
 		for (k = 0; k < (size_t)ns; k++) {
+			for (o = 0; o < 2; o++) {
+				lz[o] += step[o][k];
+				lq[o] += step[o][k];
+			}
 			if (++cur[k] < cnt[k])
 				break;
+			for (o = 0; o < 2; o++) {
+				lz[o] -= cnt[k] * step[o][k];
+				lq[o] -= cnt[k] * step[o][k];
+			}
 			cur[k] = 0;
 		}
 		if (k == (size_t)ns)
@@ -278,20 +327,23 @@ forward_consistent(const xm_tensor_t *a, const xm_tensor_t *b,
     const xm_tensor_t *dc, const char *idxa, const char *idxb,
     const char *idxc)
 {
-	xm_dim_t nb = xm_block_space_get_nblocks(dc->bs), idx;
+	struct bcode *ca = block_codes(a), *cb = block_codes(b);
 	size_t i;
+	int ok = 1;
 
-	idx = xm_dim_zero(nb.n);
-	for (i = 0; i < dc->nblocks_total; i++, xm_dim_inc(&idx, &nb)) {
+	for (i = 0; i < dc->nblocks_total && ok; i++) {
 		xm_scalar_t sig;
 		int r;
 		if (dc->blocks[i].type != XM_BLOCK_TYPE_DERIVATIVE)
 			continue;
-		r = equivariant(dc, idxc, a, idxa, b, idxb, idx, &sig);
+		r = equivariant(dc, idxc, a, idxa, ca, b, idxb, cb,
+		    unlinear(dc, i), &sig);
 		if (r == EQV_NO || (r == EQV_YES && sig != dc->blocks[i].scalar))
-			return 0;
+			ok = 0;
 	}
-	return 1;
+	free(ca);
+	free(cb);
+	return ok;
 }
 
 /* Per-block factors m (indexed by t's linear block index; nonzero only
@@ -302,26 +354,30 @@ canonical_factors(const xm_tensor_t *t, const char *it,
     const xm_tensor_t *x, const char *ix, const xm_tensor_t *y,
     const char *iy, xm_scalar_t *m)
 {
-	xm_dim_t nb = xm_block_space_get_nblocks(t->bs), idx;
+	struct bcode *cx = block_codes(x), *cy = block_codes(y);
 	size_t i;
+	int ok = 1;
 
 	for (i = 0; i < t->nblocks_total; i++)
 		m[i] = t->blocks[i].type == XM_BLOCK_TYPE_CANONICAL ? 1 : 0;
-	idx = xm_dim_zero(nb.n);
-	for (i = 0; i < t->nblocks_total; i++, xm_dim_inc(&idx, &nb)) {
+	for (i = 0; i < t->nblocks_total && ok; i++) {
 		struct xmg_block *bp = &t->blocks[i];
 		xm_scalar_t sig;
 		int r;
 		if (bp->type != XM_BLOCK_TYPE_DERIVATIVE)
 			continue;
-		r = equivariant(t, it, x, ix, y, iy, idx, &sig);
-		if (r == EQV_NO)
-			return 0;
+		r = equivariant(t, it, x, ix, cx, y, iy, cy, unlinear(t, i), &sig);
+		if (r == EQV_NO) {
+			ok = 0;
+			break;
+		}
 		/* EQV_EMPTY: the gradient is zero at p and at q, any factor
 		 * serves; count the position like a consistent one */
 		m[bp->data] += r == EQV_YES ? bp->scalar * sig : 1;
 	}
-	return 1;
+	free(cx);
+	free(cy);
+	return ok;
 }
 
 /* dst_q += m_q * src_q for every canonical block q of t (dst and src on
@@ -368,29 +424,49 @@ scale_add_canonical(const xm_tensor_t *t, xm_tensor_t *dst,
 }
 
 /* Tensor on t's block space whose canonical blocks sit at t's canonical
- * positions only (or at every nonzero position of t), zero-filled. */
+ * positions only (or at every nonzero position of t).  In GPU memory its
+ * blocks share one allocation, *mem (an allocation per block costs more than
+ * the small gradients' kernels). */
 static xm_tensor_t *
-gradient_tensor(const xm_tensor_t *t, int all_nonzero)
+gradient_tensor(const xm_tensor_t *t, int all_nonzero, uint64_t *mem)
 {
 	xm_tensor_t *g = xm_tensor_create(t->bs, t->type, t->allocator);
-	xm_dim_t nb = xm_block_space_get_nblocks(t->bs), idx = xm_dim_zero(nb.n);
-	size_t i;
+	xm_dim_t nb = xm_block_space_get_nblocks(t->bs), idx;
+	size_t i, off;
+	int pass, one = xmg_alloc_is_device(t->allocator);
 
-	for (i = 0; i < t->nblocks_total; i++, xm_dim_inc(&idx, &nb)) {
-		if (t->blocks[i].type == XM_BLOCK_TYPE_CANONICAL ||
-		    (all_nonzero && t->blocks[i].type == XM_BLOCK_TYPE_DERIVATIVE))
-			xm_tensor_set_canonical_block(g, idx);
+	*mem = XM_NULL_PTR;
+	for (pass = one ? 0 : 1; pass < 2; pass++) {
+		idx = xm_dim_zero(nb.n);
+		off = 0;
+		for (i = 0; i < t->nblocks_total; i++, xm_dim_inc(&idx, &nb)) {
+			if (!(t->blocks[i].type == XM_BLOCK_TYPE_CANONICAL ||
+			    (all_nonzero && t->blocks[i].type ==
+			    XM_BLOCK_TYPE_DERIVATIVE)))
+				continue;
+			if (pass == 1 && one)
+				xm_tensor_set_canonical_block_raw(g, idx, *mem + off);
+			else if (pass == 1)
+				xm_tensor_set_canonical_block(g, idx);
+			off += (xm_tensor_get_block_bytes(t, idx) + 511) & ~(size_t)511;
+		}
+		if (pass == 0 && off > 0 && (*mem = xm_allocator_allocate(
+		    t->allocator, off)) == XM_NULL_PTR)
+			xm_fatal("%s: unable to allocate block data", __func__);
 	}
 	return g;
 }
 
 static void
-drop(xm_tensor_t *t)
+drop(xm_tensor_t *t, uint64_t mem)
 {
-	if (t) {
+	if (t == NULL)
+		return;
+	if (mem != XM_NULL_PTR)
+		xm_allocator_deallocate(t->allocator, mem);
+	else
 		xm_tensor_free_block_data(t);
-		xm_tensor_free(t);
-	}
+	xm_tensor_free(t);
 }
 
 static int
@@ -417,6 +493,7 @@ struct adj_side {
 	int mode;
 	xm_scalar_t *m;		/* SIDE_SYM: factors per block of a (b) */
 	xm_tensor_t *g;		/* gradient at canonical or every position */
+	uint64_t mem;		/* its storage (gradient_tensor) */
 };
 
 static struct {
@@ -427,6 +504,7 @@ static struct {
 	char idx[3][XM_MAX_DIM + 1];
 	int fwd;		/* forward check: -1 not run, 0 failed, 1 passed */
 	xm_tensor_t *w;
+	uint64_t wmem;
 	struct adj_side s[2];	/* 0: a, 1: b */
 } g_adj = { .fwd = -1 };
 
@@ -435,9 +513,9 @@ xmg_adjoint_release(void)
 {
 	int k;
 
-	drop(g_adj.w);
+	drop(g_adj.w, g_adj.wmem);
 	for (k = 0; k < 2; k++) {
-		drop(g_adj.s[k].g);
+		drop(g_adj.s[k].g, g_adj.s[k].mem);
 		free(g_adj.s[k].m);
 	}
 	memset(&g_adj, 0, sizeof g_adj);
@@ -555,7 +633,7 @@ xm_contract_adjoint(xm_scalar_t alpha, const xm_tensor_t *a,
 			/* G = alpha * (dc * b) or alpha * (a * dc) at t's
 			 * canonical positions; d_q += m_q G_q */
 			if (sd->g == NULL)
-				sd->g = gradient_tensor(t, 0);
+				sd->g = gradient_tensor(t, 0, &sd->mem);
 			st = k == 0 ?
 			    xmg_contract(alpha, dc, b, 0, sd->g, idxc, idxb, idxa) :
 			    xmg_contract(alpha, a, dc, 0, sd->g, idxa, idxc, idxb);
@@ -567,7 +645,7 @@ xm_contract_adjoint(xm_scalar_t alpha, const xm_tensor_t *a,
 		 * share their block structure; the structure tensor is dc) */
 		if (!w_ready) {
 			if (g_adj.w == NULL)
-				g_adj.w = gradient_tensor(dc, 0);
+				g_adj.w = gradient_tensor(dc, 0, &g_adj.wmem);
 			if ((st = xmg_set(g_adj.w, 0)) != XMG_OK ||
 			    (st = fold_onto_canonical(dc, g_adj.w, dc, 1)) !=
 			    XMG_OK)
@@ -575,7 +653,7 @@ xm_contract_adjoint(xm_scalar_t alpha, const xm_tensor_t *a,
 			w_ready = 1;
 		}
 		if (sd->g == NULL)
-			sd->g = gradient_tensor(t, 1);
+			sd->g = gradient_tensor(t, 1, &sd->mem);
 		st = k == 0 ?
 		    xmg_contract(alpha, g_adj.w, b, 0, sd->g, idxc, idxb, idxa) :
 		    xmg_contract(alpha, a, g_adj.w, 0, sd->g, idxa, idxc, idxb);

@@ -248,8 +248,8 @@ pow2_factor(xm_scalar_t s, int *sign, int *shift)
 }
 
 struct cand {
-	xm_dim_t ia, ib;
-	const struct xmg_block *pa, *pb;    /* the blocks at ia, ib */
+	size_t la, lb;                      /* linear block positions */
+	const struct xmg_block *pa, *pb;    /* the blocks there */
 	xm_scalar_t al;
 	uint64_t da, db;
 };
@@ -357,6 +357,116 @@ k_order(const xm_dim_t *cidxa, const xm_dim_t *cidxb, const int64_t *sa,
 	}
 }
 
+/*
+ * What the plan needs of one operand block: shape and strides, the offset
+ * table and exponent slot of its free indices, and per order of the
+ * contracted ones (at most two in practice) the row table and view.  A
+ * block takes part in many pairs; its tables are looked up once.
+ */
+struct opblock {
+	xm_dim_t dims;
+	int64_t st[XM_MAX_DIM], size;
+	uint64_t ptr;
+	int32_t col, e;
+	int norder;
+	uint32_t order[2];
+	int32_t row[2], view[2];
+};
+
+struct opcache {
+	const xm_tensor_t *t;
+	const xm_dim_t *freemask;
+	int32_t *at;                        /* entry + 1 per block position */
+	struct opblock *v;
+	int n, cap;
+};
+
+static void
+opcache_init(struct opcache *c, const xm_tensor_t *t, const xm_dim_t *freemask)
+{
+	memset(c, 0, sizeof *c);
+	c->t = t;
+	c->freemask = freemask;
+	if ((c->at = calloc(t->nblocks_total, sizeof *c->at)) == NULL)
+		xm_fatal("%s: out of memory", __func__);
+}
+
+static void
+opcache_free(struct opcache *c)
+{
+	free(c->at);
+	free(c->v);
+}
+
+/* Block `lin` of the operand; *err receives a status.  The entry stays valid
+ * until the next call. */
+static struct opblock *
+opblock_get(struct opcache *c, size_t lin, uint64_t handle, plan_t *p,
+    xmg_hmap_t *eindex, int32_t *nexp, int32_t ncols, int device, int *err)
+{
+	xm_dim_t nb, idx;
+	struct opblock *o;
+	size_t k, r = lin;
+
+	*err = XMG_OK;
+	if (c->at[lin] != 0)
+		return &c->v[c->at[lin] - 1];
+	if (c->n == c->cap) {
+		c->cap = c->cap ? 2 * c->cap : 64;
+		if ((c->v = realloc(c->v, (size_t)c->cap * sizeof *c->v)) == NULL)
+			xm_fatal("%s: out of memory", __func__);
+	}
+	nb = xm_block_space_get_nblocks(c->t->bs);
+	idx = xm_dim_zero(nb.n);
+	for (k = 0; k < nb.n; k++) {
+		idx.i[k] = r % nb.i[k];
+		r /= nb.i[k];
+	}
+	o = &c->v[c->n++];
+	memset(o, 0, sizeof *o);
+	c->at[lin] = c->n;
+	o->dims = xm_block_space_get_block_dims(c->t->bs, idx);
+	o->size = (int64_t)xm_dim_dot(&o->dims);
+	xmg_tensor_block_strides(c->t, idx, o->st);
+	if (o->size > INT32_MAX || !device)
+		return o;
+	o->col = mask_table(&p->tabs, &o->dims, o->st, c->freemask);
+	o->e = exp_slot(eindex, nexp, c->t, idx, c->freemask, ncols);
+	o->ptr = handle;
+	if (device == 1)
+		*err = xmg_alloc_device_view(c->t->allocator, handle,
+		    xm_tensor_get_block_bytes(c->t, idx), &o->ptr);
+	return o;
+}
+
+/* Row table and view of a block for contracted indices in the order `ord`. */
+static void
+opblock_rows(struct opblock *o, plan_t *p, const xm_dim_t *ord,
+    xmgd_view_t **views, int *n, int *cap, xmg_hmap_t *index, int32_t k,
+    int32_t mn, int32_t *row, int32_t *view)
+{
+	uint32_t code = 0;
+	size_t q;
+	int i;
+
+	for (q = 0; q < ord->n; q++)
+		code |= (uint32_t)ord->i[q] << (4 * q);
+	for (i = 0; i < o->norder; i++)
+		if (o->order[i] == code) {
+			*row = o->row[i];
+			*view = o->view[i];
+			return;
+		}
+	*row = mask_table(&p->tabs, &o->dims, o->st, ord);
+	*view = view_id(views, n, cap, index, o->ptr, k, mn, *row, o->col, o->e);
+	if (o->norder < 2) {
+		i = o->norder++;
+		o->order[i] = code;
+		o->row[i] = *row;
+		o->view[i] = *view;
+	}
+}
+
 double
 xmg_now_ms(void)
 {
@@ -424,12 +534,13 @@ xmg_plan_build(xm_scalar_t alpha, const xm_tensor_t *a, const xm_tensor_t *b,
 	/* device: 0 pairs only; 1 the full device plan (blocks staged);
 	 * 2 the full structure with data handles in place of device
 	 * addresses (no device needed: work-list checks) */
-	xm_dim_t *list, nba, nbb, blkc, ia, ib, dims, dA, dB, ka, kb;
+	xm_dim_t *list, nba, nbb, blkc, ia, ib, dims, ka, kb;
+	struct opcache oca, ocb;
+	struct opblock *oa, *ob;
 	size_t nlist, nblkk, l, i, la, lb, sta[XM_MAX_DIM], stb[XM_MAX_DIM];
 	struct cand *cand = NULL;
 	xmg_hmap_t merge;
-	int64_t sa[XM_MAX_DIM], sb[XM_MAX_DIM], sc[XM_MAX_DIM];
-	int32_t arow, acol, brow, bcol, ea = 0, eb = 0;
+	int64_t sc[XM_MAX_DIM];
 	struct xmg_block *ba, *bb;
 	uint64_t rep, dptr;
 	xmgd_cblock_t *cb;
@@ -449,6 +560,8 @@ xmg_plan_build(xm_scalar_t alpha, const xm_tensor_t *a, const xm_tensor_t *b,
 	if (nblkk > 0 && (cand = malloc(nblkk * sizeof *cand)) == NULL)
 		xm_fatal("%s: out of memory", __func__);
 	xmg_hmap_init(&merge);
+	opcache_init(&oca, a, &p->aidxa);
+	opcache_init(&ocb, b, &p->aidxb);
 	for (l = 0; l < nlist && st == XMG_OK; l++) {
 		blkc = list[l];
 		dims = xm_block_space_get_block_dims(c->bs, blkc);
@@ -488,8 +601,8 @@ xmg_plan_build(xm_scalar_t alpha, const xm_tensor_t *a, const xm_tensor_t *b,
 		for (i = 0; i < nblkk; i++) {
 			ba = &a->blocks[la];
 			bb = &b->blocks[lb];
-			cand[i].ia = ia;
-			cand[i].ib = ib;
+			cand[i].la = la;
+			cand[i].lb = lb;
 			cand[i].pa = ba;
 			cand[i].pb = bb;
 			cand[i].al = 0;
@@ -525,6 +638,14 @@ xmg_plan_build(xm_scalar_t alpha, const xm_tensor_t *a, const xm_tensor_t *b,
 		for (i = 0; i < nblkk; i++) {
 			if (cand[i].al == 0)
 				continue;
+			oa = opblock_get(&oca, cand[i].la, cand[i].da, p,
+			    &p->ea_index, &p->nexp_a, cb->m, device, &st);
+			if (st != XMG_OK)
+				break;
+			ob = opblock_get(&ocb, cand[i].lb, cand[i].db, p,
+			    &p->eb_index, &p->nexp_b, cb->n, device, &st);
+			if (st != XMG_OK)
+				break;
 			if (p->collect) {
 				if (p->nbh == p->capbh) {
 					p->capbh = p->capbh ? 2 * p->capbh : 256;
@@ -534,11 +655,10 @@ xmg_plan_build(xm_scalar_t alpha, const xm_tensor_t *a, const xm_tensor_t *b,
 						xm_fatal("%s: out of memory", __func__);
 				}
 				p->bh[p->nbh] = cand[i].db;
-				p->bsz[p->nbh++] = xm_tensor_get_block_bytes(b, cand[i].ib);
+				p->bsz[p->nbh++] = (uint64_t)ob->size *
+				    xm_scalar_sizeof(b->type);
 			}
-			dA = xm_block_space_get_block_dims(a->bs, cand[i].ia);
-			dB = xm_block_space_get_block_dims(b->bs, cand[i].ib);
-			if (xm_dim_dot(&dA) > INT32_MAX || xm_dim_dot(&dB) > INT32_MAX) {
+			if (oa->size > INT32_MAX || ob->size > INT32_MAX) {
 				st = xmg_seterr(XMG_EINVAL, "xm_contract: a block of a "
 				    "or b has more than 2^31 - 1 elements");
 				break;
@@ -546,7 +666,7 @@ xmg_plan_build(xm_scalar_t alpha, const xm_tensor_t *a, const xm_tensor_t *b,
 			GROW(p->pr, p->npr, p->cappr);
 			pr = &p->pr[p->npr++];
 			memset(pr, 0, sizeof *pr);
-			pr->k = (int32_t)xm_dim_dot_mask(&dA, &p->cidxa);
+			pr->k = (int32_t)xm_dim_dot_mask(&oa->dims, &p->cidxa);
 			xmg_scalar_pack(xm_scalar_mul(alpha, cand[i].al, c->type),
 			    pr->al);
 			p->flops += mult * cb->m * (double)cb->n * pr->k;
@@ -558,36 +678,18 @@ xmg_plan_build(xm_scalar_t alpha, const xm_tensor_t *a, const xm_tensor_t *b,
 			}
 			if (!device)
 				continue;
-			xmg_tensor_block_strides(a, cand[i].ia, sa);
-			xmg_tensor_block_strides(b, cand[i].ib, sb);
-			k_order(&p->cidxa, &p->cidxb, sa, sb,
+			k_order(&p->cidxa, &p->cidxb, oa->st, ob->st,
 			    (int64_t)pr->k * cb->m, (int64_t)pr->k * cb->n, &ka, &kb);
-			arow = mask_table(&p->tabs, &dA, sa, &ka);
-			acol = mask_table(&p->tabs, &dA, sa, &p->aidxa);
-			brow = mask_table(&p->tabs, &dB, sb, &kb);
-			bcol = mask_table(&p->tabs, &dB, sb, &p->aidxb);
-			pr->arow = arow; pr->acol = acol;
-			pr->brow = brow; pr->bcol = bcol;
-			dptr = cand[i].da;
-			if (device == 1 && (st = xmg_alloc_device_view(a->allocator,
-			    cand[i].da, xm_tensor_get_block_bytes(a, cand[i].ia), &dptr)))
-				break;
-			pr->a_ptr = dptr;
-			dptr = cand[i].db;
-			if (device == 1 && (st = xmg_alloc_device_view(b->allocator,
-			    cand[i].db, xm_tensor_get_block_bytes(b, cand[i].ib), &dptr)))
-				break;
-			pr->b_ptr = dptr;
-			ea = exp_slot(&p->ea_index, &p->nexp_a, a, cand[i].ia,
-			    &p->aidxa, cb->m);
-			eb = exp_slot(&p->eb_index, &p->nexp_b, b, cand[i].ib,
-			    &p->aidxb, cb->n);
-			pr->aview = view_id(&p->va, &p->nva, &p->capva,
-			    &p->va_index, pr->a_ptr, pr->k, cb->m, arow, acol, ea);
-			pr->bview = view_id(&p->vb, &p->nvb, &p->capvb,
-			    &p->vb_index, pr->b_ptr, pr->k, cb->n, brow, bcol, eb);
-			cb->eA = ea;
-			cb->eB = eb;
+			opblock_rows(oa, p, &ka, &p->va, &p->nva, &p->capva,
+			    &p->va_index, pr->k, cb->m, &pr->arow, &pr->aview);
+			opblock_rows(ob, p, &kb, &p->vb, &p->nvb, &p->capvb,
+			    &p->vb_index, pr->k, cb->n, &pr->brow, &pr->bview);
+			pr->acol = oa->col;
+			pr->bcol = ob->col;
+			pr->a_ptr = oa->ptr;
+			pr->b_ptr = ob->ptr;
+			cb->eA = oa->e;
+			cb->eB = ob->e;
 		}
 next:
 		cb->npairs = p->npr - cb->first_pair;
@@ -595,6 +697,8 @@ next:
 		p->ncb++;
 	}
 	xmg_hmap_free(&merge);
+	opcache_free(&oca);
+	opcache_free(&ocb);
 	free(cand);
 	free(list);
 	if (st == XMG_OK && p->tabs.overflow)
