@@ -407,25 +407,26 @@ __device__ __forceinline__ bool pack_f64(long long V, int e, unsigned long long 
 }
 
 /* A pipeline stage holds KSTEPS consecutive 16-wide K steps (each the
- * M-side chunk then the N-side chunk).  The per-stage synchronisation of
- * the producer and MMA threads (barrier round trips, copy issue, commit)
- * weighs on the stage's MMAs, so both forms take several steps per stage.
- * The 3-slice form (6 MMAs per K step) three, in three stages of 72 KiB
- * (measured on the float32 ring term's GEMM: one step per stage 30.3-32.3
- * ms, two 27.8, three 27.0, four in two stages 26.5 with a one-stage head,
- * 32.6 with two); the 6-slice form (21 MMAs per step) two, in two stages
- * of 96 KiB (FP64 ring term 59.6 -> 56.5 ms, cfg2 ladder 32.4-32.9 ->
- * 32.0 ms, with a head and tail of both stages). */
+ * M-side chunk then the N-side chunk).  Smaller stages come back to the
+ * producer sooner and leave less of a chunk to its head and tail; the price
+ * is a barrier wait, a commit and the copies' arrival per stage.  With the
+ * producer and MMA warps in step (mma_bf16_split) a stage costs the MMAs
+ * nothing, and four stages of 48 KiB are best in both forms: one step of
+ * the 6-slice form (GEMM of a 24 x 64 ladder 118 us with two steps in two
+ * stages, 107 with one in four; 1.72 and 1.68 ms at 53 x 187; equal at 96 x
+ * 384), two steps of the 3-slice form (float32 ring term, 64 x 256: 19.9 ms
+ * with one step in eight stages, 19.2 with two in four, 19.8 with three in
+ * three). */
 template <int S>
 struct stage_cfg {
 #ifndef EMU_KSTEPS32
-#define EMU_KSTEPS32 3
+#define EMU_KSTEPS32 2
 #endif
 #ifndef EMU_BUDGET32
-#define EMU_BUDGET32 221184                   /* 3 stages of 72 KiB */
+#define EMU_BUDGET32 196608                   /* 4 stages of 48 KiB */
 #endif
 #ifndef EMU_KSTEPS64
-#define EMU_KSTEPS64 2                        /* 2 stages of 96 KiB */
+#define EMU_KSTEPS64 1                        /* 4 stages of 48 KiB */
 #endif
 	static constexpr int KSTEPS = S == fin<float>::S ? EMU_KSTEPS32 : EMU_KSTEPS64;
 	static constexpr int BUDGET = S == fin<float>::S ? EMU_BUDGET32 : STAGE_BUDGET;
@@ -495,11 +496,14 @@ __device__ __forceinline__ int chunk_end(int c0, int nks, int cplx, int kchunk)
  * Y.  A slice of the M side times w consecutive slices of the N side is one
  * MMA of w * N columns when the accumulators of its w groups lie side by
  * side, since the slices of the N side follow one another in shared memory.
- * An MMA reads its operands from shared memory at 128 B per cycle, the
- * M-side slice (4 KiB) again each time, and costs max(cols / 2, 32 + cols /
- * 4) + 6 cycles (measured), so fewer, wider ones win: a step of 21 products
- * took 1450 cycles at N = 128, 1311 at 96, 1210 at 64 and 32 as single
- * products; as below 1353, 1125, 698 and 560.  By the width N of a tile:
+ * An MMA costs max(cols / 2, 28 + cols / 6) cycles, so fewer, wider ones
+ * win.  Operands are read from shared memory at 128 B per cycle; the MMAs of
+ * one M-side slice (4 KiB) follow one another and keep it in the tensor
+ * core's buffer (at N = 128 a step's reads and copies then take 1248 cycles
+ * against the MMAs' 1344, 1728 if each MMA read it again).  A step of 21
+ * products, measured without copies: 1344 cycles at N = 128, 1014 at 96, 747
+ * at 64 as in class 2; issued from one lane alone, with a barrier wait per
+ * step, 1524, 1419 and 1419.  By the width N of a tile:
  *   class 0 (N <= 80): six accumulators, up to three slices: 9 MMAs;
  *   class 1 (N = 96): five (groups 4 and 5 share one), two slices: 15;
  *   class 2 (N > 96): four (3, 4, 5 share one), two slices: 17 (19 where X
@@ -542,16 +546,16 @@ struct mma_item {
  * acc0: 0 where they start the set's accumulators */
 template <int S, int KEEP, int CLS, int SET, bool PAIR, int P = 0, int Q = -1>
 __device__ __forceinline__ void
-issue_set(const mma_item &m, uint32_t tmem, uint32_t xcol, uint32_t alo, uint32_t ahi,
+issue_set(const mma_item &m, uint32_t el, uint32_t tmem, uint32_t xcol, uint32_t alo, uint32_t ahi,
     uint32_t blo, uint32_t bhi, uint32_t acc0)
 {
 	using R = prod<S, KEEP, CLS, SET>;
 	if constexpr (Q < 0) {
 		constexpr int q0 = R::GLO > P ? R::GLO - P : 0;
 		if constexpr (P < S)
-			issue_set<S, KEEP, CLS, SET, PAIR, P, q0>(m, tmem, xcol, alo, ahi, blo, bhi, acc0);
+			issue_set<S, KEEP, CLS, SET, PAIR, P, q0>(m, el, tmem, xcol, alo, ahi, blo, bhi, acc0);
 	} else if constexpr (Q >= S || P + Q > R::GHI) {
-		issue_set<S, KEEP, CLS, SET, PAIR, P + 1, -1>(m, tmem, xcol, alo, ahi, blo, bhi, acc0);
+		issue_set<S, KEEP, CLS, SET, PAIR, P + 1, -1>(m, el, tmem, xcol, alo, ahi, blo, bhi, acc0);
 	} else {
 		constexpr int w = R::width(P, Q), a = R::acc(P + Q);
 		/* the first product of its accumulators: slice 0 of the M side
@@ -560,12 +564,17 @@ issue_set(const mma_item &m, uint32_t tmem, uint32_t xcol, uint32_t alo, uint32_
 		/* FP32 alternates X between two fixed places */
 		const uint32_t d = tmem + (KEEP == 2 && !PAIR && a == 2 ? xcol : a * m.n);
 		const uint32_t acc = first ? acc0 : 1u;
+		/* slice P stays in the buffer over its row of MMAs */
+		constexpr bool row0 = Q == (R::GLO > P ? R::GLO - P : 0);
+		constexpr bool row1 = Q + w >= S || P + Q + w > R::GHI;
+		constexpr int COL = row0 && row1 ? COL_NONE : row0 ? COL_KEEP :
+		    row1 ? COL_LAST : COL_USE;
 		if constexpr (PAIR)
-			mma_bf16_pair(d, alo + P * m.sa, ahi, blo + Q * m.sb, bhi, m.idesc[0], acc);
+			mma_bf16_pair<COL>(el, d, alo + P * m.sa, ahi, blo + Q * m.sb, bhi, m.idesc[0], acc);
 		else
-			mma_bf16_split(d, alo + P * m.sa, ahi, blo + Q * m.sb, bhi,
+			mma_bf16_split<COL>(el, d, alo + P * m.sa, ahi, blo + Q * m.sb, bhi,
 			    m.idesc[w - 1], acc);
-		issue_set<S, KEEP, CLS, SET, PAIR, P, Q + w>(m, tmem, xcol, alo, ahi, blo, bhi, acc0);
+		issue_set<S, KEEP, CLS, SET, PAIR, P, Q + w>(m, el, tmem, xcol, alo, ahi, blo, bhi, acc0);
 	}
 }
 
@@ -630,7 +639,7 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 	 * nothing, the host recomputes these blocks on the FP64 path */
 	if (*(volatile int *)flags & 1)
 		return;
-	const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+	const int warp = __shfl_sync(0xffffffffu, threadIdx.x / 32, 0), lane = threadIdx.x % 32;
 	const uint32_t rank = PAIR ? cluster_rank() : 0;
 	/* bounded waits; in a pair, with cluster-scope acquire */
 	auto wait = [&](uint32_t bar, uint32_t parity, int code) -> bool {
@@ -694,26 +703,36 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 	tc_fence_after();
 	const uint32_t tmem = s_tmem;
 
+	/* for the roles whose warp runs in step: the issuing lane, a value of
+	 * lane 0 as a uniform one, a wait with one verdict */
+	const uint32_t el = elect_lane();
+	auto uni = [](auto v) { return __shfl_sync(0xffffffffu, v, 0); };
+	auto wwait = [&](uint64_t *bar, uint32_t parity, int code) -> bool {
+		return __all_sync(0xffffffffu, wait(smem_u32(bar), parity, code));
+	};
+
 	/* persistent: the producer takes the next item of the cost-sorted list
 	 * from a global counter and passes its index to the MMA and drain
 	 * warps through a two-slot ring (-1 ends); the stage ring and the
 	 * accumulator phases carry across items */
 	if (warp == 0) {
-		/* ---------------- producer ---------------- */
-		if (lane == 0) {
-			int s = 0;
-			uint32_t ph = 0;
-			int lastp[NST];
+		/* ---------------- producer ----------------
+		 * (in step, as the MMA warp; one lane issues) */
+		int s = 0;
+		uint32_t ph = 0;
+		int lastp[NST];
 #pragma unroll
-			for (int q = 0; q < NST; q++)
-				lastp[q] = -1;
-			uint32_t iph = 0;
-			for (int slot = 0; !s_err; ) {
-				int t;
-				if (!PAIR || rank == 0) {
-					/* fetch the next item and hand it to every role */
-					if (!wait(smem_u32(&bar_iempty[slot]), iph ^ 1, 5))
-						break;
+		for (int q = 0; q < NST; q++)
+			lastp[q] = -1;
+		uint32_t iph = 0;
+		bool ok = true;
+		for (int slot = 0; ok; ) {
+			int t = 0;
+			if (!PAIR || rank == 0) {
+				/* fetch the next item and hand it to every role */
+				if (!wwait(&bar_iempty[slot], iph ^ 1, 5))
+					break;
+				if (lane == 0) {
 					t = atomicAdd(g_next, 1);
 					t = t < nitems ? t : -1;
 					s_item[slot] = t;
@@ -722,149 +741,149 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 						mbar_arrive_remote(map_shared(smem_u32(&bar_ifull[slot]), 1));
 					}
 					mbar_arrive(smem_u32(&bar_ifull[slot]));
-				} else {
-					if (!wait(smem_u32(&bar_ifull[slot]), iph, 5))
-						break;
+				}
+			} else {
+				if (!wwait(&bar_ifull[slot], iph, 5))
+					break;
+				if (lane == 0) {
 					t = s_item[slot];
 					arrive0(&bar_iempty[slot]);
 				}
-				if (++slot == 2) { slot = 0; iph ^= 1; }
-				if (t < 0)
-					break;
-				const emu_item it = items[t];
-				const int nmem = it.mcount;
-				const xmgd_cblock_t cb = cbs[members[it.mfirst].cblock];
-				const int pass = it.pr & 1, swp = (it.pr >> 1) & 1;
-				const int mstk = (it.pr >> 2) & 1;
-				constexpr uint32_t ROWB = S * EMU_KS * 2;  /* a row's slices */
-				/* the shared side: the M side's tile (this CTA's of the two
-				 * in a pair) or, M-stacked, the N side's */
-				const int stile = it.m0 / EMU_TM + (mstk ? 0 : (int)rank);
-				const int slen = mstk == swp ? cb.n : cb.m;
-				/* (a pair's second M tile may lie past the view: its rows
-				 * are then never stored) */
-				const uint32_t sby = stile * EMU_TM < slen ?
-				    tile_rows(slen, stile * EMU_TM) * ROWB : 0;
-				/* the members: bytes copied per K step, bytes of their
-				 * tile's chunk, place in the stage; one member, unless the
-				 * list is stacked (row-major chunks); a pair stages half of
-				 * its rows in each CTA */
-				int mfp[EMU_MAXMEM], mrt[EMU_MAXMEM];
-				uint32_t mby[EMU_MAXMEM], mch[EMU_MAXMEM], mdo[EMU_MAXMEM], stb = 0;
+			}
+			t = uni(t);
+			if (++slot == 2) { slot = 0; iph ^= 1; }
+			if (t < 0)
+				break;
+			const emu_item it = items[t];
+			const xmgd_cblock_t cb = cbs[members[it.mfirst].cblock];
+			const int nmem = uni(it.mcount), npairs = uni(cb.npairs), pair0 = uni(cb.first_pair);
+			const int pr0 = uni(it.pr), m0 = uni(it.m0);
+			const int pass = pr0 & 1, swp = (pr0 >> 1) & 1, mstk = (pr0 >> 2) & 1;
+			constexpr uint32_t ROWB = S * EMU_KS * 2;  /* a row's slices */
+			/* the shared side: the M side's tile (this CTA's of the two
+			 * in a pair) or, M-stacked, the N side's */
+			const int stile = m0 / EMU_TM + (mstk ? 0 : (int)rank);
+			const int slen = uni(mstk == swp ? cb.n : cb.m);
+			/* (a pair's second M tile may lie past the view: its rows
+			 * are then never stored) */
+			const uint32_t sby = stile * EMU_TM < slen ?
+			    tile_rows(slen, stile * EMU_TM) * ROWB : 0;
+			/* the members: bytes copied per K step, bytes of their
+			 * tile's chunk, place in the stage; one member, unless the
+			 * list is stacked (row-major chunks); a pair stages half of
+			 * its rows in each CTA */
+			int mfp[EMU_MAXMEM], mrt[EMU_MAXMEM];
+			uint32_t mby[EMU_MAXMEM], mch[EMU_MAXMEM], mdo[EMU_MAXMEM], stb = 0;
+#pragma unroll
+			for (int j = 0; j < EMU_MAXMEM; j++) {
+				const emu_member mb = members[it.mfirst + (j < nmem ? j : 0)];
+				const xmgd_cblock_t cj = cbs[mb.cblock];
+				mfp[j] = uni(cj.first_pair);
+				mrt[j] = uni(mb.n0) / EMU_TM;
+				/* the stacked side: the N side (without swap a's rows)
+				 * or, M-stacked, the M side */
+				mch[j] = uni(tile_rows(mstk == swp ? cj.m : cj.n, mb.n0)) * ROWB;
+				mby[j] = PAIR ? mch[j] / 2 : mch[j];
+				mdo[j] = (mstk ? 0u : C::CHUNK_BYTES) + (uint32_t)uni(mb.off) * ROWB;
+				stb += j < nmem ? mby[j] : 0;
+			}
+			const uint32_t mso = PAIR ? rank * mby[0] : 0;
+			/* shared side from a's views when it is a's side */
+			const bool sha = (mstk ^ swp) != 0;
+			/* a pair's operand chunks: the shared side's tile and each
+			 * member's */
+			struct pair_src {
+				unsigned long long gs, gn[EMU_MAXMEM];
+				int k;
+			};
+			auto load_pair = [&](int p, pair_src &o) {
+				/* the members' pair lists run in step: pair p of
+				 * every member has member 0's view and K on the
+				 * shared side */
+				const xmgd_pair_t pr = prs[pair0 + p];
+				o.k = pr.k;
+				o.gs = sha ? va[pr.aview].slices : vb[pr.bview].slices;
 #pragma unroll
 				for (int j = 0; j < EMU_MAXMEM; j++) {
-					const emu_member mb = members[it.mfirst + (j < nmem ? j : 0)];
-					const xmgd_cblock_t cj = cbs[mb.cblock];
-					mfp[j] = cj.first_pair;
-					mrt[j] = mb.n0 / EMU_TM;
-					/* the stacked side: the N side (without swap a's rows)
-					 * or, M-stacked, the M side */
-					mch[j] = tile_rows(mstk == swp ? cj.m : cj.n, mb.n0) * ROWB;
-					mby[j] = PAIR ? mch[j] / 2 : mch[j];
-					mdo[j] = (mstk ? 0u : C::CHUNK_BYTES) + (uint32_t)mb.off * ROWB;
-					stb += j < nmem ? mby[j] : 0;
+					if (j >= nmem)
+						break;
+					const xmgd_pair_t pj = prs[mfp[j] + p];
+					o.gn[j] = sha ? vb[pj.bview].slices : va[pj.aview].slices;
 				}
-				const uint32_t mso = PAIR ? rank * mby[0] : 0;
-				/* shared side from a's views when it is a's side */
-				const bool sha = (mstk ^ swp) != 0;
-				/* a pair's operand chunks: the shared side's tile and each
-				 * member's */
-				struct pair_src {
-					const uint8_t *gs, *gn[EMU_MAXMEM];
-					int nks;
-				};
-				auto load_pair = [&](int p, pair_src &o) {
-					/* the members' pair lists run in step: pair p of
-					 * every member has member 0's view and K on the
-					 * shared side */
-					const xmgd_pair_t pr = prs[cb.first_pair + p];
-					o.nks = pair_steps(pr.k, cplx);
-					o.gs = reinterpret_cast<const uint8_t *>(sha ?
-					    va[pr.aview].slices : vb[pr.bview].slices) +
-					    (size_t)stile * o.nks * C::CHUNK_BYTES;
+			};
+			/* a view's tile, for all of the warp */
+			auto tile_at = [&](unsigned long long slices, int tile, int nks) {
+				return reinterpret_cast<const uint8_t *>(uni(slices)) +
+				    (size_t)tile * nks * C::CHUNK_BYTES;
+			};
+			/* K step ks of a pair: the shared side reads at its own
+			 * K index (the M side's or the N side's), the members at
+			 * the other; the imaginary pass swaps B's re/im halves */
+			auto kidx = [&](int ks, int nks, int &ksh, int &kst) {
+				const int nh = nks / 2;
+				const int kb = (cplx && pass) ? (ks < nh ? ks + nh : ks - nh) : ks;
+				const int km = swp ? ks : kb, kn = swp ? kb : ks;
+				ksh = mstk ? kn : km;
+				kst = mstk ? km : kn;
+			};
+			/* the next pair's operand addresses are loaded while this
+			 * one's steps are staged (two dependent loads) */
+			pair_src nxt;
+			load_pair(0, nxt);
+			for (int p = 0; p < npairs && ok; p++) {
+				const int nks = pair_steps(uni(nxt.k), cplx);
+				const uint8_t *gs = tile_at(nxt.gs, stile, nks), *gn[EMU_MAXMEM];
 #pragma unroll
-					for (int j = 0; j < EMU_MAXMEM; j++) {
-						if (j >= nmem)
-							break;
-						const xmgd_pair_t pj = prs[mfp[j] + p];
-						o.gn[j] = reinterpret_cast<const uint8_t *>(sha ?
-						    vb[pj.bview].slices : va[pj.aview].slices) +
-						    (size_t)mrt[j] * o.nks * C::CHUNK_BYTES + mso;
-					}
-				};
-				/* K step ks of a pair: the shared side reads at its own
-				 * K index (the M side's or the N side's), the members at
-				 * the other; the imaginary pass swaps B's re/im halves */
-				auto kidx = [&](int ks, int nks, int &ksh, int &kst) {
-					const int nh = nks / 2;
-					const int kb = (cplx && pass) ? (ks < nh ? ks + nh : ks - nh) : ks;
-					const int km = swp ? ks : kb, kn = swp ? kb : ks;
-					ksh = mstk ? kn : km;
-					kst = mstk ? km : kn;
-				};
-				/* the next pair's operand addresses are loaded while this
-				 * one's steps are staged (two dependent loads) */
-				pair_src cur, nxt;
-				load_pair(0, nxt);
-				for (int p = 0; p < cb.npairs && !s_err; p++) {
-					cur = nxt;
-					if (p + 1 < cb.npairs)
-						load_pair(p + 1, nxt);
-					for (int ks = 0; ks < cur.nks; ) {
-						const int ke = super_end<S>(ks, cur.nks, cplx);
-						if (!wait(smem_u32(&bar_empty[s]), ph ^ 1, 1))
-							break;
-						uint32_t dst = smem_u32(stages + (size_t)s * C::STAGE_BYTES);
-						const uint32_t fb = smem_u32(&bar_full[s]);
+				for (int j = 0; j < EMU_MAXMEM; j++)
+					if (j < nmem)
+						gn[j] = tile_at(nxt.gn[j], mrt[j], nks) + mso;
+				if (p + 1 < npairs)
+					load_pair(p + 1, nxt);
+				for (int ks = 0; ks < nks; ) {
+					const int ke = super_end<S>(ks, nks, cplx);
+					if (!(ok = wwait(&bar_empty[s], ph ^ 1, 1)))
+						break;
+					uint32_t dst = smem_u32(stages + (size_t)s * C::STAGE_BYTES);
+					const uint32_t fb = smem_u32(&bar_full[s]);
+					if (el)
 						mbar_expect_tx(fb, (uint32_t)(ke - ks) * (sby + stb));
-						/* (a stage's steps lie in one half of a realified view,
-						 * so that both operands' chunks follow one another) */
-						int ksh, kst;
-						kidx(ks, cur.nks, ksh, kst);
-						const uint8_t *g = cur.gs + (size_t)ksh * sby;
-						if (nmem == 1 && !PAIR) {
-							const uint8_t *x = cur.gn[0] + (size_t)kst * mch[0];
-							const uint32_t xb = mch[0];
-							for (int k = ks; k < ke; k++) {
-								bulk_g2s(dst, g, sby, fb);
-								bulk_g2s(dst + C::CHUNK_BYTES, x, xb, fb);
-								dst += C::STEP_BYTES;
-								g += sby;
-								x += xb;
-							}
-						} else
-						for (int k = ks; k < ke; k++, kst++) {
-							if (!PAIR || sby)
-								bulk_g2s(dst + (mstk ? C::CHUNK_BYTES : 0u), g, sby, fb);
+					__syncwarp();
+					/* (a stage's steps lie in one half of a realified view,
+					 * so that both operands' chunks follow one another) */
+					int ksh, kst;
+					kidx(ks, nks, ksh, kst);
+					const uint8_t *g = gs + (size_t)ksh * sby;
+					for (int k = ks; k < ke; k++, kst++) {
+						if (!PAIR || sby)
+							bulk_g2s_el(el, dst + (mstk ? C::CHUNK_BYTES : 0u), g, sby, fb);
 #pragma unroll
-							for (int j = 0; j < EMU_MAXMEM; j++)
-								if (j < nmem)
-									bulk_g2s(dst + mdo[j],
-									    cur.gn[j] + (size_t)kst * mch[j], mby[j], fb);
-							dst += C::STEP_BYTES;
-							g += sby;
-						}
-#pragma unroll
-						for (int q = 0; q < NST; q++)
-							if (q == s)
-								lastp[q] = (int)ph;
-						if (++s == NST) { s = 0; ph ^= 1; }
-						ks = ke;
+						for (int j = 0; j < EMU_MAXMEM; j++)
+							if (j < nmem)
+								bulk_g2s_el(el, dst + mdo[j],
+								    gn[j] + (size_t)kst * mch[j], mby[j], fb);
+						dst += C::STEP_BYTES;
+						g += sby;
 					}
+#pragma unroll
+					for (int q = 0; q < NST; q++)
+						if (q == s)
+							lastp[q] = (int)ph;
+					if (++s == NST) { s = 0; ph ^= 1; }
+					ks = ke;
 				}
 			}
-			/* on failure, let this CTA's copies still in flight land
-			 * before it exits (bounded): the last phase issued on each
-			 * stage completes when its bytes have arrived */
-			if (s_err) {
-				uint64_t t0 = gtimer();
+		}
+		/* on failure, let this CTA's copies still in flight land
+		 * before it exits (bounded): the last phase issued on each
+		 * stage completes when its bytes have arrived */
+		if (s_err) {
+			uint64_t t0 = gtimer();
 #pragma unroll
-				for (int q = 0; q < NST; q++)
-					if (lastp[q] >= 0)
-						while (!mbar_try(smem_u32(&bar_full[q]), (uint32_t)lastp[q]) &&
-						    gtimer() - t0 < WAIT_NS)
-							;
-			}
+			for (int q = 0; q < NST; q++)
+				if (lastp[q] >= 0)
+					while (!mbar_try(smem_u32(&bar_full[q]), (uint32_t)lastp[q]) &&
+					    gtimer() - t0 < WAIT_NS)
+						;
 		}
 	} else if (warp == 1 && PAIR && rank == 1) {
 		/* ---------- rank 1: forward stage completions to rank 0 ---------- */
@@ -897,8 +916,12 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 				;
 		}
 	} else if (warp == 1) {
-		/* ---------------- MMA issuer ---------------- */
-		if (lane == 0) {
+		/* ---------------- MMA issuer ----------------
+		 * The warp runs in step, one lane issues (mma_bf16_split); what
+		 * comes from memory is broadcast from lane 0, so that the MMAs'
+		 * operands are uniform. */
+		{
+			const uint32_t tm = uni(tmem);
 			int s = 0, prevn = 0;
 			bool first = true;
 			uint32_t ph = 0, xph = 0, yph = 0, nch = 0;
@@ -906,34 +929,39 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 			/* a stage is ready once this CTA's copies (and, in a pair,
 			 * the peer's, forwarded) have landed */
 			auto ready = [&](int st_, uint32_t par) -> bool {
-				if (!wait(smem_u32(&bar_full[st_]), par, 3))
+				if (!wwait(&bar_full[st_], par, 3))
 					return false;
-				if (PAIR && !wait(smem_u32(&bar_pfull[st_]), par, 10))
+				if (PAIR && !wwait(&bar_pfull[st_], par, 10))
 					return false;
 				tc_fence_after();
 				return true;
 			};
-			/* one item of a width class; returns on failure (s_err set) */
-			auto item = [&](auto cls, const emu_item &it, const xmgd_cblock_t &cb) {
+			auto done = [&](uint64_t *bar) {
+				if (el)
+					commit(bar);
+				__syncwarp();
+			};
+			/* one item of a width class: its blocks' pairs, N side and M
+			 * side slice strides; false on failure (s_err set) */
+			auto item = [&](auto cls, int n, uint32_t sa, int pair0, int npairs) -> bool {
 				constexpr int CLS = decltype(cls)::value;
 				constexpr int KS = C::KSTEPS;
 				mma_item mi;
-				mi.n = it.pr >> 8;
-				const int swp = (it.pr >> 1) & 1;
+				mi.n = n;
 				for (int w = 0; w < 3; w++)
 					mi.idesc[w] = PAIR ? idesc_pair_n(mi.n) : idesc_n((w + 1) * mi.n);
 				mi.sbo = rowmajor ? S * 256 : 256;
-				mi.sa = rowmajor ? 16 : 2 * tile_rows(swp ? cb.m : cb.n, it.m0);
+				mi.sa = sa;
 				mi.sb = rowmajor ? 16 : 2 * mi.n;
 				/* accumulators of another width than the last item's lie
 				 * across them: wait for both sets' drains */
 				bool both = !XDB && !first && (int)mi.n != prevn;
 				prevn = mi.n;
-				int knext = prs[cb.first_pair].k;
-				for (int p = 0; p < cb.npairs; p++) {
-					const int nks = pair_steps(knext, cplx);
-					if (p + 1 < cb.npairs)
-						knext = prs[cb.first_pair + p + 1].k;
+				int knext = prs[pair0].k;
+				for (int p = 0; p < npairs; p++) {
+					const int nks = pair_steps(uni(knext), cplx);
+					if (p + 1 < npairs)
+						knext = prs[pair0 + p + 1].k;
 					for (int c0 = 0; c0 < nks; ) {
 						const int c1 = chunk_end<S>(c0, nks, cplx, kchunk);
 						/* the chunk's stages: KSTEPS steps each, the last
@@ -960,17 +988,17 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 								const uint32_t blo = (uint32_t)db, bhi = (uint32_t)(db >> 32);
 								if constexpr (WH == 3 && CLS == 2 && KEEP > 2) {
 									/* (a middle stage: both sets have started) */
-									issue_set<S, KEEP, CLS, SET_ALL, PAIR>(mi, tmem, xcol, alo,
+									issue_set<S, KEEP, CLS, SET_ALL, PAIR>(mi, el, tm, xcol, alo,
 									    ahi, blo, bhi, 1u);
 									continue;
 								}
 								if constexpr (WH & 2) {
-									issue_set<S, KEEP, CLS, SET_Y, PAIR>(mi, tmem, xcol, alo, ahi,
+									issue_set<S, KEEP, CLS, SET_Y, PAIR>(mi, el, tm, xcol, alo, ahi,
 									    blo, bhi, ay);
 									ay = 1;
 								}
 								if constexpr (WH & 1) {
-									issue_set<S, KEEP, CLS, SET_X, PAIR>(mi, tmem, xcol, alo, ahi,
+									issue_set<S, KEEP, CLS, SET_X, PAIR>(mi, el, tm, xcol, alo, ahi,
 									    blo, bhi, ax);
 									ax = 1;
 								}
@@ -990,32 +1018,32 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 						 * the previous chunk (of the one before it, where X
 						 * has two copies) */
 						if (XDB) {
-							if (nch >= 2 && !wait(smem_u32(&bar_xempty[nch & 1]),
+							if (nch >= 2 && !wwait(&bar_xempty[nch & 1],
 							    ((nch >> 1) - 1) & 1, 2))
-								return;
+								return false;
 						} else if (!first) {
-							if (!wait(smem_u32(&bar_xempty[0]), xph, 2))
-								return;
+							if (!wwait(&bar_xempty[0], xph, 2))
+								return false;
 							xph ^= 1;
 						}
 						if (both) {
-							if (!wait(smem_u32(&bar_yempty), yph, 8))
-								return;
+							if (!wwait(&bar_yempty, yph, 8))
+								return false;
 							yph ^= 1;
 						}
 						tc_fence_after();
 						for (int j = 0; j < H; j++) {
 							const int sj = s + j < NST ? s + j : s + j - NST;
 							if (!ready(sj, s + j < NST ? ph : ph ^ 1))
-								return;
+								return false;
 							issue(sj, j, X);
 						}
 						if (T == 0 && !XDB)
-							commit(&bar_xfull);
+							done(&bar_xfull);
 						/* head, set Y, once Y is read too */
 						if (!first && !both) {
-							if (!wait(smem_u32(&bar_yempty), yph, 8))
-								return;
+							if (!wwait(&bar_yempty, yph, 8))
+								return false;
 							yph ^= 1;
 						}
 						first = both = false;
@@ -1023,16 +1051,16 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 						for (int j = 0; j < H; j++) {
 							const int sj = s + j < NST ? s + j : s + j - NST;
 							issue(sj, j, Y);
-							commit(&bar_empty[sj]);
+							done(&bar_empty[sj]);
 						}
 						s += H;
 						if (s >= NST) { s -= NST; ph ^= 1; }
 						/* middle: every product per stage */
 						for (int j = H; j < nss - T; j++) {
 							if (!ready(s, ph))
-								return;
+								return false;
 							issue(s, j, XY);
-							commit(&bar_empty[s]);
+							done(&bar_empty[s]);
 							if (++s == NST) { s = 0; ph ^= 1; }
 						}
 						/* tail: set X of the last T stages, then X is
@@ -1041,58 +1069,60 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 						for (int j = 0; j < T; j++) {
 							const int sj = s + j < NST ? s + j : s + j - NST;
 							if (!ready(sj, s + j < NST ? ph : ph ^ 1))
-								return;
+								return false;
 							issue(sj, nss - T + j, X);
 						}
 						if (T > 0) {
-							commit(&bar_xfull);
+							done(&bar_xfull);
 							for (int j = 0; j < T; j++) {
 								const int sj = s + j < NST ? s + j : s + j - NST;
 								issue(sj, nss - T + j, Y);
-								commit(&bar_empty[sj]);
+								done(&bar_empty[sj]);
 							}
 							s += T;
 							if (s >= NST) { s -= NST; ph ^= 1; }
 						}
-						commit(&bar_yfull);
+						done(&bar_yfull);
 						nch++;
 						c0 = c1;
 					}
 				}
+				return true;
 			};
-			for (int slot = 0; !s_err; ) {
-				if (!wait(smem_u32(&bar_ifull[slot]), iph, 6))
+			for (int slot = 0, ok = 1; ok; ) {
+				if (!wwait(&bar_ifull[slot], iph, 6))
 					break;
-				const int t = s_item[slot];
-				mbar_arrive(smem_u32(&bar_iempty[slot]));
+				const int t = uni(*(volatile int *)&s_item[slot]);
+				if (lane == 0)
+					mbar_arrive(smem_u32(&bar_iempty[slot]));
+				__syncwarp();
 				if (++slot == 2) { slot = 0; iph ^= 1; }
 				if (t < 0)
 					break;
 				const emu_item it = items[t];
 				const xmgd_cblock_t cb = cbs[members[it.mfirst].cblock];
-				if (PAIR || rowmajor) {
-					item(std::integral_constant<int, 4>{}, it, cb);
-					continue;
-				}
-				if constexpr (PAIR)
+				const int n = uni(it.pr) >> 8, p0 = uni(cb.first_pair), np = uni(cb.npairs);
+				const uint32_t sa = rowmajor ? 16 :
+				    2 * uni(tile_rows((it.pr >> 1) & 1 ? cb.m : cb.n, it.m0));
+				auto run = [&](auto cls) { return item(cls, n, sa, p0, np); };
+				if (PAIR || rowmajor)
+					ok = run(std::integral_constant<int, 4>{});
+				else if constexpr (PAIR)
 					;
 				else if constexpr (KEEP == 2)
-					item(std::integral_constant<int, 3>{}, it, cb);
-				else {
-					const int n = it.pr >> 8;
-					if (n <= 80)
-						item(std::integral_constant<int, 0>{}, it, cb);
-					else if (n <= 96)
-						item(std::integral_constant<int, 1>{}, it, cb);
-					else
-						item(std::integral_constant<int, 2>{}, it, cb);
-				}
+					ok = run(std::integral_constant<int, 3>{});
+				else if (n <= 80)
+					ok = run(std::integral_constant<int, 0>{});
+				else if (n <= 96)
+					ok = run(std::integral_constant<int, 1>{});
+				else
+					ok = run(std::integral_constant<int, 2>{});
 			}
 			/* every MMA issued by this CTA has completed once bar_fin
 			 * fires; TMEM is released only after that */
-			commit(&bar_fin);
+			done(&bar_fin);
 			uint64_t t0 = gtimer();
-			while (!(PAIR ? mbar_try_cl(smem_u32(&bar_fin), 0) :
+			while (lane == 0 && !(PAIR ? mbar_try_cl(smem_u32(&bar_fin), 0) :
 			    mbar_try(smem_u32(&bar_fin), 0)) && gtimer() - t0 < WAIT_NS)
 				;
 		}
@@ -1187,43 +1217,46 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 #pragma unroll
 			for (int c = 0; c < NC; c++)
 				V[c] = 0;
+			/* columns per TMEM load and wait (8 took 3 % off the FP64
+			 * drains, 4 is 1 % faster in FP32) */
+			constexpr int W = LOW ? 8 : 4;
 			/* set X.  FP64: the low band, L in units of 2^-16 (|L| <
 			 * 2^19: 15 products of 256 times 2^14 at 2^-24, with the pair
 			 * factor's 2), to units of 2^(-16-F): V += 2^F h + l, h =
 			 * rint(L), l = rint(2^F (L - h)).  FP32: group 2, an integer */
 			auto drain_x = [&](uint32_t at, const float *s0) {
 #pragma unroll
-				for (int b4 = 0; b4 < NC / 4; b4++) {
-					if (b4 * 4 >= cw || col0 + b4 * 4 >= rows)
+				for (int b = 0; b < NC; b += W) {
+					if (b >= cw || col0 + b >= rows)
 						break;	/* warp-uniform: columns past the tile */
-					const int g = b4 / 4;
-					float ax[4];
-					tmem_ld4(trow + at + col0 + b4 * 4, ax);
+					const int g = b / 16;
+					float ax[W];
+					tmem_ld(trow + at + col0 + b, ax);
 					if (LOW && nacc3 > 1) {
 						/* groups 4 (and 5) have their own accumulators,
 						 * in the same units */
-						float a4[4], a5[4] = {0, 0, 0, 0};
-						tmem_ld4(trow + at + rows + col0 + b4 * 4, a4);
+						float a4[W], a5[W] = {};
+						tmem_ld(trow + at + rows + col0 + b, a4);
 						if (nacc3 > 2)
-							tmem_ld4(trow + at + 2 * rows + col0 + b4 * 4, a5);
+							tmem_ld(trow + at + 2 * rows + col0 + b, a5);
 						tmem_wait_ld();
 #pragma unroll
-						for (int c = 0; c < 4; c++)
+						for (int c = 0; c < W; c++)
 							ax[c] += a4[c] + a5[c];
 					} else
 						tmem_wait_ld();
 #pragma unroll
-					for (int c = 0; c < 4; c++) {
+					for (int c = 0; c < W; c++) {
 						const float sx = s0[g] * 65536.0f;
 						if (LOW) {
 							const float t = fmaf(ax[c], sx, MAGICF);
 							const float r = fmaf(ax[c], sx, MAGICF - t);
 							const float l = fmaf(r, __int_as_float((127 + sF[g]) << 23),
 							    MAGICF);
-							V[b4 * 4 + c] += shl64(__float_as_uint(t), sF[g]) +
+							V[b + c] += shl64(__float_as_uint(t), sF[g]) +
 							    __float_as_uint(l);
 						} else
-							V[b4 * 4 + c] += (long long)__float2int_rn(ax[c] * sx);
+							V[b + c] += (long long)__float2int_rn(ax[c] * sx);
 					}
 				}
 			};
@@ -1235,18 +1268,18 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 			 * conversions serve three groups, one serves two in FP32 */
 			auto drain_y = [&](const float *s0) {
 #pragma unroll
-				for (int b4 = 0; b4 < NC / 4; b4++) {
-					if (b4 * 4 >= cw || col0 + b4 * 4 >= rows)
+				for (int b = 0; b < NC; b += W) {
+					if (b >= cw || col0 + b >= rows)
 						break;
-					const int g = b4 / 4, F = sF[g];
-					float a0[4], a1[4], a2[4];
-					tmem_ld4(trow + col0 + b4 * 4, a0);
-					tmem_ld4(trow + rows + col0 + b4 * 4, a1);
+					const int g = b / 16, F = sF[g];
+					float a0[W], a1[W], a2[W];
+					tmem_ld(trow + col0 + b, a0);
+					tmem_ld(trow + rows + col0 + b, a1);
 					if (LOW)
-						tmem_ld4(trow + 2 * rows + col0 + b4 * 4, a2);
+						tmem_ld(trow + 2 * rows + col0 + b, a2);
 					tmem_wait_ld();
 #pragma unroll
-					for (int c = 0; c < 4; c++) {
+					for (int c = 0; c < W; c++) {
 						const float h = fmaf(a1[c], s0[g], MAGICF) - MAGICF;
 						const float r = fmaf(a1[c], s0[g], -h);
 						const int d = __float2int_rn(fmaf(a0[c], s0[g], h));
@@ -1257,12 +1290,12 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 							    ((uint32_t)d << (16 + F));
 							const uint64_t ev = ((uint64_t)(uint32_t)(e >> (32 - F)) << 32) |
 							    ((uint32_t)e << F);
-							V[b4 * 4 + c] += dv + ev;
+							V[b + c] += dv + ev;
 						} else {
 							const float l = fmaf(r, 65536.0f, MAGICF);
 							const uint64_t dv = ((uint64_t)(uint32_t)(d >> 16) << 32) |
 							    ((uint32_t)d << 16);
-							V[b4 * 4 + c] += dv + __float_as_uint(l);
+							V[b + c] += dv + __float_as_uint(l);
 						}
 					}
 				}
@@ -1417,10 +1450,8 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
  *      decreasing cost, each block's tiles together;
  *   1  the same orientation; blocks grouped by their M-side free block and
  *      the group run M tile by M tile across its blocks;
- *   2  grouped as 1, orientation from a shared-memory model of one K step,
- *      max(N / 2, 32 + N / 4) cycles: the M-side operand (4 KiB) and the
- *      N-side operand (N * 32 B) are read from shared memory at 128 B per
- *      cycle while the tensor core needs N / 2 cycles.
+ *   2  grouped as 1, orientation by max(N / 2, 32 + N / 4) per tile, which
+ *      prefers wide tiles (an MMA's cost does not fall below 28 cycles).
  * (and 6, the stacked form below).  The first runs of a plan replay each
  * distinct policy within a quarter of the modelled best once, in the model's
  * order (list_cycles), timed with events, then keep the fastest; the choice
@@ -1956,17 +1987,19 @@ items_ok(const xmgd_contract_t *p, const std::vector<emu_item> &items,
 }
 
 /* Modelled cycles of one K step of a tile of n columns: its MMAs (issue_set)
- * at max(columns / 2, 32 + columns / 4) + 6 cycles each, and the stage's
- * bytes written to shared memory at the 128 per cycle the MMAs read with. */
+ * at max(columns / 2, 28 + columns / 6) cycles each, or the shared memory's
+ * traffic at 128 B per cycle if that takes longer: each M-side slice once,
+ * an N-side slice per product, the copied bytes. */
 static double
 step_cycles(bool dbl, bool rowmajor, int n)
 {
+	const int S = dbl ? fin<double>::S : fin<float>::S, products = dbl ? 21 : 6;
 	double c = 0;
 	auto mma = [&](int slices, int count) {
-		c += count * (std::max(slices * n / 2.0, 32 + slices * n / 4.0) + 6);
+		c += count * std::max(slices * n / 2.0, 28 + slices * n / 6.0);
 	};
 	if (rowmajor)
-		mma(1, dbl ? 21 : 6);
+		mma(1, products);
 	else if (!dbl) {
 		mma(2, 1);
 		mma(1, 4);
@@ -1978,7 +2011,7 @@ step_cycles(bool dbl, bool rowmajor, int n)
 		mma(2, n <= 96 ? 6 : 4);
 		mma(1, n <= 96 ? 9 : 13);
 	}
-	return c + (dbl ? fin<double>::S : fin<float>::S) * (EMU_TM + n) / 4.0;
+	return std::max(c, (S * EMU_TM + products * n + S * (EMU_TM + n)) / 4.0);
 }
 
 /* modelled cycles of a work list on the chip: the SMs' share, at least the
@@ -2040,7 +2073,7 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 		const int nst = dbl ? stage_cfg<fin<double>::S>::NST : stage_cfg<fin<float>::S>::NST;
 		/* head/tail length in stages */
 		const char *h = getenv("XMG_EMU_HEAD");
-		e->hmax = h ? atoi(h) : 2;
+		e->hmax = h ? atoi(h) : 3;
 		e->hmax = std::max(1, std::min(nst, e->hmax));
 		/* FP64 chunks in whole stages (they start at a segment's first
 		 * step, as the stages do) */

@@ -108,6 +108,17 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src,
 	    : "memory");
 }
 
+/* the same, executed by the whole warp in step and issued by the lane where el
+ * is nonzero (as mma_bf16_split) */
+__device__ __forceinline__ void bulk_g2s_el(uint32_t el, uint32_t dst, const void *src,
+    uint32_t bytes, uint32_t bar)
+{
+	asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %4, 0;\n\t"
+	    "@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes"
+	    " [%0], [%1], %2, [%3];\n\t}" :: "r"(dst), "l"(src), "r"(bytes), "r"(bar), "r"(el)
+	    : "memory");
+}
+
 /* bring [src, src + bytes) into L2 ahead of its shared-memory copy
  * (address and size multiples of 16 bytes) */
 __device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes)
@@ -145,15 +156,47 @@ __device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t a, uint64_t b,
 	    :: "r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc));
 }
 
-/* the same with each descriptor passed as (low, high) words */
-__device__ __forceinline__ void mma_bf16_split(uint32_t d, uint32_t alo,
+/* What an MMA does with the M-side operand's buffer (the collector): load it
+ * for this MMA alone, load and keep it, take what the last MMA kept, take it
+ * for the last time.  Between KEEP and LAST every MMA of the thread has the
+ * same M-side descriptor. */
+enum { COL_NONE, COL_KEEP, COL_USE, COL_LAST };
+
+/* The same with each descriptor passed as (low, high) words, executed by the
+ * whole warp in step and issued by the lane where el is nonzero.  Descriptors
+ * live in the warp's uniform registers: in code that one lane runs alone each
+ * operand is moved there for each MMA (54 cycles per MMA, and some 300 more
+ * after every barrier wait); in code that the warp runs together they are
+ * computed there (31 cycles). */
+#define XMG_MMA(GROUP, COL)                                                  \
+	asm volatile("{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"           \
+	    "mov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"                \
+	    "setp.ne.b32 p, %6, 0;\n\tsetp.ne.b32 q, %7, 0;\n\t"              \
+	    "@q tcgen05.mma.cta_group::" GROUP ".kind::f16" COL                \
+	    " [%0], a, b, %5, p;\n\t}"                                        \
+	    :: "r"(d), "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc),     \
+	    "r"(acc), "r"(el))
+/* one lane of the converged warp: the same at each call */
+__device__ __forceinline__ uint32_t elect_lane()
+{
+	uint32_t r;
+	asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\t"
+	    "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+	return r;
+}
+
+template <int COL>
+__device__ __forceinline__ void mma_bf16_split(uint32_t el, uint32_t d, uint32_t alo,
     uint32_t ahi, uint32_t blo, uint32_t bhi, uint32_t idesc, uint32_t acc)
 {
-	asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
-	    "mov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
-	    "setp.ne.b32 p, %6, 0;\n\t"
-	    "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n\t}"
-	    :: "r"(d), "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc), "r"(acc));
+	if constexpr (COL == COL_KEEP)
+		XMG_MMA("1", ".collector::a::fill");
+	else if constexpr (COL == COL_USE)
+		XMG_MMA("1", ".collector::a::use");
+	else if constexpr (COL == COL_LAST)
+		XMG_MMA("1", ".collector::a::lastuse");
+	else
+		XMG_MMA("1", "");
 }
 
 __device__ __forceinline__ void mma_commit(uint32_t bar)
@@ -162,7 +205,7 @@ __device__ __forceinline__ void mma_commit(uint32_t bar)
 	    :: "r"(bar) : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8])
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, float (&v)[8])
 {
 	uint32_t r[8];
 	asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 "
@@ -175,7 +218,7 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8])
 		v[i] = __uint_as_float(r[i]);
 }
 
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4])
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, float (&v)[4])
 {
 	uint32_t r[4];
 	asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
@@ -276,14 +319,18 @@ __device__ __forceinline__ void cluster_sync()
 /* tensor-core MMA over the CTA pair: M = 256 (128 rows from each CTA's
  * shared memory at the same offset), the N side split between the CTAs'
  * shared memory, each CTA's TMEM receiving its 128 rows */
-__device__ __forceinline__ void mma_bf16_pair(uint32_t d, uint32_t alo,
+template <int COL>
+__device__ __forceinline__ void mma_bf16_pair(uint32_t el, uint32_t d, uint32_t alo,
     uint32_t ahi, uint32_t blo, uint32_t bhi, uint32_t idesc, uint32_t acc)
 {
-	asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\t"
-	    "mov.b64 a, {%1, %2};\n\tmov.b64 b, {%3, %4};\n\t"
-	    "setp.ne.b32 p, %6, 0;\n\t"
-	    "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %5, p;\n\t}"
-	    :: "r"(d), "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc), "r"(acc));
+	if constexpr (COL == COL_KEEP)
+		XMG_MMA("2", ".collector::a::fill");
+	else if constexpr (COL == COL_USE)
+		XMG_MMA("2", ".collector::a::use");
+	else if constexpr (COL == COL_LAST)
+		XMG_MMA("2", ".collector::a::lastuse");
+	else
+		XMG_MMA("2", "");
 }
 
 /* arrive on the barrier at this offset in both CTAs once every earlier
