@@ -73,14 +73,6 @@ template <typename T> struct fin;
 template <> struct fin<double> {
 	static constexpr int S = 6, KEEP = 5, T1 = 47, MANT = 52, EMAX = 0x7ff;
 	static constexpr int EXPOFF = 47 + 1022 - 8 * (6 - 1);    /* 1029 */
-	__device__ static inline void parts(double x, long long &m, int &eb, bool &neg)
-	{
-		long long b = __double_as_longlong(x);
-		eb = (int)((b >> 52) & 0x7ff);
-		m = b & 0xFFFFFFFFFFFFFll;
-		if (eb == 0) eb = 1; else m |= 1ll << 52;
-		neg = b < 0;
-	}
 	/* the 32-bit word that holds the exponent, and the exponent in it */
 	__device__ static inline int eword(const double *p)
 	{ return __ldg(reinterpret_cast<const int *>(p) + 1); }
@@ -89,14 +81,6 @@ template <> struct fin<double> {
 template <> struct fin<float> {
 	static constexpr int S = 3, KEEP = 2, T1 = 23, MANT = 23, EMAX = 0xff;
 	static constexpr int EXPOFF = 23 + 126 - 8 * (3 - 1);     /* 133 */
-	__device__ static inline void parts(float x, long long &m, int &eb, bool &neg)
-	{
-		unsigned b = __float_as_uint(x);
-		eb = (int)((b >> 23) & 0xff);
-		m = b & 0x7fffff;
-		if (eb == 0) eb = 1; else m |= 1ll << 23;
-		neg = (b >> 31) != 0;
-	}
 	__device__ static inline int eword(const float *p)
 	{ return __ldg(reinterpret_cast<const int *>(p)); }
 	__device__ static inline int bexp(int w) { return (w >> 23) & 0xff; }
@@ -278,17 +262,82 @@ emu_exp_kernel(const xmgd_view_t *__restrict__ views,
 /* ------------------------------------------------------------------ */
 /* 2. unfold + split                                                   */
 
-/* bf16 bits of d * w, exact for |d| <= 256 and w a power of two */
-__device__ __forceinline__ uint32_t digit_bf16(int d, float w)
+/*
+ * An element as digits: Z = X + 128 (1 + 2^8 + ... + 2^(8 (S - 1))), X =
+ * round(m * 2^(eb - er - (MANT + 1 - T1))) with the element's sign, halves
+ * away from zero, |X| <= 2^T1.  The bias turns X's balanced digits into the
+ * bytes of Z (the top one may be 256): no carries between digits.  With y =
+ * 2 |X| cut to an integer, X is floor((y + 1) / 2) or -floor((y + 1) / 2) =
+ * floor(-y / 2), so one complement, one addition of the doubled bias and one
+ * shift serve both signs and the rounding.
+ */
+struct digits64 { uint32_t lo, hi; };
+__device__ __forceinline__ digits64 digits_of(double x, int er)
 {
-	/* exact int -> float for |d| < 2^22 without a conversion unit */
-	float f = __int_as_float(0x4B400000 + d) - 12582912.0f;
-	return __float_as_uint(f * w) >> 16;
+	const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+	const uint32_t lo = (uint32_t)b, hi = (uint32_t)(b >> 32);
+	const uint32_t e = (hi >> 20) & 0x7ff;
+	const uint32_t mh = (hi & 0xFFFFF) | (e ? 0x100000u : 0u);
+	const uint32_t sh = min(er - (int)max(e, 1u) + (fin<double>::MANT - fin<double>::T1), 63);
+	/* (a funnel shift clamps at 32) */
+	const uint32_t yl = __funnelshift_rc(lo, mh, sh) >> max((int)sh - 32, 0);
+	const uint32_t yh = __funnelshift_rc(mh, 0, sh);
+	const uint32_t s = (uint32_t)((int)hi >> 31);
+	const unsigned long long z = (((unsigned long long)(yh ^ s) << 32) | (yl ^ s)) +
+	    0x1010101010101ull;
+	return digits64{(uint32_t)(z >> 1), (uint32_t)(z >> 33)};
 }
 
-/* CTA = (view, 128-row tile, group of 4 K steps); thread = (row, K octet) */
+struct digits32 { uint32_t lo; };
+__device__ __forceinline__ digits32 digits_of(float x, int er)
+{
+	const uint32_t b = __float_as_uint(x), e = (b >> 23) & 0xff;
+	const uint32_t m2 = (b << 1 & 0xFFFFFE) | (e ? 0x1000000u : 0u);
+	const uint32_t sh = min(er - (int)max(e, 1u) + 1, 31);
+	return digits32{((m2 >> sh ^ (uint32_t)((int)b >> 31)) + 0x1010101u) >> 1};
+}
+
+/* digit t of S as the float d * 2^(-8 t): its byte below the magic number
+ * whose last place is 2^(-8 t), less that number and the bias */
+template <int S, int T, typename D>
+__device__ __forceinline__ uint32_t digit_bits(const D &z)
+{
+	constexpr uint32_t magic = (uint32_t)(0x4B - 4 * T) << 24;
+	constexpr int byte = S - 1 - T;
+	uint32_t w;
+	if constexpr (S == 3)
+		w = T == 0 ? magic | z.lo >> 16 : __byte_perm(z.lo, magic, 0x7540 | byte);
+	else if constexpr (T <= 1)
+		w = T == 0 ? magic | z.hi >> 8 : __byte_perm(z.hi, magic, 0x7540);
+	else
+		w = __byte_perm(z.lo, magic, 0x7540 | byte);
+	constexpr float c = (8388608.0f + 128.0f) / (float)(1ull << (8 * T));
+	return __float_as_uint(__uint_as_float(w) - c);
+}
+
+template <int S, int T, typename D>
+__device__ __forceinline__ void digit_pairs(const D &a, const D &b, uint32_t (&bits)[S][4],
+    int q)
+{
+	if constexpr (T < S) {
+		/* (bf16 is exact: the digits' upper halves) */
+		bits[T][q] = __byte_perm(digit_bits<S, T>(a), digit_bits<S, T>(b), 0x7632);
+		digit_pairs<S, T + 1>(a, b, bits, q);
+	}
+}
+
+/* CTA = (view, 128-row tile, group of 4 K steps); thread = (row, K octet).
+ * The bytes (8 read and 12 written per double, 4 and 6 per float) bound it;
+ * the digits take some 40 and 25 instructions per element.  Where K is one
+ * contiguous run and a thread's octet lies on a 16-byte boundary, it is
+ * loaded as 16-byte words, a quarter to a half of the requests for the same
+ * sectors.  With 64-bit shifts, a carry from digit to digit and 8-byte loads
+ * (some 100 and 76 instructions) both kernels of this pass together took 587
+ * us for the operands of a 53 x 187 ladder (0.87 GB read twice, 1.2 GB
+ * written), 1807 us for a float32 ring term's (2.1 GB, 3.2 GB); now 475 and
+ * 1418. */
 template <typename T>
-__global__ void __launch_bounds__(256, 6)
+__global__ void __launch_bounds__(256, 5)
 emu_split_kernel(const xmgd_view_t *__restrict__ views,
     const view_meta *__restrict__ meta, int nviews,
     const int32_t *__restrict__ tabs, const int32_t *__restrict__ E, int rowmajor)
@@ -311,48 +360,46 @@ emu_split_kernel(const xmgd_view_t *__restrict__ views,
 	/* a contiguous K run: direct loads, no offset table */
 	const bool direct = w.kcontig && !w.cplx;
 	const T *Xr = X + co + (direct ? rowt[0] : 0);
+	/* (an octet is 32 or 64 bytes: the row's alignment is every octet's) */
+	const bool wide = live && direct && ((uintptr_t)Xr & 15) == 0;
+	if (rr >= tr)
+		return;
 
 	for (int ks = g * 4; ks < min(w.n_ks, g * 4 + 4); ks++) {
+		const int k0 = ks * EMU_KS + oct * 8;
+		T x[8];
+		if (wide && k0 + 8 <= w.k) {
+			constexpr int NW = 8 * sizeof(T) / 16, PER = 16 / sizeof(T);
+			const uint4 *p = reinterpret_cast<const uint4 *>(Xr + k0);
+			uint4 u[NW];
+#pragma unroll
+			for (int i = 0; i < NW; i++)
+				u[i] = __ldg(p + i);
+#pragma unroll
+			for (int e = 0; e < 8; e++) {
+				const uint4 q = u[e / PER];
+				if constexpr (sizeof(T) == 8)
+					x[e] = e % 2 ? __hiloint2double((int)q.w, (int)q.z) :
+					    __hiloint2double((int)q.y, (int)q.x);
+				else
+					x[e] = __uint_as_float(e % 4 == 0 ? q.x : e % 4 == 1 ? q.y :
+					    e % 4 == 2 ? q.z : q.w);
+			}
+		} else {
+#pragma unroll
+			for (int e = 0; e < 8; e++)
+				x[e] = !live ? T(0) : direct ? (k0 + e < w.k ? Xr[k0 + e] : T(0)) :
+				    fetch(X, rowt, co, w, k0 + e);
+		}
 		uint32_t bits[S][4];
 #pragma unroll
-		for (int t = 0; t < S; t++)
-#pragma unroll
-			for (int q = 0; q < 4; q++)
-				bits[t][q] = 0;
-#pragma unroll
-		for (int e = 0; e < 8; e++) {
-			const int k = ks * EMU_KS + oct * 8 + e;
-			T x = !live ? T(0) : direct ? (k < w.k ? Xr[k] : T(0)) :
-			    fetch(X, rowt, co, w, k);
-			long long m;
-			int eb;
-			bool neg;
-			fin<T>::parts(x, m, eb, neg);
-			/* X = round(m * 2^(eb - er - (MANT + 1 - T1))), |X| <= 2^T1 */
-			const int sh = er - eb + (fin<T>::MANT + 1 - fin<T>::T1);
-			long long xi = sh >= 63 ? 0 : ((m + (1ll << (sh - 1))) >> sh);
-			if (neg)
-				xi = -xi;
-			int d[S];
-#pragma unroll
-			for (int t = S - 1; t >= 1; t--) {
-				d[t] = (int)(((xi + 128) & 255) - 128);
-				xi = (xi - d[t]) >> 8;
-			}
-			d[0] = (int)xi;
-#pragma unroll
-			for (int t = 0; t < S; t++) {
-				uint32_t h = digit_bf16(d[t], __int_as_float((127 - 8 * t) << 23));
-				bits[t][e >> 1] |= h << (16 * (e & 1));
-			}
-		}
+		for (int q = 0; q < 4; q++)
+			digit_pairs<S, 0>(digits_of(x[2 * q], er), digits_of(x[2 * q + 1], er), bits, q);
 		/* chunk of a tile's live rows, rounded up to 16, in core matrices
 		 * of 8 rows x 16 B, two per row group and slice.  Slice-major,
 		 * [slice][8-row group]: consecutive slices follow one another
 		 * like the rows of one wider operand.  Row-major, [8-row
 		 * group][slice]: members' chunks stack by plain concatenation */
-		if (rr >= tr)
-			continue;
 		const size_t chunk = (size_t)rt * w.n_ks * CHUNK_ELEMS +
 		    (size_t)ks * (tr * EMU_KS * S);
 		const size_t within = (size_t)(rr >> 3) * (rowmajor ? S * 128 : 128) +
