@@ -47,6 +47,7 @@
  * frees TMEM and returns, and the host reports XMG_ETIMEOUT.
  */
 #include <algorithm>
+#include <map>
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
@@ -61,7 +62,7 @@ namespace xmg {
 constexpr int EMU_TM = 128;              /* rows per tile, both operands */
 constexpr int EMU_KS = 16;               /* K per stage = K per MMA */
 constexpr int EMU_CHUNK = 16;            /* K steps per chunk, FP64 (256) */
-constexpr int EMU_CHUNK32 = 20;          /* K steps per chunk at most, FP32 */
+constexpr int EMU_CHUNK32 = 16;          /* K steps per chunk, FP32 (256) */
 constexpr int SLICE_BYTES = EMU_TM * EMU_KS * 2;          /* 4096 */
 #ifndef EMU_DW
 #define EMU_DW 16                        /* drain warps: 8 or 16 */
@@ -102,6 +103,7 @@ template <> struct fin<float> {
  * pair index. */
 struct emu_item {
 	int32_t m0, mfirst, mcount, pr;
+	int32_t cfirst;              /* first of its chunks */
 };
 
 /* a member: output block, first row of its tile in that block's view on
@@ -511,30 +513,34 @@ __device__ __forceinline__ int stages_of(int nks, int cplx)
 	return (nh + KS - 1) / KS + (nks - nh + KS - 1) / KS;
 }
 
-/* K steps [c0, c1) of the next chunk: chunks never straddle the re/im
- * boundary of a realified complex view.  An exact group g accumulates at
- * most 3 products of |d_p d_q| <= 2^14 per K element, so its integer sum
- * stays below 2^24 (exact in fp32) for chunks of up to 341 elements.
- * FP64 takes 256 (XMG_EMU_CHUNK steps, at most 20): its rounded low
- * band's error grows with the chunk (cfg2 ladder: 3.1e-13 at 160, 4.4e-13
- * at 224, 6.2e-13 at 320, against GEMM times of 35.8, 34.2 and 33.2 ms);
- * FP32, all exact, takes up to 20 steps, the steps left split into equal
- * chunks rounded up to whole stages (at most 21 steps, 336 elements; 32
- * steps: 18 + 14), so that the stages of a segment, which start at its
- * first step, never straddle a chunk boundary. */
-template <int S>
-__device__ __forceinline__ int chunk_end(int c0, int nks, int cplx, int kchunk)
-{
-	const int lim = segment_end(c0, nks, cplx);
-	if constexpr (S == fin<float>::S) {
-		constexpr int KS = stage_cfg<S>::KSTEPS;
-		const int left = lim - c0;
-		const int n = (left + EMU_CHUNK32 - 1) / EMU_CHUNK32;
-		const int len = ((left + n - 1) / n + KS - 1) / KS * KS;
-		return min(lim, c0 + len);
-	}
-	return min(lim, c0 + kchunk);
-}
+/*
+ * Chunks and runs.  Set X (see below) is drained after each chunk of K steps,
+ * set Y after each run of chunks.  An exact group g accumulates at most 3
+ * products of |d_p d_q| <= 2^14 per K element, whose integer sum is exact in
+ * fp32 up to 2^24, 341 elements.
+ *   FP64: chunks of 256 elements of one pair, or half of a realified pair
+ * (XMG_EMU_CHUNK steps, at most 20), each a run: the rounded low band's error
+ * grows with the chunk (96 x 384 ladder: 3.1e-13 at 160, 4.4e-13 at 224,
+ * 6.2e-13 at 320, against GEMM times of 35.8, 34.2 and 33.2 ms; chunks over
+ * several short pairs took 15 % off an adjoint contraction's GEMM and doubled
+ * its error).
+ *   FP32, all exact: chunks of 256 elements that go on from one pair, or half,
+ * to the next if their factors differ by a sign at most, the same for every
+ * member of a stacked tile (the MMAs negate the M side then).  Group 2 (set X,
+ * with two copies) is drained after each chunk, groups 0 and 1 (one and two
+ * products) after two of them, unless a factor is 2: D0 is then at most 2^23,
+ * D1 2^24, and D0 + D1 2^-8 below 2^24.  The drain of Y, 2700 cycles, had been
+ * in the way of each chunk (float32 ring term, 64 x 256: 19.3 ms, now 16.9).
+ * The host lists the chunks (chunk_lists); the MMA warp, short of issue slots
+ * while the drains work, took some 500 cycles to put one together.
+ */
+struct emu_chunk {
+	int32_t head;                /* stages | flags << 8 | the run's factors << 16:
+				      * two bits per member, negative and twice */
+	uint32_t neg, part;          /* per stage: negated; of one step (of two) */
+	int32_t pad;
+};
+enum { RUN_FIRST = 1, RUN_LAST = 2, ITEM_LAST = 4 };
 
 /*
  * Accumulators and MMAs of one K step.  Weight groups p + q = 0, 1, 2 have
@@ -587,6 +593,7 @@ struct mma_item {
 	uint32_t sa, sb;             /* slice strides of the descriptors */
 	uint32_t sbo;                /* bytes between 8-row groups */
 	uint32_t n;                  /* columns per accumulator */
+	uint32_t neg;                /* instruction bit: M side negated */
 };
 
 /* the products of a set for one K step whose stage step starts at base;
@@ -617,10 +624,11 @@ issue_set(const mma_item &m, uint32_t el, uint32_t tmem, uint32_t xcol, uint32_t
 		constexpr int COL = row0 && row1 ? COL_NONE : row0 ? COL_KEEP :
 		    row1 ? COL_LAST : COL_USE;
 		if constexpr (PAIR)
-			mma_bf16_pair<COL>(el, d, alo + P * m.sa, ahi, blo + Q * m.sb, bhi, m.idesc[0], acc);
+			mma_bf16_pair<COL>(el, d, alo + P * m.sa, ahi, blo + Q * m.sb, bhi,
+			    m.idesc[0] | m.neg, acc);
 		else
 			mma_bf16_split<COL>(el, d, alo + P * m.sa, ahi, blo + Q * m.sb, bhi,
-			    m.idesc[w - 1], acc);
+			    m.idesc[w - 1] | m.neg, acc);
 		issue_set<S, KEEP, CLS, SET, PAIR, P, Q + w>(m, el, tmem, xcol, alo, ahi, blo, bhi, acc0);
 	}
 }
@@ -643,12 +651,6 @@ __device__ __forceinline__ int pair_steps(int k, int cplx)
 constexpr float MAGICF = 12582912.0f;
 constexpr int MAGIC = 0x4B400000;
 
-/* V += (uint64)a << sh, 1 <= sh < 32 */
-__device__ __forceinline__ uint64_t shl64(uint32_t a, int sh)
-{
-	return ((uint64_t)(a >> (32 - sh)) << 32) | (uint32_t)(a << sh);
-}
-
 /* PAIR: a cluster of two CTAs runs each 256-row tile with cta_group::2
  * MMAs issued by rank 0: each CTA stages its own 128 M-side rows and half
  * of the N side, rank 1 forwards its stage completions to rank 0, the
@@ -661,7 +663,8 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
     const xmgd_view_t *__restrict__ va, const xmgd_view_t *__restrict__ vb,
     const int32_t *__restrict__ tabs, const int32_t *__restrict__ EA,
     const int32_t *__restrict__ EB, const int32_t *__restrict__ cbF,
-    double alpha, double beta, int expoff2, int cplx, int hmax, int kchunk, int rowmajor,
+    const emu_chunk *__restrict__ chunks, double alpha, double beta, int expoff2, int cplx,
+    int hmax, int rowmajor,
     int *__restrict__ flags)
 {
 	using C = stage_cfg<S>;
@@ -674,8 +677,14 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 	 * used by the chunks in turn */
 	constexpr bool XDB = KEEP == 2 && !PAIR;
 	constexpr uint32_t XCOL = 256;       /* their columns: 256, 384 */
-	__shared__ __align__(8) uint64_t bar_xfull, bar_yfull, bar_xempty[2], bar_yempty, bar_fin;
+	__shared__ __align__(8) uint64_t bar_xfull, bar_xempty[2], bar_yempty, bar_fin;
+	/* a chunk's products are done: two, since the MMA warp may finish a chunk
+	 * whose Y goes on before the drains have seen the end of the last one */
+	__shared__ __align__(8) uint64_t bar_yfull[2];
 	__shared__ __align__(8) uint64_t bar_ifull[2], bar_iempty[2];
+	/* the MMA warp's chunk, for the drains: its head */
+	__shared__ __align__(8) uint64_t bar_info[2];
+	__shared__ int s_head[2];
 	__shared__ __align__(8) uint64_t bar_pfull[PAIR ? NST : 1];
 	__shared__ int s_item[2];
 	__shared__ uint32_t s_tmem;
@@ -715,13 +724,15 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 			mbar_init(smem_u32(&bar_empty[s]), 1);
 		}
 		mbar_init(smem_u32(&bar_xfull), 1);
-		mbar_init(smem_u32(&bar_yfull), 1);
-		for (int q = 0; q < 2; q++)
+		for (int q = 0; q < 2; q++) {
+			mbar_init(smem_u32(&bar_yfull[q]), 1);
 			mbar_init(smem_u32(&bar_xempty[q]), PAIR ? 2 * DW : DW);
+		}
 		mbar_init(smem_u32(&bar_yempty), PAIR ? 2 * DW : DW);
 		mbar_init(smem_u32(&bar_fin), 1);
 		for (int q = 0; q < 2; q++) {
 			mbar_init(smem_u32(&bar_ifull[q]), 1);
+			mbar_init(smem_u32(&bar_info[q]), 1);
 			/* pair: both CTAs' drains, rank 0's MMA warp, rank 1's
 			 * producer and forwarder */
 			mbar_init(smem_u32(&bar_iempty[q]), PAIR ? 2 * DW + 3 : 1 + DW);
@@ -988,9 +999,9 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 					commit(bar);
 				__syncwarp();
 			};
-			/* one item of a width class: its blocks' pairs, N side and M
-			 * side slice strides; false on failure (s_err set) */
-			auto item = [&](auto cls, int n, uint32_t sa, int pair0, int npairs) -> bool {
+			/* one item of a width class: its columns, M-side slice stride,
+			 * chunks; false on failure (s_err set) */
+			auto item = [&](auto cls, int n, uint32_t sa, int cfirst) -> bool {
 				constexpr int CLS = decltype(cls)::value;
 				constexpr int KS = C::KSTEPS;
 				mma_item mi;
@@ -1004,29 +1015,32 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 				 * across them: wait for both sets' drains */
 				bool both = !XDB && !first && (int)mi.n != prevn;
 				prevn = mi.n;
-				int knext = prs[pair0].k;
-				for (int p = 0; p < npairs; p++) {
-					const int nks = pair_steps(uni(knext), cplx);
-					if (p + 1 < npairs)
-						knext = prs[pair0 + p + 1].k;
-					for (int c0 = 0; c0 < nks; ) {
-						const int c1 = chunk_end<S>(c0, nks, cplx, kchunk);
-						/* the chunk's stages: KSTEPS steps each, the last
-						 * one shorter at a segment's end */
-						const int nss = (c1 - c0 + KS - 1) / KS;
+				const int4 *cp = reinterpret_cast<const int4 *>(chunks) + cfirst;
+				int4 next = __ldg(cp);
+				uint32_t ay = 0;
+				for (bool more = true; more; ) {
+						/* (the next chunk is loaded during this one) */
+						const int head = uni(next.x), fl = head >> 8, nss = head & 0xff;
+						const uint32_t neg = uni(next.y), part = KS == 1 ? 0u : uni(next.z);
+						more = !(fl & ITEM_LAST);
+						if (more)
+							next = __ldg(++cp);
 						const uint32_t xcol = XCOL + (nch & 1) * 128;
-						/* every accumulator restarts each chunk: the exact
-						 * groups for their 2^24 bound, the low band because
-						 * the tensor core's fp32 accumulation error grows
-						 * with the accumulation length (per-pair
+						/* every accumulator restarts each chunk or run: the
+						 * exact groups for their 2^24 bound, the low band
+						 * because the tensor core's fp32 accumulation error
+						 * grows with the accumulation length (per-pair
 						 * accumulation measured 10x larger error) */
-						uint32_t ax = 0, ay = 0;
+						uint32_t ax = 0;
+						if (fl & RUN_FIRST)
+							ay = 0;
 						/* the products of stage sj, the chunk's j-th: set X
 						 * (1), set Y (2) or both (3) */
 						auto issue = [&](int sj, int j, auto which) {
 							constexpr int WH = decltype(which)::value;
 							const uint32_t base = smem_u32(stages + (size_t)sj * C::STAGE_BYTES);
-							const int nk = min(KS, c1 - c0 - j * KS);
+							const int nk = KS == 1 || (part >> j & 1) ? 1 : KS;
+							mi.neg = (neg >> j & 1) << 13;
 							for (int u = 0; u < nk; u++) {
 								const uint32_t b0 = base + u * C::STEP_BYTES;
 								const uint64_t da = sdesc(b0, mi.sbo);
@@ -1054,12 +1068,14 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 						const std::integral_constant<int, 1> X{};
 						const std::integral_constant<int, 2> Y{};
 						const std::integral_constant<int, 3> XY{};
-						/* head: the first H (staged) stages; tail: the last T
-						 * stages; middle: the rest.  H, T <= hmax <= NST: the
-						 * stages a head or tail holds are released only after
-						 * its set-Y products, so hmax < NST leaves stages for
-						 * the producer to prefetch the steps after them */
-						const int H = min(hmax, nss);
+						/* head: the first H (staged) stages, while Y is read;
+						 * tail: the last T stages; middle: the rest.  H, T <=
+						 * hmax <= NST: the stages a head or tail holds are
+						 * released only after its set-Y products, so hmax < NST
+						 * leaves stages for the producer to prefetch the steps
+						 * after them */
+						const bool ywait = !first && !both && (fl & RUN_FIRST);
+						const int H = XDB && !ywait ? 0 : min(hmax, nss);
 						const int T = XDB ? 0 : min(hmax, nss - H);
 						/* head, set X, as soon as the drain has read X of
 						 * the previous chunk (of the one before it, where X
@@ -1079,6 +1095,17 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 							yph ^= 1;
 						}
 						tc_fence_after();
+						/* (the drains have read what this slot held) */
+						if (lane == 0) {
+							const int z = nch & 1;
+							s_head[z] = head;
+							mbar_arrive(smem_u32(&bar_info[z]));
+							if (PAIR) {
+								st_remote_u32(map_shared(smem_u32(&s_head[z]), 1), (uint32_t)head);
+								mbar_arrive_remote(map_shared(smem_u32(&bar_info[z]), 1));
+							}
+						}
+						__syncwarp();
 						for (int j = 0; j < H; j++) {
 							const int sj = s + j < NST ? s + j : s + j - NST;
 							if (!ready(sj, s + j < NST ? ph : ph ^ 1))
@@ -1088,7 +1115,7 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 						if (T == 0 && !XDB)
 							done(&bar_xfull);
 						/* head, set Y, once Y is read too */
-						if (!first && !both) {
+						if (ywait) {
 							if (!wwait(&bar_yempty, yph, 8))
 								return false;
 							yph ^= 1;
@@ -1129,10 +1156,8 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 							s += T;
 							if (s >= NST) { s -= NST; ph ^= 1; }
 						}
-						done(&bar_yfull);
+						done(&bar_yfull[nch & 1]);
 						nch++;
-						c0 = c1;
-					}
 				}
 				return true;
 			};
@@ -1147,11 +1172,11 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 				if (t < 0)
 					break;
 				const emu_item it = items[t];
-				const xmgd_cblock_t cb = cbs[members[it.mfirst].cblock];
-				const int n = uni(it.pr) >> 8, p0 = uni(cb.first_pair), np = uni(cb.npairs);
-				const uint32_t sa = rowmajor ? 16 :
-				    2 * uni(tile_rows((it.pr >> 1) & 1 ? cb.m : cb.n, it.m0));
-				auto run = [&](auto cls) { return item(cls, n, sa, p0, np); };
+				const int n = uni(it.pr) >> 8, c0 = uni(it.cfirst);
+				const uint32_t sa = rowmajor ? 16 : 2 * uni(tile_rows((it.pr >> 1) & 1 ?
+				    cbs[members[it.mfirst].cblock].m : cbs[members[it.mfirst].cblock].n,
+				    it.m0));
+				auto run = [&](auto cls) { return item(cls, n, sa, c0); };
 				if (PAIR || rowmajor)
 					ok = run(std::integral_constant<int, 4>{});
 				else if constexpr (PAIR)
@@ -1181,7 +1206,7 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 		constexpr int NSEG = NC / 16;
 		const int quad = warp & 3, half = (warp - 2) >> 2;
 		const uint32_t trow = tmem + ((uint32_t)(quad * 32) << 16);
-		uint32_t fph = 0, xb = 0;
+		uint32_t nch = 0;
 		bool ok = true;
 		uint32_t iph = 0;
 		/* one lane waits, the warp follows its verdict, so the
@@ -1226,10 +1251,11 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 			 * member's output block (N-stacked members hold
 			 * multiples of 16 columns; M-stacked ones multiples of 32
 			 * lanes, so one member holds all of this warp's lanes): per
-			 * segment the output block, its first pair, its F and the
+			 * segment the output block, its member, its F and the
 			 * N-side row of the segment's first column; and the M-side
 			 * row of this warp's first lane */
-			int scb[NSEG], sfp[NSEG], sF[NSEG], sq0[NSEG], mrow0;
+			int scb[NSEG], sF[NSEG], sq0[NSEG], mrow0;
+			uint32_t smj = 0;            /* (per segment: its factor's place) */
 			if (mstk) {
 				const int row0 = quad * 32;
 				int j = 0;
@@ -1239,7 +1265,7 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 #pragma unroll
 				for (int g = 0; g < NSEG; g++) {
 					scb[g] = mb.cblock;
-					sfp[g] = cbs[mb.cblock].first_pair;
+					smj |= (uint32_t)(16 + 2 * j) << (8 * g);
 					sF[g] = cbF[mb.cblock];
 					sq0[g] = it.m0 + col0 + g * 16;
 				}
@@ -1253,13 +1279,12 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 						j += col >= members[it.mfirst + jj].off;
 					const emu_member mb = members[it.mfirst + j];
 					scb[g] = mb.cblock;
-					sfp[g] = cbs[mb.cblock].first_pair;
+					smj |= (uint32_t)(16 + 2 * j) << (8 * g);
 					sF[g] = cbF[mb.cblock];
 					sq0[g] = mb.n0 + col - mb.off;
 				}
 				mrow0 = it.m0 + (int)rank * EMU_TM + quad * 32;
 			}
-			const int npairs = cbs[scb[0]].npairs;
 			uint64_t V[NC];                  /* two's complement */
 #pragma unroll
 			for (int c = 0; c < NC; c++)
@@ -1269,8 +1294,9 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 			constexpr int W = LOW ? 8 : 4;
 			/* set X.  FP64: the low band, L in units of 2^-16 (|L| <
 			 * 2^19: 15 products of 256 times 2^14 at 2^-24, with the pair
-			 * factor's 2), to units of 2^(-16-F): V += 2^F h + l, h =
-			 * rint(L), l = rint(2^F (L - h)).  FP32: group 2, an integer */
+			 * factor's 2), to units of 2^(-16-F): V += 2^12 h + l, h =
+			 * rint(2^(F-12) L), l = rint(2^F L - 2^12 h).  FP32: group 2,
+			 * an integer */
 			auto drain_x = [&](uint32_t at, const float *s0) {
 #pragma unroll
 				for (int b = 0; b < NC; b += W) {
@@ -1294,13 +1320,13 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 						tmem_wait_ld();
 #pragma unroll
 					for (int c = 0; c < W; c++) {
-						const float sx = s0[g] * 65536.0f;
+						const float sx = s0[g] * (LOW ?
+						    __int_as_float((127 + 4 + sF[g]) << 23) : 65536.0f);
 						if (LOW) {
 							const float t = fmaf(ax[c], sx, MAGICF);
 							const float r = fmaf(ax[c], sx, MAGICF - t);
-							const float l = fmaf(r, __int_as_float((127 + sF[g]) << 23),
-							    MAGICF);
-							V[b + c] += shl64(__float_as_uint(t), sF[g]) +
+							const float l = fmaf(r, 4096.0f, MAGICF);
+							V[b + c] += ((uint64_t)__float_as_uint(t) << 12) +
 							    __float_as_uint(l);
 						} else
 							V[b + c] += (long long)__float2int_rn(ax[c] * sx);
@@ -1347,72 +1373,54 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 					}
 				}
 			};
-			int nchunk = 0;
-			/* the next pair's extent and factors are loaded during this
-			 * one's chunks */
-			int knext = prs[sfp[0]].k, esn[NSEG], ehn[NSEG];
+			/* values rounded by the magic number (FP64: in X, FP32: in Y) */
+			int nround = 0;
+			for (bool more = true; more; nch++) {
+				const int z = nch & 1;
+				if (!(ok = wwait(&bar_info[z], (nch >> 1) & 1, 11)))
+					break;
+				const int head = *(volatile int *)&s_head[z], fl = head >> 8;
+				more = !(fl & ITEM_LAST);
+				nround += LOW || (fl & RUN_LAST);
+				/* each segment's factor, sign * 2^shift (shift 0 or 1,
+				 * checked by the planner), rides on the exact fp32 -> int
+				 * scales */
+				float s0[NSEG];
 #pragma unroll
-			for (int g = 0; g < NSEG; g++) {
-				esn[g] = prs[sfp[g]].esign;
-				ehn[g] = prs[sfp[g]].eshift;
-			}
-			for (int p = 0; p < npairs && ok; p++) {
-				const int nks = pair_steps(knext, cplx);
-				float f0[NSEG];
-#pragma unroll
-				for (int g = 0; g < NSEG; g++)
-					f0[g] = (esn[g] > 0 ? 1.0f : -1.0f) *
-					    __int_as_float((127 + ehn[g]) << 23);
-				if (p + 1 < npairs) {
-					knext = prs[sfp[0] + p + 1].k;
-#pragma unroll
-					for (int g = 0; g < NSEG; g++) {
-						esn[g] = prs[sfp[g] + p + 1].esign;
-						ehn[g] = prs[sfp[g] + p + 1].eshift;
-					}
+				for (int g = 0; g < NSEG; g++) {
+					const uint32_t q = (uint32_t)head >> (smj >> (8 * g) & 0xff);
+					s0[g] = __uint_as_float((q & 1) << 31 | (127 + (q >> 1 & 1)) << 23);
 				}
-				for (int c0 = 0; c0 < nks; ) {
-					const int c1 = chunk_end<S>(c0, nks, cplx, kchunk);
-					/* each segment's pair factor sign * 2^shift (shift 0
-					 * or 1, checked by the planner) rides on the exact
-					 * fp32 -> int scales; the real pass negates the im * im
-					 * half */
-					const bool negh = cplx && !pass && c0 >= nks / 2;
-					float s0[NSEG];
-#pragma unroll
-					for (int g = 0; g < NSEG; g++)
-						s0[g] = negh ? -f0[g] : f0[g];
-					if (XDB) {
-						/* Y first: X's copy is not needed for a chunk yet */
-						if (!(ok = wait_warp(&bar_yfull, fph, 9)))
-							break;
-						drain_y(s0);
-						release(&bar_yempty);
-						drain_x(XCOL + xb * 128, s0);
-						release(&bar_xempty[xb]);
-						xb ^= 1;
-					} else {
-						/* X first, then it is free for the next chunk's head;
-						 * Y once its last products have landed */
-						if (!(ok = wait_warp(&bar_xfull, fph, 4)))
-							break;
-						drain_x((LOW ? 3 : 2) * rows, s0);
-						release(&bar_xempty[0]);
-						if (!(ok = wait_warp(&bar_yfull, fph, 9)))
-							break;
+				if (XDB) {
+					/* Y first: X's copy is not needed for a chunk yet */
+					if (!(ok = wait_warp(&bar_yfull[z], (nch >> 1) & 1, 9)))
+						break;
+					if (fl & RUN_LAST) {
 						drain_y(s0);
 						release(&bar_yempty);
 					}
-					fph ^= 1;
-					nchunk++;
-					c0 = c1;
+					drain_x(XCOL + z * 128, s0);
+					release(&bar_xempty[z]);
+				} else {
+					/* X first, then it is free for the next chunk's head;
+					 * Y once its last products have landed */
+					if (!(ok = wait_warp(&bar_xfull, nch & 1, 4)))
+						break;
+					drain_x((LOW ? 3 : 2) * rows, s0);
+					release(&bar_xempty[0]);
+					if (!(ok = wait_warp(&bar_yfull[z], (nch >> 1) & 1, 9)))
+						break;
+					if (LOW || (fl & RUN_LAST)) {
+						drain_y(s0);
+						release(&bar_yempty);
+					}
 				}
 			}
 			/* the magic numbers' bits out of the sums (modulo 2^64) */
 #pragma unroll
 			for (int c = 0; c < NC; c++)
-				V[c] -= (uint64_t)nchunk * (LOW ?
-				    shl64(MAGIC, sF[c / 16]) + MAGIC : (uint64_t)MAGIC);
+				V[c] -= (uint64_t)nround * (LOW ?
+				    ((uint64_t)MAGIC << 12) + MAGIC : (uint64_t)MAGIC);
 			if (__any_sync(0xffffffffu, !ok || s_err))
 				break;
 			/* epilogue (overlaps the next item's first chunk of MMAs):
@@ -1578,7 +1586,7 @@ struct emu_plan {
 	uint64_t d_va = 0, d_vb = 0, d_meta[2][2] = {{0, 0}, {0, 0}};
 	int64_t nctas[2][2] = {{0, 0}, {0, 0}};
 	int kr[2] = {256, 256};              /* exponent pass: K per CTA */
-	uint64_t d_E = 0, d_F = 0;
+	uint64_t d_E = 0, d_F = 0, d_chunks = 0;
 	uint64_t dbuf = 0;                   /* the allocation of all of these */
 	std::vector<xmgd_view_t> vstage;     /* bound views on their way up */
 	int64_t nE = 0;
@@ -1700,7 +1708,8 @@ launch_gemm(emu_plan *e)
 		    e->d_cbs, e->d_prs,
 		    (const xmgd_view_t *)e->d_va, (const xmgd_view_t *)e->d_vb, e->d_tabs,
 		    (const int32_t *)EA, (const int32_t *)EB, (const int32_t *)e->d_F,
-		    e->alpha, e->beta, 2 * fin<TIN>::EXPOFF, e->cplx, e->hmax, e->kchunk,
+		    (const emu_chunk *)e->d_chunks, e->alpha, e->beta, 2 * fin<TIN>::EXPOFF,
+		    e->cplx, e->hmax,
 		    (int)row_major(c.policy), flags));
 	} else {
 		emu_gemm_kernel<S, KEEP, LOW, TOUT, EMU_DW, false><<<(unsigned)c.grid,
@@ -1708,8 +1717,8 @@ launch_gemm(emu_plan *e)
 		    (const emu_item *)c.d_items, c.nitems, (const emu_member *)c.d_members,
 		    e->d_cbs, e->d_prs,
 		    (const xmgd_view_t *)e->d_va, (const xmgd_view_t *)e->d_vb, e->d_tabs,
-		    EA, EB, (const int32_t *)e->d_F, e->alpha, e->beta,
-		    2 * fin<TIN>::EXPOFF, e->cplx, e->hmax, e->kchunk,
+		    EA, EB, (const int32_t *)e->d_F, (const emu_chunk *)e->d_chunks, e->alpha,
+		    e->beta, 2 * fin<TIN>::EXPOFF, e->cplx, e->hmax,
 		    (int)row_major(c.policy), flags);
 	}
 	g_launches++;
@@ -1788,7 +1797,7 @@ make_items(const xmgd_contract_t *p, const std::vector<int> &cblocks, int cplx,
 			tot = ncols;
 		for (int ps = 0; ps < (cplx ? 2 : 1); ps++) {
 			items.push_back(emu_item{m0, (int)members.size(), (int)mem.size(),
-			    ps | (swp ? 2 : 0) | (mstk ? 4 : 0) | (tot << 8)});
+			    ps | (swp ? 2 : 0) | (mstk ? 4 : 0) | (tot << 8), 0});
 			members.insert(members.end(), mem.begin(), mem.end());
 		}
 	};
@@ -1957,6 +1966,101 @@ make_items(const xmgd_contract_t *p, const std::vector<int> &cblocks, int cplx,
 			else
 				push(t0.n0, swp, mem, 1, t0.ncols);
 		}
+	}
+}
+
+/*
+ * The chunks of every item of a list (see emu_chunk): one list per set of
+ * members and pass, shared by the items with the same ones (the index spans
+ * the candidates of a plan).
+ */
+struct chunk_index {
+	std::vector<int> one;                      /* [2 * block + pass], or -1 */
+	std::map<std::vector<int>, int> stacked;   /* pass, blocks */
+};
+
+static void
+chunk_lists(const xmgd_contract_t *p, int cplx, int kchunk, std::vector<emu_item> &items,
+    const std::vector<emu_member> &members, chunk_index &seen, std::vector<emu_chunk> &out)
+{
+	const bool dbl = p->dtype >= 2;
+	const int KS = dbl ? stage_cfg<fin<double>::S>::KSTEPS : stage_cfg<fin<float>::S>::KSTEPS;
+	std::vector<int> key;
+
+	seen.one.resize(2 * (size_t)p->ncblocks, -1);
+	for (emu_item &it : items) {
+		const int pass = it.pr & 1, nmem = it.mcount, signs = 0x55 >> (8 - 2 * nmem);
+		key.assign(1, pass);
+		for (int j = 0; j < nmem; j++)
+			key.push_back(members[it.mfirst + j].cblock);
+		int &slot = nmem == 1 ? seen.one[2 * (size_t)key[1] + pass] :
+		    seen.stacked.insert(std::make_pair(key, -1)).first->second;
+		it.cfirst = slot;
+		if (slot >= 0)
+			continue;
+		it.cfirst = slot = (int)out.size();
+		const xmgd_cblock_t &cb = p->cblocks[key[1]];
+		emu_chunk c = {};
+		int nss = 0, room = 0, code = 0, last = 0, neg = 0, run = 0;
+		bool fresh = true;
+		auto close = [&](int flags) {
+			c.head = nss | (c.head | flags) << 8 | code << 16;
+			out.push_back(c);
+			fresh = flags & RUN_LAST;
+			nss = room = 0;
+		};
+		for (int q = 0; q < cb.npairs; q++) {
+			const int steps = (p->pairs[cb.first_pair + q].k + EMU_KS - 1) / EMU_KS;
+			int pc = 0;
+			for (int j = 0; j < nmem; j++) {
+				const xmgd_pair_t &pr = p->pairs[p->cblocks[key[1 + j]].first_pair + q];
+				pc |= ((pr.esign < 0) | (pr.eshift ? 2 : 0)) << (2 * j);
+			}
+			for (int h = 0; h < (cplx ? 2 : 1); h++) {
+				/* this half's factors; after the last one's */
+				const int fc = pc ^ (h && !pass ? signs : 0);
+				if (q || h) {
+					const int x = fc ^ last;
+					if (x && x != signs) {
+						if (nss)
+							close(RUN_LAST);
+						else if (!fresh) {
+							out.back().head |= RUN_LAST << 8;
+							fresh = true;
+						}
+					} else if (x)
+						neg ^= 1;
+				}
+				last = fc;
+				for (int of = 0; of < steps; ) {
+					if (!nss) {
+						c = emu_chunk{};
+						if (fresh) {
+							code = fc;
+							neg = run = 0;
+							c.head = RUN_FIRST;
+							fresh = false;
+						}
+						room = dbl ? kchunk : EMU_CHUNK32;
+					}
+					/* a stage holds KS steps, fewer at a half's end */
+					const int left = steps - of, take = left <= room ? left : room / KS * KS;
+					const int n = (take + KS - 1) / KS;
+					if (neg)
+						c.neg |= ((1u << n) - 1) << nss;
+					nss += n;
+					if (KS == 2 && (take & 1))
+						c.part |= 1u << (nss - 1);
+					room -= take;
+					of += take;
+					if (room == 0 || take < left || (dbl && of == steps))
+						close(dbl || ++run == 2 || (code & 0xAA) ? RUN_LAST : 0);
+				}
+			}
+		}
+		if (nss)
+			close(RUN_LAST);
+		out.back().head |= (RUN_LAST | ITEM_LAST) << 8;
 	}
 }
 
@@ -2272,6 +2376,8 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 	std::vector<std::vector<emu_item>> lists;
 	std::vector<std::vector<emu_member>> mlists;
 	std::vector<double> est;
+	chunk_index seen;
+	std::vector<emu_chunk> chunks;
 	for (int pol : pols) {
 		if (known >= 0 && pol != known)
 			continue;
@@ -2282,6 +2388,7 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 		 * stand in for it */
 		if (!items_ok(p, items, mem, pair_policy(pol)))
 			continue;
+		chunk_lists(p, cplx, e->kchunk, items, mem, seen, chunks);
 		bool dup = false;
 		for (size_t l = 0; l < lists.size(); l++)
 			dup |= row_major(e->cand[l].policy) == row_major(pol) &&
@@ -2327,6 +2434,7 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 			    &e->cand[i].d_members);
 		}
 	}
+	up.add(chunks.data(), chunks.size() * sizeof(emu_chunk), &e->d_chunks);
 	if (e->cand.empty()) {
 		st = xmg_seterr(XMG_EINVAL, "split-precision path: no work list "
 		    "passed its checks");
