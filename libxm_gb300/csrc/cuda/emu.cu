@@ -418,41 +418,40 @@ emu_split_kernel(const xmgd_view_t *__restrict__ views,
 /* ------------------------------------------------------------------ */
 /* 3. grouped tcgen05 GEMM with exact drains and the fused fold        */
 
-/* V * 2^e (sign flipped by sx) as a double, assembled in integer
- * arithmetic: |V| rounded once to 53 bits (to nearest, ties to even), the
- * exponent field written directly.  Bit-identical to ldexp((double)V, e)
- * whenever the result is a normal number; false otherwise (the caller
- * takes the FP64 path).  GB300's FP64 pipe is ~1/64 of its FP32 rate, so
- * the epilogue keeps the conversion and the scaling off it. */
-__device__ __forceinline__ bool pack_f64(long long V, int e, unsigned long long sx,
-    double &out)
+/* |V| shifted up until its top bit is bit 63 (0 stays 0): words and shift */
+struct norm64 { uint32_t hi, lo; int sh; };
+__device__ __forceinline__ norm64 normalize(long long V)
 {
-	if (V == 0) {
-		out = __longlong_as_double((long long)sx);
-		return true;
-	}
-	const unsigned long long sg = (V < 0 ? 1ull << 63 : 0ull) ^ sx;
 	const unsigned long long a = V < 0 ? 0ull - (unsigned long long)V :
 	    (unsigned long long)V;
-	int msb = 63 - __clzll((long long)a);
-	const int sh = msb - 52;
-	unsigned long long m;
-	if (sh > 0) {
-		const unsigned long long rem = a & ((1ull << sh) - 1), half = 1ull << (sh - 1);
-		m = a >> sh;
-		m += (rem > half) || (rem == half && (m & 1));
-		if (m >> 53) {
-			m >>= 1;
-			msb++;
-		}
-	} else
-		m = a << -sh;
-	const int be = msb + e + 1023;
-	if (be < 1 || be > 2046)
-		return false;
-	out = __longlong_as_double((long long)(sg | ((unsigned long long)be << 52) |
-	    (m & 0xFFFFFFFFFFFFFull)));
-	return true;
+	uint32_t hi = (uint32_t)(a >> 32), lo = (uint32_t)a;
+	const bool low = hi == 0;
+	hi = low ? lo : hi;
+	lo = low ? 0 : lo;
+	const int z = __clz(hi);
+	return norm64{__funnelshift_l(lo, hi, z), lo << (z & 31), low ? z + 32 : z};
+}
+
+/* V * 2^e (sign flipped by sx) as a double, assembled in integer
+ * arithmetic: |V| rounded once to 53 bits (to nearest, ties to even), the
+ * exponent added to the mantissa with its leading bit, so that a carry out of
+ * the rounding lands in the exponent.  A result out of the normal range is
+ * scaled there by one multiplication.  Bit-identical to ldexp((double)V, e).
+ * GB300's FP64 pipe is ~1/64 of its FP32 rate, so the epilogue keeps the
+ * conversion and the scaling off it. */
+__device__ __forceinline__ double pack_f64(long long V, int e, unsigned long long sx)
+{
+	const norm64 n = normalize(V);
+	const int be = 63 - n.sh + e + 1023, bc = min(max(be, 1), 2045);
+	const uint32_t lo = __funnelshift_r(n.lo, n.hi, 11), hi = n.hi >> 11;
+	const uint32_t up = (n.lo & 0x7ff) + (lo & 1) > 0x400;
+	const unsigned long long b = (((unsigned long long)hi << 32) | lo) + up +
+	    ((unsigned long long)(bc - 1) << 52);
+	const double v = __longlong_as_double((long long)((V ? b : 0ull) |
+	    ((V < 0 ? 1ull << 63 : 0ull) ^ sx)));
+	if (be == bc)
+		return v;
+	return v * __longlong_as_double((long long)(1023 + min(max(be - bc, -1022), 1023)) << 52);
 }
 
 /* A pipeline stage holds KSTEPS consecutive 16-wide K steps (each the
@@ -1438,38 +1437,59 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 			const int esa = apow2 ? aex - 1023 : 0;
 			const unsigned long long asx = apow2 ?
 			    (unsigned long long)ab & (1ull << 63) : 0ull;
+			/* a segment's 16 columns: their exponents and offsets are
+			 * loaded once, a column per lane, and C's old values eight at a
+			 * time, before any is stored: one by one, each waits for the
+			 * last one's store and for memory (complex128 ring term, 21 x
+			 * 75: 90600 cycles a CTA, now 62200 of 550000) */
 #pragma unroll
 			for (int g = 0; g < NSEG; g++) {
 				if (g * 16 >= cw)
 					break;
 				const xmgd_cblock_t cb = cbs[scb[g]];
 				const int flim = swp ? cb.m : cb.n, vlim = swp ? cb.n : cb.m;
-				if (ms >= flim)
-					continue;
-				TOUT *Cp = reinterpret_cast<TOUT *>(cb.c_ptr);
-				const int32_t *vtab = tabs + (swp ? cb.ccol : cb.crow);
-				const int32_t *vexp = swp ? EB + cb.eB : EA + cb.eA;
-				const int32_t fo = tabs[(swp ? cb.crow : cb.ccol) + ms];
-				const int fe = (swp ? EA + cb.eA : EB + cb.eB)[ms];
-				const int F = sF[g];
+				const int nq = min(min(vlim - sq0[g], rows - col0 - g * 16), 16);
+				TOUT *Cp = reinterpret_cast<TOUT *>(cb.c_ptr) + pass;
+				int ve = 0, vo = 0, fo = 0, fe = 0;
+				if ((lane & 15) < nq) {
+					const int q = sq0[g] + (lane & 15);
+					ve = (swp ? EB + cb.eB : EA + cb.eA)[q];
+					vo = tabs[(swp ? cb.ccol : cb.crow) + q];
+				}
+				const bool live = ms < flim;
+				if (live) {
+					fo = tabs[(swp ? cb.crow : cb.ccol) + ms];
+					fe = (swp ? EA + cb.eA : EB + cb.eB)[ms];
+				}
+				const int e0 = fe - expoff2 - 16 - sF[g];
 #pragma unroll
-				for (int c = 0; c < 16; c++) {
-					const int q = sq0[g] + c;
-					if (q < vlim && col0 + g * 16 + c < rows) {
-						const int e = vexp[q] + fe - expoff2 - 16 - F;
-						double v;
-						if (!pack_f64((long long)V[g * 16 + c], e + esa, asx, v))
-							v = alpha * ldexp((double)(long long)V[g * 16 + c], e);
-						else if (!apow2)
-							v *= alpha;
-						TOUT *cp = Cp + (size_t)cm * (vtab[q] + fo) + pass;
-						*cp = bz ? (TOUT)v : (TOUT)fma(beta, (double)*cp, v);
+				for (int c0 = 0; c0 < 16; c0 += 8) {
+					TOUT old[8];
+					if (!bz) {
+#pragma unroll
+						for (int c = 0; c < 8; c++) {
+							const int o = __shfl_sync(0xffffffffu, vo, c0 + c) + fo;
+							old[c] = live && c0 + c < nq ? Cp[(size_t)cm * o] : TOUT(0);
+						}
+					}
+#pragma unroll
+					for (int c = 0; c < 8; c++) {
+						const int e = __shfl_sync(0xffffffffu, ve, c0 + c) + e0;
+						const int o = __shfl_sync(0xffffffffu, vo, c0 + c) + fo;
+						if (live && c0 + c < nq) {
+							const long long x = (long long)V[g * 16 + c0 + c];
+							TOUT *cp = Cp + (size_t)cm * o;
+							double v = pack_f64(x, e + esa, asx);
+							if (!apow2)
+								v *= alpha;
+							*cp = bz ? (TOUT)v : (TOUT)fma(beta, (double)old[c], v);
+						}
 					}
 				}
 			}
 		}
 	}
-	/* the producer, MMA and forwarder roles run on lane 0 alone: their
+	/* the forwarder role runs on lane 0 alone, waits may leave lanes apart: the
 	 * warps reconverge first, because an aligned barrier counts a whole
 	 * warp as arrived when any of its lanes arrives, and TMEM must stay
 	 * allocated until the MMA lane has seen its last commit land */
