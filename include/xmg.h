@@ -35,7 +35,9 @@ const char *xmg_last_error(void);
  *                    FP32 partial sums drained into 64-bit integers, FP64
  *                    only for scaling and the alpha*AB + beta*C fold.
  *   XMG_PREC_AUTO  - EMU64 where it applies (power-of-two block-pair
- *                    factors), FP64 elsewhere.  Default.
+ *                    factors) and pays (a contraction that one FP64 kernel
+ *                    finishes in a few microseconds runs there), FP64
+ *                    elsewhere.  Default.
  * float uses a compensated bf16 split in EMU modes and FP32 FMA in FP64
  * mode; complex types decompose into real products.  The environment
  * variable XMG_PRECISION=fp64|emu64|auto sets the initial mode. */

@@ -6,8 +6,8 @@
  * precision tensor-core path or the plain path, and stages the work lists.
  * xmgd_plan_run replays the whole launch sequence -- beta-only blocks,
  * exponent and split kernels, the persistent grouped GEMM, the plain GEMM
- * -- as one CUDA graph captured on first use (one graph per autotuner
- * candidate while tuning), then reads the device flags once.  Operands with
+ * -- directly for the first runs, which also tune, and as CUDA graphs from
+ * the third on, then reads the device flags once.  Operands with
  * Inf/NaN make the split-precision GEMM write nothing; those blocks are then
  * recomputed on the plain FP64 path (AUTO) or reported (EMU64).
  */

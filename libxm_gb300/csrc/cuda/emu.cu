@@ -31,12 +31,13 @@
  *     ~1 TFLOP/s.  The output is pre-tiled in the exact shared-memory image
  *     the MMA reads (no-swizzle K-major core matrices), so the GEMM loads a
  *     K step of a tile with one 1-D bulk copy per operand.
- *  3. emu_gemm_kernel  - one CTA per (output block, 128 x 128 tile, pass);
+ *  3. emu_gemm_kernel  - persistent, items of (output blocks, 128 x <= 128
+ *     tile, pass);
  *     warp 0 streams stages with cp.async.bulk, warp 1 issues the slice
  *     products per 16-wide K step with tcgen05.mma.kind::f16 (bf16 x bf16 ->
  *     fp32) into TMEM accumulators, warps 2..17 drain them every 256 K
- *     elements for FP64 and every <= 336 for FP32 (the exact groups stay
- *     below 3 * 336 * 2^14 < 2^24, exact in fp32) into
+ *     elements (groups 0 and 1 of FP32 every 512; the exact groups stay
+ *     below 2^24, exact in fp32) into
  *     per-thread int64 fixed-point sums in units of 2^(-16-F), applying the
  *     pair factor exactly.  The epilogue is the only FP64 work:
  *     C = alpha * 2^(eA + eB - 2 * EXPOFF - 16 - F) * V + beta * C, scattered
