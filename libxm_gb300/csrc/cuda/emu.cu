@@ -104,8 +104,18 @@ template <> struct fin<float> {
  * pair index. */
 struct emu_item {
 	int32_t m0, mfirst, mcount, pr;
-	int32_t cfirst;              /* first of its chunks */
+	int32_t cfirst, ccount;      /* its chunks */
+	int32_t p0, k0, steps;       /* first pair, first K step in it, K steps */
+	int32_t slot, parts;         /* sums shared by this many items (below) */
 };
+
+/* Where a list leaves SMs idle, the K steps of an item are divided among
+ * several (split_items).  Each adds its 64-bit sums to the slot's, warp by warp,
+ * and the warp that finds itself the last one of its place runs the epilogue on
+ * the total: integers, so that the order does not matter.  A slot: 16 warps x
+ * 32 columns x 32 lanes of sums, then the warps' counters. */
+constexpr size_t SLOT_SUMS = (size_t)EMU_DW * (128 / (EMU_DW / 4)) * 32;
+constexpr size_t SLOT_BYTES = SLOT_SUMS * 8 + 256;
 
 /* a member: output block, first row of its tile in that block's view on
  * the stacked side, live rows (rounded up), first TMEM column or lane */
@@ -665,7 +675,7 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
     const int32_t *__restrict__ EB, const int32_t *__restrict__ cbF,
     const emu_chunk *__restrict__ chunks, double alpha, double beta, int expoff2, int cplx,
     int hmax, int rowmajor,
-    int *__restrict__ flags)
+    unsigned char *__restrict__ slots, int *__restrict__ flags)
 {
 	using C = stage_cfg<S>;
 	constexpr int NST = C::NST;
@@ -887,8 +897,9 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 			/* the next pair's operand addresses are loaded while this
 			 * one's steps are staged (two dependent loads) */
 			pair_src nxt;
-			load_pair(0, nxt);
-			for (int p = 0; p < npairs && ok; p++) {
+			int p = uni(it.p0), ks = uni(it.k0), todo = uni(it.steps);
+			load_pair(p, nxt);
+			for (; todo > 0 && ok; p++, ks = 0) {
 				const int nks = pair_steps(uni(nxt.k), cplx);
 				const uint8_t *gs = tile_at(nxt.gs, stile, nks), *gn[EMU_MAXMEM];
 #pragma unroll
@@ -897,7 +908,7 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 						gn[j] = tile_at(nxt.gn[j], mrt[j], nks) + mso;
 				if (p + 1 < npairs)
 					load_pair(p + 1, nxt);
-				for (int ks = 0; ks < nks; ) {
+				while (ks < nks && todo > 0) {
 					const int ke = super_end<S>(ks, nks, cplx);
 					if (!(ok = wwait(&bar_empty[s], ph ^ 1, 1)))
 						break;
@@ -927,6 +938,7 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 						if (q == s)
 							lastp[q] = (int)ph;
 					if (++s == NST) { s = 0; ph ^= 1; }
+					todo -= ke - ks;
 					ks = ke;
 				}
 			}
@@ -1001,7 +1013,7 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 			};
 			/* one item of a width class: its columns, M-side slice stride,
 			 * chunks; false on failure (s_err set) */
-			auto item = [&](auto cls, int n, uint32_t sa, int cfirst) -> bool {
+			auto item = [&](auto cls, int n, uint32_t sa, int cfirst, int ccount) -> bool {
 				constexpr int CLS = decltype(cls)::value;
 				constexpr int KS = C::KSTEPS;
 				mma_item mi;
@@ -1020,9 +1032,10 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 				uint32_t ay = 0;
 				for (bool more = true; more; ) {
 						/* (the next chunk is loaded during this one) */
-						const int head = uni(next.x), fl = head >> 8, nss = head & 0xff;
+						more = --ccount > 0;
+						const int head = uni(next.x) | (more ? 0 : ITEM_LAST << 8);
+						const int fl = head >> 8, nss = head & 0xff;
 						const uint32_t neg = uni(next.y), part = KS == 1 ? 0u : uni(next.z);
-						more = !(fl & ITEM_LAST);
 						if (more)
 							next = __ldg(++cp);
 						const uint32_t xcol = XCOL + (nch & 1) * 128;
@@ -1172,11 +1185,11 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 				if (t < 0)
 					break;
 				const emu_item it = items[t];
-				const int n = uni(it.pr) >> 8, c0 = uni(it.cfirst);
+				const int n = uni(it.pr) >> 8, c0 = uni(it.cfirst), cn = uni(it.ccount);
 				const uint32_t sa = rowmajor ? 16 : 2 * uni(tile_rows((it.pr >> 1) & 1 ?
 				    cbs[members[it.mfirst].cblock].m : cbs[members[it.mfirst].cblock].n,
 				    it.m0));
-				auto run = [&](auto cls) { return item(cls, n, sa, c0); };
+				auto run = [&](auto cls) { return item(cls, n, sa, c0, cn); };
 				if (PAIR || rowmajor)
 					ok = run(std::integral_constant<int, 4>{});
 				else if constexpr (PAIR)
@@ -1423,6 +1436,29 @@ emu_gemm_kernel(const emu_item *__restrict__ items, int nitems,
 				    ((uint64_t)MAGIC << 12) + MAGIC : (uint64_t)MAGIC);
 			if (__any_sync(0xffffffffu, !ok || s_err))
 				break;
+			if (it.parts > 1) {
+				unsigned long long *sum = reinterpret_cast<unsigned long long *>(slots +
+				    it.slot * SLOT_BYTES) + (size_t)(warp - 2) * NC * 32 + lane;
+				int *count = reinterpret_cast<int *>(slots + it.slot * SLOT_BYTES +
+				    SLOT_SUMS * 8) + warp - 2;
+#pragma unroll
+				for (int c = 0; c < NC; c++)
+					if (c < cw)
+						atomicAdd(sum + c * 32, (unsigned long long)V[c]);
+				__threadfence();
+				__syncwarp();
+				int before = 0;
+				if (lane == 0)
+					before = atomicAdd(count, 1);
+				before = __shfl_sync(0xffffffffu, before, 0);
+				if (before != it.parts - 1)
+					continue;
+				__threadfence();
+#pragma unroll
+				for (int c = 0; c < NC; c++)
+					if (c < cw)
+						V[c] = __ldcg(sum + c * 32);
+			}
 			/* epilogue (overlaps the next item's first chunk of MMAs):
 			 * this thread's TMEM lane is one M-side row; its columns are
 			 * N-side rows of the segments' output blocks.  Without swap
@@ -1595,7 +1631,7 @@ static std::vector<tune_entry> g_tuned;
 struct emu_cand {
 	int policy;
 	uint64_t d_items, d_members;
-	int nitems, grid;
+	int nitems, grid, nslots;
 	float ms;
 };
 
@@ -1612,7 +1648,7 @@ struct emu_plan {
 	std::vector<xmgd_view_t> vstage;     /* bound views on their way up */
 	int64_t nE = 0;
 	int32_t nexp_a = 0;
-	size_t slice_bytes = 0;
+	size_t slice_bytes = 0, slot_bytes = 0;  /* slots follow the slices */
 	uint64_t ws = 0;                     /* workspace the views point into */
 	const xmgd_cblock_t *d_cbs;
 	const xmgd_pair_t *d_prs;
@@ -1652,6 +1688,13 @@ launch_side(emu_plan *e, int side, int kind, int32_t *E, int *flags, cudaStream_
 	return XMG_OK;
 }
 
+/* the slots' place in the workspace */
+static size_t
+slot_offset(const emu_plan *e)
+{
+	return (e->slice_bytes + 255) & ~(size_t)255;
+}
+
 /* exponent tables, then unfold + split of every used view of both sides.
  * The two sides are independent chains of two kernels: a's runs on a second
  * stream beside b's (two branches of the captured graph), since on small
@@ -1668,6 +1711,9 @@ launch_split(emu_plan *e)
 
 	XMG_CK(cudaMemsetAsync((void *)e->d_E, 0, (e->nE + 64) * sizeof(int32_t),
 	    stream()));
+	if (e->cand[e->cur].nslots)
+		XMG_CK(cudaMemsetAsync((void *)(e->ws + slot_offset(e)), 0,
+		    e->cand[e->cur].nslots * SLOT_BYTES, stream()));
 	if (!e->a_mode) {
 		cudaStream_t aux;
 		if ((st = fork_aux(&aux)) ||
@@ -1710,6 +1756,8 @@ launch_gemm(emu_plan *e)
 	if (e->a_mode)
 		EA = (int32_t *)e->a_E;	/* the shared a side's table */
 
+	unsigned char *slots = (unsigned char *)(e->ws + slot_offset(e));
+
 	if (pair_policy(c.policy)) {
 		/* clusters of two CTAs */
 		cudaLaunchConfig_t cfg = {};
@@ -1731,7 +1779,7 @@ launch_gemm(emu_plan *e)
 		    (const int32_t *)EA, (const int32_t *)EB, (const int32_t *)e->d_F,
 		    (const emu_chunk *)e->d_chunks, e->alpha, e->beta, 2 * fin<TIN>::EXPOFF,
 		    e->cplx, e->hmax,
-		    (int)row_major(c.policy), flags));
+		    (int)row_major(c.policy), slots, flags));
 	} else {
 		emu_gemm_kernel<S, KEEP, LOW, TOUT, EMU_DW, false><<<(unsigned)c.grid,
 		    64 + 32 * EMU_DW, stage_cfg<S>::SMEM, stream()>>>(
@@ -1740,7 +1788,7 @@ launch_gemm(emu_plan *e)
 		    (const xmgd_view_t *)e->d_va, (const xmgd_view_t *)e->d_vb, e->d_tabs,
 		    EA, EB, (const int32_t *)e->d_F, (const emu_chunk *)e->d_chunks, e->alpha,
 		    e->beta, 2 * fin<TIN>::EXPOFF, e->cplx, e->hmax,
-		    (int)row_major(c.policy), flags);
+		    (int)row_major(c.policy), slots, flags);
 	}
 	g_launches++;
 	XMG_CK(cudaGetLastError());
@@ -1818,7 +1866,7 @@ make_items(const xmgd_contract_t *p, const std::vector<int> &cblocks, int cplx,
 			tot = ncols;
 		for (int ps = 0; ps < (cplx ? 2 : 1); ps++) {
 			items.push_back(emu_item{m0, (int)members.size(), (int)mem.size(),
-			    ps | (swp ? 2 : 0) | (mstk ? 4 : 0) | (tot << 8), 0});
+			    ps | (swp ? 2 : 0) | (mstk ? 4 : 0) | (tot << 8)});
 			members.insert(members.end(), mem.begin(), mem.end());
 		}
 	};
@@ -1998,6 +2046,8 @@ make_items(const xmgd_contract_t *p, const std::vector<int> &cblocks, int cplx,
 struct chunk_index {
 	std::vector<int> one;                      /* [2 * block + pass], or -1 */
 	std::map<std::vector<int>, int> stacked;   /* pass, blocks */
+	std::vector<std::pair<int, int>> size;     /* chunks, steps of the list that
+	                                            * starts there */
 };
 
 static void
@@ -2016,9 +2066,14 @@ chunk_lists(const xmgd_contract_t *p, int cplx, int kchunk, std::vector<emu_item
 			key.push_back(members[it.mfirst + j].cblock);
 		int &slot = nmem == 1 ? seen.one[2 * (size_t)key[1] + pass] :
 		    seen.stacked.insert(std::make_pair(key, -1)).first->second;
+		it.p0 = it.k0 = it.slot = it.steps = 0;
+		it.parts = 1;
 		it.cfirst = slot;
-		if (slot >= 0)
+		if (slot >= 0) {
+			it.ccount = seen.size[slot].first;
+			it.steps = seen.size[slot].second;
 			continue;
+		}
 		it.cfirst = slot = (int)out.size();
 		const xmgd_cblock_t &cb = p->cblocks[key[1]];
 		emu_chunk c = {};
@@ -2033,6 +2088,7 @@ chunk_lists(const xmgd_contract_t *p, int cplx, int kchunk, std::vector<emu_item
 		for (int q = 0; q < cb.npairs; q++) {
 			const int steps = (p->pairs[cb.first_pair + q].k + EMU_KS - 1) / EMU_KS;
 			int pc = 0;
+			it.steps += (cplx ? 2 : 1) * steps;
 			for (int j = 0; j < nmem; j++) {
 				const xmgd_pair_t &pr = p->pairs[p->cblocks[key[1 + j]].first_pair + q];
 				pc |= ((pr.esign < 0) | (pr.eshift ? 2 : 0)) << (2 * j);
@@ -2081,7 +2137,10 @@ chunk_lists(const xmgd_contract_t *p, int cplx, int kchunk, std::vector<emu_item
 		}
 		if (nss)
 			close(RUN_LAST);
-		out.back().head |= (RUN_LAST | ITEM_LAST) << 8;
+		out.back().head |= RUN_LAST << 8;
+		it.ccount = (int)out.size() - slot;
+		seen.size.resize(out.size());
+		seen.size[slot] = std::make_pair(it.ccount, it.steps);
 	}
 }
 
@@ -2203,6 +2262,120 @@ list_cycles(const xmgd_contract_t *p, const std::vector<emu_item> &items,
 		top = std::max(top, c);
 	}
 	return std::max(top, sum / std::max(1, num_sms()));
+}
+
+/*
+ * Lists of a few items per SM: the longest ones first, in eight classes (the
+ * order within a class, which shares operands, stays), and items divided along
+ * K where that ends a list sooner by a model: the SMs' share and 0.6 of the
+ * longest item, or the rounds of the longest; parts of at least four chunks and
+ * about all, a half, a third or a quarter of an SM's share.  A part costs some
+ * 8000 cycles beside its steps (the pipeline's ends, the sums' way through L2).
+ * GEMM of a 53 x 187 ladder (some 900 items, ordered) 1619 -> 1486 us, of a
+ * complex128 ring term, 21 x 75 (divided) 428 -> 383 us; 16 items per SM and
+ * more are even enough.  Returns the number of slots.
+ */
+static int
+split_items(const xmgd_contract_t *p, int cplx, bool rowmajor,
+    const std::vector<emu_chunk> &chunks, const std::vector<emu_member> &members,
+    std::vector<emu_item> &items)
+{
+	const double over = 8000;
+	const int KS = p->dtype >= 2 ? stage_cfg<fin<double>::S>::KSTEPS :
+	    stage_cfg<fin<float>::S>::KSTEPS;
+	std::vector<double> cost;
+	double sum = 0, top = 0;
+
+	if ((int)items.size() >= 16 * num_sms())
+		return 0;
+	for (const emu_item &it : items) {
+		cost.push_back(over + it.steps * step_cycles(p->dtype >= 2, rowmajor, it.pr >> 8));
+		sum += cost.back();
+		top = std::max(top, cost.back());
+	}
+	/* parts of an item at a target */
+	auto parts = [&](size_t i, double target) {
+		const int most = std::max(1, items[i].ccount / 4);
+		return std::max(1, std::min(most, (int)ceil(cost[i] / target - 0.25)));
+	};
+	auto model = [&](double total, double longest, size_t n) {
+		const double rounds = (double)((n + num_sms() - 1) / num_sms());
+		return std::min(total / num_sms() + 0.6 * longest, rounds * longest);
+	};
+	double best = 0.93 * model(sum, top, items.size()), target = 0;
+	for (int w = 1; w <= 4 && (int)items.size() < 8 * num_sms(); w++) {
+		const double t = sum / num_sms() / w;
+		double total = 0, longest = 0;
+		size_t count = 0;
+		for (size_t i = 0; i < items.size(); i++) {
+			const int n = parts(i, t);
+			const double c = (cost[i] - over) / n + over;
+			total += n * c;
+			count += n;
+			longest = std::max(longest, c);
+		}
+		if (model(total, longest, count) < best) {
+			best = model(total, longest, count);
+			target = t;
+		}
+	}
+	std::vector<std::pair<double, emu_item>> out;
+	int slots = 0;
+	for (size_t i = 0; i < items.size(); i++) {
+		const emu_item &it = items[i];
+		const int n = target > 0 ? parts(i, target) : 1;
+		if (n == 1) {
+			out.push_back(std::make_pair(cost[i], it));
+			continue;
+		}
+		/* cut after the run in which each part's share of steps ends */
+		const xmgd_cblock_t &cb = p->cblocks[members[it.mfirst].cblock];
+		emu_item x = it;
+		x.slot = slots;
+		x.steps = 0;
+		x.cfirst = it.cfirst;
+		std::vector<emu_item> mine;
+		int done = 0, pair = 0, k = 0;
+		for (int c = 0; c < it.ccount; c++) {
+			const emu_chunk &ch = chunks[it.cfirst + c];
+			const int st = (ch.head & 0xff) * KS - __builtin_popcount(ch.part);
+			x.steps += st;
+			const bool last = c + 1 == it.ccount;
+			if (last || ((ch.head >> 8 & RUN_LAST) && (int)mine.size() + 1 < n &&
+			    done + x.steps >= (long long)it.steps * ((int)mine.size() + 1) / n)) {
+				x.ccount = it.cfirst + c + 1 - x.cfirst;
+				x.p0 = pair;
+				x.k0 = k;
+				mine.push_back(x);
+				done += x.steps;
+				/* where the next part starts */
+				for (k += x.steps; pair < cb.npairs; pair++) {
+					const int nks = (cplx ? 2 : 1) *
+					    ((p->pairs[cb.first_pair + pair].k + EMU_KS - 1) / EMU_KS);
+					if (k < nks)
+						break;
+					k -= nks;
+				}
+				x.cfirst += x.ccount;
+				x.steps = 0;
+			}
+		}
+		for (emu_item &y : mine) {
+			y.parts = (int)mine.size();
+			out.push_back(std::make_pair((cost[i] - over) * y.steps / it.steps + over, y));
+		}
+		slots += mine.size() > 1;
+	}
+	top = 0;
+	for (const auto &o : out)
+		top = std::max(top, o.first);
+	std::stable_sort(out.begin(), out.end(),
+	    [&](const std::pair<double, emu_item> &x, const std::pair<double, emu_item> &y) {
+		return (int)(8 * x.first / top) > (int)(8 * y.first / top); });
+	items.clear();
+	for (const auto &o : out)
+		items.push_back(o.second);
+	return slots;
 }
 
 /* bytes of one K step of a view with mn rows: whole tiles, then the last
@@ -2394,7 +2567,7 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 		pols.erase(std::remove_if(pols.begin(), pols.end(),
 		    [](int q) { return !row_major(q); }), pols.end());
 	}
-	std::vector<std::vector<emu_item>> lists;
+	std::vector<std::vector<emu_item>> lists, whole;   /* whole: undivided */
 	std::vector<std::vector<emu_member>> mlists;
 	std::vector<double> est;
 	chunk_index seen;
@@ -2410,23 +2583,28 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 		if (!items_ok(p, items, mem, pair_policy(pol)))
 			continue;
 		chunk_lists(p, cplx, e->kchunk, items, mem, seen, chunks);
+		const double cycles = list_cycles(p, items, mem, cplx, row_major(pol));
 		bool dup = false;
 		for (size_t l = 0; l < lists.size(); l++)
 			dup |= row_major(e->cand[l].policy) == row_major(pol) &&
 			    pair_policy(e->cand[l].policy) == pair_policy(pol) &&
-			    lists[l].size() == items.size() && mlists[l].size() == mem.size() &&
-			    memcmp(lists[l].data(), items.data(), items.size() * sizeof(emu_item)) == 0 &&
+			    whole[l].size() == items.size() && mlists[l].size() == mem.size() &&
+			    memcmp(whole[l].data(), items.data(), items.size() * sizeof(emu_item)) == 0 &&
 			    memcmp(mlists[l].data(), mem.data(), mem.size() * sizeof(emu_member)) == 0;
 		if (dup)
 			continue;
 		emu_cand c;
 		c.policy = pol;
+		whole.push_back(items);
+		c.nslots = pair_policy(pol) ? 0 :
+		    split_items(p, cplx, row_major(pol), chunks, mem, items);
+		e->slot_bytes = std::max(e->slot_bytes, c.nslots * SLOT_BYTES);
 		c.nitems = (int)items.size();
 		c.grid = pair_policy(pol) ? 2 * std::min(c.nitems, num_sms() / 2) :
 		    std::min(c.nitems, num_sms());
 		c.ms = -1;
 		c.d_items = c.d_members = 0;
-		est.push_back(list_cycles(p, items, mem, cplx, row_major(pol)));
+		est.push_back(cycles);
 		e->cand.push_back(c);
 		lists.push_back(std::move(items));
 		mlists.push_back(std::move(mem));
@@ -2484,7 +2662,7 @@ emu_bind(emu_plan *e, bool *moved)
 	int st;
 
 	*moved = false;
-	if ((st = xmgd_scratch(8, e->slice_bytes + 16, &ws)) != XMG_OK)
+	if ((st = xmgd_scratch(8, slot_offset(e) + e->slot_bytes + 16, &ws)) != XMG_OK)
 		return st;
 	if (ws == e->ws)
 		return XMG_OK;
