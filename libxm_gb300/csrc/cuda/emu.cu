@@ -2266,10 +2266,13 @@ list_cycles(const xmgd_contract_t *p, const std::vector<emu_item> &items,
 
 /*
  * Lists of a few items per SM: the longest ones first, in eight classes (the
- * order within a class, which shares operands, stays), and items divided along
- * K where that ends a list sooner by a model: the SMs' share and 0.6 of the
+ * order within a class, which shares operands, stays; not worth the host's 10
+ * to 20 us for lists of less than 0.8 ms), and items divided along K where that
+ * ends a list sooner by a model: the SMs' share and 0.6 of the
  * longest item, or the rounds of the longest; parts of at least four chunks and
- * about all, a half, a third or a quarter of an SM's share.  A part costs some
+ * about all, a half, a third or a quarter of an SM's share.  (Dividing lists of
+ * less than a quarter of a millisecond costs the host more than it gives: an
+ * adjoint of new tensors, two GEMMs of 0.2 ms, 1575 -> 1680 us with it.)  A part costs some
  * 8000 cycles beside its steps (the pipeline's ends, the sums' way through L2).
  * GEMM of a 53 x 187 ladder (some 900 items, ordered) 1619 -> 1486 us, of a
  * complex128 ring term, 21 x 75 (divided) 428 -> 383 us; 16 items per SM and
@@ -2283,35 +2286,43 @@ split_items(const xmgd_contract_t *p, int cplx, bool rowmajor,
 	const double over = 8000;
 	const int KS = p->dtype >= 2 ? stage_cfg<fin<double>::S>::KSTEPS :
 	    stage_cfg<fin<float>::S>::KSTEPS;
-	std::vector<double> cost;
-	double sum = 0, top = 0;
+	const size_t n = items.size(), sms = (size_t)num_sms();
+	double width[EMU_TM / 16 + 1], sum = 0, top = 0;
 
-	if ((int)items.size() >= 16 * num_sms())
+	if (n >= 16 * sms)
 		return 0;
-	for (const emu_item &it : items) {
-		cost.push_back(over + it.steps * step_cycles(p->dtype >= 2, rowmajor, it.pr >> 8));
-		sum += cost.back();
-		top = std::max(top, cost.back());
+	for (int w = 1; w <= EMU_TM / 16; w++)
+		width[w] = step_cycles(p->dtype >= 2, rowmajor, 16 * w);
+	std::vector<double> cost(n);
+	for (size_t i = 0; i < n; i++) {
+		cost[i] = over + items[i].steps * width[items[i].pr >> 12];
+		sum += cost[i];
+		top = std::max(top, cost[i]);
 	}
-	/* parts of an item at a target */
+	/* parts of an item at a target (none below a quarter above it) */
 	auto parts = [&](size_t i, double target) {
-		const int most = std::max(1, items[i].ccount / 4);
-		return std::max(1, std::min(most, (int)ceil(cost[i] / target - 0.25)));
+		if (cost[i] <= 1.25 * target)
+			return 1;
+		return std::max(1, std::min(items[i].ccount / 4, (int)ceil(cost[i] / target - 0.25)));
 	};
-	auto model = [&](double total, double longest, size_t n) {
-		const double rounds = (double)((n + num_sms() - 1) / num_sms());
-		return std::min(total / num_sms() + 0.6 * longest, rounds * longest);
+	auto model = [&](double total, double longest, size_t count) {
+		const double rounds = (double)((count + sms - 1) / sms);
+		return std::min(total / sms + 0.6 * longest, rounds * longest);
 	};
-	double best = 0.93 * model(sum, top, items.size()), target = 0;
-	for (int w = 1; w <= 4 && (int)items.size() < 8 * num_sms(); w++) {
-		const double t = sum / num_sms() / w;
+	double best = 0.93 * model(sum, top, n), target = 0;
+	const char *div = getenv("XMG_EMU_DIVIDE");  /* 1: short lists too */
+	const bool divide = n < 8 * sms && (sum / sms >= 2.8e5 || (div && atoi(div) == 1));
+	for (int w = 1; w <= 4 && divide; w++) {
+		const double t = sum / sms / w;
 		double total = 0, longest = 0;
 		size_t count = 0;
-		for (size_t i = 0; i < items.size(); i++) {
-			const int n = parts(i, t);
-			const double c = (cost[i] - over) / n + over;
-			total += n * c;
-			count += n;
+		if (top <= 1.25 * t)
+			continue;
+		for (size_t i = 0; i < n; i++) {
+			const int q = parts(i, t);
+			const double c = q == 1 ? cost[i] : (cost[i] - over) / q + over;
+			total += q * c;
+			count += q;
 			longest = std::max(longest, c);
 		}
 		if (model(total, longest, count) < best) {
@@ -2319,62 +2330,73 @@ split_items(const xmgd_contract_t *p, int cplx, bool rowmajor,
 			target = t;
 		}
 	}
-	std::vector<std::pair<double, emu_item>> out;
+	if (target == 0 && sum / sms < 1.5e6)
+		return 0;
+	std::vector<emu_item> out;
 	int slots = 0;
-	for (size_t i = 0; i < items.size(); i++) {
+	out.reserve(n);
+	std::vector<double> c2;
+	for (size_t i = 0; i < n && target > 0; i++) {
 		const emu_item &it = items[i];
-		const int n = target > 0 ? parts(i, target) : 1;
-		if (n == 1) {
-			out.push_back(std::make_pair(cost[i], it));
+		const int q = parts(i, target);
+		const size_t at = out.size();
+		if (q == 1) {
+			out.push_back(it);
+			c2.push_back(cost[i]);
 			continue;
 		}
 		/* cut after the run in which each part's share of steps ends */
 		const xmgd_cblock_t &cb = p->cblocks[members[it.mfirst].cblock];
 		emu_item x = it;
+		int done = 0, pair = 0, k = 0;
 		x.slot = slots;
 		x.steps = 0;
-		x.cfirst = it.cfirst;
-		std::vector<emu_item> mine;
-		int done = 0, pair = 0, k = 0;
 		for (int c = 0; c < it.ccount; c++) {
 			const emu_chunk &ch = chunks[it.cfirst + c];
-			const int st = (ch.head & 0xff) * KS - __builtin_popcount(ch.part);
-			x.steps += st;
-			const bool last = c + 1 == it.ccount;
-			if (last || ((ch.head >> 8 & RUN_LAST) && (int)mine.size() + 1 < n &&
-			    done + x.steps >= (long long)it.steps * ((int)mine.size() + 1) / n)) {
-				x.ccount = it.cfirst + c + 1 - x.cfirst;
-				x.p0 = pair;
-				x.k0 = k;
-				mine.push_back(x);
-				done += x.steps;
-				/* where the next part starts */
-				for (k += x.steps; pair < cb.npairs; pair++) {
-					const int nks = (cplx ? 2 : 1) *
-					    ((p->pairs[cb.first_pair + pair].k + EMU_KS - 1) / EMU_KS);
-					if (k < nks)
-						break;
-					k -= nks;
-				}
-				x.cfirst += x.ccount;
-				x.steps = 0;
+			const int mine = (int)(out.size() - at) + 1;
+			x.steps += (ch.head & 0xff) * KS - __builtin_popcount(ch.part);
+			if (c + 1 < it.ccount && (!(ch.head >> 8 & RUN_LAST) || mine == q ||
+			    done + x.steps < (long long)it.steps * mine / q))
+				continue;
+			x.ccount = it.cfirst + c + 1 - x.cfirst;
+			x.p0 = pair;
+			x.k0 = k;
+			out.push_back(x);
+			c2.push_back((cost[i] - over) * x.steps / it.steps + over);
+			done += x.steps;
+			/* where the next part starts */
+			for (k += x.steps; pair < cb.npairs; pair++) {
+				const int nks = (cplx ? 2 : 1) *
+				    ((p->pairs[cb.first_pair + pair].k + EMU_KS - 1) / EMU_KS);
+				if (k < nks)
+					break;
+				k -= nks;
 			}
+			x.cfirst += x.ccount;
+			x.steps = 0;
 		}
-		for (emu_item &y : mine) {
-			y.parts = (int)mine.size();
-			out.push_back(std::make_pair((cost[i] - over) * y.steps / it.steps + over, y));
-		}
-		slots += mine.size() > 1;
+		for (size_t y = at; y < out.size(); y++)
+			out[y].parts = (int)(out.size() - at);
+		slots += out.size() - at > 1;
 	}
-	top = 0;
-	for (const auto &o : out)
-		top = std::max(top, o.first);
-	std::stable_sort(out.begin(), out.end(),
-	    [&](const std::pair<double, emu_item> &x, const std::pair<double, emu_item> &y) {
-		return (int)(8 * x.first / top) > (int)(8 * y.first / top); });
-	items.clear();
-	for (const auto &o : out)
-		items.push_back(o.second);
+	if (target > 0) {
+		items.swap(out);
+		cost.swap(c2);
+		top = 0;
+		for (double c : cost)
+			top = std::max(top, c);
+	}
+	/* by class, longest first */
+	size_t first[10] = {};
+	auto cls = [&](size_t i) { return 8 - (int)(8 * cost[i] / top); };
+	for (size_t i = 0; i < items.size(); i++)
+		first[cls(i) + 1]++;
+	for (int c = 1; c < 10; c++)
+		first[c] += first[c - 1];
+	out.resize(items.size());
+	for (size_t i = 0; i < items.size(); i++)
+		out[first[cls(i)]++] = items[i];
+	items.swap(out);
 	return slots;
 }
 
@@ -2513,13 +2535,15 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 		std::vector<char> &use = side ? e->useB : e->useA;
 		/* the exponent pass: K ranges of 256 (one atomic per row and CTA
 		 * from the fewest CTAs), halved down to 32 while the grid is
-		 * below eight CTAs per SM */
+		 * below two CTAs per SM (24 x 64 ladder, exponent and split pass:
+		 * 54 us with eight, 48 with four, 47 with two; more CTAs, whose
+		 * warps' sums outweigh their loads) */
 		for (int &kr = e->kr[side]; kr > 32; kr /= 2) {
 			int64_t n = 0;
 			for (size_t v = 0; v < V.size(); v++)
 				if (use[v])
 					n += (int64_t)V[v].n_rt * ((V[v].k + kr - 1) / kr);
-			if (n >= 8 * num_sms())
+			if (n >= 2 * num_sms())
 				break;
 		}
 		for (int kind = 0; kind < 2; kind++) {
@@ -2567,7 +2591,8 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 		pols.erase(std::remove_if(pols.begin(), pols.end(),
 		    [](int q) { return !row_major(q); }), pols.end());
 	}
-	std::vector<std::vector<emu_item>> lists, whole;   /* whole: undivided */
+	std::vector<std::vector<emu_item>> lists;
+	std::vector<uint64_t> whole;
 	std::vector<std::vector<emu_member>> mlists;
 	std::vector<double> est;
 	chunk_index seen;
@@ -2584,18 +2609,22 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 			continue;
 		chunk_lists(p, cplx, e->kchunk, items, mem, seen, chunks);
 		const double cycles = list_cycles(p, items, mem, cplx, row_major(pol));
+		/* (lists are divided later: their sums tell them apart) */
+		uint64_t sum = items.size();
+		for (const emu_item &it : items)
+			sum = (sum ^ ((uint64_t)(uint32_t)it.m0 << 32 | (uint32_t)it.pr) ^
+			    (uint64_t)it.mfirst << 20) * 0x9e3779b97f4a7c15ull;
 		bool dup = false;
 		for (size_t l = 0; l < lists.size(); l++)
 			dup |= row_major(e->cand[l].policy) == row_major(pol) &&
 			    pair_policy(e->cand[l].policy) == pair_policy(pol) &&
-			    whole[l].size() == items.size() && mlists[l].size() == mem.size() &&
-			    memcmp(whole[l].data(), items.data(), items.size() * sizeof(emu_item)) == 0 &&
+			    whole[l] == sum && mlists[l].size() == mem.size() &&
 			    memcmp(mlists[l].data(), mem.data(), mem.size() * sizeof(emu_member)) == 0;
 		if (dup)
 			continue;
 		emu_cand c;
 		c.policy = pol;
-		whole.push_back(items);
+		whole.push_back(sum);
 		c.nslots = pair_policy(pol) ? 0 :
 		    split_items(p, cplx, row_major(pol), chunks, mem, items);
 		e->slot_bytes = std::max(e->slot_bytes, c.nslots * SLOT_BYTES);

@@ -1,7 +1,8 @@
 """GPU: the split-precision GEMM over pairs whose factors change.  Blocks of a
 are derivatives of one block with factors from a list (the same ones; signs
 only; twos too), different ones in the two rows of blocks, which share b's
-views and stack into one tile (work list 6).  Contracted extents of a block
+views and stack into one tile (work list 6); items are divided along K where
+that ends the list sooner, however short it is.  Contracted extents of a block
 below, at and above a K step, a stage and a chunk.  The elements are 14-bit
 integers times a power of two per row, so that every sum is exact: the exact
 result, rounded once in the float types, is expected."""
@@ -33,6 +34,7 @@ def _values(rng, rows, k, dtype):
 @pytest.mark.parametrize("factors", sorted(FACTORS))
 def test_factors(engine, monkeypatch, factors, dtype, policy):
     monkeypatch.setenv("XMG_POLICY", policy)
+    monkeypatch.setenv("XMG_EMU_DIVIDE", "1")
     engine.check(engine.xmg_set_precision(api.PREC_EMU64))
     al = api.Allocator(engine)
     nt = api.NP_TYPES[dtype]
