@@ -2271,9 +2271,9 @@ list_cycles(const xmgd_contract_t *p, const std::vector<emu_item> &items,
  * ends a list sooner by a model: the SMs' share and 0.6 of the
  * longest item, or the rounds of the longest; parts of at least four chunks and
  * about all, a half, a third or a quarter of an SM's share.  (Dividing lists of
- * less than a quarter of a millisecond costs the host more than it gives: an
- * adjoint of new tensors, two GEMMs of 0.2 ms, 1575 -> 1680 us with it.)  A part costs some
- * 8000 cycles beside its steps (the pipeline's ends, the sums' way through L2).
+ * a modelled 0.15 ms and less costs the host more than it gives: an adjoint of
+ * new tensors, two such GEMMs, 1575 -> 1680 us with it.)  A part costs some 8000
+ * cycles beside its steps (the pipeline's ends, the sums' way through L2).
  * GEMM of a 53 x 187 ladder (some 900 items, ordered) 1619 -> 1486 us, of a
  * complex128 ring term, 21 x 75 (divided) 428 -> 383 us; 16 items per SM and
  * more are even enough.  Returns the number of slots.
