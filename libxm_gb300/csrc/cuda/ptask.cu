@@ -133,13 +133,11 @@ combine(D x, S y, const scalars<D, S> &c, double &dre, double &dim_)
 		return num<D>::mul(unit<ONE>(c.al, x), conv<D, S>(y));
 	else if constexpr (OP == XMGD_OP_DIV)
 		return num<D>::div(x, unit<ONE>(c.al, conv<D, S>(y)));
-	else if constexpr (std::is_same<D, cd>::value) {
-		/* four fused steps, no product rounded on its own */
-		const cd z = conv<D, S>(y);
-		dre = ::fma(x.x, z.x, ::fma(-x.y, z.y, dre));
-		dim_ = ::fma(x.x, z.y, ::fma(x.y, z.x, dim_));
-		return x;
-	} else {
+	else {
+		/* a complex product is formed before it is added: two fused steps
+		 * into the sum would round the sum, not the product, twice, and the
+		 * halves of a product that cancel (|x| |y| large, re or im small)
+		 * would take the sum's low bits with them */
 		const D pr = num<D>::mul(x, conv<D, S>(y));
 		dre += num<D>::re(pr);
 		dim_ += num<D>::im(pr);
