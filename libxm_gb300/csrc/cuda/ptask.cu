@@ -147,12 +147,13 @@ combine(D x, S y, const scalars<D, S> &c, double &dre, double &dim_)
 
 /* f.run<OP, ONE>() for a task's operation; scalar conversions exist for
  * xm_copy alone, and ONE is set apart where FP64 work bounds the kernel or
- * costs nothing to leave out */
+ * costs nothing to leave out (not for a complex float source, whose products
+ * with 1 + 0i are no FP64 work and spread NaN) */
 template <typename D, typename S, typename F>
 __device__ __forceinline__ void
 with_op(const xmgd_ptask_t &t, F f)
 {
-	constexpr bool special = !std::is_same<D, cf>::value;
+	constexpr bool special = !std::is_same<D, cf>::value && !std::is_same<S, cf>::value;
 	/* by their bits: a compare would be an FP64 instruction */
 	bool one = special && __double_as_longlong(t.alpha[0]) == 0x3ff0000000000000ll;
 	if (std::is_same<D, cd>::value)
