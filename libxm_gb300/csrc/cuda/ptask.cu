@@ -643,6 +643,27 @@ elem_bytes(int type)
 	return type == 0 ? 4 : type == 3 ? 16 : 8;	/* float, cd; double, cf */
 }
 
+static bool
+reads_src(const xmgd_ptask_t &t)
+{
+	return t.op != XMGD_OP_SET && t.op != XMGD_OP_SCALE;
+}
+
+/* the schedule of a task (task_meta.mode); tile_n: elements of a tile */
+static int
+schedule_of(const xmgd_ptask_t &t, int tile_n)
+{
+	const int64_t far = 1 << 24;
+
+	if (t.ndim == 1 && t.dst_stride[0] == 1 && (!reads_src(t) || t.src_stride[0] == 1))
+		return 2;
+	if (t.ndim < 2 || t.src_stride[1] != 1 || t.src_stride[0] == 1 || !reads_src(t))
+		return 0;
+	return t.size[0] <= SLICE_MAX && t.size[1] <= SLICE_MAX &&
+	    t.size[0] * t.size[1] <= tile_n && t.src_stride[0] < far &&
+	    t.dst_stride[0] < far && t.dst_stride[1] < far ? 3 : 1;
+}
+
 /*
  * Schedule of every task of a batch.  Tasks are grouped by schedule (stable
  * within a group, order[] maps group position -> caller's index) so that
@@ -663,26 +684,16 @@ plan_tasks(const xmgd_ptask_t *tasks, int ntasks, int dtype, int stype,
 		const xmgd_ptask_t &t = tasks[i];
 		task_meta &m = m0[i];
 		memset(&m, 0, sizeof m);
-		const bool nosrc = t.op == XMGD_OP_SET || t.op == XMGD_OP_SCALE;
-		const bool tile = t.ndim >= 2 && t.src_stride[1] == 1 &&
-		    t.src_stride[0] != 1 && !nosrc;
-		const bool flat = t.ndim == 1 && t.dst_stride[0] == 1 &&
-		    (nosrc || t.src_stride[0] == 1);
-		if (flat) {
-			m.mode = 2;
-			m.nouter = 1;
+		m.mode = schedule_of(t, tile_n);
+		m.nouter = 1;
+		if (m.mode == 2) {
 			nflat += t.size[0];
-		} else if (tile) {
+		} else if (m.mode != 0) {
 			const int s0 = t.size[0], s1 = t.size[1];
-			const int64_t far = 1 << 24;
-			m.nouter = 1;
 			for (int d = 2; d < t.ndim; d++)
 				m.nouter *= t.size[d];
-			if (s0 <= SLICE_MAX && s1 <= SLICE_MAX && s0 * s1 <= tile_n &&
-			    t.src_stride[0] < far && t.dst_stride[0] < far &&
-			    t.dst_stride[1] < far) {
+			if (m.mode == 3) {
 				/* as many slices as the elements and the tile hold */
-				m.mode = 3;
 				const int q = std::min({tile_n / (s0 * s1),
 				    tile_cap(tile_n) / (s1 * (s0 | 1)), SLICE_MAXQ});
 				m.rows_per_cta = std::max(1, q);
@@ -691,7 +702,6 @@ plan_tasks(const xmgd_ptask_t *tasks, int ntasks, int dtype, int stype,
 				/* t1: the source's run in equal parts of at most 32;
 				 * t0: what fills the steps of 2^l1 lanes, in whole
 				 * 32-lane blocks */
-				m.mode = 1;
 				const int parts = (s1 + 31) / 32;
 				m.t1 = (s1 + parts - 1) / parts;
 				m.l1 = lanes_log2(m.t1);
@@ -704,9 +714,7 @@ plan_tasks(const xmgd_ptask_t *tasks, int ntasks, int dtype, int stype,
 				cnt[i] = (int64_t)m.ctas_d0 * m.ctas_d1 * m.nouter;
 			}
 		} else {
-			m.mode = 0;
 			m.ctas_d0 = (t.size[0] + ROW_ELEMS - 1) / ROW_ELEMS;
-			m.nouter = 1;
 			for (int d = 1; d < t.ndim; d++)
 				m.nouter *= t.size[d];
 			int64_t rows = t.size[0] >= ROW_ELEMS ? 1 :
@@ -841,9 +849,8 @@ batch_pinned(size_t bytes, void **p)
 	return XMG_OK;
 }
 
-extern "C" int
-xmgd_ptasks(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks,
-    double *dots)
+static int
+run_batch(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks, double *dots)
 {
 	std::vector<xmgd_ptask_t> sorted;
 	std::vector<task_meta> meta;
@@ -909,4 +916,81 @@ xmgd_ptasks(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks,
 	if (dots)
 		memcpy(dots, sums, db);
 	return XMG_OK;
+}
+
+/* Whether a task would read elements that it may already have overwritten:
+ * a permuted operation of a block onto itself, unless each CTA's slices, all
+ * loaded before any is stored, map onto themselves. */
+static bool
+overtakes(const xmgd_ptask_t &t, int tile_n)
+{
+	bool same = true, outer = true;
+
+	if (t.src != t.dst || !reads_src(t) || t.op == XMGD_OP_DOT)
+		return false;
+	for (int d = 0; d < t.ndim; d++) {
+		const bool eq = t.size[d] == 1 || t.dst_stride[d] == t.src_stride[d];
+		same = same && eq;
+		outer = outer && (d < 2 || eq);
+	}
+	return !same && !(outer && schedule_of(t, tile_n) == 3 && t.dst_stride[0] == 1 &&
+	    t.size[0] == t.size[1] && t.dst_stride[1] == t.src_stride[0]);
+}
+
+/* bytes from a task's first source element to the end of its last */
+static size_t
+src_bytes(const xmgd_ptask_t &t, int esz)
+{
+	size_t n = 1;
+
+	for (int d = 0; d < t.ndim; d++)
+		n += (size_t)(t.size[d] - 1) * (size_t)t.src_stride[d];
+	return n * esz;
+}
+
+/* The tasks of a batch.  Those of a block onto itself whose stores could
+ * overtake their loads read a copy of the block made before, of COPY_MAX
+ * bytes of blocks at a time: as in the reference, which reads a block whole
+ * before it writes it (xm.c:66-413), the block's old elements count. */
+extern "C" int
+xmgd_ptasks(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks,
+    double *dots)
+{
+	constexpr size_t COPY_MAX = (size_t)256 << 20;
+	const int esz = elem_bytes(stype), tile_n = tile_elems(elem_bytes(dtype), esz);
+	std::vector<xmgd_ptask_t> now, copied;
+	int st;
+
+	for (int i = 0; i < ntasks; i++)
+		if (overtakes(tasks[i], tile_n))
+			copied.push_back(tasks[i]);
+	if (copied.empty())
+		return run_batch(dtype, stype, tasks, ntasks, dots);
+	for (int i = 0; i < ntasks; i++)
+		if (!overtakes(tasks[i], tile_n))
+			now.push_back(tasks[i]);
+	st = run_batch(dtype, stype, now.data(), (int)now.size(), dots);
+	for (size_t first = 0, end; first < copied.size() && st == XMG_OK; first = end) {
+		uint64_t mem, at;
+		size_t n = 0;
+		for (end = first; end < copied.size(); end++) {
+			const size_t b = src_bytes(copied[end], esz);
+			if (end > first && n + b > COPY_MAX)
+				break;
+			n += (b + 255) & ~(size_t)255;
+		}
+		if ((st = xmgd_alloc(n, &mem)) != XMG_OK)
+			return st;
+		at = mem;
+		for (size_t i = first; i < end && st == XMG_OK; i++) {
+			const size_t b = src_bytes(copied[i], esz);
+			st = xmgd_d2d(at, copied[i].src, b);
+			copied[i].src = at;
+			at += (b + 255) & ~(size_t)255;
+		}
+		if (st == XMG_OK)
+			st = run_batch(dtype, stype, &copied[first], (int)(end - first), nullptr);
+		xmgd_free(mem);
+	}
+	return st;
 }
