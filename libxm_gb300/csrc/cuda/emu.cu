@@ -142,6 +142,14 @@ __device__ __forceinline__ int find_view(const view_meta *m, int n, int64_t cta)
 	return last_at_most(n, cta, [&](int i) { return m[i].first_cta; });
 }
 
+/* Place of the real (half 0) or imaginary part of the element at row + col of
+ * a complex block, counted in parts: a block's elements number below 2^31, its
+ * parts do not. */
+__host__ __device__ __forceinline__ int64_t part_at(int32_t row, int32_t col, int half)
+{
+	return 2 * ((int64_t)row + col) + half;
+}
+
 /* Element (k', r) of a view: real views directly, complex views realified
  * along K as [re | im] with halves of w.khp (zero padding). */
 template <typename T>
@@ -153,7 +161,7 @@ __device__ __forceinline__ T fetch(const T *X, const int32_t *rowt, int32_t co,
 	}
 	const int half = k >= w.khp;
 	const int kk = k - half * w.khp;
-	return kk < w.k ? X[2 * (rowt[kk] + co) + half] : T(0);
+	return kk < w.k ? X[part_at(rowt[kk], co, half)] : T(0);
 }
 
 /* ------------------------------------------------------------------ */
@@ -215,10 +223,9 @@ emu_exp_kernel(const xmgd_view_t *__restrict__ views,
 					const int32_t ra = rowt[ka], rc = rowt[kc];
 #pragma unroll
 					for (int j = 0; j < 4; j++) {
-						const int a = fin<T>::eword(X + 2 * (ra + co[j]));
-						const int b = fin<T>::eword(X + 2 * (rc + co[j]));
-						const int p = fin<T>::eword(X + 2 * (ra + co[j]) + 1);
-						const int q = fin<T>::eword(X + 2 * (rc + co[j]) + 1);
+						const T *pa = X + part_at(ra, co[j], 0), *pc = X + part_at(rc, co[j], 0);
+						const int a = fin<T>::eword(pa), b = fin<T>::eword(pc);
+						const int p = fin<T>::eword(pa + 1), q = fin<T>::eword(pc + 1);
 						x[j][0] = fin<T>::bexp(a) > fin<T>::bexp(p) ? a : p;
 						x[j][1] = fin<T>::bexp(b) > fin<T>::bexp(q) ? b : q;
 					}
@@ -2750,6 +2757,13 @@ int emu_record_split(emu_plan *e) { return e->split(e); }
 int emu_record_gemm(emu_plan *e) { return e->gemm(e); }
 int64_t emu_slice_bytes(const emu_plan *e) { return (int64_t)e->slice_bytes; }
 int emu_a_mode(const emu_plan *e) { return e->a_mode; }
+
+/* part_at on the host: what the kernels of the operand pass index with */
+extern "C" int64_t
+xmgd_emu_part_at(int32_t row, int32_t col, int half)
+{
+	return part_at(row, col, half);
+}
 
 /* the slice bytes tile() gives one view */
 extern "C" int64_t
