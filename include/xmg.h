@@ -81,6 +81,16 @@ int xmg_work_list_check(const xm_tensor_t *a, const xm_tensor_t *b,
     const xm_tensor_t *c, const char *idxa, const char *idxb,
     const char *idxc, int policy, long long out[4]);
 
+/* The same list with its items divided along K for a chip of `sms` SMs (0:
+ * the engine's device), however short the list (XMG_EMU_DIVIDE=1): out =
+ * {items, slots (items that were divided), chunks, 1 if the parts of every
+ * slot cover the item's K steps once, the chunks are the stages the kernel
+ * fills, with their factors and exact ranges, and the list's own invariants
+ * hold}.  For tests. */
+int xmg_work_list_parts(const xm_tensor_t *a, const xm_tensor_t *b,
+    const xm_tensor_t *c, const char *idxa, const char *idxb,
+    const char *idxc, int policy, int sms, long long out[4]);
+
 /* The out-of-core batch plans, cut on the host without a device from the
  * whole plan, for b's blocks (in the streamed path's order: file order,
  * or the output blocks' with XMG_STREAM_ORDER=output) in the

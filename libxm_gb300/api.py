@@ -125,6 +125,8 @@ _GB_SIGS = {
     "xmg_contract_flops": (C.c_double, [_P, _P, _P, C.c_char_p, C.c_char_p, C.c_char_p]),
     "xmg_work_list_check": (C.c_int, [_P, _P, _P, C.c_char_p, C.c_char_p, C.c_char_p,
                                       C.c_int, C.POINTER(C.c_longlong)]),
+    "xmg_work_list_parts": (C.c_int, [_P, _P, _P, C.c_char_p, C.c_char_p, C.c_char_p,
+                                      C.c_int, C.c_int, C.POINTER(C.c_longlong)]),
     "xmg_batch_plan_check": (C.c_int, [_P, _P, _P, C.c_char_p, C.c_char_p, C.c_char_p,
                                        C.c_int, C.c_longlong, C.c_int,
                                        C.POINTER(C.c_longlong)]),

@@ -2283,17 +2283,18 @@ list_cycles(const xmgd_contract_t *p, const std::vector<emu_item> &items,
  * cycles beside its steps (the pipeline's ends, the sums' way through L2).
  * GEMM of a 53 x 187 ladder (some 900 items, ordered) 1619 -> 1486 us, of a
  * complex128 ring term, 21 x 75 (divided) 428 -> 383 us; 16 items per SM and
- * more are even enough.  Returns the number of slots.
+ * more are even enough.  all: short lists too (XMG_EMU_DIVIDE=1, for tests).
+ * Returns the number of slots.
  */
 static int
-split_items(const xmgd_contract_t *p, int cplx, bool rowmajor,
+split_items(const xmgd_contract_t *p, int cplx, bool rowmajor, size_t sms, bool all,
     const std::vector<emu_chunk> &chunks, const std::vector<emu_member> &members,
     std::vector<emu_item> &items)
 {
 	const double over = 8000;
 	const int KS = p->dtype >= 2 ? stage_cfg<fin<double>::S>::KSTEPS :
 	    stage_cfg<fin<float>::S>::KSTEPS;
-	const size_t n = items.size(), sms = (size_t)num_sms();
+	const size_t n = items.size();
 	double width[EMU_TM / 16 + 1], sum = 0, top = 0;
 
 	if (n >= 16 * sms)
@@ -2317,8 +2318,7 @@ split_items(const xmgd_contract_t *p, int cplx, bool rowmajor,
 		return std::min(total / sms + 0.6 * longest, rounds * longest);
 	};
 	double best = 0.93 * model(sum, top, n), target = 0;
-	const char *div = getenv("XMG_EMU_DIVIDE");  /* 1: short lists too */
-	const bool divide = n < 8 * sms && (sum / sms >= 2.8e5 || (div && atoi(div) == 1));
+	const bool divide = n < 8 * sms && (sum / sms >= 2.8e5 || all);
 	for (int w = 1; w <= 4 && divide; w++) {
 		const double t = sum / sms / w;
 		double total = 0, longest = 0;
@@ -2405,6 +2405,129 @@ split_items(const xmgd_contract_t *p, int cplx, bool rowmajor,
 		out[first[cls(i)]++] = items[i];
 	items.swap(out);
 	return slots;
+}
+
+/* What the kernel takes from a list with its chunks and parts beyond
+ * items_ok, in O(items): an item's chunks lie in the array; an undivided one
+ * starts at its first step and holds all of them; the parts of a slot are as
+ * many as each of them says, share tile and members, and follow one another
+ * from the first step and chunk to the last. */
+static bool
+parts_ok(const xmgd_contract_t *p, int cplx, const std::vector<emu_item> &items,
+    const std::vector<emu_member> &mem, const std::vector<emu_chunk> &chunks, int nslots)
+{
+	struct place { int steps, chunk, item; };
+	std::vector<std::vector<place>> slot(nslots);
+	auto total = [&](const xmgd_cblock_t &cb, int pair) {
+		long long n = 0;
+		for (int q = 0; q < pair; q++)
+			n += (cplx ? 2 : 1) * ((p->pairs[cb.first_pair + q].k + EMU_KS - 1) / EMU_KS);
+		return n;
+	};
+	for (size_t i = 0; i < items.size(); i++) {
+		const emu_item &it = items[i];
+		const xmgd_cblock_t &cb = p->cblocks[mem[it.mfirst].cblock];
+		if (it.cfirst < 0 || it.ccount < 1 || it.steps < 1 ||
+		    (size_t)it.cfirst + it.ccount > chunks.size() || it.p0 < 0 || it.k0 < 0 ||
+		    it.p0 >= cb.npairs || it.parts < 1)
+			return false;
+		if (it.parts == 1) {
+			if (it.p0 || it.k0 || it.steps != total(cb, cb.npairs))
+				return false;
+			continue;
+		}
+		if (it.slot < 0 || it.slot >= nslots)
+			return false;
+		slot[it.slot].push_back(place{(int)total(cb, it.p0) + it.k0, it.cfirst, (int)i});
+	}
+	for (std::vector<place> &v : slot) {
+		std::sort(v.begin(), v.end(),
+		    [](const place &x, const place &y) { return x.steps < y.steps; });
+		int steps = 0, chunk = v.empty() ? 0 : v[0].chunk;
+		for (const place &x : v) {
+			const emu_item &it = items[x.item], &f = items[v[0].item];
+			if (it.parts != (int)v.size() || x.steps != steps || x.chunk != chunk ||
+			    it.m0 != f.m0 || it.pr != f.pr || it.mfirst != f.mfirst ||
+			    it.mcount != f.mcount)
+				return false;
+			steps += it.steps;
+			chunk += it.ccount;
+		}
+		if (v.size() < 2 || steps != total(p->cblocks[mem[items[v[0].item].mfirst].cblock],
+		    p->cblocks[mem[items[v[0].item].mfirst].cblock].npairs))
+			return false;
+	}
+	return true;
+}
+
+/* The same against the roles of the kernel, stage by stage: the stages the
+ * producer fills from (p0, k0) on are the ones the chunks count, of one step
+ * where they say so, with the members' factors; chunks and runs stay below
+ * the accumulators' exact ranges (see emu_chunk).  As long as the list's K
+ * steps: for the host checks. */
+static bool
+chunks_ok(const xmgd_contract_t *p, int cplx, int kchunk, const std::vector<emu_item> &items,
+    const std::vector<emu_member> &mem, const std::vector<emu_chunk> &chunks)
+{
+	const bool dbl = p->dtype >= 2;
+	const int KS = dbl ? stage_cfg<fin<double>::S>::KSTEPS : stage_cfg<fin<float>::S>::KSTEPS;
+
+	for (const emu_item &it : items) {
+		const int pass = it.pr & 1;
+		const xmgd_cblock_t &cb = p->cblocks[mem[it.mfirst].cblock];
+		int q = it.p0, k = it.k0, left = it.steps, run = 0, code = 0;
+		for (int c = 0; c < it.ccount; c++) {
+			const emu_chunk &ch = chunks[it.cfirst + c];
+			const int nss = ch.head & 0xff, fl = ch.head >> 8 & 0xff;
+			const bool last = c + 1 == it.ccount;
+			int steps = 0, from = -1;
+			if (nss < 1 || nss > 32 || (run == 0) != ((fl & RUN_FIRST) != 0) ||
+			    (fl & ITEM_LAST) || (last && !(fl & RUN_LAST)))
+				return false;
+			if (run++ == 0)
+				code = ch.head >> 16;
+			if (ch.head >> 16 != code || code >> (2 * it.mcount))
+				return false;
+			for (int j = 0; j < nss; j++) {
+				if (q >= cb.npairs)
+					return false;
+				const int nks = (cplx ? 2 : 1) *
+				    ((p->pairs[cb.first_pair + q].k + EMU_KS - 1) / EMU_KS);
+				const int half = cplx && k >= nks / 2;
+				const int end = cplx && !half ? nks / 2 : nks, n = std::min(KS, end - k);
+				if (n != (KS == 2 && !(ch.part >> j & 1) ? 2 : 1))
+					return false;
+				for (int m = 0; m < it.mcount; m++) {
+					const xmgd_pair_t &pr =
+					    p->pairs[p->cblocks[mem[it.mfirst + m].cblock].first_pair + q];
+					const int neg = (pr.esign < 0) ^ (half && !pass);
+					const int has = code >> (2 * m) & 3;
+					if ((has & 1) != (neg ^ (int)(ch.neg >> j & 1)) ||
+					    (has >> 1) != (pr.eshift ? 1 : 0))
+						return false;
+				}
+				/* FP64: one segment, as the drains' error asks */
+				if (dbl && from >= 0 && from != 2 * q + half)
+					return false;
+				from = 2 * q + half;
+				steps += n;
+				k += n;
+				if (k == nks) {
+					k = 0;
+					q++;
+				}
+			}
+			left -= steps;
+			if (steps > (dbl ? kchunk : EMU_CHUNK32) ||
+			    run > (dbl || (code & 0xAA) ? 1 : 2))
+				return false;
+			if (fl & RUN_LAST)
+				run = 0;
+		}
+		if (left != 0)
+			return false;
+	}
+	return true;
 }
 
 /* bytes of one K step of a view with mn rows: whole tiles, then the last
@@ -2604,6 +2727,8 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 	std::vector<double> est;
 	chunk_index seen;
 	std::vector<emu_chunk> chunks;
+	const char *div = getenv("XMG_EMU_DIVIDE");
+	const bool divide_all = div && atoi(div) == 1;
 	for (int pol : pols) {
 		if (known >= 0 && pol != known)
 			continue;
@@ -2631,9 +2756,11 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 			continue;
 		emu_cand c;
 		c.policy = pol;
+		c.nslots = pair_policy(pol) ? 0 : split_items(p, cplx, row_major(pol),
+		    (size_t)num_sms(), divide_all, chunks, mem, items);
+		if (!parts_ok(p, cplx, items, mem, chunks, c.nslots))
+			continue;
 		whole.push_back(sum);
-		c.nslots = pair_policy(pol) ? 0 :
-		    split_items(p, cplx, row_major(pol), chunks, mem, items);
 		e->slot_bytes = std::max(e->slot_bytes, c.nslots * SLOT_BYTES);
 		c.nitems = (int)items.size();
 		c.grid = pair_policy(pol) ? 2 * std::min(c.nitems, num_sms() / 2) :
@@ -2717,9 +2844,14 @@ emu_bind(emu_plan *e, bool *moved)
 	return XMG_OK;
 }
 
-/* the work list of one policy, built and checked on the host (no device) */
-extern "C" int
-xmgd_work_list_check(const xmgd_contract_t *p, int policy, long long out[4])
+/* The work list of one policy, built and checked on the host (no device) as
+ * emu_prepare uploads it.  sms: the SMs it is divided for (0: the device's;
+ * below 0: not divided), with short lists if all; slots, chunks: its numbers
+ * of both. */
+static int
+checked_list(const xmgd_contract_t *p, int policy, int sms, bool all,
+    std::vector<emu_item> &items, std::vector<emu_member> &mem, int *slots, size_t *nchunks,
+    bool *ok)
 {
 	int cplx;
 
@@ -2736,16 +2868,59 @@ xmgd_work_list_check(const xmgd_contract_t *p, int policy, long long out[4])
 	for (int i = 0; i < p->ncblocks; i++)
 		if (p->cblocks[i].npairs > 0 && p->emulatable[i])
 			cblocks.push_back(i);
+	make_items(p, cblocks, cplx, policy, items, mem);
+	chunk_index seen;
+	std::vector<emu_chunk> chunks;
+	*slots = 0;
+	if ((*ok = items_ok(p, items, mem, pair_policy(policy)))) {
+		chunk_lists(p, cplx, EMU_CHUNK, items, mem, seen, chunks);
+		if (sms >= 0 && !pair_policy(policy))
+			*slots = split_items(p, cplx, row_major(policy),
+			    (size_t)(sms ? sms : std::max(1, num_sms())), all, chunks, mem, items);
+		*ok = parts_ok(p, cplx, items, mem, chunks, *slots) &&
+		    chunks_ok(p, cplx, EMU_CHUNK, items, mem, chunks);
+	}
+	*nchunks = chunks.size();
+	return XMG_OK;
+}
+
+extern "C" int
+xmgd_work_list_check(const xmgd_contract_t *p, int policy, long long out[4])
+{
 	std::vector<emu_item> items;
 	std::vector<emu_member> mem;
-	make_items(p, cblocks, cplx, policy, items, mem);
+	size_t nchunks;
+	int slots, st;
+	bool ok;
+
+	if ((st = checked_list(p, policy, -1, false, items, mem, &slots, &nchunks, &ok)) != XMG_OK)
+		return st;
 	long long stacked = 0;
 	for (const emu_item &it : items)
 		stacked += it.mcount > 1;
 	out[0] = (long long)items.size();
 	out[1] = (long long)mem.size();
 	out[2] = stacked;
-	out[3] = items_ok(p, items, mem, pair_policy(policy)) ? 1 : 0;
+	out[3] = ok;
+	return XMG_OK;
+}
+
+extern "C" int
+xmgd_work_list_parts(const xmgd_contract_t *p, int policy, int sms, long long out[4])
+{
+	std::vector<emu_item> items;
+	std::vector<emu_member> mem;
+	size_t nchunks;
+	int slots, st;
+	bool ok;
+
+	if ((st = checked_list(p, policy, std::max(0, sms), true, items, mem, &slots, &nchunks,
+	    &ok)) != XMG_OK)
+		return st;
+	out[0] = (long long)items.size();
+	out[1] = slots;
+	out[2] = (long long)nchunks;
+	out[3] = ok;
 	return XMG_OK;
 }
 

@@ -781,10 +781,11 @@ fill_contract(xmgd_contract_t *dp, const plan_t *p, xm_scalar_t alpha,
 	dp->emulatable = p->emulatable;
 }
 
-int
-xmg_work_list_check(const xm_tensor_t *a, const xm_tensor_t *b,
-    const xm_tensor_t *c, const char *idxa, const char *idxb,
-    const char *idxc, int policy, long long out[4])
+/* a work-list check of a contraction's device plan, built without a device */
+static int
+list_check(const xm_tensor_t *a, const xm_tensor_t *b, const xm_tensor_t *c,
+    const char *idxa, const char *idxb, const char *idxc, int policy, int sms,
+    long long out[4])
 {
 	xmgd_contract_t dp;
 	plan_t p;
@@ -794,10 +795,29 @@ xmg_work_list_check(const xm_tensor_t *a, const xm_tensor_t *b,
 	if ((st = xmg_plan_check(a, b, c, idxa, idxb, idxc, &p)) == XMG_OK &&
 	    (st = xmg_plan_build(1, a, b, c, &p, 2)) == XMG_OK) {
 		fill_contract(&dp, &p, 1, 0, XMG_PREC_EMU64);
-		st = xmgd_work_list_check(&dp, policy, out);
+		st = sms < 0 ? xmgd_work_list_check(&dp, policy, out) :
+		    xmgd_work_list_parts(&dp, policy, sms, out);
 	}
 	xmg_plan_free(&p);
 	return st;
+}
+
+int
+xmg_work_list_check(const xm_tensor_t *a, const xm_tensor_t *b,
+    const xm_tensor_t *c, const char *idxa, const char *idxb,
+    const char *idxc, int policy, long long out[4])
+{
+	return list_check(a, b, c, idxa, idxb, idxc, policy, -1, out);
+}
+
+int
+xmg_work_list_parts(const xm_tensor_t *a, const xm_tensor_t *b,
+    const xm_tensor_t *c, const char *idxa, const char *idxb,
+    const char *idxc, int policy, int sms, long long out[4])
+{
+	if (sms < 0)
+		return xmg_seterr(XMG_EINVAL, "work list: number of SMs");
+	return list_check(a, b, c, idxa, idxb, idxc, policy, sms, out);
 }
 
 /* ------------------------------------------------------------------ */
