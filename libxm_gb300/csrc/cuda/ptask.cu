@@ -582,27 +582,59 @@ ptask_kernel(const __grid_constant__ task_pack pack,
 	}
 }
 
-/* Sums of the per-CTA partial dot products: a warp per task (in the
- * caller's order, order[]), lanes striding over its CTAs, so the order of
- * the additions depends on the batch alone. */
-__global__ void __launch_bounds__(256)
+/*
+ * Sums of the per-CTA partial dot products, per task (in the caller's order,
+ * order[]): LANES threads stride over a task's CTAs, four loads in flight, so
+ * the order of the additions depends on the batch alone.  A warp per task for
+ * batches of short tasks; 1024 threads where a task has more than 256 CTAs: a
+ * lone warp takes 360 us for the 37 000 partial sums of a 40-million-element
+ * block, longer than its products.
+ */
+template <int LANES>
+__global__ void __launch_bounds__(LANES == 32 ? 256 : LANES)
 dot_sum_kernel(const __grid_constant__ task_pack pack,
     const task_meta *__restrict__ dmeta, const int *__restrict__ order, int ntasks,
     int64_t nctas, const double *__restrict__ partial, double *__restrict__ out)
 {
+	constexpr int U = 4;
+	__shared__ double s_red[2][LANES / 32];
 	const task_meta *meta = dmeta ? dmeta : pack.m;
-	const int t = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x & 31;
+	const int t = LANES == 32 ? blockIdx.x * 8 + threadIdx.x / 32 : blockIdx.x;
+	const int lane = threadIdx.x % LANES;
 	if (t >= ntasks)
 		return;
 	const int64_t end = t + 1 < ntasks ? meta[t + 1].first_cta : nctas;
+	const double2 *p2 = reinterpret_cast<const double2 *>(partial);
 	double a = 0, b = 0;
-	for (int64_t c = meta[t].first_cta + lane; c < end; c += 32) {
-		a += partial[2 * c];
-		b += partial[2 * c + 1];
+	for (int64_t c = meta[t].first_cta + lane; c < end; c += U * LANES) {
+		double2 v[U];
+#pragma unroll
+		for (int u = 0; u < U; u++)
+			v[u] = c + u * LANES < end ? p2[c + u * LANES] : make_double2(0, 0);
+#pragma unroll
+		for (int u = 0; u < U; u++) {
+			a += v[u].x;
+			b += v[u].y;
+		}
 	}
 	for (int off = 16; off > 0; off >>= 1) {
 		a += __shfl_down_sync(0xffffffffu, a, off);
 		b += __shfl_down_sync(0xffffffffu, b, off);
+	}
+	if constexpr (LANES > 32) {
+		if (lane % 32 == 0) {
+			s_red[0][lane / 32] = a;
+			s_red[1][lane / 32] = b;
+		}
+		__syncthreads();
+		if (lane >= 32)
+			return;
+		a = lane < LANES / 32 ? s_red[0][lane] : 0;
+		b = lane < LANES / 32 ? s_red[1][lane] : 0;
+		for (int off = 16; off > 0; off >>= 1) {
+			a += __shfl_down_sync(0xffffffffu, a, off);
+			b += __shfl_down_sync(0xffffffffu, b, off);
+		}
 	}
 	if (lane == 0) {
 		const int o = order ? order[t] : t;
@@ -904,8 +936,16 @@ run_batch(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks, double *d
 	st = launch_types(dtype, stype, pack, (const xmgd_ptask_t *)dbuf, dmeta, ntasks,
 	    begin, (double *)dpart);
 	if (st == XMG_OK && dots) {
-		dot_sum_kernel<<<(unsigned)((ntasks + 7) / 8), 256, 0, stream()>>>(pack,
-		    dmeta, dorder, ntasks, nctas, (const double *)dpart, sums);
+		int64_t longest = 0;
+		for (int i = 0; i < ntasks; i++)
+			longest = std::max(longest, (i + 1 < ntasks ? meta[i + 1].first_cta : nctas) -
+			    meta[i].first_cta);
+		if (longest <= 256)
+			dot_sum_kernel<32><<<(unsigned)((ntasks + 7) / 8), 256, 0, stream()>>>(pack,
+			    dmeta, dorder, ntasks, nctas, (const double *)dpart, sums);
+		else
+			dot_sum_kernel<1024><<<(unsigned)ntasks, 1024, 0, stream()>>>(pack,
+			    dmeta, dorder, ntasks, nctas, (const double *)dpart, sums);
 		g_launches++;
 		st = check(cudaGetLastError(), "dot_sum_kernel");
 	}
