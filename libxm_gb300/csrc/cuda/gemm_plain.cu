@@ -85,9 +85,12 @@ plain_gemm_kernel(const pg_item *__restrict__ items,
 	const pg_item it = items[blockIdx.x];
 	const xmgd_cblock_t cb = cbs[it.cblock];
 	const int tx = threadIdx.x % P::NX, ty = threadIdx.x / P::NX;
-	/* rows and columns of threads that reach into the block */
-	const int mi = min(TM, (cb.m - it.m0 + P::NX - 1) / P::NX);
-	const int nj = min(TN, (cb.n - it.n0 + P::NY - 1) / P::NY);
+	/* rows and columns of threads that reach into the block (all of them for
+	 * float, whose multiply-adds cost less than the branches: 1500 x 1500 x
+	 * 1500 in 25 blocks 461 us, 756 with them) */
+	constexpr bool ALL = std::is_same<T, float>::value;
+	const int mi = ALL ? TM : min(TM, (cb.m - it.m0 + P::NX - 1) / P::NX);
+	const int nj = ALL ? TN : min(TN, (cb.n - it.n0 + P::NY - 1) / P::NY);
 	T acc[TM][TN];
 #pragma unroll
 	for (int i = 0; i < TM; i++)
