@@ -85,9 +85,11 @@ plain_gemm_kernel(const pg_item *__restrict__ items,
 	const pg_item it = items[blockIdx.x];
 	const xmgd_cblock_t cb = cbs[it.cblock];
 	const int tx = threadIdx.x % P::NX, ty = threadIdx.x / P::NX;
-	/* rows and columns of threads that reach into the block (all of them for
-	 * float, whose multiply-adds cost less than the branches: 1500 x 1500 x
-	 * 1500 in 25 blocks 461 us, 756 with them) */
+	/* rows and columns of threads that reach into the block; all of them, and
+	 * whole K tiles, for float, whose multiply-adds cost less than the branches
+	 * (1500 x 1500 x 1500 in 25 blocks 396 us, 756 with them); float loads a
+	 * tile when it is due (16 x 16 x 5000: 475 us with the next one in flight,
+	 * 412 without; large ones the same) */
 	constexpr bool ALL = std::is_same<T, float>::value;
 	const int mi = ALL ? TM : min(TM, (cb.m - it.m0 + P::NX - 1) / P::NX);
 	const int nj = ALL ? TN : min(TN, (cb.n - it.n0 + P::NY - 1) / P::NY);
@@ -108,18 +110,24 @@ plain_gemm_kernel(const pg_item *__restrict__ items,
 		const bool bkf = pr.k > 1 && brow[1] - brow[0] == 1;
 		const T al = num<T>::mk(pr.al);
 		T va[P::NL], vb[P::NL];
-		P::fetch(va, A, arow, acol, 0, pr.k, it.m0, cb.m, akf);
-		P::fetch(vb, B, brow, bcol, 0, pr.k, it.n0, cb.n, bkf);
+		if (!ALL) {
+			P::fetch(va, A, arow, acol, 0, pr.k, it.m0, cb.m, akf);
+			P::fetch(vb, B, brow, bcol, 0, pr.k, it.n0, cb.n, bkf);
+		}
 		for (int k0 = 0; k0 < pr.k; k0 += PG_BK) {
+			if (ALL) {
+				P::fetch(va, A, arow, acol, k0, pr.k, it.m0, cb.m, akf);
+				P::fetch(vb, B, brow, bcol, k0, pr.k, it.n0, cb.n, bkf);
+			}
 			__syncthreads();
 			P::put(As, va, akf, &al);
 			P::put(Bs, vb, bkf, nullptr);
 			__syncthreads();
-			if (k0 + PG_BK < pr.k) {	/* the next tile, in flight below */
+			if (!ALL && k0 + PG_BK < pr.k) {	/* the next tile, in flight below */
 				P::fetch(va, A, arow, acol, k0 + PG_BK, pr.k, it.m0, cb.m, akf);
 				P::fetch(vb, B, brow, bcol, k0 + PG_BK, pr.k, it.n0, cb.n, bkf);
 			}
-			const int kn = min(PG_BK, pr.k - k0);
+			const int kn = ALL ? PG_BK : min(PG_BK, pr.k - k0);
 #pragma unroll 4
 			for (int kk = 0; kk < kn; kk++) {
 				T a[TM], b[TN];
