@@ -94,8 +94,9 @@ static __device__ __noinline__ cd axpy_any(cd al, cd x, cd be, cd y)
 
 static __device__ __noinline__ cd mul_any(cd a, cd b) { return num<cd>::mul(a, b); }
 
-/* s * v; ONE: s is 1, left out for real types and for finite complex ones
- * (Inf and NaN take the product, which spreads NaN to both parts) */
+/* s * v; ONE: s is 1, left out for real types and for finite complex doubles;
+ * Inf and NaN take the product, which spreads NaN to both parts (complex
+ * floats: what is left of it) */
 template <bool ONE, typename T>
 __device__ __forceinline__ T unit(const T &s, const T &v)
 {
@@ -103,6 +104,8 @@ __device__ __forceinline__ T unit(const T &s, const T &v)
 		return num<T>::mul(s, v);
 	else if constexpr (std::is_same<T, cd>::value)
 		return finite(v) ? v : mul_any(s, v);
+	else if constexpr (std::is_same<T, cf>::value)
+		return cf{fmaf(-v.y, 0.0f, v.x), fmaf(v.x, 0.0f, v.y)};
 	else
 		return v;
 }
@@ -147,13 +150,12 @@ combine(D x, S y, const scalars<D, S> &c, double &dre, double &dim_)
 
 /* f.run<OP, ONE>() for a task's operation; scalar conversions exist for
  * xm_copy alone, and ONE is set apart where FP64 work bounds the kernel or
- * costs nothing to leave out (not for a complex float source, whose products
- * with 1 + 0i are no FP64 work and spread NaN) */
+ * costs nothing to leave out */
 template <typename D, typename S, typename F>
 __device__ __forceinline__ void
 with_op(const xmgd_ptask_t &t, F f)
 {
-	constexpr bool special = !std::is_same<D, cf>::value && !std::is_same<S, cf>::value;
+	constexpr bool special = !std::is_same<D, cf>::value;
 	/* by their bits: a compare would be an FP64 instruction */
 	bool one = special && __double_as_longlong(t.alpha[0]) == 0x3ff0000000000000ll;
 	if (std::is_same<D, cd>::value)
