@@ -228,8 +228,9 @@ struct flat_run {
 	template <int OP, bool ONE>
 	__device__ __forceinline__ int vectors()
 	{
-		/* (a division needs the registers of two vectors more) */
-		constexpr int W = 16 / sizeof(D), U = OP == XMGD_OP_DIV ? 2 : 4;
+		/* (an FP64 division needs the registers of two vectors more) */
+		constexpr bool f64 = std::is_same<D, double>::value || std::is_same<D, cd>::value;
+		constexpr int W = 16 / sizeof(D), U = OP == XMGD_OP_DIV && f64 ? 2 : 4;
 		vec16<D> *dv = reinterpret_cast<vec16<D> *>(dp);
 		const vec16<D> *sv = reinterpret_cast<const vec16<D> *>(sp);
 		const int nv = n / W;
