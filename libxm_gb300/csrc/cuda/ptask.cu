@@ -38,14 +38,22 @@ constexpr int FLAT_ELEMS = 8192;   /* elements per CTA in flat mode, at most */
 constexpr int FLAT_MIN = 1024;     /* ... and at least */
 constexpr int SLICE_MAX = 48;      /* slices: extents at most */
 constexpr int SLICE_MAXQ = 64;     /* slices per CTA at most */
-/* tile and slices: elements per CTA (eight per thread; sixteen of the
- * 4-byte type, four of the 16-byte ones), and the shared tile with the
- * padding of its rows */
+/* tile: elements per CTA (eight per thread, four of the 16-byte types), and
+ * the shared tile with the padding of its rows */
 static constexpr int tile_elems(int dbytes, int sbytes)
 {
-	return dbytes == 4 && sbytes == 4 ? 4096 : dbytes <= 8 && sbytes <= 8 ? 2048 : 1024;
+	return dbytes <= 8 && sbytes <= 8 ? 2048 : 1024;
 }
 static constexpr int tile_cap(int n) { return n + 256; }
+/* slices: the same (one slice of 48 x 48 or two of 33 x 33 of the 8-byte
+ * types; sixteen elements per thread of the 4-byte one; copies between types
+ * hold the source alone) */
+static constexpr int slice_elems(int dbytes, int sbytes)
+{
+	return dbytes == 4 && sbytes == 4 ? 4096 :
+	    sbytes <= 8 && (dbytes <= 8 || dbytes != sbytes) ? 2304 : 1024;
+}
+static constexpr int slice_cap(int n) { return n == 2304 ? 48 * 49 : n + 256; }
 /* log2 of the lanes along a run of n <= 32 elements: 8 to 32 */
 static inline int lanes_log2(int n) { return n <= 8 ? 3 : n <= 16 ? 4 : 5; }
 
@@ -390,7 +398,11 @@ struct slice_run {
 	template <int OP, bool ONE>
 	__device__ __forceinline__ void run()
 	{
-		constexpr int U = tile_elems(sizeof(D), sizeof(S)) / PT_THREADS;
+		constexpr int U = slice_elems(sizeof(D), sizeof(S)) / PT_THREADS;
+		/* steps that no thread has an element in are left out (20 million
+		 * floats added in 4 x 4 slices: 327 us, now 240); four steps of
+		 * 16-byte elements cost less than the branches (1.06) */
+		constexpr bool SKIP = sizeof(D) <= 8;
 		const int n = w0 * w1, ld = w0 | 1;
 		const fastdiv by_n(n), by_w1(w1), by_w0(w0);
 		S y[U];
@@ -398,6 +410,8 @@ struct slice_run {
 		uint32_t e0 = threadIdx.x;
 #pragma unroll
 		for (int u = 0; u < U; u++) {
+			if (SKIP && u * PT_THREADS >= total)
+				break;
 			const uint32_t e = e0 + u * PT_THREADS;
 			if ((int)e < total) {
 				const uint32_t q = by_n(e), r = e - q * n;
@@ -408,6 +422,8 @@ struct slice_run {
 		if (op_reads_dst(OP)) {
 #pragma unroll
 			for (int u = 0; u < U; u++) {
+				if (SKIP && u * PT_THREADS >= total)
+					break;
 				const uint32_t e = e0 + u * PT_THREADS;
 				if ((int)e < total) {
 					const uint32_t q = by_n(e), r = e - q * n;
@@ -421,6 +437,8 @@ struct slice_run {
 		asm volatile("" : "+r"(e0));
 #pragma unroll
 		for (int u = 0; u < U; u++) {
+			if (SKIP && u * PT_THREADS >= total)
+				break;
 			const uint32_t e = e0 + u * PT_THREADS;
 			if ((int)e < total) {
 				const uint32_t q = by_n(e), r = e - q * n;
@@ -432,6 +450,8 @@ struct slice_run {
 		const scalars<D, S> c(t);
 #pragma unroll
 		for (int u = 0; u < U; u++) {
+			if (SKIP && u * PT_THREADS >= total)
+				break;
 			const uint32_t e = e0 + u * PT_THREADS;
 			if ((int)e < total) {
 				const uint32_t g = by_w0(e), q = by_n(e);
@@ -540,7 +560,8 @@ ptask_kernel(const __grid_constant__ task_pack pack,
 		with_op<D, S>(t, row_run<D, S>{dst, src, rows, (int)w0, t.dst_stride[0],
 		    t.src_stride[0], so, t, dre, dim_});
 	} else {
-		__shared__ S tile[tile_cap(tile_elems(sizeof(D), sizeof(S)))];
+		__shared__ S tile[MODE == 1 ? tile_cap(tile_elems(sizeof(D), sizeof(S))) :
+		    slice_cap(slice_elems(sizeof(D), sizeof(S)))];
 		if constexpr (MODE == 1) {
 			const uint32_t x = (uint32_t)local, d0 = m.ctas_d0, d1 = m.ctas_d1;
 			const uint32_t y = x / d0, c0 = x - y * d0, o = y / d1, c1 = y - o * d1;
@@ -693,9 +714,10 @@ reads_src(const xmgd_ptask_t &t)
 	return t.op != XMGD_OP_SET && t.op != XMGD_OP_SCALE;
 }
 
-/* the schedule of a task (task_meta.mode); tile_n: elements of a tile */
+/* the schedule of a task (task_meta.mode); slice_n: elements of a CTA's
+ * slices */
 static int
-schedule_of(const xmgd_ptask_t &t, int tile_n)
+schedule_of(const xmgd_ptask_t &t, int slice_n)
 {
 	const int64_t far = 1 << 24;
 
@@ -704,7 +726,7 @@ schedule_of(const xmgd_ptask_t &t, int tile_n)
 	if (t.ndim < 2 || t.src_stride[1] != 1 || t.src_stride[0] == 1 || !reads_src(t))
 		return 0;
 	return t.size[0] <= SLICE_MAX && t.size[1] <= SLICE_MAX &&
-	    t.size[0] * t.size[1] <= tile_n && t.src_stride[0] < far &&
+	    t.size[0] * t.size[1] <= slice_n && t.src_stride[0] < far &&
 	    t.dst_stride[0] < far && t.dst_stride[1] < far ? 3 : 1;
 }
 
@@ -722,13 +744,14 @@ plan_tasks(const xmgd_ptask_t *tasks, int ntasks, int dtype, int stype,
 	std::vector<task_meta> m0((size_t)ntasks);
 	std::vector<int64_t> cnt((size_t)ntasks);
 	const int tile_n = tile_elems(elem_bytes(dtype), elem_bytes(stype));
+	const int slice_n = slice_elems(elem_bytes(dtype), elem_bytes(stype));
 
-	int64_t nflat = 0;
+	int64_t nflat = 0, nslice = 0;
 	for (int i = 0; i < ntasks; i++) {
 		const xmgd_ptask_t &t = tasks[i];
 		task_meta &m = m0[i];
 		memset(&m, 0, sizeof m);
-		m.mode = schedule_of(t, tile_n);
+		m.mode = schedule_of(t, slice_n);
 		m.nouter = 1;
 		if (m.mode == 2) {
 			nflat += t.size[0];
@@ -738,10 +761,10 @@ plan_tasks(const xmgd_ptask_t *tasks, int ntasks, int dtype, int stype,
 				m.nouter *= t.size[d];
 			if (m.mode == 3) {
 				/* as many slices as the elements and the tile hold */
-				const int q = std::min({tile_n / (s0 * s1),
-				    tile_cap(tile_n) / (s1 * (s0 | 1)), SLICE_MAXQ});
+				const int q = std::min({slice_n / (s0 * s1),
+				    slice_cap(slice_n) / (s1 * (s0 | 1)), SLICE_MAXQ});
 				m.rows_per_cta = std::max(1, q);
-				cnt[i] = (m.nouter + m.rows_per_cta - 1) / m.rows_per_cta;
+				nslice += m.nouter * s0 * s1;
 			} else {
 				/* t1: the source's run in equal parts of at most 32;
 				 * t0: what fills the steps of 2^l1 lanes, in whole
@@ -775,11 +798,18 @@ plan_tasks(const xmgd_ptask_t *tasks, int ntasks, int dtype, int stype,
 	int32_t chunk = FLAT_ELEMS;
 	while (chunk > FLAT_MIN && nflat < (int64_t)chunk * 4 * num_sms())
 		chunk /= 2;
+	/* slices of a small batch: spread over two CTAs per SM in the same way */
+	const int64_t each = std::max<int64_t>(PT_THREADS, nslice / (2 * num_sms()));
 	for (int i = 0; i < ntasks; i++)
 		if (m0[i].mode == 2) {
 			m0[i].rows_per_cta = chunk;
 			m0[i].ctas_d0 = (int32_t)((tasks[i].size[0] + chunk - 1) / chunk);
 			cnt[i] = m0[i].ctas_d0;
+		} else if (m0[i].mode == 3) {
+			int32_t &q = m0[i].rows_per_cta;
+			q = (int32_t)std::max<int64_t>(1, std::min<int64_t>(q, each /
+			    (tasks[i].size[0] * tasks[i].size[1])));
+			cnt[i] = (m0[i].nouter + q - 1) / q;
 		}
 	sorted.clear();
 	meta.clear();
@@ -974,7 +1004,7 @@ run_batch(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks, double *d
  * a permuted operation of a block onto itself, unless each CTA's slices, all
  * loaded before any is stored, map onto themselves. */
 static bool
-overtakes(const xmgd_ptask_t &t, int tile_n)
+overtakes(const xmgd_ptask_t &t, int slice_n)
 {
 	bool same = true, outer = true;
 
@@ -985,7 +1015,7 @@ overtakes(const xmgd_ptask_t &t, int tile_n)
 		same = same && eq;
 		outer = outer && (d < 2 || eq);
 	}
-	return !same && !(outer && schedule_of(t, tile_n) == 3 && t.dst_stride[0] == 1 &&
+	return !same && !(outer && schedule_of(t, slice_n) == 3 && t.dst_stride[0] == 1 &&
 	    t.size[0] == t.size[1] && t.dst_stride[1] == t.src_stride[0]);
 }
 
@@ -1009,17 +1039,17 @@ xmgd_ptasks(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks,
     double *dots)
 {
 	constexpr size_t COPY_MAX = (size_t)256 << 20;
-	const int esz = elem_bytes(stype), tile_n = tile_elems(elem_bytes(dtype), esz);
+	const int esz = elem_bytes(stype), slice_n = slice_elems(elem_bytes(dtype), esz);
 	std::vector<xmgd_ptask_t> now, copied;
 	int st;
 
 	for (int i = 0; i < ntasks; i++)
-		if (overtakes(tasks[i], tile_n))
+		if (overtakes(tasks[i], slice_n))
 			copied.push_back(tasks[i]);
 	if (copied.empty())
 		return run_batch(dtype, stype, tasks, ntasks, dots);
 	for (int i = 0; i < ntasks; i++)
-		if (!overtakes(tasks[i], tile_n))
+		if (!overtakes(tasks[i], slice_n))
 			now.push_back(tasks[i]);
 	st = run_batch(dtype, stype, now.data(), (int)now.size(), dots);
 	for (size_t first = 0, end; first < copied.size() && st == XMG_OK; first = end) {
