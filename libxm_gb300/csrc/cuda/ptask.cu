@@ -36,6 +36,11 @@ constexpr int PT_THREADS = 256;
 constexpr int ROW_ELEMS = 4096;    /* elements per CTA in row mode */
 constexpr int FLAT_ELEMS = 8192;   /* elements per CTA in flat mode, at most */
 constexpr int FLAT_MIN = 1024;     /* ... and at least */
+/* rows of at most this many elements whose source runs are longer than a
+ * slice go by the row schedule: a tile would hold 32 of them in a CTA, 256
+ * go in one there (dot of 2 x 1 000 000 floats 432 us as tiles, 73 as rows;
+ * quotient of 12 x 200 001 doubles 62 and 31) */
+constexpr int ROW_THIN = 16;
 constexpr int SLICE_MAX = 48;      /* slices: extents at most */
 constexpr int SLICE_MAXQ = 64;     /* slices per CTA at most */
 /* tile: elements per CTA (eight per thread, four of the 16-byte types), and
@@ -723,7 +728,8 @@ schedule_of(const xmgd_ptask_t &t, int slice_n)
 
 	if (t.ndim == 1 && t.dst_stride[0] == 1 && (!reads_src(t) || t.src_stride[0] == 1))
 		return 2;
-	if (t.ndim < 2 || t.src_stride[1] != 1 || t.src_stride[0] == 1 || !reads_src(t))
+	if (t.ndim < 2 || t.src_stride[1] != 1 || t.src_stride[0] == 1 || !reads_src(t) ||
+	    (t.size[0] <= ROW_THIN && t.size[1] > SLICE_MAX))
 		return 0;
 	return t.size[0] <= SLICE_MAX && t.size[1] <= SLICE_MAX &&
 	    t.size[0] * t.size[1] <= slice_n && t.src_stride[0] < far &&
