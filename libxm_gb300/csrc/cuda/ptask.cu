@@ -9,7 +9,7 @@
  * unfold -> scale -> fold -> axpy host loops (tensor.c:436-639,
  * scalar.c:123-239, xm.c:28-508) with one HBM pass.
  *
- * Four schedules, chosen per task on the host after xmg_ptask_shape has
+ * Five schedules, chosen per task on the host after xmg_ptask_shape has
  * normalised the iteration space; each schedule is its own kernel
  * instantiation (so the lean ones keep few registers),
  * and a batch launches one kernel per schedule present:
@@ -22,13 +22,20 @@
  *    memory (loads along the source's runs, stores along the
  *    destination's): the gather-transpose of unfold/fold;
  *  - tile: the same for larger extents, a t0 x t1 tile per CTA;
+ *  - slab: xm_copy's transposes when each s0 x s1 slice lies contiguously
+ *    on both sides and consecutive slices follow one another (whole
+ *    blocks whose permutation swaps the two leading dimensions): a CTA
+ *    brings its slices in with one bulk copy into shared memory,
+ *    transposes there and stores along the destination's run.
  */
+#include <stdlib.h>
 #include <string.h>
 #include <algorithm>
 #include <type_traits>
 #include <vector>
 
 #include "common.cuh"
+#include "tc.cuh"
 
 namespace xmg {
 
@@ -43,6 +50,12 @@ constexpr int FLAT_MIN = 1024;     /* ... and at least */
 constexpr int ROW_THIN = 16;
 constexpr int SLICE_MAX = 48;      /* slices: extents at most */
 constexpr int SLICE_MAXQ = 64;     /* slices per CTA at most */
+/* slab: about SLAB_CHUNK bytes of slices per CTA (one slice at least), at
+ * most SLAB_SMEM bytes of shared memory (the source's slices and the padded
+ * tile) */
+constexpr int64_t SLAB_CHUNK = 16384;
+constexpr int64_t SLAB_SMEM = 64 * 1024;
+constexpr int64_t SLAB_MIN = 32 << 20;   /* bytes of a batch's slabs */
 /* tile: elements per CTA (eight per thread, four of the 16-byte types), and
  * the shared tile with the padding of its rows */
 static constexpr int tile_elems(int dbytes, int sbytes)
@@ -64,9 +77,9 @@ static inline int lanes_log2(int n) { return n <= 8 ? 3 : n <= 16 ? 4 : 5; }
 
 struct task_meta {
 	int64_t first_cta;
-	int32_t mode;          /* 0 row, 1 tile, 2 flat, 3 slices */
+	int32_t mode;          /* 0 row, 1 tile, 2 flat, 3 slices, 4 slab */
 	int32_t rows_per_cta;  /* row mode: outer rows per CTA; flat mode:
-	                          elements per CTA; slices: slices */
+	                          elements per CTA; slices and slab: slices */
 	int64_t nouter;        /* row: product of dims 1..; tile: dims 2.. */
 	int32_t ctas_d0, ctas_d1;
 	int32_t t0, t1;        /* tile mode: extents of a tile */
@@ -620,6 +633,119 @@ ptask_kernel(const __grid_constant__ task_pack pack,
 	}
 }
 
+/* a bounded wait of the slab schedule gave up (set on the device, read
+ * and cleared by the host after the launches) */
+__device__ int g_slab_err;
+
+/*
+ * Slab schedule: rows_per_cta consecutive s0 x s1 slices per CTA, each
+ * contiguous on both sides (source: dim 1 unit stride, dim 0 stride s1;
+ * destination: dim 0 unit stride, dim 1 stride s0; slice q at q * s0 * s1
+ * on both), 16-byte aligned.  One bulk copy brings the CTA's slices of the
+ * source into shared memory (one instruction, where the slices schedule
+ * issues a load per element); the source goes into a tile with an odd row
+ * pitch, so that both the transposing pass (threads along the source's
+ * run) and the storing pass (threads along the destination's run) touch
+ * distinct banks; stores follow the destination's run.
+ */
+template <typename T>
+__global__ void __launch_bounds__(PT_THREADS, 6)
+slab_kernel(const __grid_constant__ task_pack pack,
+    const xmgd_ptask_t *__restrict__ dtasks,
+    const task_meta *__restrict__ dmeta, int ntasks, int64_t cta0)
+{
+	extern __shared__ __align__(16) unsigned char dsm[];
+	__shared__ __align__(8) uint64_t bar;
+	__shared__ int s_err;
+
+	const int64_t cta = cta0 + blockIdx.x;
+	const xmgd_ptask_t *tasks = dtasks ? dtasks : pack.t;
+	const task_meta *meta = dtasks ? dmeta : pack.m;
+	const int lo = last_at_most(ntasks, cta, [&](int i) { return meta[i].first_cta; });
+	const xmgd_ptask_t &t = tasks[lo];
+	const task_meta &m = meta[lo];
+	const int s0 = t.size[0], s1 = t.size[1], n = s0 * s1;
+	const int ld = s0 | 1;
+	const int64_t o0 = (cta - m.first_cta) * m.rows_per_cta;
+	const int k = (int)(m.nouter - o0 < m.rows_per_cta ? m.nouter - o0 :
+	    m.rows_per_cta);
+	const int kn = k * n;
+	const uint32_t cbytes = (uint32_t)kn * (uint32_t)sizeof(T);
+	const T *sb = reinterpret_cast<const T *>(dsm);
+	T *tb = reinterpret_cast<T *>(dsm + cbytes);
+	T *dst = reinterpret_cast<T *>(t.dst) + o0 * n;
+	const T *src = reinterpret_cast<const T *>(t.src) + o0 * n;
+	const T al = num<T>::mk(t.alpha);
+
+	const uint32_t b = smem_u32(&bar);
+	if (threadIdx.x == 0) {
+		s_err = 0;
+		mbar_init(b, 1);
+		asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+	}
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		mbar_expect_tx(b, cbytes);
+		bulk_g2s(smem_u32(dsm), src, cbytes, b);
+	}
+	const bool ok = mbar_wait(b, 0, &s_err, &g_slab_err, 1);
+	/* every thread leaves together when the wait gave up */
+	if (__syncthreads_or(!ok))
+		return;
+	/* source order e = q n + i0 s1 + i1 -> tile q s1 ld + i1 ld + i0 */
+	{
+		int q = threadIdx.x / n, r = threadIdx.x - q * n;
+		int i0 = r / s1, i1 = r - i0 * s1;
+		const int dq = PT_THREADS / n, dr = PT_THREADS - dq * n;
+		const int d0 = dr / s1, d1 = dr - d0 * s1;
+		for (int e = threadIdx.x; e < kn; e += PT_THREADS) {
+			tb[(q * s1 + i1) * ld + i0] = sb[e];
+			i1 += d1;
+			if (i1 >= s1) { i1 -= s1; i0++; }
+			i0 += d0;
+			if (i0 >= s0) { i0 -= s0; q++; }
+			q += dq;
+		}
+	}
+	__syncthreads();
+	/* destination order e = q n + i1 s0 + i0 */
+	int q = threadIdx.x / n, r = threadIdx.x - q * n;
+	int i1 = r / s0, i0 = r - i1 * s0;
+	const int dq = PT_THREADS / n, dr = PT_THREADS - dq * n;
+	const int d1 = dr / s0, d0 = dr - d1 * s0;
+	for (int e = threadIdx.x; e < kn; e += PT_THREADS) {
+		dst[e] = num<T>::mul(al, tb[(q * s1 + i1) * ld + i0]);
+		i0 += d0;
+		if (i0 >= s0) { i0 -= s0; i1++; }
+		i1 += d1;
+		if (i1 >= s1) { i1 -= s1; q++; }
+		q += dq;
+	}
+}
+
+/* the slab schedule for a task: slices per CTA (0 when the schedule does
+ * not apply: xm_copy of one scalar type only), and the CTA's shared memory */
+static int64_t
+slab_shape(const xmgd_ptask_t &t, int dbytes, int sbytes, int64_t *smem)
+{
+	if (dbytes != sbytes || t.op != XMGD_OP_COPY || t.ndim < 2 || t.ndim > 3)
+		return 0;
+	const int64_t s0 = t.size[0], s1 = t.size[1], n = s0 * s1;
+	const int64_t mt = sbytes <= 8 ? 48 : 32;
+	if (s0 > mt || s1 > mt || s0 < 2 || s1 < 2 ||
+	    t.dst_stride[0] != 1 || t.dst_stride[1] != s0 ||
+	    t.src_stride[1] != 1 || t.src_stride[0] != s1 ||
+	    (t.ndim == 3 && (t.dst_stride[2] != n || t.src_stride[2] != n)) ||
+	    (n * sbytes) % 16 != 0 || ((t.dst | t.src) & 15) != 0)
+		return 0;
+	int64_t k = n * sbytes >= SLAB_CHUNK ? 1 : SLAB_CHUNK / (n * sbytes);
+	const int64_t cap = t.ndim == 3 ? t.size[2] : 1;
+	if (k > cap)
+		k = cap;
+	*smem = k * n * sbytes + k * s1 * (s0 | 1) * sbytes;
+	return *smem <= SLAB_SMEM ? k : 0;
+}
+
 /*
  * Sums of the per-CTA partial dot products, per task (in the caller's order,
  * order[]): LANES threads stride over a task's CTAs, four loads in flight, so
@@ -683,9 +809,37 @@ dot_sum_kernel(const __grid_constant__ task_pack pack,
 
 template <typename D, typename S>
 static int
-launch(const task_pack &pack, const xmgd_ptask_t *dtasks, const task_meta *dmeta,
-    int ntasks, const int64_t *begin, double *dpartial)
+launch_slab(const task_pack &pack, const xmgd_ptask_t *dtasks, const task_meta *dmeta,
+    int ntasks, int64_t cta0, int64_t n, int64_t smem)
 {
+	if constexpr (std::is_same<D, S>::value) {
+		static bool attr = false;
+		if (!attr) {
+			XMG_CK(cudaFuncSetAttribute(slab_kernel<D>,
+			    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SLAB_SMEM));
+			attr = true;
+		}
+		slab_kernel<D><<<(unsigned)n, PT_THREADS, (size_t)smem, stream()>>>(
+		    pack, dtasks, dmeta, ntasks, cta0);
+		g_launches++;
+		XMG_CK(cudaGetLastError());
+		return XMG_OK;
+	} else {
+		return xmg_seterr(XMG_EINVAL, "slab schedule: scalar conversion");
+	}
+}
+
+template <typename D, typename S>
+static int
+launch(const task_pack &pack, const xmgd_ptask_t *dtasks, const task_meta *dmeta,
+    int ntasks, const int64_t *begin, int64_t slab_smem, double *dpartial)
+{
+	if (begin[5] > begin[4]) {
+		int st = launch_slab<D, S>(pack, dtasks, dmeta, ntasks, begin[4],
+		    begin[5] - begin[4], slab_smem);
+		if (st)
+			return st;
+	}
 	/* one launch per schedule, over that schedule's CTA range */
 	for (int mode = 0; mode < 4; mode++) {
 		const int64_t n = begin[mode + 1] - begin[mode];
@@ -719,8 +873,8 @@ reads_src(const xmgd_ptask_t &t)
 	return t.op != XMGD_OP_SET && t.op != XMGD_OP_SCALE;
 }
 
-/* the schedule of a task (task_meta.mode); slice_n: elements of a CTA's
- * slices */
+/* the schedule of a task without slab (task_meta.mode); slice_n: elements of
+ * a CTA's slices */
 static int
 schedule_of(const xmgd_ptask_t &t, int slice_n)
 {
@@ -745,18 +899,49 @@ schedule_of(const xmgd_ptask_t &t, int slice_n)
 static void
 plan_tasks(const xmgd_ptask_t *tasks, int ntasks, int dtype, int stype,
     std::vector<xmgd_ptask_t> &sorted, std::vector<task_meta> &meta,
-    std::vector<int> &order, int64_t begin[5])
+    std::vector<int> &order, int64_t begin[6], int64_t *slab_smem)
 {
 	std::vector<task_meta> m0((size_t)ntasks);
 	std::vector<int64_t> cnt((size_t)ntasks);
 	const int tile_n = tile_elems(elem_bytes(dtype), elem_bytes(stype));
 	const int slice_n = slice_elems(elem_bytes(dtype), elem_bytes(stype));
+	const char *e = getenv("XMG_PTASK_SLAB");
+	const bool slab_on = !(e && strcmp(e, "0") == 0);
+
+	/* slab beats slices on what does not stay in L2 (copies of 40 million
+	 * elements in 16 x 16 slices: float 89 against 134 us, double 119 against
+	 * 151; of 3 million 28 against 26, its flag's way to the host); with
+	 * 16-byte elements only where slices leave a quarter of their CTAs empty
+	 * or products with the scalar to do (20 million in 24 x 24: 167 against
+	 * 190 us; in 20 x 20: 173 against 164, scaled 173 against 203) */
+	const int esz = elem_bytes(stype);
+	int64_t need = 0, whole = 0;
+	auto slab_task = [&](const xmgd_ptask_t &t) {
+		const int64_t k = slab_shape(t, elem_bytes(dtype), esz, &need);
+		const int n = k > 0 ? t.size[0] * t.size[1] : 1;
+		const bool one = t.alpha[0] == 1 && t.alpha[1] == 0;
+		return esz == 16 && one && slice_n / n * n * 4 >= slice_n * 3 ? 0 : k;
+	};
+	for (int i = 0; i < ntasks && slab_on; i++)
+		if (slab_task(tasks[i]) > 0)
+			whole += (int64_t)tasks[i].size[0] * tasks[i].size[1] *
+			    (tasks[i].ndim == 3 ? tasks[i].size[2] : 1) * esz;
 
 	int64_t nflat = 0, nslice = 0;
+	*slab_smem = 0;	/* the slab launch's: the largest of its CTAs' */
 	for (int i = 0; i < ntasks; i++) {
 		const xmgd_ptask_t &t = tasks[i];
 		task_meta &m = m0[i];
 		memset(&m, 0, sizeof m);
+		const int64_t k = whole >= SLAB_MIN ? slab_task(t) : 0;
+		if (k > 0) {
+			m.mode = 4;
+			m.nouter = t.ndim == 3 ? t.size[2] : 1;
+			m.rows_per_cta = (int32_t)k;
+			cnt[i] = (m.nouter + k - 1) / k;
+			*slab_smem = std::max(*slab_smem, need);
+			continue;
+		}
 		m.mode = schedule_of(t, slice_n);
 		m.nouter = 1;
 		if (m.mode == 2) {
@@ -821,7 +1006,7 @@ plan_tasks(const xmgd_ptask_t *tasks, int ntasks, int dtype, int stype,
 	meta.clear();
 	order.clear();
 	int64_t n = 0;
-	for (int mode = 0; mode < 4; mode++) {
+	for (int mode = 0; mode < 5; mode++) {
 		begin[mode] = n;
 		for (int i = 0; i < ntasks; i++)
 			if (m0[i].mode == mode) {
@@ -833,16 +1018,16 @@ plan_tasks(const xmgd_ptask_t *tasks, int ntasks, int dtype, int stype,
 				order.push_back(i);
 			}
 	}
-	begin[4] = n;
+	begin[5] = n;
 }
 
 static int
 launch_types(int dtype, int stype, const task_pack &pack, const xmgd_ptask_t *dt, const task_meta *dm,
-    int ntasks, const int64_t *begin, double *dp)
+    int ntasks, const int64_t *begin, int64_t slab_smem, double *dp)
 {
 	int st;
 
-#define L(D, S) st = launch<D, S>(pack, dt, dm, ntasks, begin, dp)
+#define L(D, S) st = launch<D, S>(pack, dt, dm, ntasks, begin, slab_smem, dp)
 	if (dtype == stype) {
 		switch (dtype) {
 		case 0: L(float, float); break;
@@ -884,7 +1069,8 @@ xmgd_ptask_stage(const xmgd_ptask_t *tasks, int ntasks, int stype,
 	if (ntasks <= 0)
 		return XMG_OK;
 	/* batches staged for replay carry one type on both sides */
-	plan_tasks(tasks, ntasks, stype, stype, sorted, meta, order, b->begin);
+	plan_tasks(tasks, ntasks, stype, stype, sorted, meta, order, b->begin,
+	    &b->slab_smem);
 	if ((st = xmgd_alloc(tb + meta.size() * sizeof(task_meta), &b->dbuf)))
 		return st;
 	b->ntasks = ntasks;
@@ -905,11 +1091,12 @@ xmgd_ptask_launch(int dtype, int stype, const xmgd_ptask_batch_t *b)
 	static const task_pack none = {};
 	return launch_types(dtype, stype, none, (const xmgd_ptask_t *)b->dbuf,
 	    (const task_meta *)(b->dbuf + task_bytes(b->ntasks)), b->ntasks,
-	    b->begin, nullptr);
+	    b->begin, b->slab_smem, nullptr);
 }
 
 /* page-locked host memory of the element-wise calls: the batch on its way
- * to the device, or the sums a dot product's last kernel writes.  Grow-only;
+ * to the device, the sums a dot product's last kernel writes, the slab
+ * schedule's flag on its way back.  Grow-only;
  * every call that uses it waits for its kernels before it returns. */
 static int
 batch_pinned(size_t bytes, void **p)
@@ -936,18 +1123,20 @@ run_batch(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks, double *d
 	std::vector<task_meta> meta;
 	std::vector<int> order;
 	task_pack pack;
-	int64_t begin[5], nctas;
+	int64_t begin[6], nctas, slab_smem;
 	uint64_t dbuf = 0, dpart = 0;
 	const task_meta *dmeta = nullptr;
 	const int *dorder = nullptr;
 	void *pin = nullptr;
 	double *sums = nullptr;
+	int *slab_err = nullptr;
 	int st;
 
 	if (ntasks <= 0)
 		return XMG_OK;
-	plan_tasks(tasks, ntasks, dtype, stype, sorted, meta, order, begin);
-	nctas = begin[4];
+	plan_tasks(tasks, ntasks, dtype, stype, sorted, meta, order, begin, &slab_smem);
+	nctas = begin[5];
+	const bool slab = begin[5] > begin[4];
 	const size_t tb = task_bytes(ntasks);
 	const size_t mb = ((size_t)ntasks * sizeof(task_meta) + 255) & ~(size_t)255;
 	const size_t ob = ((size_t)ntasks * sizeof(int) + 255) & ~(size_t)255;
@@ -958,10 +1147,11 @@ run_batch(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks, double *d
 		inorder = inorder && order[i] == i;
 	/* an out-of-order batch of dots needs its order on the device */
 	const size_t up = small && (inorder || !dots) ? 0 : tb + mb + ob;
-	if (up + db > 0) {
-		if ((st = batch_pinned(up + db, &pin)) != XMG_OK)
+	if (up + db + slab > 0) {
+		if ((st = batch_pinned(up + db + 256, &pin)) != XMG_OK)
 			return st;
 		sums = (double *)((char *)pin + up);
+		slab_err = (int *)((char *)pin + up + db);
 	}
 	if (up > 0) {
 		char *h = (char *)pin;
@@ -982,7 +1172,7 @@ run_batch(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks, double *d
 	    &dpart)) != XMG_OK)
 		return st;
 	st = launch_types(dtype, stype, pack, (const xmgd_ptask_t *)dbuf, dmeta, ntasks,
-	    begin, (double *)dpart);
+	    begin, slab_smem, (double *)dpart);
 	if (st == XMG_OK && dots) {
 		int64_t longest = 0;
 		for (int i = 0; i < ntasks; i++)
@@ -997,10 +1187,19 @@ run_batch(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks, double *d
 		g_launches++;
 		st = check(cudaGetLastError(), "dot_sum_kernel");
 	}
+	if (st == XMG_OK && slab)
+		st = check(cudaMemcpyFromSymbolAsync(slab_err, g_slab_err, sizeof(int), 0,
+		    cudaMemcpyDeviceToHost, stream()), "slab flag");
 	/* the buffers are reused by the next batch: wait here */
 	const int st2 = check(cudaStreamSynchronize(stream()), "ptask_kernel");
 	if (st != XMG_OK || (st = st2) != XMG_OK)
 		return st;
+	if (slab && *slab_err) {
+		const int zero = 0;
+		XMG_CK(cudaMemcpyToSymbol(g_slab_err, &zero, sizeof zero));
+		return xmg_seterr(XMG_ETIMEOUT, "slab schedule: a bulk copy did not complete "
+		    "within the bounded wait");
+	}
 	if (dots)
 		memcpy(dots, sums, db);
 	return XMG_OK;
