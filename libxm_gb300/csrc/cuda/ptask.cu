@@ -1096,8 +1096,8 @@ xmgd_ptask_launch(int dtype, int stype, const xmgd_ptask_batch_t *b)
 
 /* page-locked host memory of the element-wise calls: the batch on its way
  * to the device, the sums a dot product's last kernel writes, the slab
- * schedule's flag on its way back.  Grow-only;
- * every call that uses it waits for its kernels before it returns. */
+ * schedule's flag on its way back.  Grow-only; every call that uses it
+ * waits for its kernels before it returns. */
 static int
 batch_pinned(size_t bytes, void **p)
 {
@@ -1147,6 +1147,12 @@ run_batch(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks, double *d
 		inorder = inorder && order[i] == i;
 	/* an out-of-order batch of dots needs its order on the device */
 	const size_t up = small && (inorder || !dots) ? 0 : tb + mb + ob;
+	/* (all memory before the first copy: from there on the page-locked buffer
+	 * is in use until the wait below) */
+	if ((up > 0 && (st = xmgd_scratch(2, up, &dbuf)) != XMG_OK) ||
+	    (dots && (st = xmgd_scratch(3, (size_t)nctas * 2 * sizeof(double), &dpart)) !=
+	    XMG_OK))
+		return st;
 	if (up + db + slab > 0) {
 		if ((st = batch_pinned(up + db + 256, &pin)) != XMG_OK)
 			return st;
@@ -1158,8 +1164,6 @@ run_batch(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks, double *d
 		memcpy(h, sorted.data(), (size_t)ntasks * sizeof(xmgd_ptask_t));
 		memcpy(h + tb, meta.data(), (size_t)ntasks * sizeof(task_meta));
 		memcpy(h + tb + mb, order.data(), (size_t)ntasks * sizeof(int));
-		if ((st = xmgd_scratch(2, up, &dbuf)) != XMG_OK)
-			return st;
 		XMG_CK(cudaMemcpyAsync((void *)dbuf, pin, up, cudaMemcpyHostToDevice,
 		    stream()));
 		dmeta = (const task_meta *)(dbuf + tb);
@@ -1168,9 +1172,6 @@ run_batch(int dtype, int stype, const xmgd_ptask_t *tasks, int ntasks, double *d
 		memcpy(pack.t, sorted.data(), (size_t)ntasks * sizeof(xmgd_ptask_t));
 		memcpy(pack.m, meta.data(), (size_t)ntasks * sizeof(task_meta));
 	}
-	if (dots && (st = xmgd_scratch(3, (size_t)nctas * 2 * sizeof(double),
-	    &dpart)) != XMG_OK)
-		return st;
 	st = launch_types(dtype, stype, pack, (const xmgd_ptask_t *)dbuf, dmeta, ntasks,
 	    begin, slab_smem, (double *)dpart);
 	if (st == XMG_OK && dots) {
