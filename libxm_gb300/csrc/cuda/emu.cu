@@ -1723,12 +1723,16 @@ launch_split(emu_plan *e)
 		    e->cand[e->cur].nslots * SLOT_BYTES, stream()));
 	if (!e->a_mode) {
 		cudaStream_t aux;
-		if ((st = fork_aux(&aux)) ||
-		    (st = launch_side<TIN>(e, 0, 0, EA, flags, aux)) ||
+		if ((st = fork_aux(&aux)))
+			return st;
+		if ((st = launch_side<TIN>(e, 0, 0, EA, flags, aux)) ||
 		    (st = launch_side<TIN>(e, 0, 1, EA, flags, aux)) ||
 		    (st = launch_side<TIN>(e, 1, 0, EB, flags, stream())) ||
-		    (st = launch_side<TIN>(e, 1, 1, EB, flags, stream())))
+		    (st = launch_side<TIN>(e, 1, 1, EB, flags, stream()))) {
+			/* what the second stream got is waited for on the engine's */
+			join_aux();
 			return st;
+		}
 		return join_aux();
 	}
 	/* a shared a side: the preparing plan fills the shared exponent table
