@@ -6,8 +6,9 @@
  * precision tensor-core path or the plain path, and stages the work lists.
  * xmgd_plan_run replays the whole launch sequence -- beta-only blocks,
  * exponent and split kernels, the persistent grouped GEMM, the plain GEMM
- * -- directly for the first runs, which also tune, and as CUDA graphs from
- * the third on, then reads the device flags once.  Operands with
+ * -- directly in the first run and in those that tune, as CUDA graphs (but
+ * for the plain GEMM) from the next one on, then reads the device flags
+ * once.  Operands with
  * Inf/NaN make the split-precision GEMM write nothing; those blocks are then
  * recomputed on the plain FP64 path (AUTO) or reported (EMU64).
  */
@@ -78,11 +79,10 @@ struct xmgd_plan {
 	uint64_t d_pg = 0;                   /* plain GEMM work list */
 	int n_pg = 0, pg_tile = 0;
 	emu_plan *ep = nullptr;
-	/* three captured segments, timed by events recorded between their
-	 * launches: 0 beta-only blocks + operand split, 1 split-precision
-	 * GEMM (one graph each per autotuner candidate, whose form fixes the
-	 * operands' layout), 2 plain GEMM */
-	segment seg2;
+	/* three segments, timed by events recorded between their launches:
+	 * 0 beta-only blocks + operand split, 1 split-precision GEMM, both
+	 * captured (one graph each per autotuner candidate, whose form fixes
+	 * the operands' layout), 2 plain GEMM, one direct launch */
 	std::vector<segment> seg0, seg1;
 	cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
 };
@@ -222,7 +222,6 @@ drop(segment &g)
 static void
 drop_graphs(xmgd_plan *dp)
 {
-	drop(dp->seg2);
 	for (segment &g : dp->seg0)
 		drop(g);
 	for (segment &g : dp->seg1)
@@ -362,17 +361,16 @@ capture(xmgd_plan *dp, int seg, segment &out)
 }
 
 static int
-run_segment(xmgd_plan *dp, int seg, segment &g)
+run_segment(xmgd_plan *dp, int seg, int cand)
 {
 	int st;
 
-	if (seg_empty(dp, seg))
-		return XMG_OK;
-	/* a graph pays from the third launch on: a plan's first run, its tuning
-	 * runs and the plain GEMM, one kernel, launch directly */
+	/* a graph pays only if it is launched again: a plan's first run, its
+	 * tuning runs and the plain GEMM, one kernel, launch directly */
 	if (!graphs_enabled() || dp->one_shot || seg == 2 || !dp->ran ||
 	    (dp->ep && !emu_tuned(dp->ep)))
 		return record(dp, seg);
+	segment &g = seg == 0 ? dp->seg0[cand] : dp->seg1[cand];
 	if (!g.x && (st = capture(dp, seg, g)))
 		return st;
 	XMG_CK(cudaGraphLaunch(g.x, stream()));
@@ -404,8 +402,7 @@ xmgd_plan_run(xmgd_plan *dp, int *precision_used)
 		at[seg + 1] = at[seg];
 		if (seg_empty(dp, seg))
 			continue;
-		if ((st = run_segment(dp, seg, seg == 0 ? dp->seg0[cand] :
-		    seg == 1 ? dp->seg1[cand] : dp->seg2)))
+		if ((st = run_segment(dp, seg, cand)))
 			return st;
 		at[seg + 1] = seg + 1;
 		XMG_CK(cudaEventRecord(dp->ev[seg + 1], stream()));

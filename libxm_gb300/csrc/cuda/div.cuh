@@ -72,9 +72,6 @@ __host__ __device__ __forceinline__ uint32_t recip22(uint32_t frac)
 	memcpy(&f, &u, sizeof f);
 	f = 1.0f / f;
 	memcpy(&u, &f, sizeof u);
-#ifdef DIV_NUDGE
-	u += DIV_NUDGE;
-#endif
 #endif
 	/* the approximation may leave [1/2, 1) by its last bit */
 	if (u < 0x3f000000u)

@@ -119,14 +119,6 @@ __device__ __forceinline__ void bulk_g2s_el(uint32_t el, uint32_t dst, const voi
 	    : "memory");
 }
 
-/* bring [src, src + bytes) into L2 ahead of its shared-memory copy
- * (address and size multiples of 16 bytes) */
-__device__ __forceinline__ void bulk_prefetch_l2(const void *src, uint32_t bytes)
-{
-	asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;"
-	    :: "l"(src), "r"(bytes) : "memory");
-}
-
 __device__ __forceinline__ void tc_fence_before()
 {
 	asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -148,21 +140,13 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t saddr, uint32_t sbo)
 	    (1ull << 46);
 }
 
-__device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t a, uint64_t b,
-    uint32_t idesc, uint32_t acc)
-{
-	asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-	    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-	    :: "r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc));
-}
-
 /* What an MMA does with the M-side operand's buffer (the collector): load it
  * for this MMA alone, load and keep it, take what the last MMA kept, take it
  * for the last time.  Between KEEP and LAST every MMA of the thread has the
  * same M-side descriptor. */
 enum { COL_NONE, COL_KEEP, COL_USE, COL_LAST };
 
-/* The same with each descriptor passed as (low, high) words, executed by the
+/* One MMA, each descriptor passed as (low, high) words, executed by the
  * whole warp in step and issued by the lane where el is nonzero.  Descriptors
  * live in the warp's uniform registers: in code that one lane runs alone each
  * operand is moved there for each MMA (54 cycles per MMA, and some 300 more
@@ -225,21 +209,6 @@ __device__ __forceinline__ void tmem_ld(uint32_t taddr, float (&v)[4])
 	    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr));
 #pragma unroll
 	for (int i = 0; i < 4; i++)
-		v[i] = __uint_as_float(r[i]);
-}
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
-{
-	uint32_t r[16];
-	asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-	    "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-	    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]),
-	      "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-	      "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
-	      "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-	    : "r"(taddr));
-#pragma unroll
-	for (int i = 0; i < 16; i++)
 		v[i] = __uint_as_float(r[i]);
 }
 
