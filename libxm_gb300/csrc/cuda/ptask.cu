@@ -10,13 +10,13 @@
  * scalar.c:123-239, xm.c:28-508) with one HBM pass.
  *
  * Five schedules, chosen per task on the host after xmg_ptask_shape has
- * normalised the iteration space; each schedule is its own kernel
- * instantiation (so the lean ones keep few registers),
- * and a batch launches one kernel per schedule present:
+ * normalised the iteration space; each schedule is its own kernel, and a
+ * batch launches one kernel per schedule present:
  *  - flat: one contiguous run on both sides (whole canonical blocks);
  *  - row: dimension 0 unit-stride on the destination side; a CTA covers
  *    ROW_ELEMS elements along dim 0 for as many outer rows as fit, with
- *    per-row outer offsets precomputed in shared memory;
+ *    per-row outer offsets precomputed in shared memory (outer permutations,
+ *    transposes of thin blocks);
  *  - slices: the source's unit-stride dimension is dim 1 and both extents
  *    are small: a CTA moves whole s0 x s1 slices through padded shared
  *    memory (loads along the source's runs, stores along the
@@ -530,6 +530,8 @@ struct row_run {
 	}
 };
 
+/* Four CTAs per SM for every schedule: with five (48 registers) flat runs
+ * spill, and their sums and copies take 3 to 12 % longer. */
 template <typename D, typename S, int MODE>
 __global__ void __launch_bounds__(PT_THREADS, 4)
 ptask_kernel(const __grid_constant__ task_pack pack,
