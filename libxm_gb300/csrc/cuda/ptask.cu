@@ -985,10 +985,12 @@ plan_tasks(const xmgd_ptask_t *tasks, int ntasks, int dtype, int stype,
 			cnt[i] = (int64_t)m.ctas_d0 * ((m.nouter + rows - 1) / rows);
 		}
 	}
-	/* flat CTAs of 8192 elements, halved while they leave SMs without
-	 * four of them (a small batch is bound by the latency of a CTA's
-	 * passes: 33 000 elements divided in 6 CTAs took 52 us) */
-	int32_t chunk = FLAT_ELEMS;
+	/* flat CTAs of 8192 elements (4096 of 16 bytes: setting a block of 196
+	 * million complex doubles 450 us with 8192, 430 with 4096), halved while
+	 * they leave SMs without four of them (a small batch is bound by the
+	 * latency of a CTA's passes: 33 000 elements divided in 6 CTAs took 52
+	 * us) */
+	int32_t chunk = elem_bytes(dtype) == 16 ? FLAT_ELEMS / 2 : FLAT_ELEMS;
 	while (chunk > FLAT_MIN && nflat < (int64_t)chunk * 4 * num_sms())
 		chunk /= 2;
 	/* slices of a small batch: spread over two CTAs per SM in the same way */
