@@ -147,7 +147,7 @@ __device__ __forceinline__ int find_view(const view_meta *m, int n, int64_t cta)
  * parts do not. */
 __host__ __device__ __forceinline__ int64_t part_at(int32_t row, int32_t col, int half)
 {
-	return 2 * ((int64_t)row + col) + half;
+	return 2 * (int64_t)(row + col) + half;
 }
 
 /* Element (k', r) of a view: real views directly, complex views realified
@@ -2411,38 +2411,50 @@ split_items(const xmgd_contract_t *p, int cplx, bool rowmajor, size_t sms, bool 
 	return slots;
 }
 
+/* K steps of every block's pairs in all */
+static std::vector<int>
+block_steps(const xmgd_contract_t *p, int cplx)
+{
+	std::vector<int> steps(p->ncblocks, 0);
+	for (int i = 0; i < p->ncblocks; i++)
+		for (int q = 0; q < p->cblocks[i].npairs; q++)
+			steps[i] += (cplx ? 2 : 1) *
+			    ((p->pairs[p->cblocks[i].first_pair + q].k + EMU_KS - 1) / EMU_KS);
+	return steps;
+}
+
 /* What the kernel takes from a list with its chunks and parts beyond
  * items_ok, in O(items): an item's chunks lie in the array; an undivided one
  * starts at its first step and holds all of them; the parts of a slot are as
  * many as each of them says, share tile and members, and follow one another
  * from the first step and chunk to the last. */
 static bool
-parts_ok(const xmgd_contract_t *p, int cplx, const std::vector<emu_item> &items,
-    const std::vector<emu_member> &mem, const std::vector<emu_chunk> &chunks, int nslots)
+parts_ok(const xmgd_contract_t *p, int cplx, const std::vector<int> &steps_of,
+    const std::vector<emu_item> &items, const std::vector<emu_member> &mem,
+    const std::vector<emu_chunk> &chunks, int nslots)
 {
 	struct place { int steps, chunk, item; };
 	std::vector<std::vector<place>> slot(nslots);
-	auto total = [&](const xmgd_cblock_t &cb, int pair) {
-		long long n = 0;
-		for (int q = 0; q < pair; q++)
-			n += (cplx ? 2 : 1) * ((p->pairs[cb.first_pair + q].k + EMU_KS - 1) / EMU_KS);
-		return n;
-	};
 	for (size_t i = 0; i < items.size(); i++) {
 		const emu_item &it = items[i];
-		const xmgd_cblock_t &cb = p->cblocks[mem[it.mfirst].cblock];
+		const int ci = mem[it.mfirst].cblock;
+		const xmgd_cblock_t &cb = p->cblocks[ci];
 		if (it.cfirst < 0 || it.ccount < 1 || it.steps < 1 ||
 		    (size_t)it.cfirst + it.ccount > chunks.size() || it.p0 < 0 || it.k0 < 0 ||
 		    it.p0 >= cb.npairs || it.parts < 1)
 			return false;
 		if (it.parts == 1) {
-			if (it.p0 || it.k0 || it.steps != total(cb, cb.npairs))
+			if (it.p0 || it.k0 || it.steps != steps_of[ci])
 				return false;
 			continue;
 		}
 		if (it.slot < 0 || it.slot >= nslots)
 			return false;
-		slot[it.slot].push_back(place{(int)total(cb, it.p0) + it.k0, it.cfirst, (int)i});
+		int before = it.k0;
+		for (int q = 0; q < it.p0; q++)
+			before += (cplx ? 2 : 1) *
+			    ((p->pairs[cb.first_pair + q].k + EMU_KS - 1) / EMU_KS);
+		slot[it.slot].push_back(place{before, it.cfirst, (int)i});
 	}
 	for (std::vector<place> &v : slot) {
 		std::sort(v.begin(), v.end(),
@@ -2457,8 +2469,7 @@ parts_ok(const xmgd_contract_t *p, int cplx, const std::vector<emu_item> &items,
 			steps += it.steps;
 			chunk += it.ccount;
 		}
-		if (v.size() < 2 || steps != total(p->cblocks[mem[items[v[0].item].mfirst].cblock],
-		    p->cblocks[mem[items[v[0].item].mfirst].cblock].npairs))
+		if (v.size() < 2 || steps != steps_of[mem[items[v[0].item].mfirst].cblock])
 			return false;
 	}
 	return true;
@@ -2733,6 +2744,7 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 	std::vector<emu_chunk> chunks;
 	const char *div = getenv("XMG_EMU_DIVIDE");
 	const bool divide_all = div && atoi(div) == 1;
+	const std::vector<int> steps_of = block_steps(p, cplx);
 	for (int pol : pols) {
 		if (known >= 0 && pol != known)
 			continue;
@@ -2762,7 +2774,7 @@ emu_prepare(const xmgd_contract_t *p, const std::vector<int> &cblocks,
 		c.policy = pol;
 		c.nslots = pair_policy(pol) ? 0 : split_items(p, cplx, row_major(pol),
 		    (size_t)num_sms(), divide_all, chunks, mem, items);
-		if (!parts_ok(p, cplx, items, mem, chunks, c.nslots))
+		if (!parts_ok(p, cplx, steps_of, items, mem, chunks, c.nslots))
 			continue;
 		whole.push_back(sum);
 		e->slot_bytes = std::max(e->slot_bytes, c.nslots * SLOT_BYTES);
@@ -2881,7 +2893,7 @@ checked_list(const xmgd_contract_t *p, int policy, int sms, bool all,
 		if (sms >= 0 && !pair_policy(policy))
 			*slots = split_items(p, cplx, row_major(policy),
 			    (size_t)(sms ? sms : std::max(1, num_sms())), all, chunks, mem, items);
-		*ok = parts_ok(p, cplx, items, mem, chunks, *slots) &&
+		*ok = parts_ok(p, cplx, block_steps(p, cplx), items, mem, chunks, *slots) &&
 		    chunks_ok(p, cplx, EMU_CHUNK, items, mem, chunks);
 	}
 	*nchunks = chunks.size();
