@@ -22,8 +22,8 @@
 namespace xmg {
 
 template <typename T>
-int plain_gemm_launch(const void *items, int nitems, int tile, const xmgd_cblock_t *cbs,
-    const xmgd_pair_t *prs, const int32_t *tabs, const double *beta);
+int plain_gemm_launch(const void *items, int nitems, int tile, bool full,
+    const xmgd_cblock_t *cbs, const xmgd_pair_t *prs, const int32_t *tabs, const double *beta);
 int plain_tile(int dtype, int64_t tiles32);
 
 /* split-precision path (emu.cu) */
@@ -78,6 +78,7 @@ struct xmgd_plan {
 	int n_scale = 0;
 	uint64_t d_pg = 0;                   /* plain GEMM work list */
 	int n_pg = 0, pg_tile = 0;
+	bool pg_full = false;
 	emu_plan *ep = nullptr;
 	/* three segments, timed by events recorded between their launches:
 	 * 0 beta-only blocks + operand split, 1 split-precision GEMM, both
@@ -97,7 +98,7 @@ xmgd_last_timing(xmgd_timing_t *t)
 static int
 stage_plain(int dtype, const std::vector<xmgd_cblock_t> &cbs,
     const std::vector<xmgd_pair_t> &prs, const std::vector<int> &blocks,
-    uint64_t *d, int *n, int *tile)
+    uint64_t *d, int *n, int *tile, bool *full)
 {
 	std::vector<pg_item> items;
 	std::vector<int64_t> cost(cbs.size(), 0);
@@ -105,6 +106,7 @@ stage_plain(int dtype, const std::vector<xmgd_cblock_t> &cbs,
 
 	*d = 0;
 	*n = *tile = 0;
+	*full = false;
 	if (blocks.empty())
 		return XMG_OK;
 	int64_t t32 = 0;
@@ -120,9 +122,13 @@ stage_plain(int dtype, const std::vector<xmgd_cblock_t> &cbs,
 	std::vector<int> order(blocks);
 	std::stable_sort(order.begin(), order.end(),
 	    [&](int x, int y) { return cost[x] > cost[y]; });
-	size_t nt = 0;
-	for (int ci : order)
+	/* full: a quarter of the tiles or more, in 16 x 16 parts, lies in blocks */
+	size_t nt = 0, parts = 0;
+	for (int ci : order) {
 		nt += (size_t)((cbs[ci].m + tb - 1) / tb) * ((cbs[ci].n + tb - 1) / tb);
+		parts += (size_t)((cbs[ci].m + 15) / 16) * ((cbs[ci].n + 15) / 16);
+	}
+	*full = 4 * parts >= nt * (size_t)(tb / 16) * (tb / 16);
 	items.reserve(nt);
 	for (int ci : order)
 		for (int m0 = 0; m0 < cbs[ci].m; m0 += tb)
@@ -137,7 +143,7 @@ stage_plain(int dtype, const std::vector<xmgd_cblock_t> &cbs,
 }
 
 static int
-launch_plain(xmgd_plan *dp, uint64_t items, int n, int tile)
+launch_plain(xmgd_plan *dp, uint64_t items, int n, int tile, bool full)
 {
 	const xmgd_cblock_t *dc = (const xmgd_cblock_t *)dp->d_cbs;
 	const xmgd_pair_t *pr = (const xmgd_pair_t *)dp->d_prs;
@@ -145,10 +151,10 @@ launch_plain(xmgd_plan *dp, uint64_t items, int n, int tile)
 	const void *di = (const void *)items;
 
 	switch (dp->dtype) {
-	case 0: return plain_gemm_launch<float>(di, n, tile, dc, pr, dt, dp->beta);
-	case 1: return plain_gemm_launch<cf>(di, n, tile, dc, pr, dt, dp->beta);
-	case 2: return plain_gemm_launch<double>(di, n, tile, dc, pr, dt, dp->beta);
-	case 3: return plain_gemm_launch<cd>(di, n, tile, dc, pr, dt, dp->beta);
+	case 0: return plain_gemm_launch<float>(di, n, tile, full, dc, pr, dt, dp->beta);
+	case 1: return plain_gemm_launch<cf>(di, n, tile, full, dc, pr, dt, dp->beta);
+	case 2: return plain_gemm_launch<double>(di, n, tile, full, dc, pr, dt, dp->beta);
+	case 3: return plain_gemm_launch<cd>(di, n, tile, full, dc, pr, dt, dp->beta);
 	}
 	return xmg_seterr(XMG_EINVAL, "bad scalar type");
 }
@@ -197,7 +203,7 @@ record(xmgd_plan *dp, int seg)
 	case 1:
 		return dp->ep ? emu_record_gemm(dp->ep) : XMG_OK;
 	default:
-		return dp->n_pg ? launch_plain(dp, dp->d_pg, dp->n_pg, dp->pg_tile) : XMG_OK;
+		return dp->n_pg ? launch_plain(dp, dp->d_pg, dp->n_pg, dp->pg_tile, dp->pg_full) : XMG_OK;
 	}
 }
 
@@ -320,7 +326,7 @@ xmgd_plan_create(const xmgd_contract_t *p, xmgd_plan **out)
 			goto fail;
 	}
 	if ((st = stage_plain(dp->dtype, dp->cbs, dp->prs, dp->plain, &dp->d_pg, &dp->n_pg,
-	    &dp->pg_tile)))
+	    &dp->pg_tile, &dp->pg_full)))
 		goto fail;
 	dp->seg0.resize(dp->ep ? emu_ncand(dp->ep) : 1);
 	dp->seg1.resize(dp->seg0.size());
@@ -450,9 +456,10 @@ xmgd_plan_run(xmgd_plan *dp, int *precision_used)
 			    "in operands");
 		uint64_t d;
 		int n, tile;
-		if ((st = stage_plain(dp->dtype, dp->cbs, dp->prs, dp->emu, &d, &n, &tile)))
+		bool full;
+		if ((st = stage_plain(dp->dtype, dp->cbs, dp->prs, dp->emu, &d, &n, &tile, &full)))
 			return st;
-		st = launch_plain(dp, d, n, tile);
+		st = launch_plain(dp, d, n, tile, full);
 		xmgd_free(d);
 		if (st == XMG_OK)
 			st = check(cudaStreamSynchronize(stream()), "plain fallback");

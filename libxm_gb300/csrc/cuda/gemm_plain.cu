@@ -72,7 +72,13 @@ struct pg {
 	}
 };
 
-template <typename T, int TB, int TM, int TN>
+/* ALL (float lists whose tiles are not mostly empty): every thread computes
+ * its TM x TN outputs, past the block too, and a tile is loaded when it is due.
+ * A float's multiply-add costs less than the branches around it (1500 x 1500 x
+ * 1500 in 25 blocks 398 us, 756 with them; 16 x 16 x 5000, one sixteenth of a
+ * tile, 475 and 353); the next tile's loads in flight change little there
+ * (402). */
+template <typename T, int TB, int TM, int TN, bool ALL = false>
 __global__ void __launch_bounds__(pg<T, TB, TM, TN>::THREADS)
 plain_gemm_kernel(const pg_item *__restrict__ items,
     const xmgd_cblock_t *__restrict__ cbs, const xmgd_pair_t *__restrict__ prs,
@@ -85,12 +91,7 @@ plain_gemm_kernel(const pg_item *__restrict__ items,
 	const pg_item it = items[blockIdx.x];
 	const xmgd_cblock_t cb = cbs[it.cblock];
 	const int tx = threadIdx.x % P::NX, ty = threadIdx.x / P::NX;
-	/* rows and columns of threads that reach into the block; all of them, and
-	 * whole K tiles, for float, whose multiply-adds cost less than the branches
-	 * (1500 x 1500 x 1500 in 25 blocks 396 us, 756 with them); float loads a
-	 * tile when it is due (16 x 16 x 5000: 475 us with the next one in flight,
-	 * 412 without; large ones the same) */
-	constexpr bool ALL = std::is_same<T, float>::value;
+	/* rows and columns of threads that reach into the block */
 	const int mi = ALL ? TM : min(TM, (cb.m - it.m0 + P::NX - 1) / P::NX);
 	const int nj = ALL ? TN : min(TN, (cb.n - it.n0 + P::NY - 1) / P::NY);
 	T acc[TM][TN];
@@ -127,7 +128,7 @@ plain_gemm_kernel(const pg_item *__restrict__ items,
 				P::fetch(va, A, arow, acol, k0 + PG_BK, pr.k, it.m0, cb.m, akf);
 				P::fetch(vb, B, brow, bcol, k0 + PG_BK, pr.k, it.n0, cb.n, bkf);
 			}
-			const int kn = ALL ? PG_BK : min(PG_BK, pr.k - k0);
+			const int kn = min(PG_BK, pr.k - k0);
 #pragma unroll 4
 			for (int kk = 0; kk < kn; kk++) {
 				T a[TM], b[TN];
@@ -161,14 +162,34 @@ plain_gemm_kernel(const pg_item *__restrict__ items,
 		int n = it.n0 + ty + P::NY * j;
 		if (n >= cb.n)
 			continue;
-		int32_t co = ccol[n];
+		if constexpr (ALL) {
+			/* a column's old values together: each load would wait for the
+			 * last one's store (4000 x 4000 x 8 floats, beta 1/2: 114 us one by
+			 * one, now 95; the FP64 forms take longer with it, a 20 x 57
+			 * ladder 2525 -> 2680 us) */
+			T *cn = C + ccol[n], old[TM];
 #pragma unroll
-		for (int i = 0; i < TM; i++) {
-			int m = it.m0 + tx + P::NX * i;
-			if (m >= cb.m)
-				continue;
-			T *cp = C + crow[m] + co;
-			*cp = bzero ? acc[i][j] : num<T>::fma(beta, *cp, acc[i][j]);
+			for (int i = 0; i < TM; i++) {
+				int m = it.m0 + tx + P::NX * i;
+				old[i] = bzero || m >= cb.m ? num<T>::zero() : cn[crow[m]];
+			}
+#pragma unroll
+			for (int i = 0; i < TM; i++) {
+				int m = it.m0 + tx + P::NX * i;
+				if (m >= cb.m)
+					continue;
+				cn[crow[m]] = bzero ? acc[i][j] : num<T>::fma(beta, old[i], acc[i][j]);
+			}
+		} else {
+			int32_t co = ccol[n];
+#pragma unroll
+			for (int i = 0; i < TM; i++) {
+				int m = it.m0 + tx + P::NX * i;
+				if (m >= cb.m)
+					continue;
+				T *cp = C + crow[m] + co;
+				*cp = bzero ? acc[i][j] : num<T>::fma(beta, *cp, acc[i][j]);
+			}
 		}
 	}
 }
@@ -183,8 +204,8 @@ plain_tile(int dtype, int64_t tiles32)
 
 template <typename T>
 int
-plain_gemm_launch(const void *items, int nitems, int tile, const xmgd_cblock_t *cbs,
-    const xmgd_pair_t *prs, const int32_t *tabs, const double *beta)
+plain_gemm_launch(const void *items, int nitems, int tile, bool full,
+    const xmgd_cblock_t *cbs, const xmgd_pair_t *prs, const int32_t *tabs, const double *beta)
 {
 	const pg_item *it = (const pg_item *)items;
 	const double2 b2 = make_double2(beta[0], beta[1]);
@@ -198,20 +219,23 @@ plain_gemm_launch(const void *items, int nitems, int tile, const xmgd_cblock_t *
 		else
 			plain_gemm_kernel<T, 32, 4, 2><<<nitems, 128, 0, stream()>>>(it, cbs, prs,
 			    tabs, b2);
-	} else
+	} else if (std::is_same<T, float>::value && full)
+		plain_gemm_kernel<T, 64, 4, 4, std::is_same<T, float>::value><<<nitems, 256, 0,
+		    stream()>>>(it, cbs, prs, tabs, b2);
+	else
 		plain_gemm_kernel<T, 64, 4, 4><<<nitems, 256, 0, stream()>>>(it, cbs, prs, tabs,
 		    b2);
 	g_launches++;
 	return check(cudaGetLastError(), "plain_gemm_kernel launch");
 }
 
-template int plain_gemm_launch<float>(const void *, int, int, const xmgd_cblock_t *,
+template int plain_gemm_launch<float>(const void *, int, int, bool, const xmgd_cblock_t *,
     const xmgd_pair_t *, const int32_t *, const double *);
-template int plain_gemm_launch<double>(const void *, int, int, const xmgd_cblock_t *,
+template int plain_gemm_launch<double>(const void *, int, int, bool, const xmgd_cblock_t *,
     const xmgd_pair_t *, const int32_t *, const double *);
-template int plain_gemm_launch<cf>(const void *, int, int, const xmgd_cblock_t *,
+template int plain_gemm_launch<cf>(const void *, int, int, bool, const xmgd_cblock_t *,
     const xmgd_pair_t *, const int32_t *, const double *);
-template int plain_gemm_launch<cd>(const void *, int, int, const xmgd_cblock_t *,
+template int plain_gemm_launch<cd>(const void *, int, int, bool, const xmgd_cblock_t *,
     const xmgd_pair_t *, const int32_t *, const double *);
 
 } /* namespace xmg */
